@@ -33,6 +33,7 @@ UNITS = [
     ("host_io.cpp", []),
     ("metrics.cpp", []),
     ("build.cu", ["-fmad=false"]),
+    ("pairs.cu", []),
     ("step64.cu", ["-fmad=false"]),
     ("compat.cu", []),
     ("engine.cu", []),

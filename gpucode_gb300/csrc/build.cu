@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 
 #include "dem_device.cuh"
+#include "pairs.cuh"
 
 namespace dem {
 
@@ -140,6 +141,29 @@ __global__ void k_cell_ranges(int* __restrict__ cell_start, int* __restrict__ ce
       }
     }
     off += c[e];
+  }
+}
+
+/* the same scan over any counts: out[i] = sum of in[0 .. i), the total last,
+ * into the pair set that is not current */
+__global__ void k_scan_apply(const int* __restrict__ in, int n, const int* __restrict__ tile_off, int* out0, int* out1,
+                             const int* __restrict__ ctl) {
+  int* __restrict__ out = ctl[0] ? out0 : out1;
+  const long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanPerThread;
+  int c[kScanPerThread];
+  int s = 0;
+#pragma unroll
+  for (int e = 0; e < kScanPerThread; e++) {
+    c[e] = base + e < n ? in[base + e] : 0;
+    s += c[e];
+  }
+  int total;
+  int off = block_exclusive_scan(s, total) + tile_off[blockIdx.x];
+#pragma unroll
+  for (int e = 0; e < kScanPerThread; e++) {
+    if (base + e < n) out[base + e] = off;
+    off += c[e];
+    if (base + e == n - 1) out[n] = off;
   }
 }
 
@@ -443,6 +467,16 @@ dem_status cell_sort(const double3* pos, const int* plevel, const int* order_key
                                                       order_key, n);
   }
   return cuda_check(cudaGetLastError(), "cell_sort launch");
+}
+
+dem_status exclusive_scan(const int* in, int n, int* out0, int* out1, const int* ctl, void* scratch, cudaStream_t s) {
+  if (n <= 0) return DEM_OK;
+  int* tile = (int*)scratch;
+  const int ntiles = div_up(n, kScanTile);
+  k_tile_sums<<<ntiles, kScanThreads, 0, s>>>(in, n, tile);
+  k_scan_tiles<<<1, kScanThreads, 0, s>>>(tile, ntiles);
+  k_scan_apply<<<ntiles, kScanThreads, 0, s>>>(in, n, tile, out0, out1, ctl);
+  return cuda_check(cudaGetLastError(), "scan launch");
 }
 
 dem_status neighbor_find(const double3* pos, const double* rad, const int* sorted_src,

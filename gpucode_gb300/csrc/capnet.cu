@@ -82,13 +82,21 @@ struct SampleArgs {
   const double3* pos;
   const double* rad;
   const int *nebor, *num_nebor, *plevel, *nidx, *npars, *nneb, *lqd, *id;
-  const unsigned char* brg;
+  PairSet ps; /* the slots' pairs and their bridge flags */
   int n;
   double vol, gapmn, layer, stension;
   float theta_max;
   unsigned long long theta_seed;
   LiquidModel lm; /* mode 1: per-contact volumes and angles (liquid.cuh) */
 };
+
+/* slot s's bridge flag */
+__device__ __forceinline__ bool slot_bridged(const SampleArgs& a, int cur, long long s) {
+  const int e = a.ps.eidx[s];
+  if (e == kNoPair) return false;
+  const long long p = e < 0 ? ~e : e;
+  return (cur ? a.ps.brg[1] : a.ps.brg[0])[a.ps.sides * p + (a.ps.sides == 2 && e < 0 ? 1 : 0)] != 0;
+}
 
 __global__ void k_sample_count(SampleArgs a, int* cnt) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -97,7 +105,8 @@ __global__ void k_sample_count(SampleArgs a, int* cnt) {
   const long long stride = a.npars[L];
   const long long base = slot_base(L, a.npars, a.nneb) + a.nidx[q];
   int c = 0;
-  for (int k = 0; k < a.num_nebor[q]; k++) c += a.brg[base + k * stride] ? 1 : 0;
+  const int cur = a.ps.ctl[0];
+  for (int k = 0; k < a.num_nebor[q]; k++) c += slot_bridged(a, cur, base + k * stride) ? 1 : 0;
   cnt[q] = c;
 }
 
@@ -127,6 +136,7 @@ __global__ void k_sample_write(SampleArgs a, const long long* off, long long cap
   const long long stride = a.npars[L];
   const long long base = slot_base(L, a.npars, a.nneb) + a.nidx[q];
   long long o = off[q];
+  const int cur = a.ps.ctl[0];
   const double3 pi = a.pos[q];
   const double ri = a.rad[q];
   const int inl = max(12, a.lqd[q]);
@@ -136,7 +146,7 @@ __global__ void k_sample_write(SampleArgs a, const long long* off, long long cap
   lq.stension = a.stension; lq.vol = a.vol; lq.gapmn = a.gapmn; lq.layer = a.layer; lq.brknmx = 0.0;
   for (int k = 0; k < a.num_nebor[q]; k++) {
     const long long s = base + k * stride;
-    if (!a.brg[s]) continue;
+    if (!slot_bridged(a, cur, s)) continue;
     if (o >= capacity) return;
     const int j = a.nebor[s];
     const double3 pj = a.pos[j];
@@ -1062,7 +1072,7 @@ dem_status dem_capnet_samples(dem_ctx* c, float* x_dev, float* y_dev, long long 
   SampleArgs a;
   a.pos = c->b.pos; a.rad = c->b.rad; a.nebor = c->b.nebor; a.num_nebor = c->b.num_nebor; a.plevel = c->b.plevel;
   a.nidx = c->b.nidx; a.npars = c->b.npars; a.nneb = c->b.nneb; a.lqd = c->b.lqd; a.id = c->b.id;
-  a.brg = c->b.brg; a.n = c->n;
+  a.ps = c->b.ps; a.n = c->n;
   a.vol = c->s.lqd.vol; a.gapmn = c->s.lqd.gapmn; a.layer = c->s.lqd.layer; a.stension = c->s.lqd.stension;
   a.theta_max = c->theta_max;
   a.theta_seed = c->theta_seed;

@@ -84,7 +84,7 @@ __device__ __forceinline__ float cap_formula32(float sep, float vol) {
   const float f3 = 1.268f + 0.198f * L + 0.02232f * L2 + 0.0008585f * L3;
   const float f4 = -0.010703f + 0.03345f * L + 0.0018574f * L2;
   const float ls = __logf(sp);
-  return __expf(f1 - f2 * __expf(f3 * ls + f4 * ls * ls));
+  return __expf(f1 - f2 * __expf(fmaf(f3, ls, f4 * ls * ls)));
 }
 
 /* SiLU for the BF16 tiles: z sigmoid(z) = h + h tanh(h) with h = z / 2, one

@@ -55,37 +55,15 @@ dem_status dalloc(dem_ctx* c, T** p, size_t count) {
   return DEM_OK;
 }
 
-__global__ void k_zero_int(int* p, long long n) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    p[i] = 0;
-}
-
-/* R1: copy the used slots (and wall slots) to the *_old buffers */
-__global__ void k_copy_old(const int* __restrict__ nebor, const int* __restrict__ num_nebor,
-                           const int* __restrict__ nidx, const int* __restrict__ plevel,
-                           const int* __restrict__ npars, const int* __restrict__ nneb,
-                           const ContactRec* __restrict__ rec, const unsigned char* __restrict__ brg,
-                           const int* __restrict__ wlist, const int* __restrict__ nwall,
-                           const ContactRec* __restrict__ wrec, int* __restrict__ nebor_old,
-                           int* __restrict__ num_nebor_old, int* __restrict__ nidx_old,
-                           ContactRec* __restrict__ rec_old, unsigned char* __restrict__ brg_old,
-                           int* __restrict__ wlist_old, int* __restrict__ nwall_old,
-                           ContactRec* __restrict__ wrec_old, int n, unsigned long long* counters) {
-  const int p = reversed_block_thread(); /* the longest slot lists first */
+/* R1: copy the used wall slots to the *_old buffers (pair histories are not
+ * copied: the rebuild writes the other pair set) */
+__global__ void k_copy_old(const int* __restrict__ wlist, const int* __restrict__ nwall,
+                           const ContactRec* __restrict__ wrec, int* __restrict__ wlist_old,
+                           int* __restrict__ nwall_old, ContactRec* __restrict__ wrec_old, int n,
+                           unsigned long long* counters) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p == 0 && counters) counters[4] += 1; /* rebuilds */
   if (p >= n) return;
-  const int L = plevel[p];
-  const long long stride = npars[L];
-  const long long base = slot_base(L, npars, nneb) + nidx[p];
-  const int nn = num_nebor[p];
-  for (int a = 0; a < nn; a++) {
-    const long long s = base + a * stride;
-    nebor_old[s] = nebor[s];
-    rec_old[s] = rec[s];
-    brg_old[s] = brg[s];
-  }
-  num_nebor_old[p] = nn;
-  nidx_old[p] = nidx[p];
   const int nw = nwall[p];
   nwall_old[p] = nw;
   for (int a = 0; a < nw; a++) {
@@ -148,46 +126,20 @@ __global__ void k_copy_back(int n, const double3* __restrict__ tpos, const doubl
   pmove[q] = 0.0;
 }
 
-/* R6: carry-over into the new lists: matched slot -> copy, else zero */
-__global__ void k_carry(const int* __restrict__ nebor, const int* __restrict__ num_nebor, const int* __restrict__ nidx,
-                        const int* __restrict__ plevel, const int* __restrict__ npars, const int* __restrict__ nneb,
-                        const int* __restrict__ nebor_old, const int* __restrict__ num_nebor_old,
-                        const int* __restrict__ nidx_old, const ContactRec* __restrict__ rec_old,
-                        const unsigned char* __restrict__ brg_old, ContactRec* __restrict__ rec,
-                        unsigned char* __restrict__ brg, const int* __restrict__ wlist, const int* __restrict__ nwall,
-                        const int* __restrict__ wlist_old, const int* __restrict__ nwall_old,
-                        const ContactRec* __restrict__ wrec_old, ContactRec* __restrict__ wrec,
-                        const int* __restrict__ src, const int* __restrict__ old_to_new, int n) {
-  const int q = reversed_block_thread(); /* the longest slot lists first */
+/* R6: carry-over of the wall history: matched wall -> copy, else zero */
+__global__ void k_carry_walls(const int* __restrict__ wlist, const int* __restrict__ nwall,
+                              const int* __restrict__ wlist_old, const int* __restrict__ nwall_old,
+                              const ContactRec* __restrict__ wrec_old, ContactRec* __restrict__ wrec,
+                              const int* __restrict__ src, int n) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
+  const int nw = nwall[q];
+  if (nw == 0) return;
   const int p = src ? src[q] : q;
-  const int L = plevel[q];
-  const long long stride = npars[L];
-  const long long lb = slot_base(L, npars, nneb);
-  const long long nb = lb + nidx[q], ob = lb + nidx_old[p];
-  const int nn = num_nebor[q], no = num_nebor_old[p];
+  const int nwo = nwall_old[p];
   ContactRec zero;
   zero.dx = zero.dy = zero.dz = zero.nDsp = zero.nDsp_mx = zero.plstRad = zero.plstDfm = 0.0;
   zero.stage = 0;
-  for (int a = 0; a < nn; a++) {
-    const long long s = nb + a * stride;
-    const int partner = nebor[s];
-    long long hit = -1;
-    for (int b = 0; b < no; b++) {
-      const long long t = ob + b * stride;
-      int j = nebor_old[t];
-      if (old_to_new) j = old_to_new[j];
-      if (j == partner) hit = t; /* the reference lets the last match win */
-    }
-    if (hit >= 0) {
-      rec[s] = rec_old[hit];
-      brg[s] = brg_old[hit];
-    } else {
-      rec[s] = zero;
-      brg[s] = 0;
-    }
-  }
-  const int nw = nwall[q], nwo = nwall_old[p];
   for (int a = 0; a < nw; a++) {
     const int w = wlist[3 * q + a];
     long long hit = -1;
@@ -320,7 +272,9 @@ __global__ void k_check_finite(int n, const double3* __restrict__ pos, const dou
 
 /* ------------------------------------------------------------------ */
 
-HistAoS hist_pp(dem_ctx* c) { return HistAoS{c->b.rec, c->b.brg}; }
+NeborLists lists_of(const EngineBufs& b) {
+  return NeborLists{b.nebor, b.num_nebor, b.nidx, b.plevel, b.npars, b.nneb};
+}
 HistAoS hist_pw(dem_ctx* c) { return HistAoS{c->b.wrec, nullptr}; }
 
 /* dem_profile_kernels: an event after the kernel(s) just enqueued */
@@ -343,10 +297,8 @@ dem_status enqueue_rebuild(dem_ctx* c, cudaStream_t s, int parity) {
     if (st != DEM_OK) return st;
     mark(c, s, "k_lqd_from_shadow");
   }
-  k_copy_old<<<grid_for(n, 128), 128, 0, s>>>(b.nebor, b.num_nebor, b.nidx, b.plevel, b.npars, b.nneb, b.rec, b.brg,
-                                               b.wlist, b.nwall, b.wrec, b.nebor_old, b.num_nebor_old, b.nidx_old,
-                                               b.rec_old, b.brg_old, b.wlist_old, b.nwall_old, b.wrec_old, n,
-                                               b.counters);
+  k_copy_old<<<grid_for(n, 256), 256, 0, s>>>(b.wlist, b.nwall, b.wrec, b.wlist_old, b.nwall_old, b.wrec_old, n,
+                                              b.counters);
   mark(c, s, "k_copy_old");
   st = cell_sort(b.pos, b.plevel, reorder ? b.id : nullptr, n, c->lv, c->k, c->s.sys_ncells, b.sorted_hash,
                  b.sorted_src, b.cell_start, b.cell_end, b.scratch, b.err, s, b.cell_off);
@@ -384,15 +336,27 @@ dem_status enqueue_rebuild(dem_ctx* c, cudaStream_t s, int parity) {
   mark(c, s, "k_neighbor_find");
   st = wall_list(b.pos, b.rad, b.cyl, b.wlist, 3 * sizeof(int), b.nwall, n, c->k, s, b.id, b.sys_of_id);
   if (st != DEM_OK) return st;
+  if (c->opt.precision == DEM_PREC_MIXED) {
+    st = mixed_wall_entries(c, s);
+    if (st != DEM_OK) return st;
+  }
   mark(c, s, "k_wall_list");
-  k_carry<<<grid_for(n, 128), 128, 0, s>>>(b.nebor, b.num_nebor, b.nidx, b.plevel, b.npars, b.nneb, b.nebor_old,
-                                           b.num_nebor_old, b.nidx_old, b.rec_old, b.brg_old, b.rec, b.brg, b.wlist,
-                                           b.nwall, b.wlist_old, b.nwall_old, b.wrec_old, b.wrec,
-                                           reorder ? b.sorted_src : nullptr, reorder ? b.old_to_new : nullptr, n);
+  k_carry_walls<<<grid_for(n, 256), 256, 0, s>>>(b.wlist, b.nwall, b.wlist_old, b.nwall_old, b.wrec_old, b.wrec,
+                                                 reorder ? b.sorted_src : nullptr, n);
+  mark(c, s, "k_carry_walls");
+  /* the sort's scratch is free again */
+  int* cnt = reinterpret_cast<int*>(b.scratch);
+  st = pair_build(b.ps, lists_of(b), n, cnt, cnt + n, b.err, s);
+  if (st != DEM_OK) return st;
+  mark(c, s, "pair list (k_pair_count .. k_pair_fill)");
+  st = pair_carry(b.ps, lists_of(b), n, reorder ? b.sorted_src : nullptr, b.err, s);
+  if (st != DEM_OK) return st;
   mark(c, s, "k_carry");
   /* the caller-order view of the new cell order, for the state import and export */
   k_inverse<<<grid_for(n, 256), 256, 0, s>>>(n, b.id, b.inv);
   mark(c, s, "k_inverse");
+  st = pair_flip(b.ps, s);
+  if (st != DEM_OK) return st;
   return cuda_check(cudaGetLastError(), "rebuild launch");
 }
 
@@ -404,9 +368,9 @@ dem_status enqueue_step(dem_ctx* c, cudaStream_t s, int parity) {
   dem_status st = var_init(b.force, b.mom, b.rmom, b.lqd, b.lqd_old, n, s);
   if (st != DEM_OK) return st;
   /* the export staging is idle during a step: it holds the spheres' liquid shares */
-  st = pp_force64<HistAoS>(b.pos, b.vel, b.angv, b.rad, b.nebor, b.plevel, b.npars, b.nneb, b.nidx, hist_pp(c),
-                           b.num_nebor, b.lqd, b.lqd_old, b.force, b.mom, b.rmom, n, c->s.force_cap,
-                           c->s.load_stage, c->k, b.counters, reinterpret_cast<double*>(b.tmp_out), s, b.id, c->lm);
+  st = pair_force64(b.ps, b.pair_out, b.pos, b.vel, b.angv, b.rad, b.plevel, b.npars, b.nneb, b.nidx, b.num_nebor,
+                    b.lqd, b.lqd_old, b.force, b.mom, b.rmom, n, c->s.force_cap, c->s.load_stage, c->k, b.counters,
+                    reinterpret_cast<double*>(b.tmp_out), s, b.id, c->lm);
   if (st != DEM_OK) return st;
   st = wall_force64<HistAoS>(b.pos, b.vel, b.angv, b.force, b.mom, b.rmom, b.rad, b.cyl, hist_pw(c), b.nwall,
                              b.wlist, 3 * sizeof(int), n, n, c->s.load_stage, c->k, b.counters,
@@ -622,7 +586,12 @@ dem_memory memory_of(long long N, long long S, long long C, const dem_options* o
                    + 2 * 3 * 64                /* wall records and their copies */
                    + 3 * 4 + 2 * 4;            /* sorted hash / source, old_to_new, sort scratch */
   if (o && o->precision == DEM_PREC_MIXED) m.per_particle += 9 * 16; /* FP32 shadows */
-  m.per_slot = 2 * (4 + 64 + 1);               /* list entry, record, bridge flag, and their copies */
+  /* the list entry and the slot's pair index (8), and for half a pair a slot two
+   * sets of pair (16), record (128) and bridge flag (2), and the pair's result
+   * (48): 105 in mixed precision, where 138 covers the wall results and the
+   * reserve of unmirrored pairs too; FP64 has a record and flag a side, and 160
+   * bytes of result */
+  m.per_slot = o && o->precision == DEM_PREC_MIXED ? 138 : 240;
   m.per_cell = 3 * 4;                         /* cell start, end, offset */
   m.slots = S;
   const long long allocations = 64;
@@ -766,8 +735,18 @@ extern "C" dem_status dem_create(const dem_setup* s, const double* rad, const in
   A(b.tmp_plevel, N);
   A(b.force, N); A(b.mom, N); A(b.rmom, N);
   A(b.nebor, S); A(b.num_nebor, N); A(b.wlist, 3 * N); A(b.nwall, N);
-  A(b.nebor_old, S); A(b.num_nebor_old, N); A(b.wlist_old, 3 * N); A(b.nwall_old, N); A(b.nidx_old, N);
-  A(b.rec, S); A(b.rec_old, S); A(b.brg, S); A(b.brg_old, S); A(b.wrec, 3 * N); A(b.wrec_old, 3 * N);
+  A(b.wlist_old, 3 * N); A(b.nwall_old, N); A(b.wrec, 3 * N); A(b.wrec_old, 3 * N);
+  const size_t P = (size_t)pair_capacity(c->n, c->slots);
+  b.ps.cap = (int)P;
+  b.ps.sides = c->opt.precision == DEM_PREC_MIXED ? 1 : 2;
+  const size_t PS = P * (size_t)b.ps.sides;
+  for (int k = 0; k < 2; k++) {
+    A(b.ps.pair[k], P); A(b.ps.off[k], N + 1); A(b.ps.rec[k], PS); A(b.ps.brg[k], PS);
+  }
+  A(b.ps.eidx, S); A(b.ps.ctl, 8);
+  char* pair_out = nullptr;
+  A(pair_out, P * (c->opt.precision == DEM_PREC_MIXED ? kPairOut32 : kPairOut64));
+  b.pair_out = pair_out;
   A(b.sorted_hash, N); A(b.sorted_src, N); A(b.old_to_new, N); A(b.cell_start, C); A(b.cell_end, C);
   A(b.cell_off, C + 1);
   A(b.cell_size, L); A(b.grid_size, L); A(b.ncell_idx, L); A(b.npars, L); A(b.nneb, L); A(b.level_size, L);
@@ -1396,36 +1375,98 @@ extern "C" dem_status dem_get_neighbors(dem_ctx* c, int* counts, int* partners, 
   return DEM_OK;
 }
 
-extern "C" dem_status dem_get_history(dem_ctx* c, double* rec, int* brg, int max_per) {
-  if (!c || !rec || max_per <= 0) return fail(DEM_ERR_ARG, "dem_get_history: bad argument");
+/* The pair histories on the host, and the used neighbour slots they belong to:
+ * visit(particle position q, entry a, slot, record (-1: no pair), whether the
+ * record is the slot's sphere's own or the mirror image of it) */
+namespace {
+struct HostPairs {
+  std::vector<ContactRec> rec;
+  std::vector<unsigned char> brg;
+  std::vector<int> eidx, num, nidx, plevel;
+};
+dem_status fetch_pairs(dem_ctx* c, HostPairs& h, bool history) {
+  EngineBufs& b = c->b;
   const size_t N = (size_t)c->n, S = (size_t)c->slots;
-  std::vector<ContactRec> r(S);
-  std::vector<unsigned char> bf(S);
-  std::vector<int> num(N), nidx(N), plevel(N), id(N);
+  int ctl[4] = {0, 0, 0, 0};
+  h.eidx.resize(S);
+  h.num.resize(N);
+  h.nidx.resize(N);
+  h.plevel.resize(N);
   cudaError_t e = cudaStreamSynchronize(c->stream);
-  if (e == cudaSuccess) e = cudaMemcpy(r.data(), c->b.rec, sizeof(ContactRec) * S, cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess) e = cudaMemcpy(bf.data(), c->b.brg, S, cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess) e = cudaMemcpy(num.data(), c->b.num_nebor, sizeof(int) * N, cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess) e = cudaMemcpy(nidx.data(), c->b.nidx, sizeof(int) * N, cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess) e = cudaMemcpy(plevel.data(), c->b.plevel, sizeof(int) * N, cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess) e = cudaMemcpy(id.data(), c->b.id, sizeof(int) * N, cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return cuda_check(e, "dem_get_history");
+  if (e == cudaSuccess) e = cudaMemcpy(ctl, b.ps.ctl, sizeof(ctl), cudaMemcpyDeviceToHost);
+  const int cur = ctl[0] & 1, P = ctl[1 + cur];
+  if (history) {
+    const size_t PS = (size_t)P * b.ps.sides;
+    h.rec.resize(PS);
+    h.brg.resize(PS);
+    if (e == cudaSuccess)
+      e = cudaMemcpy(h.rec.data(), b.ps.rec[cur], sizeof(ContactRec) * PS, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(h.brg.data(), b.ps.brg[cur], PS, cudaMemcpyDeviceToHost);
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(h.eidx.data(), b.ps.eidx, sizeof(int) * S, cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess) e = cudaMemcpy(h.num.data(), b.num_nebor, sizeof(int) * N, cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess) e = cudaMemcpy(h.nidx.data(), b.nidx, sizeof(int) * N, cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess) e = cudaMemcpy(h.plevel.data(), b.plevel, sizeof(int) * N, cudaMemcpyDeviceToHost);
+  return cuda_check(e, "pair history download");
+}
+template <class V>
+void visit_slots(const dem_ctx* c, const HostPairs& h, V visit) {
   long long base[DEM_MAX_LEVELS];
   long long acc = 0;
   for (int l = 0; l < c->s.n_levels; l++) {
     base[l] = acc;
     acc += (long long)c->s.level_nnebors[l] * c->s.level_npars[l];
   }
-  for (size_t q = 0; q < N; q++) {
-    const int i = id[q], L = plevel[q];
-    if (num[q] > max_per) return fail(DEM_ERR_ARG, "dem_get_history: max_per too small");
-    for (int a = 0; a < num[q]; a++) {
-      const long long sl = base[L] + (long long)a * c->s.level_npars[L] + nidx[q];
-      double* o = rec + ((size_t)i * max_per + a) * 8;
-      decode_record(r[(size_t)sl], c->opt.precision == DEM_PREC_MIXED, o);
-      if (brg) brg[(size_t)i * max_per + a] = bf[(size_t)sl];
+  for (size_t q = 0; q < (size_t)c->n; q++)
+    for (int a = 0; a < h.num[q]; a++) {
+      const int L = h.plevel[q];
+      const size_t sl = (size_t)(base[L] + (long long)a * c->s.level_npars[L] + h.nidx[q]);
+      const int e = h.eidx[sl];
+      const long long p = e < 0 ? ~e : e;
+      if (e == kNoPair) visit(q, a, sl, -1LL, true);
+      else if (c->b.ps.sides == 2) visit(q, a, sl, 2 * p + (e < 0 ? 1 : 0), true);
+      else visit(q, a, sl, p, e >= 0);
     }
+}
+/* a record as the slot's sphere sees it: the second sphere's spring is the
+ * mirror image of the first one's (mixed records) */
+ContactRec slot_record(const HostPairs& h, long long p, bool own) {
+  ContactRec r;
+  std::memset(&r, 0, sizeof(r));
+  if (p < 0 || (size_t)p >= h.rec.size()) return r;
+  r = h.rec[(size_t)p];
+  if (!own) {
+    r.dx = -r.dx;
+    r.dy = -r.dy;
+    r.dz = -r.dz;
+    MixedRec m;
+    std::memcpy(&m, &r, sizeof(m));
+    m.fx = -m.fx;
+    m.fy = -m.fy;
+    m.fz = -m.fz;
+    std::memcpy(&r, &m, sizeof(m));
   }
+  return r;
+}
+}  // namespace
+
+extern "C" dem_status dem_get_history(dem_ctx* c, double* rec, int* brg, int max_per) {
+  if (!c || !rec || max_per <= 0) return fail(DEM_ERR_ARG, "dem_get_history: bad argument");
+  const size_t N = (size_t)c->n;
+  const bool mixed = c->opt.precision == DEM_PREC_MIXED;
+  HostPairs h;
+  std::vector<int> id(N);
+  dem_status st = fetch_pairs(c, h, true);
+  if (st != DEM_OK) return st;
+  cudaError_t e = cudaMemcpy(id.data(), c->b.id, sizeof(int) * N, cudaMemcpyDeviceToHost);
+  if (e != cudaSuccess) return cuda_check(e, "dem_get_history");
+  for (size_t q = 0; q < N; q++)
+    if (h.num[q] > max_per) return fail(DEM_ERR_ARG, "dem_get_history: max_per too small");
+  visit_slots(c, h, [&](size_t q, int a, size_t, long long p, bool own) {
+    const size_t at = (size_t)id[q] * max_per + a;
+    decode_record(slot_record(h, p, own), mixed, rec + at * 8);
+    if (brg) brg[at] = p >= 0 && (size_t)p < h.brg.size() ? h.brg[(size_t)p] : 0;
+  });
   return DEM_OK;
 }
 
@@ -1473,20 +1514,24 @@ extern "C" dem_status dem_get_aux(dem_ctx* c, double* pmove, int* lqd, int* nwal
 
 /* ---------------- checkpoint ---------------- */
 namespace {
+/* what a checkpoint holds, in file order.  The pair histories are stored per
+ * neighbour slot, as each slot's sphere sees them (kind 1: the records, 2: the
+ * bridge flags), so a file does not depend on how the engine keeps its pairs */
 struct Blob {
   void* dev;
   size_t bytes;
+  int kind;
 };
 std::vector<Blob> checkpoint_blobs(dem_ctx* c) {
   EngineBufs& b = c->b;
   const size_t N = (size_t)c->n, S = (size_t)c->slots;
-  return {{b.pos, sizeof(double3) * N}, {b.vel, sizeof(double3) * N}, {b.angv, sizeof(double3) * N},
-          {b.rad, sizeof(double) * N},  {b.pmove, sizeof(double) * N}, {b.lqd, sizeof(int) * N},
-          {b.id, sizeof(int) * N},      {b.plevel, sizeof(int) * N},   {b.nidx, sizeof(int) * N},
-          {b.nebor, sizeof(int) * S},   {b.num_nebor, sizeof(int) * N}, {b.wlist, sizeof(int) * 3 * N},
-          {b.nwall, sizeof(int) * N},   {b.rec, sizeof(ContactRec) * S}, {b.brg, S},
-          {b.wrec, sizeof(ContactRec) * 3 * N}, {b.flag, sizeof(int)}, {b.need, sizeof(int)},
-          {b.cyl, sizeof(CylinderBC)}, {b.counters, sizeof(unsigned long long) * 8}};
+  return {{b.pos, sizeof(double3) * N, 0}, {b.vel, sizeof(double3) * N, 0}, {b.angv, sizeof(double3) * N, 0},
+          {b.rad, sizeof(double) * N, 0},  {b.pmove, sizeof(double) * N, 0}, {b.lqd, sizeof(int) * N, 0},
+          {b.id, sizeof(int) * N, 0},      {b.plevel, sizeof(int) * N, 0},   {b.nidx, sizeof(int) * N, 0},
+          {b.nebor, sizeof(int) * S, 0},   {b.num_nebor, sizeof(int) * N, 0}, {b.wlist, sizeof(int) * 3 * N, 0},
+          {b.nwall, sizeof(int) * N, 0},   {nullptr, sizeof(ContactRec) * S, 1}, {nullptr, S, 2},
+          {b.wrec, sizeof(ContactRec) * 3 * N, 0}, {b.flag, sizeof(int), 0}, {b.need, sizeof(int), 0},
+          {b.cyl, sizeof(CylinderBC), 0}, {b.counters, sizeof(unsigned long long) * 8, 0}};
 }
 const char kMagic[8] = {'D', 'E', 'M', 'G', 'B', '3', '0', '1'};
 }  // namespace
@@ -1507,12 +1552,26 @@ extern "C" dem_status dem_save(dem_ctx* c, const char* path, int nBatch) {
   long long hdr[4] = {c->iter, (long long)c->n, c->slots, (long long)c->opt.precision};
   std::fwrite(hdr, sizeof(hdr), 1, f);
   std::fwrite(&c->ctime, sizeof(double), 1, f);
+  HostPairs hp;
+  st = fetch_pairs(c, hp, true);
   for (const Blob& bl : checkpoint_blobs(c)) {
+    if (st != DEM_OK) break;
     std::vector<char> h(bl.bytes);
-    e = cudaMemcpy(h.data(), bl.dev, bl.bytes, cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) {
-      st = cuda_check(e, "dem_save copy");
-      break;
+    if (bl.kind == 0) {
+      e = cudaMemcpy(h.data(), bl.dev, bl.bytes, cudaMemcpyDeviceToHost);
+      if (e != cudaSuccess) {
+        st = cuda_check(e, "dem_save copy");
+        break;
+      }
+    } else {
+      visit_slots(c, hp, [&](size_t, int, size_t sl, long long p, bool own) {
+        if (bl.kind == 1) {
+          const ContactRec r = slot_record(hp, p, own);
+          std::memcpy(h.data() + sl * sizeof(r), &r, sizeof(r));
+        } else {
+          h[sl] = p >= 0 && (size_t)p < hp.brg.size() ? (char)hp.brg[(size_t)p] : 0;
+        }
+      });
     }
     if (std::fwrite(h.data(), 1, bl.bytes, f) != bl.bytes) {
       st = fail(DEM_ERR_IO, "dem_save: short write");
@@ -1547,11 +1606,16 @@ extern "C" dem_status dem_load(dem_ctx* c, const char* path) {
     return fail(DEM_ERR_ARG, "dem_load: checkpoint does not match this context");
   }
   dem_status st = DEM_OK;
+  std::vector<char> slot_rec, slot_brg;
   for (const Blob& bl : checkpoint_blobs(c)) {
     std::vector<char> h(bl.bytes);
     if (std::fread(h.data(), 1, bl.bytes, f) != bl.bytes) {
       st = fail(DEM_ERR_IO, "dem_load: truncated checkpoint");
       break;
+    }
+    if (bl.kind) {
+      (bl.kind == 1 ? slot_rec : slot_brg).swap(h);
+      continue;
     }
     cudaError_t e = cudaMemcpy(bl.dev, h.data(), bl.bytes, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
@@ -1561,11 +1625,38 @@ extern "C" dem_status dem_load(dem_ctx* c, const char* path) {
   }
   std::fclose(f);
   if (st != DEM_OK) return st;
+  /* the pair list of the loaded neighbour lists, and each pair's history from
+   * its owner's slot */
+  {
+    EngineBufs& b = c->b;
+    int* cnt = reinterpret_cast<int*>(b.scratch);
+    st = pair_build(b.ps, lists_of(b), c->n, cnt, cnt + c->n, b.err, c->stream);
+    /* links the slots to the pairs; what it carries over is overwritten below */
+    if (st == DEM_OK) st = pair_carry(b.ps, lists_of(b), c->n, nullptr, b.err, c->stream);
+    if (st == DEM_OK) st = pair_flip(b.ps, c->stream);
+    HostPairs hp;
+    if (st == DEM_OK) st = fetch_pairs(c, hp, true);
+    if (st != DEM_OK) return st;
+    visit_slots(c, hp, [&](size_t, int, size_t sl, long long p, bool own) {
+      if (!own || p < 0) return;
+      std::memcpy(&hp.rec[(size_t)p], slot_rec.data() + sl * sizeof(ContactRec), sizeof(ContactRec));
+      hp.brg[(size_t)p] = (unsigned char)slot_brg[sl];
+    });
+    int cur = 0;
+    cudaError_t e = cudaMemcpy(&cur, b.ps.ctl, sizeof(int), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess)
+      e = cudaMemcpy(b.ps.rec[cur], hp.rec.data(), sizeof(ContactRec) * hp.rec.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(b.ps.brg[cur], hp.brg.data(), hp.brg.size(), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return cuda_check(e, "dem_load pair history");
+  }
   c->iter = hdr[0];
   c->ctime = ct;
   c->parity = 0;
   k_inverse<<<grid_for(c->n, 256), 256, 0, c->stream>>>(c->n, c->b.id, c->b.inv);
-  if (c->opt.precision == DEM_PREC_MIXED) st = mixed_shadows(c, 0, c->stream);
+  if (c->opt.precision == DEM_PREC_MIXED) {
+    st = mixed_shadows(c, 0, c->stream);
+    if (st == DEM_OK) st = mixed_wall_entries(c, c->stream);
+  }
   if (st == DEM_OK) st = cuda_check(cudaStreamSynchronize(c->stream), "dem_load sync");
   return st;
 }

@@ -9,11 +9,12 @@
  *  - neighbour lists: nebor[S] level/slot-major (slot(q,k) = base[L] +
  *    k*npars[L] + nidx[q], coalesced across consecutive particles for a fixed
  *    k), num_nebor[N]; wall lists wlist[N][3], nwall[N];
- *  - contact history: 64-byte ContactRec per slot (+ one bridge byte), and
- *    3N wall records (slot (a, q) at a*N + q);
- *  - *_old copies of the used slots, written at the start of a rebuild and
- *    read by the carry-over (fixed pointers, so a rebuild can sit inside a
- *    CUDA-graph conditional node);
+ *  - the pair list (pairs.cuh): every pair of neighbours once, with its 64-byte
+ *    ContactRec and bridge byte, in two sets that a rebuild alternates between
+ *    (fixed pointers, so a rebuild can sit inside a CUDA graph); each slot's
+ *    pair index; the pairs' results of the running step;
+ *  - 3N wall records (slot (a, q) at a*N + q), with *_old copies a rebuild
+ *    writes first and carries over from;
  *  - mixed precision: FP32 shadow state read by neighbours, double-buffered
  *    per step (see mixed.cu).
  */
@@ -25,6 +26,7 @@
 #include <vector>
 
 #include "dem_internal.h"
+#include "pairs.cuh"
 
 namespace dem {
 
@@ -53,10 +55,13 @@ struct EngineBufs {
   double* rmom;
   /* lists */
   int *nebor, *num_nebor, *wlist, *nwall;
-  int *nebor_old, *num_nebor_old, *wlist_old, *nwall_old, *nidx_old;
-  /* history */
-  ContactRec *rec, *rec_old, *wrec, *wrec_old;
-  unsigned char *brg, *brg_old;
+  int *wlist_old, *nwall_old;
+  /* the pair list with its history, and each pair's result of the running
+   * step (mixed.cu / step64.cu) */
+  PairSet ps;
+  void* pair_out;
+  /* wall history */
+  ContactRec *wrec, *wrec_old;
   /* sort */
   int *sorted_hash, *sorted_src, *old_to_new, *cell_start, *cell_end;
   int* cell_off; /* every cell's offset in sorted order, and the total (C + 1) */
@@ -152,10 +157,10 @@ dem_status mixed_import(dem_ctx* c, int which, int has_v, int has_w, cudaStream_
  * inv[i] is caller index i's cell position */
 dem_status mixed_import_mapped(dem_ctx* c, int which, const int* inv, const double3* hp, const double3* hv,
                                const double3* hw, cudaStream_t s);
-/* the mixed step's pair loop: one thread per particle (true) or warp-cooperative */
-bool mixed_thread_loop(const dem_ctx* c);
-/* the name of the step kernel mixed_step launches, e.g. "k_step_mixed<1,0>" */
+/* the names of the kernels mixed_step launches */
 const char* mixed_step_kernel_name(const dem_ctx* c);
+/* the compact list of the wall slots in use, from fresh wall lists */
+dem_status mixed_wall_entries(dem_ctx* c, cudaStream_t s);
 /* copy the last step's bridge counts from the shadow `which` to the master */
 dem_status mixed_pre_rebuild(dem_ctx* c, int which, cudaStream_t s);
 /* download the last step's force totals into the FP64 force array */

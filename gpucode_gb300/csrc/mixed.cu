@@ -1,19 +1,28 @@
 /*
- * mixed.cu -- the fused FP32-force / FP64-state step kernel (sm_103a).
+ * mixed.cu -- the FP32-force / FP64-state step kernels (sm_103a).
  *
- * One launch per time step does, for each particle i (cell order, one thread):
- * gravity, every p-p contact and capillary bridge over i's neighbour slots,
- * the <= 3 cylinder-wall contacts, and the integrator -- the reference's
- * VarInit + PPForceCalcG + CirPWInterG + UpdateSystemG (kernel.cu:413-606,
- * 958-1023) in one pass.
+ * Two launches per time step: k_pair_mixed, one thread per pair of the pair
+ * list (pairs.cu) -- contact law and capillary bridge, the pair's history --
+ * with the listed walls as its first blocks; and k_body_mixed, one thread per
+ * sphere -- gravity, the sum of its pairs' and walls' results, the integrator.
+ * Together the reference's VarInit + PPForceCalcG + CirPWInterG + UpdateSystemG
+ * (kernel.cu:413-606, 958-1023).
+ *
+ * Why two: a thread per sphere that walks its own slots evaluates every pair
+ * twice, moves its history twice, keeps 18 of 32 lanes busy (lists of 2 to 30
+ * entries) and chains index -> shadow -> record -> law per slot.  On the packed
+ * 200k wet bed that one kernel took 114 us; the pair kernel takes 35 us (25 of
+ * 32 lanes, half the evaluations, 83 + 30 MB of DRAM traffic at 49 % occupancy;
+ * bound by the latency of its two rounds of loads) and the sphere kernel 35 us
+ * (bound by the gather of the pairs' results), 78 against 116 us a chained step;
+ * 2M spheres 710 against 912 us, 5,000 dry spheres 23 against 43 us.
  *
  * Why this shape on GB300: FP64 arithmetic runs at ~0.6 T op/s (1/58 of
  * FP32) and FP64 pow at ~6 G/s, so the reference's all-FP64 pair math is
  * bound by FP64 issue.  Here:
  *  - neighbours are read from FP32 "shadow" copies of last step's state
  *    (double-buffered: step t reads buffer t%2, writes the other), written by
- *    the integrator, so a neighbour costs one 16-byte gather until it is a
- *    contact candidate;
+ *    the integrator;
  *  - positions are shadowed as hi + lo float pairs of (x + offset), where the
  *    offset puts every coordinate in the binade [2^k, 2^(k+1)): hi_i - hi_j
  *    is then exact (Sterbenz), and the overlap d - (ri + rj) is computed as
@@ -28,7 +37,8 @@
  *    a small difference, v_t dt) so its accumulation error is relative to
  *    the increment, not to the spring;
  *  - contact records are 64 bytes (two DRAM sectors) read and written only for
- *    contacts; bridge flags are one byte per slot, coalesced across particles.
+ *    contacts, streamed past L2's reusable lines; bridge flags are one byte a
+ *    pair; a pair's two spheres get one evaluation, mirrored by its signs.
  */
 #include <cuda_runtime.h>
 
@@ -45,6 +55,8 @@ namespace dem {
 struct MixedState {
   float4 *phi[2], *plo[2], *vel[2], *angv[2];
   float4* force;
+  float4* wall_out; /* the step's wall results, two per wall slot */
+  int* wall_entry;  /* the listed wall slots (slot w of sphere q: w * n + q) */
   double3 off;
   float coarse_tol;
   int bin_exp;    /* FP64 biased exponent of the binade [2^k, 2^(k+1)) */
@@ -73,9 +85,12 @@ struct MixArgs {
   double3 *pos, *vel, *angv;
   const double* rad;
   double* pmove;
-  const int *nebor, *num_nebor, *plevel, *nidx, *npars, *nneb;
-  ContactRec* rec;
-  unsigned char* brg;
+  const int *num_nebor, *plevel, *nidx, *npars, *nneb;
+  PairSet ps;
+  float4* pair_out; /* two float4s per pair */
+  float4* wall_out; /* the same per wall slot */
+  const int* wall_entry; /* the listed wall slots, ctl[3] of them */
+  unsigned wall_blocks;
   const int *wlist, *nwall;
   ContactRec* wrec;
   float4* force_out;
@@ -135,18 +150,6 @@ struct KSum3 {
   KSum x, y, z;
   __device__ __forceinline__ void add(float3 v) { x.add(v.x); y.add(v.y); z.add(v.z); }
 };
-/* four Kahan sums kept as (sums, compensations) in two float4s of shared memory */
-__device__ __forceinline__ void kahan4(float4* acc, float3 v, float w) {
-  float4 sm = acc[0], cm = acc[1];
-  KSum t;
-  t.s = sm.x; t.c = cm.x; t.add(v.x); sm.x = t.s; cm.x = t.c;
-  t.s = sm.y; t.c = cm.y; t.add(v.y); sm.y = t.s; cm.y = t.c;
-  t.s = sm.z; t.c = cm.z; t.add(v.z); sm.z = t.s; cm.z = t.c;
-  t.s = sm.w; t.c = cm.w; t.add(w); sm.w = t.s; cm.w = t.c;
-  acc[0] = sm;
-  acc[1] = cm;
-}
-
 /* error-free transforms (Knuth two-sum, FMA two-product) */
 __device__ __forceinline__ float two_sum(float a, float b, float& err) {
   const float s = a + b;
@@ -208,12 +211,13 @@ __device__ __forceinline__ double f2d(float f) {
   return __longlong_as_double((long long)(sign | (de << 52) | ((unsigned long long)(b & 0x7fffffu) << 29)));
 }
 
-/* the elasto-plastic normal law, damping, tangential spring and rolling
- * resistance of kernel.cu:89-228 / :236-359 in FP32.  The spring is advanced
+/* the elasto-plastic normal law, damping and tangential spring of
+ * kernel.cu:89-228 / :236-359 in FP32: the normal force fN, the damping fD
+ * (both along u) and the friction fT.  The spring is advanced
  * as an FP64 update by a small FP32 increment (three FP64 adds per contact);
  * the maximum overlap stays an FP64 field. */
-__device__ __forceinline__ void law32(const Law32& c, float ijRad, float nrm, float3 u, float3 cpv, MixedRec& r,
-                                      float iRad, float rfrc, float dt, float3& dF, float3& dM, float& dR) {
+__device__ __forceinline__ void law32_forces(const Law32& c, float ijRad, float nrm, float3 u, float3 cpv, MixedRec& r,
+                                      float dt, float& fN_out, float& fD_out, float3& fT_out) {
   const float plstDfm0 = r.plstDfm, nDsp0 = r.nDsp, nDspMx0 = d2f(r.nDsp_mx);
   float plstRad = r.plstRad, plstDfm = plstDfm0;
   int st;
@@ -294,14 +298,25 @@ __device__ __forceinline__ void law32(const Law32& c, float ijRad, float nrm, fl
     const float lvt = lenf(vt);
     if (lvt > 1.0e-10f) fT = vt * __fdividef(-c.sfrc * fN * ratio, lvt);
   }
-  dF = (fN + fD) * u + fT;
-  const float arm = iRad - nrm * 0.5f;
-  dM = crossf(u * (-arm), fT);
-  dR = 0.5f * (rfrc + rfrc) * fN * iRad;
+  fN_out = fN;
+  fD_out = fD;
+  fT_out = fT;
   r.nDsp = nrm;
   r.plstRad = plstRad;
   r.plstDfm = plstDfm;
   r.stage = st;
+}
+
+/* the same with the force, moment and rolling moment on a sphere of radius iRad */
+__device__ __forceinline__ void law32(const Law32& c, float ijRad, float nrm, float3 u, float3 cpv, MixedRec& r,
+                                      float iRad, float rfrc, float dt, float3& dF, float3& dM, float& dR) {
+  float fN, fD;
+  float3 fT;
+  law32_forces(c, ijRad, nrm, u, cpv, r, dt, fN, fD, fT);
+  dF = (fN + fD) * u + fT;
+  const float arm = iRad - nrm * 0.5f;
+  dM = crossf(u * (-arm), fT);
+  dR = 0.5f * (rfrc + rfrc) * fN * iRad;
 }
 
 /* a bridge's force magnitude and rupture distance under the context's liquid
@@ -340,20 +355,6 @@ __device__ __forceinline__ void store_rec(ContactRec* p, const MixedRec& r) {
   __stcs(q + 3, o[3]);
 }
 
-/* One p-p contact (gap < 0, unit vector u from j to i): relative velocity at
- * the contact point, the law, and the 64-byte history record of slot s read
- * and written back */
-__device__ __forceinline__ void pp_contact(const Law32& law, ContactRec* rec, float ri, float rj, float3 iv,
-                                           float3 iw, float4 vj4, float4 wj4, float3 u, float gap, float rfrc,
-                                           float dt, float3& dF, float3& dM, float& dR) {
-  MixedRec rc = load_rec(rec);
-  const float3 cpv = f3(iv.x - vj4.x, iv.y - vj4.y, iv.z - vj4.z) -
-                     crossf(iw * ri + f3(wj4.x, wj4.y, wj4.z) * rj, u);
-  const float ijRad = ri * rj / (ri + rj);
-  law32(law, ijRad, -gap, u, cpv, rc, ri, rfrc, dt, dF, dM, dR);
-  store_rec(rec, rc);
-}
-
 /* hi/lo split of a coordinate already shifted into the binade [2^k, 2^(k+1)):
  * hi keeps the top 24 significand bits (exponent fixed), lo the remaining 29
  * bits as an exact integer times 2^(k-52), rounded to 24 bits.  Integer and
@@ -380,39 +381,29 @@ __device__ __forceinline__ void prefetch_l2(const void* p) {
 }
 
 __device__ __forceinline__ void warp_add(unsigned long long* ctr, unsigned v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  v = __reduce_add_sync(0xffffffffu, v);
   if ((threadIdx.x & 31) == 0 && v) atomicAdd(ctr, (unsigned long long)v);
 }
 
-/* One bridge waiting for the learned closure: 40 bytes in a per-warp queue in
- * shared memory.  After the network has run, sep and vol hold its two outputs
+/* One bridge of a warp's pairs waiting for the learned closure (16 bytes in
+ * shared memory); after the network has run, sep and vol hold its two outputs
  * (normalised force, rupture distance). */
-struct CapEntry {
+struct __align__(16) CapEntry {
   float sep, vol, theta, ratio; /* raw features */
-  float wx, wy, wz;             /* -2 pi R_eff gamma u: the force per unit normalised force */
-  float gap;
-  unsigned slot;
-  int meta; /* bit 0: the bridge forms this step (gap below the liquid layer); bits 8..: 1 + the
-               queue index of the same lane's previous entry (0: none) */
 };
-constexpr int kCapQ = 128; /* entries per warp; flushed before an iteration could overflow it */
 #ifndef DEM_NET_BLOCKS
-#define DEM_NET_BLOCKS 4
+#define DEM_NET_BLOCKS 6
 #endif
-/* resident blocks per SM the network variant is built for: 4 (no register
- * spills) measured faster than 5 on the 200k wet bed */
-constexpr int kNetBlocks = DEM_NET_BLOCKS;
-constexpr int kWarps = 4;  /* warps per block of the step kernel */
-constexpr size_t kCapSmem = ((sizeof(CapNetSmem) + 15) / 16) * 16 + sizeof(CapEntry) * kCapQ * kWarps;
+constexpr int kNetBlocks = DEM_NET_BLOCKS; /* resident blocks per SM the network variant is built for */
+constexpr int kWarps = 4;                  /* warps per block of the step kernels */
+constexpr size_t kCapSmem = ((sizeof(CapNetSmem) + 15) / 16) * 16 + sizeof(CapEntry) * 32 * kWarps;
 
 __device__ __forceinline__ uint32_t cap_pair(const CapNetSmem& w, const CapEntry& e, int t) {
   return cap_pair(w, e.sep, e.vol, e.theta, e.ratio, t);
 }
 
-/* Run the queued bridges of this warp through the network in 16-row BF16
- * tensor-core tiles; each entry's sep / vol fields receive the two outputs
- * (normalised force, rupture distance).  All 32 lanes call it. */
+/* Run this warp's queued bridges (at most 32) through the network in 16-row
+ * BF16 tensor-core tiles.  All 32 lanes call it. */
 __device__ __forceinline__ void cap_run_queue(const CapNetSmem& w, CapEntry* qw, int qn) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   __syncwarp();
@@ -440,97 +431,393 @@ __device__ __forceinline__ void cap_run_queue(const CapNetSmem& w, CapEntry* qw,
   }
 }
 
-/* Run the queue through the network, then let every lane fold in its own
- * bridges, walking its chain of entries from the newest: rupture decision,
- * bridge flag, force.  All 32 lanes call it; `last` is the lane's newest
- * entry (-1: none). */
-__device__ __forceinline__ void cap_flush(const CapNetSmem& w, CapEntry* qw, int qn, int last, unsigned char* brg,
-                                          KSum3& F, int& wet, unsigned& nbr, unsigned& nmlp) {
-  cap_run_queue(w, qw, qn);
-  for (int e = last; e >= 0;) {
-    const CapEntry& en = qw[e];
-    e = (en.meta >> 8) - 1;
-    const int b = (en.meta & 1) ? 1 : (en.gap > en.vol ? 0 : 1);
-    brg[en.slot] = (unsigned char)b;
-    nmlp++;
-    if (b) {
-      F.add(f3(en.wx, en.wy, en.wz) * en.sep);
-      wet++;
-      if (en.gap >= 0.f) nbr++;
-    }
+/* One entry of the wall list (sphere q's wall slot w) against its cylinder, the
+ * distance in FP64 (CirPWInterG, kernel.cu:958-1023).  The result: the force
+ * and the normal force, the moment and the overlap (0: no contact).  Listed walls are evaluated from a compact
+ * list (k_wall_entries), one thread each, because a listed sphere is one in
+ * six and a touching one in fifteen, spread over almost every warp of a thread
+ * per sphere, and the exact distance is two FP64 roots and three divisions. */
+__device__ __forceinline__ void wall_entry(const MixArgs& a, int e) {
+  const int w = e / a.n, q = e - w * a.n;
+  const float4 hi = ro(a.phi_in + q), lo = ro(a.plo_in + q);
+  const float ri = hi.w + lo.w;
+  const CylinderBC cy = a.cyl[a.sys_of_id ? a.sys_of_id[ro(a.id + q)] : 0];
+  const int kind = a.wlist[3 * q + w];
+  float4 f = make_float4(0.f, 0.f, 0.f, 0.f), t = f;
+  /* A wall the sphere certainly does not touch costs no FP64 work: a coarse
+   * gap from the shadow (hi part of x + offset, truncated to the binade) is
+   * within wall_tol of the exact one -- 5 binade ulps for the flat walls, 11
+   * for the curved one, bounded by 16 -- so only spheres within wall_tol of a
+   * wall take the reference's geometry. */
+  float gc;
+  if (kind == 2) {
+    const float cxo = d2f(cy.cir.x) + a.offf.x, cyo = d2f(cy.cir.y) + a.offf.y;
+    const float dx = hi.x - cxo, dy = hi.y - cyo;
+    gc = fabsf(sqrtf(dx * dx + dy * dy) - d2f(cy.R)) - ri;
+  } else {
+    gc = fabsf(hi.z - (d2f(kind == 0 ? cy.Tw : cy.Bw) + a.offf.z)) - ri;
   }
-  __syncwarp();
-}
-
-/* After the pair loop, per particle: the <= 3 cylinder-wall contacts
- * (CirPWInterG, kernel.cu:958-1023), the integrator (UpdateSystemG,
- * kernel.cu:563-606), the next step's shadows and the counters. */
-template <bool NET>
-__device__ __forceinline__ void finish_particle(const MixArgs& a, int q, int qq, bool live, int sys, float4 hi,
-                                                float4 lo, float4 wi4, float3 iv, float3 iw, float ri, float twor,
-                                                float mass_f, KSum3& F, KSum3& M, KSum& R, int wet, unsigned nn,
-                                                unsigned ncont, unsigned nbr, unsigned nmlp, unsigned nfall) {
-  /* cylinder walls (CirPWInterG), geometry in FP64 */
-  unsigned nwc = 0;
-  double3 p = a.pos[qq];
-  const int nw = live ? a.nwall[qq] : 0;
-  if (nw > 0) {
-    const double rid = a.rad[qq];
-    const CylinderBC cy = a.cyl[sys];
-    double3 jvel = make_double3(0.0, 0.0, 0.0);
-    for (int w = 0; w < nw; w++) {
-      const int kind = a.wlist[3 * qq + w];
+  if (gc <= a.wall_tol) {
+    const double3 p = a.pos[q];
+    const double rid = a.rad[q];
+    double3 jp;
+    if (kind == 2) {
+      const double ddx = cy.cir.x - p.x, ddy = cy.cir.y - p.y;
+      const double dist = sqrt(ddx * ddx + ddy * ddy);
+      jp = make_double3(cy.R * ((p.x - cy.cir.x) / dist) + cy.cir.x, cy.R * ((p.y - cy.cir.y) / dist) + cy.cir.y,
+                        p.z);
+    } else {
+      jp = make_double3(p.x, p.y, kind == 0 ? cy.Tw : cy.Bw);
+    }
+    const double3 d = make_double3(p.x - jp.x, p.y - jp.y, p.z - jp.z);
+    const double len = sqrt(d.x * d.x + d.y * d.y + d.z * d.z);
+    const float gapw = (float)(len - rid);
+    if (gapw < 0.f) {
+      const float il = (float)(1.0 / len);
+      const float3 u = f3((float)d.x * il, (float)d.y * il, (float)d.z * il);
+      const float4 vi4 = ro(a.v_in + q), wi4 = ro(a.w_in + q);
       /* the top wall's velocity carries over to the walls after it in the
        * list, as the reference's jVel does (kernel.cu:987-1020) */
-      if (kind == 0) jvel = make_double3(0.0, 0.0, cy.topv);
-      /* A wall the particle certainly does not touch costs no FP64 work:
-       * a coarse gap from the shadow (hi part of x + offset, truncated to
-       * the binade) is within wall_tol of the exact one -- 5 binade ulps for
-       * the flat walls, 11 for the curved one, bounded by 16 -- so only
-       * particles within wall_tol of a wall take the reference's geometry. */
-      float gc;
-      if (kind == 0 || kind == 1) {
-        gc = fabsf(hi.z - (d2f(kind == 0 ? cy.Tw : cy.Bw) + a.offf.z)) - ri;
-      } else if (kind == 2) {
-        const float cxo = d2f(cy.cir.x) + a.offf.x, cyo = d2f(cy.cir.y) + a.offf.y;
-        const float dx = hi.x - cxo, dy = hi.y - cyo;
-        gc = fabsf(sqrtf(dx * dx + dy * dy) - d2f(cy.R)) - ri;
-      } else {
-        continue;
+      double jv = 0.0;
+      for (int k = 0; k <= w; k++)
+        if (a.wlist[3 * q + k] == 0) jv = cy.topv;
+      const float3 cpv = (f3(vi4.x, vi4.y, vi4.z) - f3(0.f, 0.f, (float)jv)) - crossf(f3(wi4.x, wi4.y, wi4.z) * ri, u);
+      ContactRec* rp = a.wrec + (long long)w * a.n + q;
+      MixedRec rc = load_rec(rp);
+      float fN, fD;
+      float3 fT;
+      law32_forces(a.pw, ri, -gapw, u, cpv, rc, a.dtf, fN, fD, fT);
+      store_rec(rp, rc);
+      const float3 F = (fN + fD) * u + fT, M = crossf(u * (-(ri - -gapw * 0.5f)), fT);
+      f = make_float4(F.x, F.y, F.z, fN);
+      t = make_float4(M.x, M.y, M.z, -gapw);
+    }
+  }
+  a.wall_out[2 * (size_t)e] = f;
+  a.wall_out[2 * (size_t)e + 1] = t;
+}
+
+/* resident blocks per SM the pair kernel is built for: 8 (56 registers, no
+ * spills) 80.5 us a step on the packed 200k bed, 7 84.5, 6 86.4; 2M spheres 710,
+ * 746, 770 us */
+#ifndef DEM_PAIR_BLOCKS
+#define DEM_PAIR_BLOCKS 8
+#endif
+
+/* One thread per pair of the list: overlap, contact law, capillary bridge, the
+ * pair's history.  What it leaves for the two spheres (k_body_mixed) is what
+ * each would have computed for itself, in pieces that are the same for both
+ * but for their sign: the normal u and the overlap (0: no contact; the sign bit
+ * says that a bridge acts), the friction fT and the normal force with damping,
+ * and, where a bridge acts or the material rolls, fN and the bridge's force:
+ * u c_i and u c_j for the two spheres (formula, d = 1), or u c_i times the
+ * network's output, d for the first sphere and c_j for the second. */
+template <bool WET, bool NET>
+__global__ void __launch_bounds__(128, NET ? kNetBlocks : DEM_PAIR_BLOCKS) k_pair_mixed(const __grid_constant__ MixArgs a) {
+  const int4 ct = pair_ctl(a.ps);
+  if (a.gate && *a.gate) return;
+  if (blockIdx.x < a.wall_blocks) { /* the first blocks take the wall list */
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < ct.w; k += a.wall_blocks * blockDim.x)
+      wall_entry(a, a.wall_entry[k]);
+    return;
+  }
+  extern __shared__ __align__(16) unsigned char dsm[];
+  const CapNetSmem* capw = reinterpret_cast<const CapNetSmem*>(dsm);
+  CapEntry* qw = reinterpret_cast<CapEntry*>(dsm + ((sizeof(CapNetSmem) + 15) / 16) * 16) + (threadIdx.x >> 5) * 32;
+  const int P = ct.x ? ct.z : ct.y;
+  const int2* __restrict__ pair = ct.x ? a.ps.pair[1] : a.ps.pair[0];
+  ContactRec* const rec = ct.x ? a.ps.rec[1] : a.ps.rec[0];
+  unsigned char* const brg = ct.x ? a.ps.brg[1] : a.ps.brg[0];
+  if (NET) {
+    cap_stage(a.capw, reinterpret_cast<CapNetSmem*>(dsm));
+    __syncthreads();
+  }
+  unsigned nmlp = 0, nfall = 0;
+  const int lane = threadIdx.x & 31;
+  const int step = (gridDim.x - a.wall_blocks) * blockDim.x;
+  const int first = (blockIdx.x - a.wall_blocks) * blockDim.x + threadIdx.x;
+  /* NET: whole warps go round together */
+  const int last = NET ? (P + 31) / 32 * 32 : P;
+  for (int p = first; p < last; p += step) {
+    const bool act = !NET || p < P;
+    bool want = false; /* NET: this lane's bridge goes to the network */
+    bool form = false, wet = false;
+    int bprev = 0;
+    float gap = 0.f, fN = 0.f, nrm = 0.f, s_n = 0.f, ci = 0.f, cj = 0.f, d = 1.0f;
+    float3 fT = f3(0.f, 0.f, 0.f), u = f3(0.f, 0.f, 0.f);
+    CapEntry ent, ent_j;
+    bool want_j = false;
+    if (act) {
+      const int2 ij = ro(pair + p);
+      const int i = ij.x, j = ij.y;
+      const float4 hi = ro(a.phi_in + i), hj = ro(a.phi_in + j);
+      const float4 lo = ro(a.plo_in + i), lj = ro(a.plo_in + j);
+      const float4 vi = ro(a.v_in + i), vj = ro(a.v_in + j);
+      if (WET) bprev = brg[p];
+      const float ax = hi.x - hj.x, ay = hi.y - hj.y, az = hi.z - hj.z; /* exact */
+      const float ri = hi.w + lo.w;
+      float rj;
+      gap = exact_gap(hi, lo, hj, lj, ax, ay, az, u, rj);
+      if (gap < 0.f) {
+        const float4 wi = ro(a.w_in + i), wj = ro(a.w_in + j);
+        MixedRec rc = load_rec(rec + p);
+        const float3 cpv = f3(vi.x - vj.x, vi.y - vj.y, vi.z - vj.z) -
+                           crossf(f3(wi.x, wi.y, wi.z) * ri + f3(wj.x, wj.y, wj.z) * rj, u);
+        float fD;
+        nrm = -gap;
+        law32_forces(a.pp, ri * rj / (ri + rj), nrm, u, cpv, rc, a.dtf, fN, fD, fT);
+        store_rec(rec + p, rc);
+        s_n = fN + fD;
       }
-      if (gc > a.wall_tol) continue;
-      double3 jp;
-      if (kind == 0) {
-        jp = make_double3(p.x, p.y, cy.Tw);
-      } else if (kind == 1) {
-        jp = make_double3(p.x, p.y, cy.Bw);
-      } else if (kind == 2) {
-        const double ddx = cy.cir.x - p.x, ddy = cy.cir.y - p.y;
-        const double dist = sqrt(ddx * ddx + ddy * ddy);
-        jp = make_double3(cy.R * ((p.x - cy.cir.x) / dist) + cy.cir.x, cy.R * ((p.y - cy.cir.y) / dist) + cy.cir.y,
-                          p.z);
-      } else {
-        continue;
-      }
-      const double3 d = make_double3(p.x - jp.x, p.y - jp.y, p.z - jp.z);
-      const double len = sqrt(d.x * d.x + d.y * d.y + d.z * d.z);
-      const float gapw = (float)(len - rid);
-      if (gapw < 0.f) {
-        const float il = (float)(1.0 / len);
-        const float3 u = f3((float)d.x * il, (float)d.y * il, (float)d.z * il);
-        const float3 cpv = (iv - f3((float)jvel.x, (float)jvel.y, (float)jvel.z)) - crossf(iw * ri, u);
-        ContactRec* rp = a.wrec + (long long)w * a.n + qq;
-        MixedRec rc = load_rec(rp);
-        float3 dF, dM;
-        float dR;
-        law32(a.pw, ri, -gapw, u, cpv, rc, ri, a.rfrc, a.dtf, dF, dM, dR);
-        store_rec(rp, rc);
-        F.add(dF);
-        M.add(dM);
-        R.add(dR);
-        nwc++;
+      if (WET && (!a.sys_wet || a.sys_wet[a.sys_of_id[ro(a.id + i)]])) {
+        form = gap < 2.0f * a.lqd_layer * (ri + rj);
+        if (form || bprev) {
+          /* the pair's bridge volume and contact angle: the reference's split of
+           * both spheres' liquid, or the per-contact model's.  Each sphere adds
+           * the partner's share (and angle) to its own, rounded first: vol_j and
+           * th_j are what the second sphere gets, mostly the same bits. */
+          float vol, vol_j, th_i = 0.f, th_j = 0.f;
+          int id_i = 0, id_j = 0;
+          if (NET || a.lq_mode) {
+            id_i = ro(a.id + i);
+            id_j = ro(a.id + j);
+            /* the mean contact angle, the own angle rounded first */
+            const float tm = a.lq_mode ? a.lq_theta_max : a.theta_max;
+            const float xi = a.lq_mode ? cap_theta32(id_i, a.lq_seed, 1.0f) : cap_theta(id_i, a.theta_seed, 1.0f);
+            const float xj = a.lq_mode ? cap_theta32(id_j, a.lq_seed, 1.0f) : cap_theta(id_j, a.theta_seed, 1.0f);
+            th_i = 0.5f * fmaf(tm, xj, __fmul_rn(tm, xi));
+            th_j = 0.5f * fmaf(tm, xi, __fmul_rn(tm, xj));
+          }
+          if (a.lq_mode == 0) {
+            const int inl = max(__float_as_int(vi.w), 12), jnl = max(__float_as_int(vj.w), 12);
+            const float ti = 2.0f * ri, tj = 2.0f * rj;
+            const float mi = ti * ti * ti, mj = tj * tj * tj;
+            const float qi = __fdividef(1.0f, (float)inl), qj = __fdividef(1.0f, (float)jnl);
+            const float xi = a.lqd_vol * mi, xj = a.lqd_vol * mj;
+            vol = fmaf(xj, qj, __fmul_rn(xi, qi));
+            vol_j = fmaf(xi, qi, __fmul_rn(xj, qj));
+          } else {
+            vol = vol_j = pair_bridge_volume32(id_i, id_j, a.lq_seed, a.lq_vmin, a.lq_vspan, fminf(ri, rj));
+          }
+          const float lq_th_i = a.lq_mode ? th_i : 0.f, lq_th_j = a.lq_mode ? th_j : 0.f;
+          const float effR = 2.0f * ri * rj / (ri + rj);
+          if (NET) {
+            ent = CapEntry{fmaxf(a.lqd_gapmn, fmaxf(gap, 0.f)), 8.0f * vol, th_i,
+                           __fdividef(fminf(ri, rj), fmaxf(ri, rj))};
+            want = cap_in_hull(*capw, ent.sep, ent.vol, ent.theta, ent.ratio);
+            /* the second sphere's features, where their BF16 roundings differ */
+            ent_j = ent;
+            ent_j.vol = 8.0f * vol_j;
+            ent_j.theta = th_j;
+            want_j = want && (cap_pair(*capw, ent, 0) != cap_pair(*capw, ent_j, 0) ||
+                              cap_pair(*capw, ent, 1) != cap_pair(*capw, ent_j, 1));
+          }
+          if (!NET || !want) {
+            const int b = form ? 1 : (gap > bridge_rupture32(a, vol, lq_th_i) ? 0 : 1);
+            if (b != bprev) brg[p] = (unsigned char)b;
+            if (b) {
+              const float sep = gap < 0.f ? 0.f : gap;
+              ci = -bridge_force32(a, sep, vol, lq_th_i, effR);
+              cj = vol_j == vol && lq_th_j == lq_th_i ? ci : -bridge_force32(a, sep, vol_j, lq_th_j, effR);
+              wet = true;
+            }
+            if (NET) nfall++;
+          } else {
+            ci = -2.0f * kPiF * effR * a.lqd_st;
+          }
+        }
       }
     }
+    if (NET) {
+      const unsigned m = __ballot_sync(0xffffffffu, want);
+      const unsigned mj = __ballot_sync(0xffffffffu, want_j);
+      const unsigned below = (1u << lane) - 1u;
+      const int at = __popc(m & below);
+      if (want) qw[at] = ent;
+      if (m) cap_run_queue(*capw, qw, __popc(m));
+      if (want) {
+        d = cj = qw[at].sep;
+        const int b = form ? 1 : (gap > qw[at].vol ? 0 : 1);
+        if (b != bprev) brg[p] = (unsigned char)b;
+        wet = b != 0;
+        nmlp++;
+      }
+      if (mj) {
+        __syncwarp();
+        const int atj = __popc(mj & below);
+        if (want_j) qw[atj] = ent_j;
+        cap_run_queue(*capw, qw, __popc(mj));
+        if (want_j) cj = qw[atj].sep;
+      }
+      __syncwarp(); /* the queue is read before the next round fills it */
+    }
+    if (act) {
+      float4* o = a.pair_out + 2 * (size_t)p;
+      o[0] = make_float4(u.x, u.y, u.z, __uint_as_float(__float_as_uint(nrm) | (wet ? 0x80000000u : 0u)));
+      if (nrm > 0.f) o[1] = make_float4(fT.x, fT.y, fT.z, s_n);
+      if (wet || (a.rfrc != 0.f && nrm > 0.f)) a.pair_out[2 * (size_t)a.ps.cap + p] = make_float4(fN, ci, cj, d);
+    }
+  }
+  if (NET && a.counters) {
+    /* counted once per sphere, as every sphere feels its bridges */
+    warp_add(&a.counters[5], 2u * nmlp);
+    warp_add(&a.counters[6], 2u * nfall);
+  }
+}
+
+/* resident blocks per SM the sphere kernel is built for, and the pair results
+ * a sphere has in flight: 6 and 3, 81.8 us a step on the packed 200k bed; 4 in
+ * flight 86.4 (a few spills), 2 83.4, 1 89.4; 5 blocks with 4 89.0, 8 with 2 84.0 */
+#ifndef DEM_BODY_BLOCKS
+#define DEM_BODY_BLOCKS 6
+#endif
+#ifndef DEM_BODY_BATCH
+#define DEM_BODY_BATCH 3
+#endif
+constexpr int kBodyBatch = DEM_BODY_BATCH;
+
+/* a pair's vector as the slot's sphere sees it: the second sphere's (e < 0)
+ * points the other way.  Sign bits, not a product, so that no contraction
+ * touches it. */
+__device__ __forceinline__ float3 turned(float4 v, int e) {
+  const unsigned m = (unsigned)e & 0x80000000u;
+  return f3(__uint_as_float(__float_as_uint(v.x) ^ m), __uint_as_float(__float_as_uint(v.y) ^ m),
+            __uint_as_float(__float_as_uint(v.z) ^ m));
+}
+
+/* One thread per sphere: gravity, its pairs' results summed in neighbour order
+ * with Kahan compensation, the <= 3 cylinder-wall contacts (CirPWInterG,
+ * kernel.cu:958-1023), the integrator (UpdateSystemG, kernel.cu:563-606), the
+ * next step's shadows and the counters. */
+template <bool WET, bool NET>
+__global__ void __launch_bounds__(128, DEM_BODY_BLOCKS) k_body_mixed(MixArgs a) {
+  if (a.gate && *a.gate) return;
+  const int q = reversed_block_thread(); /* the spheres with the most pairs first */
+  const bool live = q < a.n;
+  const int qq = live ? q : a.n - 1;
+  __shared__ unsigned sums[5];
+  if (threadIdx.x < 5) sums[threadIdx.x] = 0u;
+  __syncthreads();
+  /* the integrator's FP64 state and the wall count are needed only after the
+   * pairs: start bringing them in now */
+  prefetch_l2(a.pos + qq);
+  prefetch_l2(a.vel + qq);
+  prefetch_l2(a.angv + qq);
+  prefetch_l2(a.pmove + qq);
+  prefetch_l2(a.nwall + qq);
+  const int L = ro(a.plevel + qq);
+  const int nn = live ? ro(a.num_nebor + qq) : 0;
+  const long long stride = ro(a.npars + L);
+  const long long base = slot_base(L, a.npars, a.nneb) + ro(a.nidx + qq);
+  const float4 hi = ro(a.phi_in + qq), lo = ro(a.plo_in + qq), wi4 = ro(a.w_in + qq);
+  const float ri = hi.w + lo.w, twor = 2.0f * ri;
+  const float mass_f = __fmul_rn(__fmul_rn(twor, twor), twor);
+  KSum3 F, M;
+  KSum R;
+  F.z.add(-mass_f); /* gravity, m = (2r)^3 */
+  int wet = 0;
+  unsigned ncont = 0, nbr = 0;
+  if (NET) {
+    /* The network's bridges join the sum a warp's queue at a time, the newest
+     * first, once more than kCapQ - 32 wait: the order in which a kernel that
+     * queues them while it walks the slots adds them. */
+    constexpr int kCapQ = 128;
+    const int nloop = __reduce_max_sync(0xffffffffu, nn);
+    int queued = 0, since = 0;
+    auto flush = [&](int end) {
+      for (int k = min(end, nn) - 1; k >= since; k--) {
+        const int e = ro(a.ps.eidx + base + (long long)k * stride);
+        if (e == kNoPair) continue;
+        const int p = e < 0 ? ~e : e;
+        const float4 nu = a.pair_out[2 * (size_t)p];
+        if (!(__float_as_uint(nu.w) >> 31)) continue;
+        const float4 br = a.pair_out[2 * (size_t)a.ps.cap + p];
+        if (br.w == 1.0f) continue;
+        F.add((turned(nu, e) * br.y) * (e < 0 ? br.z : br.w));
+      }
+      since = end;
+    };
+    for (int k = 0; k < nloop; k++) {
+      bool net = false;
+      const int e = k < nn ? ro(a.ps.eidx + base + (long long)k * stride) : kNoPair;
+      if (e != kNoPair) {
+        const int p = e < 0 ? ~e : e;
+        const float4 nu = a.pair_out[2 * (size_t)p], ft = a.pair_out[2 * (size_t)p + 1],
+                     br = a.pair_out[2 * (size_t)a.ps.cap + p];
+        const unsigned nb = __float_as_uint(nu.w);
+        const float nrm = fabsf(nu.w);
+        const float3 u = turned(nu, e);
+        if (nrm > 0.f) {
+          const float3 fT = turned(ft, e);
+          F.add(ft.w * u + fT);
+          const float arm = ri - nrm * 0.5f;
+          M.add(crossf(u * (-arm), fT));
+          if (a.rfrc != 0.f) R.add(0.5f * (a.rfrc + a.rfrc) * br.x * ri);
+          ncont++;
+        }
+        if (nb >> 31) {
+          net = br.w != 1.0f;
+          if (!net) F.add(u * (e < 0 ? br.z : br.y));
+          wet++;
+          if (!(nrm > 0.f)) nbr++;
+        }
+      }
+      queued += __popc(__ballot_sync(0xffffffffu, net));
+      if (queued > kCapQ - 32) {
+        flush(k + 1);
+        queued = 0;
+      }
+    }
+    flush(nloop);
+  }
+  for (int k0 = 0; !NET && k0 < nn; k0 += kBodyBatch) {
+    int e[kBodyBatch];
+    float4 nu[kBodyBatch], ft[kBodyBatch], br[kBodyBatch];
+#pragma unroll
+    for (int t = 0; t < kBodyBatch; t++)
+      e[t] = k0 + t < nn ? ro(a.ps.eidx + base + (long long)(k0 + t) * stride) : kNoPair;
+#pragma unroll
+    for (int t = 0; t < kBodyBatch; t++) {
+      nu[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+      ft[t] = br[t] = nu[t];
+      if (e[t] != kNoPair) {
+        const int p = e[t] < 0 ? ~e[t] : e[t];
+        nu[t] = a.pair_out[2 * (size_t)p];
+        ft[t] = a.pair_out[2 * (size_t)p + 1];
+        if (WET || a.rfrc != 0.f) br[t] = a.pair_out[2 * (size_t)a.ps.cap + p];
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < kBodyBatch; t++) {
+      const unsigned nb = __float_as_uint(nu[t].w);
+      if (nb == 0u) continue; /* neither contact nor bridge (or no pair) */
+      const float nrm = fabsf(nu[t].w);
+      const float3 u = turned(nu[t], e[t]);
+      if (nrm > 0.f) {
+        const float3 fT = turned(ft[t], e[t]);
+        F.add(ft[t].w * u + fT);
+        const float arm = ri - nrm * 0.5f;
+        M.add(crossf(u * (-arm), fT));
+        if (a.rfrc != 0.f) R.add(0.5f * (a.rfrc + a.rfrc) * br[t].x * ri);
+        ncont++;
+      }
+      if (WET && (nb >> 31)) {
+        F.add(u * (e[t] < 0 ? br[t].z : br[t].y));
+        wet++;
+        if (!(nrm > 0.f)) nbr++;
+      }
+    }
+  }
+  unsigned nwc = 0;
+  const int nw = live ? a.nwall[qq] : 0;
+  for (int w = 0; w < nw; w++) {
+    const float4* r = a.wall_out + 2 * ((size_t)w * a.n + qq);
+    const float4 t = r[1], f = r[0];
+    if (!(t.w > 0.f)) continue;
+    F.add(f3(f.x, f.y, f.z));
+    M.add(f3(t.x, t.y, t.z));
+    R.add(0.5f * (a.rfrc + a.rfrc) * f.w * ri);
+    nwc++;
   }
 
   /* integrator (UpdateSystemG) in FP64 with FP32 increments */
@@ -541,7 +828,7 @@ __device__ __forceinline__ void finish_particle(const MixArgs& a, int q, int qq,
      * goes through the integer pipe */
     const float fx = F.x.s - F.x.c, fy = F.y.s - F.y.c, fz = F.z.s - F.z.c;
     const float inv_m = a.dtf / mass_f;
-    double3 v = a.vel[q];
+    double3 p = a.pos[q], v = a.vel[q];
     v.x += f2d(fx * inv_m);
     v.y += f2d(fy * inv_m);
     v.z += f2d(fz * inv_m);
@@ -591,676 +878,47 @@ __device__ __forceinline__ void finish_particle(const MixArgs& a, int q, int qq,
   const unsigned fm = __ballot_sync(0xffffffffu, flagged);
   if ((threadIdx.x & 31) == 0 && fm) atomicAdd(a.flag, __popc(fm));
   if (a.counters) {
-    warp_add(&a.counters[0], (unsigned)nn);
-    warp_add(&a.counters[1], ncont);
-    warp_add(&a.counters[2], nbr);
-    warp_add(&a.counters[3], nwc);
-    if (NET) {
-      warp_add(&a.counters[5], nmlp);
-      warp_add(&a.counters[6], nfall);
-    }
-  }
-}
-
-/* resident blocks per SM the thread loop is built for: 6 (80 registers, a few
- * bytes of spills; its moment sums live in shared memory) measured 5 % faster
- * on the packed 200k wet bed than 5 (96 registers); 7 spills more and is slower */
-#ifndef DEM_MIXED_BLOCKS
-#define DEM_MIXED_BLOCKS 6
-#endif
-
-template <bool WET, bool NET>
-__global__ void __launch_bounds__(128, NET ? kNetBlocks : DEM_MIXED_BLOCKS) k_step_mixed(MixArgs a) {
-  if (a.n <= 0 || (a.gate && *a.gate)) return;
-  const int q = reversed_block_thread(); /* the heaviest particles first */
-  const bool live = q < a.n;
-  const int qq = live ? q : a.n - 1;
-  extern __shared__ __align__(16) unsigned char dsm[];
-  const CapNetSmem* capw = reinterpret_cast<const CapNetSmem*>(dsm);
-  CapEntry* qw = reinterpret_cast<CapEntry*>(dsm + ((sizeof(CapNetSmem) + 15) / 16) * 16) +
-                 (threadIdx.x >> 5) * kCapQ;
-  if (NET) {
-    cap_stage(a.capw, reinterpret_cast<CapNetSmem*>(dsm));
-    __syncthreads();
-  }
-  /* the integrator's FP64 state is needed only after the pair loop: start
-   * bringing it in now */
-  prefetch_l2(a.pos + qq);
-  prefetch_l2(a.vel + qq);
-  prefetch_l2(a.angv + qq);
-  prefetch_l2(a.pmove + qq);
-  /* so are the wall count and list, which would otherwise be two dependent
-   * DRAM misses at the end of the warp's work */
-  prefetch_l2(a.nwall + qq);
-  prefetch_l2(a.wlist + 3 * qq);
-
-  const float4 hi = ro(a.phi_in + qq), lo = ro(a.plo_in + qq), vi4 = ro(a.v_in + qq), wi4 = ro(a.w_in + qq);
-  const float ri = hi.w + lo.w;
-  const float3 iv = f3(vi4.x, vi4.y, vi4.z), iw = f3(wi4.x, wi4.y, wi4.z);
-  const float twor = 2.0f * ri;
-  const float mass_f = twor * twor * twor;
-  KSum3 F;
-  F.z.add(-mass_f); /* gravity, m = (2r)^3 */
-  /* the moment and rolling-moment Kahan sums (sum, compensation) wait in
-   * shared memory while the pairs are evaluated: registers for the pair loop */
-  __shared__ float4 mr_acc[2 * 128];
-  float4* const mra = mr_acc + 2 * threadIdx.x;
-  mra[0] = make_float4(0.f, 0.f, 0.f, 0.f);
-  mra[1] = make_float4(0.f, 0.f, 0.f, 0.f);
-  int wet = 0;
-  float iVol = 0.f;
-  /* batched systems: this particle's system (its cylinder, dry or wet) */
-  const int sys = a.sys_of_id ? a.sys_of_id[ro(a.id + qq)] : 0;
-  const bool wet_i = WET && (!a.sys_wet || a.sys_wet[sys]);
-  if (WET) {
-    int inl = __float_as_int(vi4.w);
-    if (inl < 12) inl = 12;
-    iVol = a.lqd_vol * mass_f / (float)inl;
-  }
-  const int L = ro(a.plevel + qq);
-  const long long stride = ro(a.npars + L);
-  const long long base = slot_base(L, a.npars, a.nneb) + ro(a.nidx + qq);
-  const int nn = live ? ro(a.num_nebor + qq) : 0;
-  unsigned ncont = 0, nbr = 0, nmlp = 0, nfall = 0;
-  /* learned closure: the warp walks its lanes' slots in lockstep so that
-   * bridges can be queued and evaluated 16 at a time on the tensor cores */
-  const int lane = threadIdx.x & 31;
-  const int nloop = NET ? __reduce_max_sync(0xffffffffu, nn) : nn;
-  const int id_i = (NET || (WET && a.lq_mode)) ? ro(a.id + qq) : 0;
-  const float th_i = (WET && a.lq_mode) ? cap_theta32(id_i, a.lq_seed, a.lq_theta_max)
-                     : NET              ? cap_theta(id_i, a.theta_seed, a.theta_max)
-                                        : 0.f;
-  int qn = 0;    /* entries in this warp's queue (warp-uniform) */
-  int last = -1; /* this lane's newest entry in it */
-  /* one slot ahead: the next partner's index and coarse shadow are in flight
-   * while the current pair is evaluated */
-  int j_next = nn > 0 ? ro(a.nebor + base) : 0;
-  float4 hj_next = ro(a.phi_in + j_next);
-  for (int k = 0; k < nloop; k++) {
-    bool want = false; /* NET: this lane queues `ent` at the end of the iteration */
-    CapEntry ent;
-    if (!NET || k < nn) { /* the slot body (lanes with a k-th neighbour) */
-    const long long s = base + k * stride;
-    const int j = j_next;
-    const float4 hj = hj_next;
-    if (k + 1 < nn) {
-      j_next = ro(a.nebor + s + stride);
-      hj_next = ro(a.phi_in + j_next);
-      /* the next pair's lo parts (and, wet, its velocity record and bridge
-       * flag) are read by every candidate: into L2 while this pair runs */
-      prefetch_l2(a.plo_in + j_next);
-      if (WET) {
-        prefetch_l2(a.v_in + j_next);
-        prefetch_l2(a.brg + s + stride);
-      }
-    }
-    const float ax = hi.x - hj.x, ay = hi.y - hj.y, az = hi.z - hj.z; /* exact */
-    const float shi = hi.w + hj.w;
-    const float coarse = sqrtf(ax * ax + ay * ay + az * az) - shi;
-    float gap = coarse;
-    float3 u = f3(0.f, 0.f, 0.f);
-    float rj = hj.w;
-    const bool cand = WET || coarse < a.coarse_tol;
-    float4 vj4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (WET) vj4 = ro(a.v_in + j);
-    if (cand) {
-      gap = exact_gap(hi, lo, hj, ro(a.plo_in + j), ax, ay, az, u, rj);
-      if (gap < 0.f) {
-        if (!WET) vj4 = ro(a.v_in + j);
-        float3 dF, dM;
-        float dR;
-        pp_contact(a.pp, a.rec + s, ri, rj, iv, iw, vj4, ro(a.w_in + j), u, gap, a.rfrc, a.dtf, dF, dM, dR);
-        F.add(dF);
-        kahan4(mra, dM, dR);
-        ncont++;
-      }
-    }
-    if (WET && wet_i) {
-      /* the pair's bridge volume and contact angle: the reference's split of
-       * both particles' liquid, or the per-contact model's */
-      float ijVol, th = 0.f;
-      int id_j = 0;
-      if (a.lq_mode == 0) {
-        int jnl = __float_as_int(vj4.w);
-        if (jnl < 12) jnl = 12;
-        const float tj = 2.0f * rj;
-        ijVol = iVol + __fdividef(a.lqd_vol * (tj * tj * tj), (float)jnl);
-      } else {
-        id_j = ro(a.id + j);
-        th = 0.5f * (th_i + cap_theta32(id_j, a.lq_seed, a.lq_theta_max));
-        ijVol = pair_bridge_volume32(id_i, id_j, a.lq_seed, a.lq_vmin, a.lq_vspan, fminf(ri, rj));
-      }
-      const int bprev = a.brg[s];
-      const bool form = gap < 2.0f * a.lqd_layer * (ri + rj);
-      if (NET && (bprev || form)) {
-        /* a bridge to evaluate: queue it for the network, or (outside the
-         * network's training box) take the plain formula right here */
-        const float sep = fmaxf(a.lqd_gapmn, fmaxf(gap, 0.f)), vol = 8.0f * ijVol;
-        const float theta =
-            a.lq_mode ? th : 0.5f * (th_i + cap_theta(ro(a.id + j), a.theta_seed, a.theta_max));
-        const float ratio = __fdividef(fminf(ri, rj), fmaxf(ri, rj));
-        const float effR = 2.0f * ri * rj / (ri + rj);
-        if (cap_in_hull(*capw, sep, vol, theta, ratio) && s <= 0xffffffffLL) {
-          const float3 wv = u * (-2.0f * kPiF * effR * a.lqd_st);
-          ent = CapEntry{sep, vol, theta, ratio, wv.x, wv.y, wv.z, gap, (unsigned)s, form ? 1 : 0};
-          want = true;
-        } else {
-          const int b = form ? 1 : (gap > bridge_rupture32(a, ijVol, th) ? 0 : 1);
-          a.brg[s] = (unsigned char)b;
-          if (b) {
-            const float fc = bridge_force32(a, gap < 0.f ? 0.f : gap, ijVol, th, effR);
-            F.add(u * (-fc));
-            wet++;
-            if (gap >= 0.f) nbr++;
-          }
-          nfall++;
-        }
-      } else if (!NET) {
-        int b = bprev;
-        if (form) b = 1;
-        else if (gap > bridge_rupture32(a, ijVol, th)) b = 0;
-        a.brg[s] = (unsigned char)b;
-        if (b) {
-          const float effR = 2.0f * ri * rj / (ri + rj);
-          const float fc = bridge_force32(a, gap < 0.f ? 0.f : gap, ijVol, th, effR);
-          F.add(u * (-fc));
-          wet++;
-          if (gap >= 0.f) nbr++;
-        }
-      }
-    }
-    }
-    if (NET) {
-      const unsigned m = __ballot_sync(0xffffffffu, want);
-      if (want) {
-        const int pos = qn + __popc(m & ((1u << lane) - 1u));
-        ent.meta |= (last + 1) << 8;
-        qw[pos] = ent;
-        last = pos;
-      }
-      qn += __popc(m);
-      if (qn > kCapQ - 32) {
-        cap_flush(*capw, qw, qn, last, a.brg, F, wet, nbr, nmlp);
-        qn = 0;
-        last = -1;
-      }
-    }
-  }
-  if (NET && qn > 0) cap_flush(*capw, qw, qn, last, a.brg, F, wet, nbr, nmlp);
-
-  KSum3 M;
-  KSum R;
-  {
-    const float4 sm = mra[0], cm = mra[1];
-    M.x.s = sm.x; M.x.c = cm.x; M.y.s = sm.y; M.y.c = cm.y; M.z.s = sm.z; M.z.c = cm.z;
-    R.s = sm.w; R.c = cm.w;
-  }
-  finish_particle<NET>(a, q, qq, live, sys, hi, lo, wi4, iv, iw, ri, twor, mass_f, F, M, R, wet, (unsigned)nn, ncont,
-                       nbr, nmlp, nfall);
-}
-
-/* ---------------- the warp-cooperative pair loop ----------------
- * One thread per particle makes a warp walk max(nn) neighbour slots with most
- * lanes idle (measured: 15 of 32 lanes active on the settled 200k wet bed) and
- * issue the whole slot body -- geometry, contact law, bridge -- once per slot
- * whatever each lane needs.  Here the 32 particles of a warp put their slots
- * end to end (inclusive shuffle scan of the slot counts) and each pass over up
- * to kChunk of them runs in phases, every lane taking the next item whichever
- * particle owns it (binary search of the scan, in shuffles):
- *   A  geometry of every pair (one 16-byte gather per partner, the exact
- *      overlap for candidates); contacts and bridges are ballot-compacted into
- *      two lists in shared memory;
- *   B  the contact law over the compacted contacts only (velocity, spin and
- *      the 64-byte record gathered together);
- *   C  the capillary bridges over the compacted bridge list (formula, or the
- *      learned closure's queue on the tensor cores);
- *   D  every lane folds its own particle's pairs, in neighbour order, into its
- *      Kahan sums.
- * so the contact law issues once per 32 contacts rather than once per 32
- * slots.  Then each lane finishes its particle (walls, integrator) as before. */
-
-struct PairOut {
-  float fx, fy, fz, mx, my, mz, rr;
-  int flags;
-};
-enum : int { kPContact = 1, kPWet = 2, kPNbr = 4, kPMlp = 8, kPFall = 16 };
-
-/* phase A's result for one pair */
-struct PairGeo {
-  float ux, uy, uz, gap;
-  int j;
-  float rj;
-  int meta;
-  int pad;
-};
-enum : int { kGContact = 1, kGBridge = 2, kGForm = 4 };
-
-/* the warp's 32 particles as the pair lanes read them */
-struct WarpOwn {
-  float4 hi[32], lo[32];
-  float4 v[32]; /* velocity, liquid volume */
-  float4 w[32]; /* spin, contact angle (learned closure) */
-  long long base[32];
-  int stride[32];
-};
-static_assert(sizeof(WarpOwn) % 16 == 0, "WarpOwn keeps 16-byte alignment");
-
-/* a lane's running sums and counts between passes (in shared memory, so
- * that they hold no registers while the pairs are evaluated) */
-struct LaneAcc {
-  KSum3 F, M;
-  KSum R;
-  int wet;
-  unsigned ncont, nbr, nmlp, nfall, pad;
-};
-static_assert(sizeof(LaneAcc) == 80, "LaneAcc is 80 bytes");
-
-/* a pass's pair geometry and pair results in shared memory, each pair as two
- * 16-byte halves in two arrays, so that a warp's 32 consecutive pairs are 16
- * bytes apart: one 128-bit access a quarter-warp per wavefront, no bank
- * conflicts (a 32-byte record would take two) */
-struct PairBuf {
-  float4* gu; /* ux, uy, uz, gap */
-  int4* gm;   /* j, rj (bits), meta, pad */
-  float4* oa; /* fx, fy, fz, mx */
-  float4* ob; /* my, mz, rr, flags (bits) */
-  __device__ __forceinline__ void put_geo(int k, const PairGeo& g) const {
-    gu[k] = make_float4(g.ux, g.uy, g.uz, g.gap);
-    gm[k] = make_int4(g.j, __float_as_int(g.rj), g.meta, g.pad);
-  }
-  __device__ __forceinline__ PairGeo geo(int k) const {
-    const float4 u = gu[k];
-    const int4 m = gm[k];
-    return PairGeo{u.x, u.y, u.z, u.w, m.x, __int_as_float(m.y), m.z, m.w};
-  }
-  __device__ __forceinline__ int meta(int k) const { return reinterpret_cast<const int*>(gm + k)[2]; }
-  __device__ __forceinline__ void put_out(int k, const PairOut& r) const {
-    oa[k] = make_float4(r.fx, r.fy, r.fz, r.mx);
-    ob[k] = make_float4(r.my, r.mz, r.rr, __int_as_float(r.flags));
-  }
-  __device__ __forceinline__ PairOut out(int k) const {
-    const float4 x = oa[k], y = ob[k];
-    return PairOut{x.x, x.y, x.z, x.w, y.x, y.y, y.z, __float_as_int(y.w)};
-  }
-};
-
-#ifndef DEM_COOP_CHUNK
-#define DEM_COOP_CHUNK 64
-#endif
-
-/* pairs per warp per pass (the learned closure's bridge queue holds a pass,
- * so it never has to be flushed inside one) and the per-warp shared memory:
- * own particles, lane sums, pair geometry and results, the two lists, queue */
-template <bool NET>
-struct Coop {
-  static constexpr int kChunk = NET ? 64 : DEM_COOP_CHUNK;
-  static constexpr size_t kOffAcc = sizeof(WarpOwn);
-  static constexpr size_t kOffGeo = kOffAcc + 32 * sizeof(LaneAcc);
-  static constexpr size_t kOffOut = kOffGeo + 32 * kChunk; /* PairBuf: two 16-byte halves per pair */
-  static constexpr size_t kOffQ = kOffOut + 32 * kChunk;
-  static constexpr size_t kOffList = kOffQ + (NET ? sizeof(CapEntry) * kChunk : 0);
-  static constexpr size_t kWarpBytes = kOffList + 2 * kChunk;
-  static constexpr size_t smem(int warps) {
-    return (NET ? ((sizeof(CapNetSmem) + 15) / 16) * 16 : 0) + warps * kWarpBytes;
-  }
-  static_assert(kChunk % 32 == 0 && kChunk <= 256, "a pass is whole rounds of 32; list entries are bytes");
-  static_assert(kWarpBytes % 16 == 0 && kOffQ % 16 == 0, "per-warp areas keep 16-byte alignment");
-};
-
-#ifndef DEM_COOP_BLOCKS
-#define DEM_COOP_BLOCKS 6
-#endif
-
-/* the particle (lane) owning pair p: the number of lanes whose inclusive slot
- * count is <= p.  Every lane of the warp calls it. */
-__device__ __forceinline__ int coop_owner(int incl, int p) {
-  int o = 0;
+    /* a block's counts go out together, by its last warp: an atomic per warp
+     * on four words of one sector would queue up behind one another, and a
+     * barrier would hold the finished warps' places */
+    const unsigned c[4] = {(unsigned)nn, ncont, nbr, nwc};
+    unsigned mine = 0;
 #pragma unroll
-  for (int b = 16; b > 0; b >>= 1) {
-    const int v = __shfl_sync(0xffffffffu, incl, o + b - 1);
-    if (v <= p) o += b;
-  }
-  return o;
-}
-
-/* phase A for one pair (owner o, partner j with coarse shadow hj): the
- * overlap -- coarse from the hi parts, exact (hi + lo, error-free
- * transforms) for candidates -- and what the later phases need */
-template <bool WET>
-__device__ __forceinline__ PairGeo coop_geo(const MixArgs& a, const WarpOwn& ow, int o, bool wet_o, long long s,
-                                            int j, float4 hj) {
-  PairGeo g;
-  const float4 hi = ow.hi[o], lo = ow.lo[o];
-  const float ax = hi.x - hj.x, ay = hi.y - hj.y, az = hi.z - hj.z; /* exact */
-  const float coarse = sqrtf(ax * ax + ay * ay + az * az) - (hi.w + hj.w);
-  g.gap = coarse;
-  g.ux = g.uy = g.uz = 0.f;
-  g.rj = hj.w;
-  g.j = j;
-  g.meta = 0;
-  g.pad = 0;
-  if (WET || coarse < a.coarse_tol) {
-    float3 u;
-    g.gap = exact_gap(hi, lo, hj, ro(a.plo_in + j), ax, ay, az, u, g.rj);
-    g.ux = u.x;
-    g.uy = u.y;
-    g.uz = u.z;
-    if (g.gap < 0.f) g.meta = kGContact;
-  }
-  if (WET && wet_o) {
-    /* a bridge to evaluate: an existing one, or one forming this step (gap
-     * below the liquid layer); the others stay unbridged (flag 0) */
-    const float ri = hi.w + lo.w;
-    const bool form = g.gap < 2.0f * a.lqd_layer * (ri + g.rj);
-    if (form) g.meta |= kGBridge | kGForm;
-    else if (a.brg[s]) g.meta |= kGBridge;
-  }
-  return g;
-}
-
-/* phase B for one contact: the elasto-plastic law with its history record */
-__device__ __forceinline__ PairOut coop_contact(const MixArgs& a, const WarpOwn& ow, int o, long long s,
-                                                const PairGeo& g) {
-  const float4 hi = ow.hi[o], lo = ow.lo[o], vi = ow.v[o], wi = ow.w[o];
-  float3 dF, dM;
-  float dR;
-  pp_contact(a.pp, a.rec + s, hi.w + lo.w, g.rj, f3(vi.x, vi.y, vi.z), f3(wi.x, wi.y, wi.z), ro(a.v_in + g.j),
-             ro(a.w_in + g.j), f3(g.ux, g.uy, g.uz), g.gap, a.rfrc, a.dtf, dF, dM, dR);
-  return PairOut{dF.x, dF.y, dF.z, dM.x, dM.y, dM.z, dR, kPContact};
-}
-
-/* phase C for one bridge: rupture decision, bridge flag and force with the
- * plain formula, added into the pair's result (NET: inside the network's
- * training box the bridge is queued in `ent` instead, want = true) */
-template <bool NET>
-__device__ __forceinline__ void coop_bridge(const MixArgs& a, const WarpOwn& ow, int o, long long s,
-                                            const PairGeo& g, PairOut& out, const CapNetSmem* capw, int pidx,
-                                            bool& want, CapEntry& ent) {
-  const float4 hi = ow.hi[o], lo = ow.lo[o];
-  const float ri = hi.w + lo.w, rj = g.rj;
-  float ijVol, th = 0.f;
-  if (a.lq_mode == 0) {
-    int jnl = __float_as_int(ro(a.v_in + g.j).w);
-    if (jnl < 12) jnl = 12;
-    const float tj = 2.0f * rj;
-    ijVol = ow.v[o].w + __fdividef(a.lqd_vol * (tj * tj * tj), (float)jnl);
-  } else {
-    const int id_j = ro(a.id + g.j);
-    th = 0.5f * (ow.w[o].w + cap_theta32(id_j, a.lq_seed, a.lq_theta_max));
-    ijVol = pair_bridge_volume32(__float_as_int(ow.v[o].w), id_j, a.lq_seed, a.lq_vmin, a.lq_vspan, fminf(ri, rj));
-  }
-  const bool form = (g.meta & kGForm) != 0;
-  const float effR = 2.0f * ri * rj / (ri + rj);
-  const float vol = 8.0f * ijVol;
-  if (NET) {
-    const float sep = fmaxf(a.lqd_gapmn, fmaxf(g.gap, 0.f));
-    const float theta =
-        a.lq_mode ? th : 0.5f * (ow.w[o].w + cap_theta(ro(a.id + g.j), a.theta_seed, a.theta_max));
-    const float ratio = __fdividef(fminf(ri, rj), fmaxf(ri, rj));
-    if (cap_in_hull(*capw, sep, vol, theta, ratio) && s <= 0xffffffffLL) {
-      const float sc = -2.0f * kPiF * effR * a.lqd_st;
-      ent = CapEntry{sep, vol, theta, ratio, g.ux * sc, g.uy * sc, g.uz * sc, g.gap, (unsigned)s,
-                     (form ? 1 : 0) | (pidx << 8)};
-      want = true;
-      return;
+    for (int t = 0; t < 4; t++) {
+      const unsigned v = __reduce_add_sync(0xffffffffu, c[t]);
+      if ((threadIdx.x & 31) == t) mine = v;
     }
-    out.flags |= kPFall;
-  }
-  const int b = form ? 1 : (g.gap > bridge_rupture32(a, ijVol, th) ? 0 : 1);
-  a.brg[s] = (unsigned char)b;
-  if (b) {
-    const float fc = bridge_force32(a, g.gap < 0.f ? 0.f : g.gap, ijVol, th, effR);
-    out.fx -= g.ux * fc;
-    out.fy -= g.uy * fc;
-    out.fz -= g.uz * fc;
-    out.flags |= kPWet | (g.gap >= 0.f ? kPNbr : 0);
-  }
-}
-
-/* run the pass's bridge queue through the network, then fold each entry into
- * its pair's result: rupture decision, bridge flag, force */
-__device__ __forceinline__ void cap_fold_coop(const CapNetSmem& w, CapEntry* qw, int qn, const PairBuf& pb,
-                                              unsigned char* brg) {
-  cap_run_queue(w, qw, qn);
-  for (int e = threadIdx.x & 31; e < qn; e += 32) {
-    const CapEntry en = qw[e];
-    const int b = (en.meta & 1) ? 1 : (en.gap > en.vol ? 0 : 1);
-    brg[en.slot] = (unsigned char)b;
-    PairOut r = pb.out(en.meta >> 8);
-    int fl = r.flags | kPMlp;
-    if (b) {
-      r.fx += en.wx * en.sep;
-      r.fy += en.wy * en.sep;
-      r.fz += en.wz * en.sep;
-      fl |= kPWet | (en.gap >= 0.f ? kPNbr : 0);
+    if ((threadIdx.x & 31) < 4) atomicAdd(&sums[threadIdx.x & 31], mine);
+    __threadfence_block();
+    __syncwarp();
+    unsigned done = 0;
+    if ((threadIdx.x & 31) == 0) done = atomicAdd(&sums[4], 1u);
+    done = __shfl_sync(0xffffffffu, done, 0);
+    if (done == blockDim.x / 32 - 1 && (threadIdx.x & 31) < 4) {
+      const unsigned v = atomicAdd(&sums[threadIdx.x & 31], 0u);
+      if (v) atomicAdd(&a.counters[threadIdx.x & 31], (unsigned long long)v);
     }
-    r.flags = fl;
-    pb.put_out(en.meta >> 8, r);
   }
-  __syncwarp();
 }
 
-/* the slot of pair p of owner o */
-__device__ __forceinline__ long long coop_slot(const WarpOwn& ow, int o, int p, int eo) {
-  return ow.base[o] + (long long)(p - eo) * ow.stride[o];
-}
-
-template <bool WET, bool NET>
-__global__ void __launch_bounds__(128, NET ? kNetBlocks : DEM_COOP_BLOCKS) k_step_coop(MixArgs a) {
-  if (a.n <= 0 || (a.gate && *a.gate)) return;
-  using CF = Coop<NET>;
-  constexpr int CH = CF::kChunk;
-  const unsigned FULL = 0xffffffffu;
+/* the listed wall slots, compact (their order does not matter: each writes its
+ * own slot's result) */
+__global__ void k_wall_entries(const int* __restrict__ nwall, int n, int* __restrict__ entry, int* __restrict__ count) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  const int nw = q < n ? nwall[q] : 0;
   const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
-  const int q = reversed_block_thread(); /* the heaviest particles first */
-  const bool live = q < a.n;
-  const int qq = live ? q : a.n - 1;
-  extern __shared__ __align__(16) unsigned char dsm[];
-  const CapNetSmem* capw = reinterpret_cast<const CapNetSmem*>(dsm);
-  unsigned char* wsm = dsm + (NET ? ((sizeof(CapNetSmem) + 15) / 16) * 16 : 0) + (threadIdx.x >> 5) * CF::kWarpBytes;
-  WarpOwn& ow = *reinterpret_cast<WarpOwn*>(wsm);
-  LaneAcc* acc = reinterpret_cast<LaneAcc*>(wsm + CF::kOffAcc);
-  const PairBuf pb{reinterpret_cast<float4*>(wsm + CF::kOffGeo), reinterpret_cast<int4*>(wsm + CF::kOffGeo + 16 * CH),
-                   reinterpret_cast<float4*>(wsm + CF::kOffOut), reinterpret_cast<float4*>(wsm + CF::kOffOut + 16 * CH)};
-  CapEntry* qw = reinterpret_cast<CapEntry*>(wsm + CF::kOffQ);
-  unsigned char* clist = wsm + CF::kOffList;
-  unsigned char* blist = clist + CH;
-  if (NET) {
-    cap_stage(a.capw, reinterpret_cast<CapNetSmem*>(dsm));
-    __syncthreads();
-  }
-  /* the integrator's FP64 state is needed only after the pair loop */
-  prefetch_l2(a.pos + qq);
-  prefetch_l2(a.vel + qq);
-  prefetch_l2(a.angv + qq);
-  prefetch_l2(a.pmove + qq);
-  /* so are the wall count and list, which would otherwise be two dependent
-   * DRAM misses at the end of the warp's work */
-  prefetch_l2(a.nwall + qq);
-  prefetch_l2(a.wlist + 3 * qq);
-
-  const int sys = a.sys_of_id ? a.sys_of_id[ro(a.id + qq)] : 0;
-  const int nn = live ? ro(a.num_nebor + qq) : 0;
-  unsigned wetm;
-  {
-    /* this lane's particle, for the lanes that evaluate its pairs and for
-     * the integrator after the loop (read back from shared memory then) */
-    const float4 hi = ro(a.phi_in + qq), lo = ro(a.plo_in + qq), vi4 = ro(a.v_in + qq), wi4 = ro(a.w_in + qq);
-    const float twor = 2.0f * (hi.w + lo.w);
-    const float mass_f = twor * twor * twor;
-    const bool wet_i = WET && (!a.sys_wet || a.sys_wet[sys]);
-    float iVol = 0.f;
-    if (WET) {
-      int inl = __float_as_int(vi4.w);
-      if (inl < 12) inl = 12;
-      iVol = a.lqd_vol * mass_f / (float)inl;
-    }
-    const int L = ro(a.plevel + qq);
-    ow.hi[lane] = hi;
-    ow.lo[lane] = lo;
-    /* .w of the own velocity: the liquid volume (reference model) or the
-     * particle's id (per-contact model); of the own spin: the contact angle */
-    const bool lqm = WET && a.lq_mode;
-    const int id_i = (NET || lqm) ? ro(a.id + qq) : 0;
-    ow.v[lane] = make_float4(vi4.x, vi4.y, vi4.z, lqm ? __int_as_float(id_i) : iVol);
-    ow.w[lane] = make_float4(wi4.x, wi4.y, wi4.z,
-                             lqm   ? cap_theta32(id_i, a.lq_seed, a.lq_theta_max)
-                             : NET ? cap_theta(id_i, a.theta_seed, a.theta_max)
-                                   : 0.f);
-    ow.base[lane] = slot_base(L, a.npars, a.nneb) + ro(a.nidx + qq);
-    ow.stride[lane] = ro(a.npars + L);
-    LaneAcc z;
-    z.F = KSum3();
-    z.M = KSum3();
-    z.R = KSum();
-    z.F.z.add(-mass_f); /* gravity, m = (2r)^3 */
-    z.wet = 0;
-    z.ncont = z.nbr = z.nmlp = z.nfall = z.pad = 0;
-    acc[lane] = z;
-    wetm = __ballot_sync(FULL, wet_i);
-  }
-  /* the warp's slots end to end */
-  int incl = nn;
+  int incl = nw;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const int t = __shfl_up_sync(FULL, incl, o);
+    const int t = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += t;
   }
-  const int excl = incl - nn;
-  const int total = __shfl_sync(FULL, incl, 31);
-  __syncwarp();
-
-  for (int c0 = 0; c0 < total; c0 += CH) {
-    const int cend = min(total, c0 + CH);
-    /* ---- A: geometry of every pair; contacts and bridges listed ---- */
-    int nc = 0, nb = 0;
-    {
-      /* pair p of this lane, and one round ahead: its partner index and
-       * coarse shadow are in flight while the current pair is evaluated */
-      int p = c0 + lane;
-      bool act = p < cend;
-      int o = coop_owner(incl, p);
-      long long s = 0;
-      int j = 0;
-      float4 hj = make_float4(0.f, 0.f, 0.f, 0.f);
-      {
-        const int eo = __shfl_sync(FULL, excl, o);
-        if (act) {
-          s = coop_slot(ow, o, p, eo);
-          j = ro(a.nebor + s);
-          hj = ro(a.phi_in + j);
-        }
-      }
-      for (int p0 = c0; p0 < cend; p0 += 32) {
-        const int pn = p + 32;
-        const bool actn = pn < cend;
-        const int on = coop_owner(incl, pn);
-        const int eon = __shfl_sync(FULL, excl, on);
-        long long sn = 0;
-        int jn = 0;
-        float4 hjn = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (actn) {
-          sn = coop_slot(ow, on, pn, eon);
-          jn = ro(a.nebor + sn);
-          hjn = ro(a.phi_in + jn);
-          /* its lo parts (read for every candidate) and bridge flag: into L2 now */
-          prefetch_l2(a.plo_in + jn);
-          if (WET) prefetch_l2(a.brg + sn);
-        }
-        int meta = 0;
-        if (act) {
-          const PairGeo g = coop_geo<WET>(a, ow, o, (wetm >> o) & 1u, s, j, hj);
-          pb.put_geo(p - c0, g);
-          meta = g.meta;
-          if (meta & kGContact) { /* phase B will need them: start bringing them in */
-            prefetch_l2(a.rec + s);
-            prefetch_l2(a.w_in + j);
-          }
-        }
-        const unsigned mc = __ballot_sync(FULL, meta & kGContact);
-        const unsigned mb = __ballot_sync(FULL, meta & kGBridge);
-        if (meta & kGContact) clist[nc + __popc(mc & lt)] = (unsigned char)(p - c0);
-        if (meta & kGBridge) blist[nb + __popc(mb & lt)] = (unsigned char)(p - c0);
-        nc += __popc(mc);
-        nb += __popc(mb);
-        p = pn;
-        act = actn;
-        o = on;
-        s = sn;
-        j = jn;
-        hj = hjn;
-      }
-    }
-    __syncwarp();
-    /* ---- B: the contact law over the compacted contacts ---- */
-    for (int k0 = 0; k0 < nc; k0 += 32) {
-      const int k = k0 + lane;
-      const int pidx = k < nc ? clist[k] : 0;
-      const int p = c0 + pidx;
-      const int o = coop_owner(incl, p);
-      const int eo = __shfl_sync(FULL, excl, o);
-      if (k < nc) pb.put_out(pidx, coop_contact(a, ow, o, coop_slot(ow, o, p, eo), pb.geo(pidx)));
-    }
-    __syncwarp();
-    /* ---- C: the bridges over the compacted list ---- */
-    if (WET) {
-      int qn = 0;
-      for (int k0 = 0; k0 < nb; k0 += 32) {
-        const int k = k0 + lane;
-        const int pidx = k < nb ? blist[k] : 0;
-        const int p = c0 + pidx;
-        const int o = coop_owner(incl, p);
-        const int eo = __shfl_sync(FULL, excl, o);
-        bool want = false;
-        CapEntry ent;
-        if (k < nb) {
-          const PairGeo g = pb.geo(pidx);
-          PairOut r;
-          if (g.meta & kGContact) r = pb.out(pidx);
-          else r = PairOut{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0};
-          coop_bridge<NET>(a, ow, o, coop_slot(ow, o, p, eo), g, r, capw, pidx, want, ent);
-          pb.put_out(pidx, r);
-        }
-        if (NET) {
-          const unsigned m = __ballot_sync(FULL, want);
-          if (want) qw[qn + __popc(m & lt)] = ent;
-          qn += __popc(m);
-        }
-      }
-      if (NET && qn > 0) cap_fold_coop(*capw, qw, qn, pb, a.brg);
-    }
-    __syncwarp();
-    /* ---- D: this lane's particle, its pairs of the pass in neighbour order ---- */
-    const int k0 = max(excl, c0), k1 = min(incl, cend);
-    if (k0 < k1) {
-      LaneAcc A = acc[lane];
-      for (int kk = k0; kk < k1; kk++) {
-        if (!(pb.meta(kk - c0) & (kGContact | kGBridge))) continue;
-        const PairOut r = pb.out(kk - c0);
-        if (r.flags & (kPContact | kPWet)) A.F.add(f3(r.fx, r.fy, r.fz));
-        if (r.flags & kPContact) {
-          A.M.add(f3(r.mx, r.my, r.mz));
-          A.R.add(r.rr);
-          A.ncont++;
-        }
-        if (r.flags & kPWet) A.wet++;
-        if (r.flags & kPNbr) A.nbr++;
-        if (NET) {
-          if (r.flags & kPMlp) A.nmlp++;
-          if (r.flags & kPFall) A.nfall++;
-        }
-      }
-      acc[lane] = A;
-    }
-    __syncwarp();
-  }
-  LaneAcc A = acc[lane];
-  const float4 hi = ow.hi[lane], lo = ow.lo[lane], v = ow.v[lane], w = ow.w[lane];
-  const float ri = hi.w + lo.w, twor = 2.0f * ri;
-  const float4 wi4 = make_float4(w.x, w.y, w.z, 0.f);
-  finish_particle<NET>(a, q, qq, live, sys, hi, lo, wi4, f3(v.x, v.y, v.z), f3(w.x, w.y, w.z), ri, twor,
-                       twor * twor * twor, A.F, A.M, A.R, A.wet, (unsigned)nn, A.ncont, A.nbr, A.nmlp, A.nfall);
+  const int total = __shfl_sync(0xffffffffu, incl, 31);
+  if (total == 0) return;
+  int at = 0;
+  if (lane == 0) at = atomicAdd(count, total);
+  at = __shfl_sync(0xffffffffu, at, 0) + incl - nw;
+  for (int w = 0; w < nw; w++) entry[at + w] = w * n + q;
 }
 
 /* CirPWInterG's wall motion (kernel.cu:966-969): every cylinder's top wall
@@ -1760,25 +1418,7 @@ MixArgs ref_args(const DevConsts& k, int n, int force_cap, int stage) {
 }
 }  // namespace
 
-#ifndef DEM_COOP_CARVEOUT
-#define DEM_COOP_CARVEOUT cudaSharedmemCarveoutMaxShared
-#endif
-
-template <class K>
-cudaError_t coop_attrs(K kernel, size_t smem) {
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess && DEM_COOP_CARVEOUT >= 0)
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, DEM_COOP_CARVEOUT);
-  return e;
-}
-
 dem_status mixed_create(dem_ctx* c) {
-  /* the cooperative step kernels: shared memory above the default 48 KB per
-   * block, and the largest shared-memory carveout (set before any capture) */
-  cudaError_t e = coop_attrs(k_step_coop<true, true>, Coop<true>::smem(kWarps));
-  if (e == cudaSuccess) e = coop_attrs(k_step_coop<true, false>, Coop<false>::smem(kWarps));
-  if (e == cudaSuccess) e = coop_attrs(k_step_coop<false, false>, Coop<false>::smem(kWarps));
-  if (e != cudaSuccess) return cuda_check(e, "mixed_create kernel attributes");
   MixedState* m = new MixedState();
   std::memset(m, 0, sizeof(*m));
   c->mx = m;
@@ -1792,6 +1432,17 @@ dem_status mixed_create(dem_ctx* c) {
     cudaMemset(p, 0, sizeof(float4) * N);
     c->allocs.push_back(p);
     *b = (float4*)p;
+  }
+  {
+    void *o = nullptr, *e = nullptr;
+    dem_status st = cuda_alloc(&o, sizeof(float4) * 6 * N);
+    if (st != DEM_OK) return st;
+    c->allocs.push_back(o);
+    m->wall_out = (float4*)o;
+    st = cuda_alloc(&e, sizeof(int) * 3 * N);
+    if (st != DEM_OK) return st;
+    c->allocs.push_back(e);
+    m->wall_entry = (int*)e;
   }
   /* offset putting every coordinate of the domain in [2^k, 2^(k+1)) */
   const PARAMETER& prm = c->s.prm;
@@ -1858,13 +1509,11 @@ Prefilter mixed_prefilter(dem_ctx* c, int which) {
   return Prefilter{c->mx->phi[which], 0.5f * c->mx->coarse_tol + 2.0e-6f};
 }
 
-bool mixed_thread_loop(const dem_ctx* c) { return c->opt.pair_mode != DEM_PAIRS_WARP; }
-
 const char* mixed_step_kernel_name(const dem_ctx* c) {
-  const bool net = c->s.force_cap == 1 && c->opt.capillary == DEM_CAP_MLP;
   const bool wet = c->s.force_cap == 1;
-  if (mixed_thread_loop(c)) return net ? "k_step_mixed<1,1>" : wet ? "k_step_mixed<1,0>" : "k_step_mixed<0,0>";
-  return net ? "k_step_coop<1,1>" : wet ? "k_step_coop<1,0>" : "k_step_coop<0,0>";
+  const bool net = wet && c->opt.capillary == DEM_CAP_MLP;
+  return net ? "k_pair_mixed<1,1> + k_body_mixed<1,1>" : wet ? "k_pair_mixed<1,0> + k_body_mixed<1,0>"
+                                                             : "k_pair_mixed<0,0> + k_body_mixed<0,0>";
 }
 
 dem_status mixed_step(dem_ctx* c, int which, cudaStream_t s) {
@@ -1876,8 +1525,10 @@ dem_status mixed_step(dem_ctx* c, int which, cudaStream_t s) {
   a.phi_out = m->phi[1 - which]; a.plo_out = m->plo[1 - which]; a.v_out = m->vel[1 - which];
   a.w_out = m->angv[1 - which];
   a.pos = b.pos; a.vel = b.vel; a.angv = b.angv; a.rad = b.rad; a.pmove = b.pmove;
-  a.nebor = b.nebor; a.num_nebor = b.num_nebor; a.plevel = b.plevel; a.nidx = b.nidx; a.npars = b.npars;
-  a.nneb = b.nneb; a.rec = b.rec; a.brg = b.brg; a.wlist = b.wlist; a.nwall = b.nwall; a.wrec = b.wrec;
+  a.num_nebor = b.num_nebor; a.plevel = b.plevel; a.nidx = b.nidx; a.npars = b.npars; a.nneb = b.nneb;
+  a.ps = b.ps; a.pair_out = reinterpret_cast<float4*>(b.pair_out);
+  a.wall_out = m->wall_out; a.wall_entry = m->wall_entry;
+  a.wlist = b.wlist; a.nwall = b.nwall; a.wrec = b.wrec;
   a.force_out = m->force; a.flag = b.flag; a.err = b.err; a.counters = b.counters; a.cyl = b.cyl;
   a.sys_of_id = b.sys_of_id; a.sys_wet = b.sys_wet;
   a.n = c->n;
@@ -1912,31 +1563,38 @@ dem_status mixed_step(dem_ctx* c, int which, cudaStream_t s) {
   a.lq_seed = c->lm.seed;
   const bool net = c->s.force_cap == 1 && c->opt.capillary == DEM_CAP_MLP;
   if (net && !c->cap_w) return fail(DEM_ERR_STATE, "DEM_CAP_MLP: no network installed (dem_set_capnet)");
-  const bool thread_loop = mixed_thread_loop(c);
-  /* threads per block: the option (a multiple of 32 up to 128), else the
-   * fastest measured: one warp for the warp-cooperative loop (a block frees
-   * its slot as soon as its only warp is done; 75.0 vs 79.5 us at 128 threads
-   * on the deposited 200k bed), four for the thread loop (118.9 vs 121.6 us
-   * at 64 and 32 threads on the packed 200k bed) and with the learned
-   * closure, whose weights are staged once per block */
+  const bool wet = c->s.force_cap == 1;
+  /* threads per block: the option (a multiple of 32 up to 128), else 128 */
   const int ob = c->opt.block_size;
-  const int bs = (ob >= 32 && ob <= 32 * kWarps && ob % 32 == 0) ? ob : (net || thread_loop) ? 32 * kWarps : 32;
+  const int bs = (ob >= 32 && ob <= 32 * kWarps && ob % 32 == 0) ? ob : 32 * kWarps;
+  /* The pair count is known on the device only: the grid covers six pairs a
+   * sphere (a packed bed lists 4.3) and strides beyond; the closure's blocks
+   * stage its weights once, so they are as many as stay resident. */
+  const long long most = std::min<long long>(c->b.ps.cap, 6LL * c->n);
   const int g = grid_for(c->n, bs);
+  int gp = grid_for(most, bs);
+  if (net) gp = std::min(gp, 152 * kNetBlocks * (32 * kWarps / bs));
   if (c->moving_walls) {
     k_move_walls<<<1, 32, 0, s>>>(b.cyl, b.n_sys > 0 ? b.n_sys : 1, c->s.prm.dt, c->step_gate);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_check(e, "mixed_step wall motion");
   }
-  if (thread_loop) {
-    if (net) k_step_mixed<true, true><<<g, bs, kCapSmem, s>>>(a);
-    else if (c->s.force_cap == 1) k_step_mixed<true, false><<<g, bs, 0, s>>>(a);
-    else k_step_mixed<false, false><<<g, bs, 0, s>>>(a);
-  } else {
-    if (net) k_step_coop<true, true><<<g, bs, Coop<true>::smem(bs / 32), s>>>(a);
-    else if (c->s.force_cap == 1) k_step_coop<true, false><<<g, bs, Coop<false>::smem(bs / 32), s>>>(a);
-    else k_step_coop<false, false><<<g, bs, Coop<false>::smem(bs / 32), s>>>(a);
-  }
+  a.wall_blocks = (unsigned)grid_for(c->n / 4 + 1, bs); /* a packed bed lists one sphere in six */
+  gp += (int)a.wall_blocks;
+  if (net) k_pair_mixed<true, true><<<gp, bs, kCapSmem, s>>>(a);
+  else if (wet) k_pair_mixed<true, false><<<gp, bs, 0, s>>>(a);
+  else k_pair_mixed<false, false><<<gp, bs, 0, s>>>(a);
+  if (net) k_body_mixed<true, true><<<g, bs, 0, s>>>(a);
+  else if (wet) k_body_mixed<true, false><<<g, bs, 0, s>>>(a);
+  else k_body_mixed<false, false><<<g, bs, 0, s>>>(a);
   return cuda_check(cudaGetLastError(), "mixed_step launch");
+}
+
+dem_status mixed_wall_entries(dem_ctx* c, cudaStream_t s) {
+  cudaError_t e = cudaMemsetAsync(c->b.ps.ctl + 3, 0, sizeof(int), s);
+  if (e != cudaSuccess) return cuda_check(e, "wall entries");
+  k_wall_entries<<<grid_for(c->n, 256), 256, 0, s>>>(c->b.nwall, c->n, c->mx->wall_entry, c->b.ps.ctl + 3);
+  return cuda_check(cudaGetLastError(), "wall entries launch");
 }
 
 dem_status mixed_pre_rebuild(dem_ctx* c, int which, cudaStream_t s) {

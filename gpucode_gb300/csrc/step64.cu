@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 
 #include "dem_device.cuh"
+#include "pairs.cuh"
 
 namespace dem {
 
@@ -147,6 +148,146 @@ __global__ void __launch_bounds__(128) k_pp_force64(
         wet = wet + 1;
         if (gap >= 0.0) nbridge++;
       }
+    }
+  }
+  force[i] = F;
+  mom[i] = M;
+  rmom[i] = R;
+  lqd[i] = wet;
+  if (counters) {
+    atomicAdd(&counters[0], (unsigned long long)nn);
+    if (ncontact) atomicAdd(&counters[1], (unsigned long long)ncontact);
+    if (nbridge) atomicAdd(&counters[2], (unsigned long long)nbridge);
+  }
+}
+
+/* ---- the native engine's pair list (pairs.cuh) in FP64 ----
+ * One thread per pair and side evaluates what k_pp_force64 evaluates for one
+ * neighbour slot, the same operations in the same order, and leaves the
+ * contact's force, moment and rolling moment and the bridge's force; one thread
+ * per sphere then adds its sides' results in neighbour order.  The loop is bound
+ * by FP64 issue, which costs a warp the same whatever lanes are active: a warp
+ * of pairs keeps them busy where a warp of spheres waits for its longest list.
+ * The two sides do not share one evaluation: the reference's overlap is dl -
+ * own radius - partner's, whose last bit depends on the order, and a contact at
+ * its loading turning point follows that bit. */
+struct SideOut64 {
+  double3 dF, dM;
+  double dR; /* -1: no contact */
+  double3 fc;
+};
+static_assert(2 * sizeof(SideOut64) == kPairOut64, "a pair's FP64 result");
+
+__global__ void __launch_bounds__(128) k_pair64(
+    PairSet ps, SideOut64* __restrict__ out, const double3* __restrict__ pos, const double3* __restrict__ vel,
+    const double3* __restrict__ angvel, const double* __restrict__ rad, int force_cap, int stage, DevConsts k,
+    const int* __restrict__ id, LiquidModel lm, const double* __restrict__ pvol) {
+  const int4 ct = pair_ctl(ps);
+  const long long items = 2LL * (ct.x ? ct.z : ct.y);
+  const int2* __restrict__ pair = ct.x ? ps.pair[1] : ps.pair[0];
+  const HistAoSAcc h{ct.x ? ps.rec[1] : ps.rec[0], ct.x ? ps.brg[1] : ps.brg[0]};
+  LawCfg64 cfg;
+  cfg.cal = &k.cal;
+  cfg.hertz_le = true;
+  cfg.rot_eps = 1.0e-7;
+  cfg.dsmx_eps = 1.0e-7;
+  cfg.damp_on = (stage == 1);
+  cfg.dmp = sqrt(k.mat[0].dmpn * k.mat[0].dmpn);
+  const bool ref_liquid = force_cap == 1 && lm.mode == 0;
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < items;
+       t += (long long)gridDim.x * blockDim.x) {
+    const int2 ij = pair[t >> 1];
+    const int i = (t & 1) ? ij.y : ij.x, j = (t & 1) ? ij.x : ij.y;
+    SideOut64* o = out + t;
+    const double3 ip = pos[i];
+    const double ir = rad[i], jr = rad[j];
+    const double3 d = sub3(ip, pos[j]);
+    const double dl = len3(d);
+    const double gap = dl - ir - jr;
+    const bool touch = gap < 0.0;
+    double3 u = make_double3(0.0, 0.0, 0.0);
+    double dR = -1.0;
+    if (touch) {
+      u = div3(d, dl);
+      const double3 cpv =
+          sub3(sub3(vel[i], vel[j]), cross3(add3(mul3(angvel[i], ir), mul3(angvel[j], jr)), u));
+      const double ijRad = ir * jr / (ir + jr);
+      HistRec rec = h.load(t);
+      double3 dF, dM;
+      contact_law64(cfg, ijRad, -gap, u, cpv, rec, ir, k.mat[0].rfrc, k.prm.dt, dF, dM, dR);
+      h.store(t, rec);
+      o->dF = dF;
+      o->dM = dM;
+    }
+    o->dR = dR;
+    if (force_cap != 1) continue;
+    const int brg0 = h.brg(t);
+    const bool film = gap < 2 * k.lqd.layer * (ir + jr);
+    if (!film && brg0 == 0) continue;
+    int brg = brg0;
+    const double Splus = gap < 0 ? 0.0 : gap;
+    const double effR = 2 * ir * jr / (ir + jr);
+    double fcap = 0.0;
+    if (ref_liquid) {
+      double ijVol = pvol[i] + pvol[j];
+      if (film) brg = 1;
+      else if (gap > 0.99 * pow(ijVol, 0.33)) brg = 0;
+      if (brg == 1) {
+        ijVol = ijVol * 8.0;
+        fcap = fcap64(Splus, ijVol, effR, k.lqd);
+      }
+    } else {
+      /* per-contact volume and contact angle (liquid.cuh) */
+      const int idi = id ? id[i] : i, idj = id ? id[j] : j;
+      const double th = 0.5 * ((double)cap_theta(idi, lm.seed, lm.theta_max) +
+                               (double)cap_theta(idj, lm.seed, lm.theta_max));
+      const double V = pair_bridge_volume(lm, idi, idj, ir < jr ? ir : jr);
+      if (film) brg = 1;
+      else if (gap > rupture64(V, th)) brg = 0;
+      if (brg == 1) fcap = 2 * kPiRef * effR * k.lqd.stension * willett64(max(k.lqd.gapmn, Splus), 8.0 * V, th);
+    }
+    if (brg != brg0) h.set_brg(t, brg);
+    if (brg == 1) {
+      if (!touch) u = div3(d, dl);
+      o->fc = smul3(-1.0 * fcap, u);
+    }
+  }
+}
+
+/* one thread per sphere: gravity and its sides' results, in neighbour order */
+__global__ void __launch_bounds__(128) k_pair_sum64(
+    PairSet ps, const SideOut64* __restrict__ out, const double* __restrict__ rad, const int* __restrict__ plevel,
+    const int* __restrict__ level_npars, const int* __restrict__ level_nnebors, const int* __restrict__ nebor_idx,
+    const int* __restrict__ num_nebor, int* __restrict__ lqd, double3* __restrict__ force, double3* __restrict__ mom,
+    double* __restrict__ rmom, int n, int force_cap, unsigned long long* __restrict__ counters) {
+  const int i = reversed_block_thread();
+  if (i >= n) return;
+  const unsigned char* __restrict__ brg = pair_ctl(ps).x ? ps.brg[1] : ps.brg[0];
+  double3 F = force[i], M = mom[i];
+  double R = rmom[i];
+  F.z = F.z - cube(2.0 * rad[i]); /* gravity, m = (2r)^3 */
+  int wet = lqd[i], ncontact = 0, nbridge = 0;
+  const int L = plevel[i];
+  const long long stride = level_npars[L];
+  const long long base = slot_base(L, level_npars, level_nnebors) + nebor_idx[i];
+  const int nn = num_nebor[i];
+  for (int a = 0; a < nn; a++) {
+    const int e = ps.eidx[base + a * stride];
+    if (e == kNoPair) continue;
+    const long long t = e < 0 ? 2LL * ~e + 1 : 2LL * e;
+    const SideOut64* o = out + t;
+    const double dR = o->dR;
+    const bool touch = !(dR < 0.0);
+    if (touch) {
+      F = add3(F, o->dF);
+      M = add3(M, o->dM);
+      R = R + dR;
+      ncontact++;
+    }
+    if (force_cap == 1 && brg[t]) {
+      F = add3(F, o->fc);
+      wet++;
+      if (!touch) nbridge++;
     }
   }
   force[i] = F;
@@ -314,6 +455,22 @@ dem_status pp_force64(const double3* pos, const double3* vel, const double3* ang
   return cuda_check(cudaGetLastError(), "pp_force64 launch");
 }
 
+dem_status pair_force64(const PairSet& ps, void* out, const double3* pos, const double3* vel, const double3* angvel,
+                        const double* rad, const int* plevel, const int* level_npars, const int* level_nnebors,
+                        const int* nebor_idx, const int* num_nebor, int* lqd, const int* lqd_old, double3* force,
+                        double3* mom, double* rmom, int n, int force_cap, int stage, const DevConsts& k,
+                        unsigned long long* counters, double* pvol, cudaStream_t stream, const int* id,
+                        LiquidModel lm) {
+  if (n <= 0) return DEM_OK;
+  if (force_cap == 1 && lm.mode == 0) k_liquid_share<<<grid_for(n, 256), 256, 0, stream>>>(rad, lqd_old, pvol, n, k);
+  const long long most = 12LL * n < 2LL * ps.cap ? 12LL * n : 2LL * ps.cap; /* beyond it the grid strides */
+  SideOut64* o = static_cast<SideOut64*>(out);
+  k_pair64<<<grid_for(most, 128), 128, 0, stream>>>(ps, o, pos, vel, angvel, rad, force_cap, stage, k, id, lm, pvol);
+  k_pair_sum64<<<grid_for(n, 128), 128, 0, stream>>>(ps, o, rad, plevel, level_npars, level_nnebors, nebor_idx,
+                                                    num_nebor, lqd, force, mom, rmom, n, force_cap, counters);
+  return cuda_check(cudaGetLastError(), "pair_force64 launch");
+}
+
 template <class H>
 dem_status wall_force64(const double3* pos, const double3* vel, const double3* angvel, double3* force,
                         double3* mom, double* rmom, const double* rad, CylinderBC* cyl, H h,
@@ -331,10 +488,6 @@ dem_status wall_force64(const double3* pos, const double3* vel, const double3* a
 
 template dem_status pp_force64<HistSoA>(const double3*, const double3*, const double3*, const double*, const int*,
                                         const int*, const int*, const int*, const int*, HistSoA, const int*, int*,
-                                        const int*, double3*, double3*, double*, int, int, int, const DevConsts&,
-                                        unsigned long long*, double*, cudaStream_t, const int*, LiquidModel);
-template dem_status pp_force64<HistAoS>(const double3*, const double3*, const double3*, const double*, const int*,
-                                        const int*, const int*, const int*, const int*, HistAoS, const int*, int*,
                                         const int*, double3*, double3*, double*, int, int, int, const DevConsts&,
                                         unsigned long long*, double*, cudaStream_t, const int*, LiquidModel);
 template dem_status wall_force64<HistSoA>(const double3*, const double3*, const double3*, double3*, double3*,

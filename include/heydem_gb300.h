@@ -268,25 +268,19 @@ dem_status dem_build_setup(const dem_input* in, const double* dia, dem_setup* ou
 enum { DEM_PREC_FP64 = 0, DEM_PREC_MIXED = 1 };
 /* capillary closure */
 enum { DEM_CAP_FORMULA = 0, DEM_CAP_MLP = 1 };
-/* pair loop of the mixed step kernel: the warp's lanes share out its particles'
- * pairs (WARP), or one thread walks one particle's pairs (THREAD); AUTO (the
- * default) takes THREAD, the faster of the two on packed and loose beds alike
- * (114.6 vs 157.2 us on the packed 200k wet bed, 6.4 contacts per sphere;
- * 505 vs 634 us on a sequentially deposited 2M bed, 2.2 contacts per sphere).
- * WARP, the same formulas in phases over the warp's compacted pairs, stays
- * selectable and tested. */
+/* pair loop of the mixed step: every mode runs the pair list (one thread per
+ * pair, then one per sphere); the names are those of two earlier loops, which
+ * it replaced on every bed, and stay accepted */
 enum { DEM_PAIRS_AUTO = 0, DEM_PAIRS_WARP = 1, DEM_PAIRS_THREAD = 2 };
 
 typedef struct dem_options {
   int precision;          /* DEM_PREC_* */
   int capillary;          /* DEM_CAP_* */
-  int block_size;         /* threads per block of the step kernel, a multiple of 32 up to 128
-                             (0 = default: 32 for the WARP loop, 128 for THREAD and with the
-                             learned closure) */
+  int block_size;         /* threads per block of the step kernels, a multiple of 32 up to 128 (0 = 128) */
   int reorder;            /* 1: keep particles in cell order (default); 0: reference order */
   int use_graph;          /* 1: replay steps through a CUDA graph (default) */
   int graph_steps;        /* time steps per graph launch (0 = 16) */
-  int pair_mode;          /* mixed step kernel: DEM_PAIRS_AUTO (default), _WARP or _THREAD */
+  int pair_mode;          /* DEM_PAIRS_AUTO (default), _WARP or _THREAD: the same */
 } dem_options;
 
 typedef struct dem_ctx dem_ctx;
@@ -387,7 +381,7 @@ typedef struct dem_liquid_model {
  * sets the learned closure's per-particle contact angles to the model's. */
 dem_status dem_set_liquid_model(dem_ctx* c, const dem_liquid_model* m);
 /* Name of the step kernel(s) dem_step launches for this context's precision,
- * closure and pair loop, e.g. "k_step_mixed<1,0>" (a static string). */
+ * closure, e.g. "k_pair_mixed<1,0> + k_body_mixed<1,0>" (a static string). */
 const char* dem_step_kernel(dem_ctx* c);
 /* Where the time of one end-to-end step goes: `reps` times the host-facing
  * sequence dem_set_state_ex(pos, vel, angvel, no rebuild request) ->

@@ -1,0 +1,123 @@
+"""The native engine's pair list (csrc/pairs.cu): what the two spheres of a pair
+hold mirrors one another through rebuilds, a list entry without its mirror image
+(a slot overflow) acts on its own sphere alone, and sizes at the edges of the
+kernels' blocks give the lists and forces of the FP64 path."""
+import copy
+
+import numpy as np
+import pytest
+
+import _workloads
+from gpucode_gb300 import _abi
+from gpucode_gb300.engine import Engine
+
+pytestmark = pytest.mark.gpu
+
+
+def _by_pair(counts, partners, rec, brg):
+    """(i, j) -> (record, flag) of every list entry"""
+    out = {}
+    for i in range(len(counts)):
+        for a in range(counts[i]):
+            out[(i, int(partners[i, a]))] = (rec[i, a], int(brg[i, a]))
+    return out
+
+
+@pytest.mark.parametrize("make", [_workloads.small_dry, _workloads.small_wet])
+def test_the_two_sides_of_a_pair_mirror_one_another(cuda, make):
+    """after steps with several rebuilds (every rebuild turns some pairs round),
+    both spheres of every pair report the same contact, the spring negated"""
+    w = make()
+    pos, vel, ang = _workloads.stirred(w)
+    e = Engine(w.setup, precision="mixed")
+    e.set_state(pos, vel, ang)
+    e.step(150)
+    e.sync()
+    assert e.stats()["rebuilds"] >= 2
+    n, p = e.neighbors()
+    rec, brg = e.history(int(n.max()))
+    e.close()
+    d = _by_pair(n, p, rec, brg)
+    held = 0
+    for (i, j), (r, b) in d.items():
+        r2, b2 = d[(j, i)]  # every entry has its mirror image
+        np.testing.assert_array_equal(r[:3], -r2[:3])
+        np.testing.assert_array_equal(r[3:], r2[3:])
+        assert b == b2
+        held += bool(r[7])
+    assert held > 100
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_an_entry_without_mirror_image_acts_on_its_own_sphere(cuda, precision):
+    """lists cut at capacity: some spheres list a partner that does not list
+    them.  From rest the first step's force on a sphere is gravity, the Hertz
+    (or plastic) forces of the partners it lists and the walls' -- checked on
+    the spheres away from the walls, one-sided entries included"""
+    w = _workloads.small_dry()
+    setup = copy.deepcopy(w.setup)
+    full = Engine(w.setup, precision="fp64")
+    pos, _, _ = _workloads.stirred(w)
+    full.set_state(pos)
+    full.step(1)
+    full.sync()
+    cap = int(full.neighbors()[0].max()) - 1
+    full.close()
+    setup.s.level_nnebors[0] = cap
+    setup.s.n_pp_slots = cap * setup.s.level_npars[0]
+    e = Engine(setup, precision=precision)
+    e.set_state(pos)
+    e.step(1)
+    with pytest.raises(_abi.DemError) as ei:
+        e.sync()
+    assert ei.value.code == _abi.DEM_ERR_OVERFLOW
+    n, p = e.neighbors()
+    f = e.get_state()["force"]
+    e.close()
+    listed = {(i, int(p[i, a])) for i in range(len(n)) for a in range(n[i])}
+    one_sided = [(i, j) for (i, j) in listed if (j, i) not in listed]
+    assert one_sided
+    s, rad = setup.s, setup.rad
+    R, bw = s.cyl.R, s.cyl.Bw
+    free = (np.hypot(pos[:, 0], pos[:, 1]) + rad < R) & (pos[:, 2] - rad > bw)
+    want = np.zeros_like(pos)
+    want[:, 2] -= (2 * rad) ** 3
+    for i, j in listed:
+        d = pos[i] - pos[j]
+        L = np.linalg.norm(d)
+        nrm = rad[i] + rad[j] - L
+        if nrm <= 0:
+            continue
+        r = rad[i] * rad[j] / (rad[i] + rad[j])
+        fn = 4 / 3 * s.cal.emod * np.sqrt(r) * nrm ** 1.5
+        if nrm > s.cal.ydsp_t * r:
+            fn = s.cal.yforce_t * r * r + s.cal.ystiff_t * r * (nrm - s.cal.ydsp_t * r)
+        want[i] += fn * d / L
+    scale = np.abs(want[free]).max()
+    # FP64: the two orders of summation; mixed: the FP32 overlap and law
+    tol = {"fp64": 1e-11, "mixed": 2e-5}[precision]
+    assert any(free[i] for i, _ in one_sided)
+    assert np.abs(f - want)[free].max() <= tol * scale
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 127, 128, 129, 255, 257])
+def test_lists_and_forces_at_block_edges(cuda, n):
+    """the mixed engine against the FP64 one at sizes around the kernels' warps
+    and blocks: the same lists, forces to the FP32 law's tolerance"""
+    w = _workloads.small_wet(n=n, n_levels=1 if n < 3 else 3)
+    pos, vel, ang = _workloads.stirred(w, vscale=0.05, wscale=0.1)
+    got = {}
+    for precision in ("fp64", "mixed"):
+        e = Engine(w.setup, precision=precision)
+        e.set_state(pos, vel, ang)
+        e.step(1)
+        e.sync()
+        c, p = e.neighbors()
+        got[precision] = (c, p, e.get_state()["force"], e.stats())
+        e.close()
+    a, b = got["fp64"], got["mixed"]
+    np.testing.assert_array_equal(a[0], b[0])
+    np.testing.assert_array_equal(a[1], b[1])
+    assert np.abs(a[2] - b[2]).max() <= 2e-5 * np.abs(a[2]).max()
+    for k in ("nb_entries", "contacts", "bridges", "wall_contacts"):
+        assert a[3][k] == b[3][k], k
