@@ -8,12 +8,9 @@
  * formula's outputs in FP64 (kernel.cu:65-81, :518), written in particle /
  * slot order (deterministic).
  *
- * Training (FP32): one block of 128 threads takes 128 samples, one sample per
- * thread for the forward pass and the per-sample backward pass, with the
- * activations in shared memory; the weight gradients are reduced over the
- * block's samples in shared memory and written as one partial per block; a
- * second kernel sums the partials in block order (so a run is reproducible)
- * and applies Adam.  Loss: mean over samples of the squared error of the two
+ * Training (FP32): blocks take 64 samples at a time through register-tiled
+ * products (k_train) and write one gradient partial each; a second kernel sums
+ * the partials in a fixed order (so a run is reproducible) and applies Adam.  Loss: mean over samples of the squared error of the two
  * standardised outputs.
  */
 #include <cuda_runtime.h>
@@ -35,6 +32,7 @@ struct dem_capnet {
   float* params;   /* device, kCapParams FP32 */
   float* adam_m;   /* device */
   float* adam_v;   /* device */
+  float* grad;     /* device, kCapParams + 1: the gradient and loss of dem_capnet_grad */
   float* partial;  /* device, per-block gradient partials */
   int partial_blocks;
   long long step;  /* Adam steps taken */
@@ -42,15 +40,22 @@ struct dem_capnet {
   bool has_norm;
   dem::CapNetSmem* packed; /* device, BF16 network as the step kernel stages it */
   bool packed_valid;
+  float host_params[4612]; /* the parameters as the FP32 network's kernel takes them */
+  bool host_valid;
+  int* gave_up; /* device: raised by a tensor-core kernel that gave up waiting */
 };
 
 namespace dem {
 namespace {
 
-constexpr int kTB = 128;           /* samples per training block */
-constexpr int kHS = kCapH + 1;     /* padded row of per-sample activations */
+constexpr int kTB = 256;           /* threads of a training block: 16 x 16 tiles of 4 x 4 */
+constexpr int kTS = 64;            /* samples per tile */
+constexpr int kTrainBlocks = 152;  /* one a multiprocessor (its operands fill the shared memory) */
+constexpr int kLd = kCapH + 4;     /* padded row of a 64-wide operand, 16-byte aligned */
+/* the gradients other than dW2, as a block collects them */
+constexpr int kSmW1 = 0, kSmB1 = kSmW1 + kCapH * kCapIn, kSmB2 = kSmB1 + kCapH, kSmW3 = kSmB2 + kCapH,
+              kSmB3 = kSmW3 + kCapOut * kCapH, kSmLoss = kSmB3 + kCapOut, kSmall = kSmLoss + 1;
 constexpr int kWPad = 4612;        /* parameters in shared memory, 16-byte multiple */
-constexpr size_t kTrainSmem = sizeof(float) * (kWPad + kTB * 4 + 3 * kTB * kHS + kTB * 2 + 32);
 
 inline int blocks_for(long long n, int b) { return n <= 0 ? 1 : (int)((n + b - 1) / b); }
 
@@ -64,10 +69,21 @@ Norm norm_of(const dem_capnet* net) {
   return z;
 }
 
-__device__ __forceinline__ float silu_acc(float z) { return z / (1.0f + expf(-z)); }
-__device__ __forceinline__ float dsilu_acc(float z) {
-  const float s = 1.0f / (1.0f + expf(-z));
-  return s * (1.0f + z * (1.0f - s));
+/* 1 / (1 + e^-z) and z / (1 + e^-z) in FP32: the hardware reciprocal with one
+ * Newton correction (within an ulp of the quotient) instead of the general
+ * division, whose range handling costs as much again as the exponential.  The
+ * exponent stops at 80, so the divisor stays finite; beyond 80 the SiLU is its
+ * argument (infinity included), and -infinity and NaN give NaN, as the plain
+ * quotient does.  No branches: a thread's units overlap. */
+__device__ __forceinline__ float sigmoid_acc(float z) {
+  const float d = 1.0f + expf(fminf(-z, 80.0f));
+  const float r = __fdividef(1.0f, d);
+  return fmaf(fmaf(-d, r, 1.0f), r, r);
+}
+__device__ __forceinline__ float silu_acc(float z) {
+  const float d = 1.0f + expf(fminf(-z, 80.0f));
+  const float r = __fdividef(1.0f, d), q = z * r;
+  return z > 80.0f ? z : fmaf(fmaf(-d, q, z), r, q);
 }
 __device__ __forceinline__ void std_inputs(const float* raw, const Norm& nz, float x[4]) {
   x[0] = (logf(raw[0]) - nz.xm[0]) / nz.xs[0];
@@ -183,124 +199,233 @@ __global__ void k_sample_write(SampleArgs a, const long long* off, long long cap
 
 /* ---------------- training ---------------- */
 
-__global__ void __launch_bounds__(kTB) k_train(const float* __restrict__ P, const float* __restrict__ xr,
-                                               const float* __restrict__ yr, const int* __restrict__ idx, int nb,
-                                               float inv_total, Norm nz, float* __restrict__ partial) {
-  extern __shared__ float sm[];
-  float* W = sm;
-  float* X = W + kWPad;
-  float* H1 = X + kTB * 4;
-  float* Z2 = H1 + kTB * kHS; /* pre-activations, then their gradients */
-  float* H2 = Z2 + kTB * kHS; /* activations, then the layer-1 gradients */
-  float* DY = H2 + kTB * kHS;
-  float* red = DY + kTB * 2;
-  const int tid = threadIdx.x;
-  for (int i = tid; i < kCapParams; i += kTB) W[i] = P[i];
-  const int gi = blockIdx.x * kTB + tid;
-  const bool valid = gi < nb;
-  float x[4] = {0.f, 0.f, 0.f, 0.f}, t[2] = {0.f, 0.f};
-  if (valid) {
-    const long long si = idx ? (long long)idx[gi] : (long long)gi;
-    std_inputs(xr + 4 * si, nz, x);
-    t[0] = (yr[2 * si] - nz.ym[0]) / nz.ys[0];
-    t[1] = (yr[2 * si + 1] - nz.ym[1]) / nz.ys[1];
-  }
-  for (int i = 0; i < 4; i++) X[tid * 4 + i] = x[i];
-  __syncthreads();
-  const float* W1 = W + kCapW1;
-  const float* B1 = W + kCapB1;
-  const float* W2 = W + kCapW2;
-  const float* B2 = W + kCapB2;
-  const float* W3 = W + kCapW3;
-  const float* B3 = W + kCapB3;
-  float* h1 = H1 + tid * kHS;
-  float* z2 = Z2 + tid * kHS;
-  float* h2 = H2 + tid * kHS;
-  /* forward */
-  for (int m = 0; m < kCapH; m++) {
-    float z = B1[m];
-    for (int i = 0; i < 4; i++) z += W1[m * 4 + i] * x[i];
-    h1[m] = silu_acc(z);
-  }
-  float y0 = B3[0], y1 = B3[1];
-  for (int n = 0; n < kCapH; n++) {
-    float z = B2[n];
-    for (int m = 0; m < kCapH; m++) z += W2[n * kCapH + m] * h1[m];
-    z2[n] = z;
-    const float a = silu_acc(z);
-    h2[n] = a;
-    y0 += W3[n] * a;
-    y1 += W3[kCapH + n] * a;
-  }
-  const float e0 = y0 - t[0], e1 = y1 - t[1];
-  const float dy0 = valid ? 2.0f * e0 * inv_total : 0.f, dy1 = valid ? 2.0f * e1 * inv_total : 0.f;
-  DY[tid * 2] = dy0;
-  DY[tid * 2 + 1] = dy1;
-  for (int n = 0; n < kCapH; n++) z2[n] = (W3[n] * dy0 + W3[kCapH + n] * dy1) * dsilu_acc(z2[n]);
-  __syncthreads();
-  float* out = partial + (size_t)blockIdx.x * (kCapParams + 1);
-  /* layer 2 and 3 weight gradients, reduced over the block's samples */
-  for (int p = tid; p < kCapH * kCapH + kCapH + kCapOut * kCapH + kCapOut; p += kTB) {
-    float acc = 0.f;
-    if (p < kCapH * kCapH) {
-      const int n = p / kCapH, m = p % kCapH;
-      for (int s = 0; s < kTB; s++) acc += Z2[s * kHS + n] * H1[s * kHS + m];
-      out[kCapW2 + p] = acc;
-    } else if (p < kCapH * kCapH + kCapH) {
-      const int n = p - kCapH * kCapH;
-      for (int s = 0; s < kTB; s++) acc += Z2[s * kHS + n];
-      out[kCapB2 + n] = acc;
-    } else if (p < kCapH * kCapH + kCapH + kCapOut * kCapH) {
-      const int q = p - kCapH * kCapH - kCapH, o = q / kCapH, n = q % kCapH;
-      for (int s = 0; s < kTB; s++) acc += DY[s * 2 + o] * H2[s * kHS + n];
-      out[kCapW3 + q] = acc;
-    } else {
-      const int o = p - kCapH * kCapH - kCapH - kCapOut * kCapH;
-      for (int s = 0; s < kTB; s++) acc += DY[s * 2 + o];
-      out[kCapB3 + o] = acc;
-    }
-  }
-  __syncthreads();
-  /* layer-1 gradients of this sample (into the H2 rows) */
-  for (int m = 0; m < kCapH; m++) {
-    float g = 0.f;
-    for (int n = 0; n < kCapH; n++) g += W2[n * kCapH + m] * z2[n];
-    float z = B1[m];
-    for (int i = 0; i < 4; i++) z += W1[m * 4 + i] * x[i];
-    h2[m] = g * dsilu_acc(z);
-  }
-  __syncthreads();
-  for (int p = tid; p < kCapH * 4 + kCapH; p += kTB) {
-    float acc = 0.f;
-    if (p < kCapH * 4) {
-      const int m = p / 4, i = p % 4;
-      for (int s = 0; s < kTB; s++) acc += H2[s * kHS + m] * X[s * 4 + i];
-      out[kCapW1 + p] = acc;
-    } else {
-      const int m = p - kCapH * 4;
-      for (int s = 0; s < kTB; s++) acc += H2[s * kHS + m];
-      out[kCapB1 + m] = acc;
-    }
-  }
-  /* loss partial */
-  float l = valid ? (e0 * e0 + e1 * e1) * inv_total : 0.f;
-  for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-  if ((tid & 31) == 0) red[tid >> 5] = l;
-  __syncthreads();
-  if (tid == 0) {
-    float s = 0.f;
-    for (int w = 0; w < kTB / 32; w++) s += red[w];
-    out[kCapParams] = s;
+/* One block of 256 threads takes 64 samples at a time.  The three 64 x 64 x 64
+ * products (layer 2 forward, its weight gradient, the gradient into layer 1)
+ * run as 4 x 4 register tiles, two 16-byte shared loads per 16 FMAs; operands
+ * that two products read along different axes are stored both ways.  Everything
+ * between the products stays in the registers of the tile's owner.  Blocks walk
+ * several tiles and keep their gradient in registers, so the partials are at
+ * most two a multiprocessor whatever the batch.
+ *
+ * Bound by the latency of one tile's chain at a batch of 8192 (128 blocks of one
+ * tile), by the FMA pipe on large sets.  Before, a thread took a sample through
+ * both layers one weight at a time (two shared loads per FMA, 128 samples a
+ * block: 64 blocks for a batch of 8192): dem_capnet_grad took 111 us on 8192
+ * samples and 1803 on 500,000, with two allocations and four waits a call; now
+ * 44 (k_train 20, k_reduce_adam 5, the rest the call) and 492.
+ */
+__device__ __forceinline__ void tile_fma(const float (*A)[kLd], const float (*B)[kLd], int r0, int c0,
+                                         float (&c)[4][4]) {
+#pragma unroll 8
+  for (int k = 0; k < 64; k++) {
+    const float4 a = *reinterpret_cast<const float4*>(&A[k][r0]), b = *reinterpret_cast<const float4*>(&B[k][c0]);
+    const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) c[i][j] = fmaf(av[i], bv[j], c[i][j]);
   }
 }
 
-/* sum the block partials in order; then an Adam step (lr > 0) and/or a copy of the gradient */
-__global__ void k_reduce_adam(float* P, float* M, float* V, const float* partial, int nblocks, float lr, float bc1,
-                              float bc2, float* grad_out, float* loss_out) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p > kCapParams) return;
+struct TrainSmem {
+  float w[kWPad];
+  float w2t[kCapH][kLd];  /* [m][n] */
+  float w2[kCapH][kLd];   /* [n][m] */
+  float h1t[kCapH][kLd];  /* [m][s] */
+  float h1[kTS][kLd];     /* [s][m] */
+  float dzt[kCapH][kLd];  /* [n][s] */
+  float dz[kTS][kLd];     /* [s][n] */
+  float x[kTS][4], t[kTS][2];
+  float red[16][kSmall];  /* the small gradients by group of four samples */
+};
+
+__global__ void __launch_bounds__(kTB) k_train(const float* __restrict__ P, const float* __restrict__ xr,
+                                               const float* __restrict__ yr, const int* __restrict__ idx, int nb,
+                                               float inv_total, Norm nz, float* __restrict__ partial) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  TrainSmem& sm = *reinterpret_cast<TrainSmem*>(raw);
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int c0 = 4 * tx, r0 = 4 * ty;
+  for (int i = tid; i < kCapParams; i += kTB) {
+    const float v = P[i];
+    sm.w[i] = v;
+    const int e = i - kCapW2;
+    if (e >= 0 && e < kCapH * kCapH) {
+      sm.w2[e / kCapH][e % kCapH] = v;
+      sm.w2t[e % kCapH][e / kCapH] = v;
+    }
+  }
+  float gw2[4][4] = {}; /* dW2[r0 + a][c0 + b] over this block's tiles */
+  float small[(kSmall + kTB - 1) / kTB] = {};
+  const int tiles = (nb + kTS - 1) / kTS;
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    __syncthreads(); /* the last tile's operands have been read */
+    if (tid < kTS) {
+      const int gi = tile * kTS + tid;
+      float x[4] = {0.f, 0.f, 0.f, 0.f}, t[2] = {0.f, 0.f};
+      if (gi < nb) {
+        const long long si = idx ? (long long)idx[gi] : (long long)gi;
+        std_inputs(xr + 4 * si, nz, x);
+        t[0] = (yr[2 * si] - nz.ym[0]) / nz.ys[0];
+        t[1] = (yr[2 * si + 1] - nz.ym[1]) / nz.ys[1];
+      }
+      for (int i = 0; i < 4; i++) sm.x[tid][i] = x[i];
+      sm.t[tid][0] = t[0];
+      sm.t[tid][1] = t[1];
+    }
+    __syncthreads();
+    /* layer 1 on samples r0.., units c0.. */
+    float d1[4][4];
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+      const float* w1 = sm.w + kCapW1 + (c0 + b) * 4;
+      const float bias = sm.w[kCapB1 + c0 + b];
+#pragma unroll
+      for (int a = 0; a < 4; a++) {
+        float z = bias;
+#pragma unroll
+        for (int i = 0; i < 4; i++) z = fmaf(w1[i], sm.x[r0 + a][i], z);
+        const float sg = sigmoid_acc(z), h = silu_acc(z);
+        d1[a][b] = sg * fmaf(z, 1.0f - sg, 1.0f);
+        sm.h1[r0 + a][c0 + b] = h;
+        sm.h1t[c0 + b][r0 + a] = h;
+      }
+    }
+    __syncthreads();
+    /* layer 2 */
+    float z2[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+      for (int b = 0; b < 4; b++) z2[a][b] = sm.w[kCapB2 + c0 + b];
+    tile_fma(sm.h1t, sm.w2t, r0, c0, z2);
+    float y0[4] = {}, y1[4] = {}, h2[4][4];
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+      const float w30 = sm.w[kCapW3 + c0 + b], w31 = sm.w[kCapW3 + kCapH + c0 + b];
+#pragma unroll
+      for (int a = 0; a < 4; a++) {
+        const float z = z2[a][b];
+        h2[a][b] = silu_acc(z);
+        y0[a] = fmaf(w30, h2[a][b], y0[a]);
+        y1[a] = fmaf(w31, h2[a][b], y1[a]);
+        const float sg = sigmoid_acc(z);
+        z2[a][b] = sg * fmaf(z, 1.0f - sg, 1.0f); /* SiLU' */
+      }
+    }
+    /* outputs: sum over the 16 threads that share the samples */
+    float dy0[4], dy1[4], loss = 0.f, s0 = 0.f, s1 = 0.f;
+#pragma unroll
+    for (int a = 0; a < 4; a++) {
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) {
+        y0[a] += __shfl_xor_sync(0xffffffffu, y0[a], o);
+        y1[a] += __shfl_xor_sync(0xffffffffu, y1[a], o);
+      }
+      const bool valid = tile * kTS + r0 + a < nb;
+      const float e0 = y0[a] + sm.w[kCapB3] - sm.t[r0 + a][0], e1 = y1[a] + sm.w[kCapB3 + 1] - sm.t[r0 + a][1];
+      dy0[a] = valid ? 2.0f * e0 * inv_total : 0.f;
+      dy1[a] = valid ? 2.0f * e1 * inv_total : 0.f;
+      loss += valid ? (e0 * e0 + e1 * e1) * inv_total : 0.f;
+      s0 += dy0[a];
+      s1 += dy1[a];
+    }
+    float* rd = sm.red[ty];
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+      const float w30 = sm.w[kCapW3 + c0 + b], w31 = sm.w[kCapW3 + kCapH + c0 + b];
+      float g0 = 0.f, g1 = 0.f, gb = 0.f;
+#pragma unroll
+      for (int a = 0; a < 4; a++) {
+        const float dz = (w30 * dy0[a] + w31 * dy1[a]) * z2[a][b];
+        sm.dz[r0 + a][c0 + b] = dz;
+        sm.dzt[c0 + b][r0 + a] = dz;
+        g0 = fmaf(dy0[a], h2[a][b], g0);
+        g1 = fmaf(dy1[a], h2[a][b], g1);
+        gb += dz;
+      }
+      rd[kSmB2 + c0 + b] = gb;
+      rd[kSmW3 + c0 + b] = g0;
+      rd[kSmW3 + kCapH + c0 + b] = g1;
+    }
+    if (tx == 0) {
+      rd[kSmB3] = s0;
+      rd[kSmB3 + 1] = s1;
+      rd[kSmLoss] = loss;
+    }
+    __syncthreads();
+    {
+      float g[4][4] = {};
+      tile_fma(sm.dz, sm.h1, r0, c0, g); /* dW2[n][m] = sum over s */
+#pragma unroll
+      for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int b = 0; b < 4; b++) gw2[a][b] += g[a][b];
+    }
+    float g1[4][4] = {};
+    tile_fma(sm.dzt, sm.w2, r0, c0, g1); /* into layer 1: [s][m] = sum over n */
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+      float gb = 0.f, gw[4] = {};
+#pragma unroll
+      for (int a = 0; a < 4; a++) {
+        const float dz1 = g1[a][b] * d1[a][b];
+        gb += dz1;
+#pragma unroll
+        for (int i = 0; i < 4; i++) gw[i] = fmaf(dz1, sm.x[r0 + a][i], gw[i]);
+      }
+      rd[kSmB1 + c0 + b] = gb;
+#pragma unroll
+      for (int i = 0; i < 4; i++) rd[kSmW1 + (c0 + b) * 4 + i] = gw[i];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < (kSmall + kTB - 1) / kTB; k++) {
+      const int e = tid + k * kTB;
+      if (e >= kSmall) break;
+      float v = 0.f;
+#pragma unroll
+      for (int g = 0; g < 16; g++) v += sm.red[g][e];
+      small[k] += v;
+    }
+  }
+  float* out = partial + (size_t)blockIdx.x * (kCapParams + 1);
+#pragma unroll
+  for (int a = 0; a < 4; a++)
+#pragma unroll
+    for (int b = 0; b < 4; b++) out[kCapW2 + (r0 + a) * kCapH + c0 + b] = gw2[a][b];
+#pragma unroll
+  for (int k = 0; k < (kSmall + kTB - 1) / kTB; k++) {
+    const int e = tid + k * kTB;
+    if (e >= kSmall) break;
+    const int to = e < kSmB1   ? kCapW1 + e
+                   : e < kSmB2 ? kCapB1 + e - kSmB1
+                   : e < kSmW3 ? kCapB2 + e - kSmB2
+                   : e < kSmB3 ? kCapW3 + e - kSmW3
+                               : kCapB3 + e - kSmB3; /* b3, then the loss */
+    out[to] = small[k];
+  }
+}
+
+/* sum the block partials in a fixed order (eight slices of the blocks, then the
+ * slices); then an Adam step (lr > 0) and/or a copy of the gradient */
+constexpr int kRedParams = 32, kRedSlices = 8;
+__global__ void __launch_bounds__(kRedParams* kRedSlices) k_reduce_adam(float* P, float* M, float* V,
+                                                                        const float* __restrict__ partial, int nblocks,
+                                                                        float lr, float bc1, float bc2,
+                                                                        float* grad_out, float* loss_out) {
+  __shared__ float part[kRedSlices][kRedParams];
+  const int lane = threadIdx.x % kRedParams, slice = threadIdx.x / kRedParams;
+  const int p = blockIdx.x * kRedParams + lane;
   float g = 0.f;
-  for (int b = 0; b < nblocks; b++) g += partial[(size_t)b * (kCapParams + 1) + p];
+  if (p <= kCapParams) {
+#pragma unroll 4
+    for (int b = slice; b < nblocks; b += kRedSlices) g += partial[(size_t)b * (kCapParams + 1) + p];
+  }
+  part[slice][lane] = g;
+  __syncthreads();
+  if (slice != 0 || p > kCapParams) return;
+  for (int k = 1; k < kRedSlices; k++) g += part[k][lane];
   if (p == kCapParams) {
     if (loss_out) *loss_out = g;
     return;
@@ -316,66 +441,126 @@ __global__ void k_reduce_adam(float* P, float* M, float* V, const float* partial
   }
 }
 
-/* FP32 forward (the training precision) on raw features -> raw outputs */
-__global__ void k_infer32(const float* __restrict__ P, const float* __restrict__ xr, long long n, Norm nz,
-                          float* __restrict__ y) {
-  __shared__ float W[kWPad];
-  for (int i = threadIdx.x; i < kCapParams; i += blockDim.x) W[i] = P[i];
-  __syncthreads();
-  const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (q >= n) return;
-  float x[4], h1[kCapH];
-  std_inputs(xr + 4 * q, nz, x);
-  for (int m = 0; m < kCapH; m++) {
-    float z = W[kCapB1 + m];
-    for (int i = 0; i < 4; i++) z += W[kCapW1 + m * 4 + i] * x[i];
-    h1[m] = silu_acc(z);
+/* FP32 forward (the training precision) on raw features -> raw outputs, R rows
+ * a thread with their hidden units in registers, A partial sums a dot product.
+ * The weights are kernel parameters: they reach the FMAs through the constant
+ * path, as uniform operands, where a shared-memory broadcast moves 512 bytes
+ * into the register file per four weights and bounded the loop.  Bound by
+ * instruction issue (82 %): 4,480 FMAs and 128 SiLUs a row.  1M rows: 271 us
+ * (one row a thread with the hidden units in local memory and weights in shared
+ * memory: 480). */
+struct __align__(16) CapParams {
+  float w[kWPad];
+};
+constexpr int kInferThreads = 128;
+template <int R, int A>
+__global__ void __launch_bounds__(kInferThreads) k_infer32(const __grid_constant__ CapParams P,
+                                                           const float* __restrict__ xr, long long n, Norm nz,
+                                                           float* __restrict__ y) {
+  const long long q0 = (long long)blockIdx.x * (kInferThreads * R) + threadIdx.x;
+  float h1[R][kCapH];
+#pragma unroll
+  for (int r = 0; r < R; r++) {
+    const long long q = q0 + r * kInferThreads;
+    float x[4] = {0.f, 0.f, 0.f, 0.f};
+    if (q < n) std_inputs(xr + 4 * q, nz, x);
+#pragma unroll
+    for (int m = 0; m < kCapH; m++) {
+      float z = P.w[kCapB1 + m];
+#pragma unroll
+      for (int i = 0; i < 4; i++) z = fmaf(P.w[kCapW1 + m * 4 + i], x[i], z);
+      h1[r][m] = silu_acc(z);
+    }
   }
-  float y0 = W[kCapB3], y1 = W[kCapB3 + 1];
+  float y0[R], y1[R];
+#pragma unroll
+  for (int r = 0; r < R; r++) {
+    y0[r] = P.w[kCapB3];
+    y1[r] = P.w[kCapB3 + 1];
+  }
+#pragma unroll 1
   for (int nn = 0; nn < kCapH; nn++) {
-    float z = W[kCapB2 + nn];
-    for (int m = 0; m < kCapH; m++) z += W[kCapW2 + nn * kCapH + m] * h1[m];
-    const float a = silu_acc(z);
-    y0 += W[kCapW3 + nn] * a;
-    y1 += W[kCapW3 + kCapH + nn] * a;
+    float z[R][A];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+#pragma unroll
+      for (int k = 0; k < A; k++) z[r][k] = k ? 0.f : P.w[kCapB2 + nn];
+    }
+    const float4* w4 = reinterpret_cast<const float4*>(P.w + kCapW2 + nn * kCapH);
+#pragma unroll
+    for (int m = 0; m < kCapH / 4; m++) {
+      const float4 w = w4[m];
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        float& c = z[r][m % A];
+        c = fmaf(w.x, h1[r][4 * m], c);
+        c = fmaf(w.y, h1[r][4 * m + 1], c);
+        c = fmaf(w.z, h1[r][4 * m + 2], c);
+        c = fmaf(w.w, h1[r][4 * m + 3], c);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      float v = z[r][0];
+#pragma unroll
+      for (int k = 1; k < A; k++) v += z[r][k];
+      const float a = silu_acc(v);
+      y0[r] = fmaf(P.w[kCapW3 + nn], a, y0[r]);
+      y1[r] = fmaf(P.w[kCapW3 + kCapH + nn], a, y1[r]);
+    }
   }
-  y[2 * q] = y0 * nz.ys[0] + nz.ym[0];
-  y[2 * q + 1] = y1 * nz.ys[1] + nz.ym[1];
+#pragma unroll
+  for (int r = 0; r < R; r++) {
+    const long long q = q0 + r * kInferThreads;
+    if (q < n) {
+      y[2 * q] = y0[r] * nz.ys[0] + nz.ym[0];
+      y[2 * q + 1] = y1[r] * nz.ys[1] + nz.ym[1];
+    }
+  }
 }
 
-/* BF16 tensor-core tiles, exactly as the fused step kernel evaluates them */
+/* BF16 tensor-core tiles, exactly as the fused step kernel evaluates them.  The
+ * next tile's features are in flight while the current one runs (1M rows: 47
+ * us, without 54; the 128 hardware tanh a row alone need 25). */
 __global__ void __launch_bounds__(128) k_infer_tc(const CapNetSmem* __restrict__ wsrc, const float* __restrict__ xr,
                                                   long long n, float* __restrict__ y) {
   __shared__ __align__(16) unsigned char wbuf[sizeof(CapNetSmem)];
   CapNetSmem& w = *reinterpret_cast<CapNetSmem*>(wbuf);
-  cap_stage(wsrc, &w);
-  __syncthreads();
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-  for (long long tile = warp; tile * 16 < n; tile += nwarps) {
-    uint32_t xa = 0u, xb = 0u;
-    const long long r0 = tile * 16 + g, r1 = r0 + 8;
-    if (t < 2) {
-      if (r0 < n) {
-        const float* f = xr + 4 * r0;
-        xa = cap_pair(w, f[0], f[1], f[2], f[3], t);
-      }
-      if (r1 < n) {
-        const float* f = xr + 4 * r1;
-        xb = cap_pair(w, f[0], f[1], f[2], f[3], t);
+  /* lane (g, t < 2) standardises features 2t, 2t + 1 of rows g and g + 8 */
+  float f[2][2];
+  auto fetch = [&](long long tile) {
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const long long r = tile * 16 + g + 8 * k;
+      if (t < 2 && r < n) {
+        f[k][0] = xr[4 * r + 2 * t];
+        f[k][1] = xr[4 * r + 2 * t + 1];
       }
     }
+  };
+  long long tile = warp;
+  fetch(tile);
+  cap_stage(wsrc, &w);
+  __syncthreads();
+  for (; tile * 16 < n; tile += nwarps) {
+    uint32_t x[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++)
+      x[k] = t < 2 && tile * 16 + g + 8 * k < n ? cap_pair(w, f[k][0], f[k][1], f[k][0], f[k][1], t) : 0u;
+    fetch(tile + nwarps);
     float o[4];
-    cap_tile16(w, xa, xb, o);
+    cap_tile16(w, x[0], x[1], o);
     if (t == 0) {
-      if (r0 < n) {
-        y[2 * r0] = o[0] * w.y_std[0] + w.y_mean[0];
-        y[2 * r0 + 1] = o[1] * w.y_std[1] + w.y_mean[1];
-      }
-      if (r1 < n) {
-        y[2 * r1] = o[2] * w.y_std[0] + w.y_mean[0];
-        y[2 * r1 + 1] = o[3] * w.y_std[1] + w.y_mean[1];
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        const long long r = tile * 16 + g + 8 * k;
+        if (r < n) {
+          y[2 * r] = o[2 * k] * w.y_std[0] + w.y_mean[0];
+          y[2 * r + 1] = o[2 * k + 1] * w.y_std[1] + w.y_mean[1];
+        }
       }
     }
   }
@@ -398,7 +583,10 @@ __global__ void __launch_bounds__(128) k_infer_tc(const CapNetSmem* __restrict__
  * adjacent along K (leading-dimension offset 128 B), 8-row groups follow
  * each other (stride-dimension offset = 128 B x cores along K). */
 constexpr int kTcRows = 128;
-constexpr uint32_t kTcCols = 128;  /* tensor-memory columns: D1 at 0, D2 at 64 */
+constexpr uint32_t kTcCols = 64;   /* tensor-memory columns: D1, then D2 over it */
+/* resident blocks a multiprocessor: 4 (1M rows 84 us a call, 100,000 34) as fast as 6 or
+ * 7 on many rows and faster on few, where each block's staging counts (44) */
+constexpr int kTcBlocks = 4;
 constexpr unsigned long long kTcWaitNs = 1000000000ull; /* give up on an MMA completion after 1 s */
 
 struct __align__(128) TcSmem {
@@ -481,7 +669,7 @@ __device__ __forceinline__ void tc_sync() {
 /* raw features -> raw outputs; err gets 1 if an MMA completion was not seen
  * within kTcWaitNs (the kernel then stops; tensor memory is freed on every
  * path) */
-__global__ void __launch_bounds__(kTcRows, 1) k_infer_tc5(const CapNetSmem* __restrict__ wsrc,
+__global__ void __launch_bounds__(kTcRows, kTcBlocks) k_infer_tc5(const CapNetSmem* __restrict__ wsrc,
                                                           const float* __restrict__ xr, long long n,
                                                           float* __restrict__ y, int* __restrict__ err) {
   __shared__ TcSmem sm;
@@ -525,19 +713,27 @@ __global__ void __launch_bounds__(kTcRows, 1) k_infer_tc5(const CapNetSmem* __re
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   tc_sync();
   const uint32_t tmem = sm.tmem_base;
-  const uint32_t d1 = tmem, d2 = tmem + (uint32_t)kCapH;
+  const uint32_t d1 = tmem, d2 = tmem; /* D1 is read before layer 2's MMAs are issued */
   const uint32_t lane_base = (uint32_t)(32 * warp) << 16; /* this warp's tensor-memory lanes */
   const unsigned long long da1 = tc_desc(smem_u32(sm.a1), 128, 2 * 128);
   const unsigned long long db1 = tc_desc(smem_u32(sm.b1), 128, 2 * 128);
   uint32_t parity = 0;
   bool ok = true;
   const long long tiles = (n + kTcRows - 1) / kTcRows;
+  /* the next tile's row is in flight while the current one runs */
+  float4 fn = make_float4(1.f, 1.f, 0.f, 0.f);
+  if (blockIdx.x * (long long)kTcRows + tid < n)
+    fn = *reinterpret_cast<const float4*>(xr + 4 * (blockIdx.x * (long long)kTcRows + tid));
   for (long long tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
     const long long row = tile * kTcRows + tid;
     /* layer 1 operand: this row's standardised inputs (k 0..3; k 4..15 stay 0) */
     float x0 = 0.f, x1 = 0.f, x2 = 0.f, x3 = 0.f;
+    const float4 f = fn;
+    {
+      const long long next = row + (long long)gridDim.x * kTcRows;
+      if (next < n) fn = *reinterpret_cast<const float4*>(xr + 4 * next);
+    }
     if (row < n) {
-      const float4 f = *reinterpret_cast<const float4*>(xr + 4 * row);
       x0 = (__logf(f.x) - sm.xm[0]) * sm.xis[0];
       x1 = (__logf(f.y) - sm.xm[1]) * sm.xis[1];
       x2 = (f.z - sm.xm[2]) * sm.xis[2];
@@ -727,6 +923,17 @@ dem_status ensure_packed(dem_capnet* net) {
   return st;
 }
 
+dem_status ensure_host_params(dem_capnet* net) {
+  if (net->host_valid) return DEM_OK;
+  dem_status st = ck(cudaMemcpy(net->host_params, net->params, sizeof(float) * kCapParams, cudaMemcpyDeviceToHost),
+                     "capnet params download");
+  net->host_valid = st == DEM_OK;
+  return st;
+}
+
+/* the parameters on the device have changed */
+void params_changed(dem_capnet* net) { net->packed_valid = net->host_valid = false; }
+
 dem_status ensure_partials(dem_capnet* net, int blocks) {
   if (blocks <= net->partial_blocks) return DEM_OK;
   if (net->partial) cudaFree(net->partial);
@@ -740,18 +947,18 @@ dem_status ensure_partials(dem_capnet* net, int blocks) {
 /* one gradient (and optionally Adam) step over `nb` samples given by idx (device) */
 dem_status train_step(dem_capnet* net, const float* x, const float* y, const int* idx, int nb, float lr,
                       float* grad_dev, float* loss_dev, cudaStream_t s) {
-  const int blocks = blocks_for(nb, kTB);
+  const int blocks = std::min(blocks_for(nb, kTS), kTrainBlocks);
   dem_status st = ensure_partials(net, blocks);
   if (st != DEM_OK) return st;
   const Norm nz = norm_of(net);
-  k_train<<<blocks, kTB, kTrainSmem, s>>>(net->params, x, y, idx, nb, 1.0f / (float)nb, nz, net->partial);
+  k_train<<<blocks, kTB, sizeof(TrainSmem), s>>>(net->params, x, y, idx, nb, 1.0f / (float)nb, nz, net->partial);
   float bc1 = 1.f, bc2 = 1.f;
   if (lr > 0.f) {
     net->step++;
     bc1 = 1.f - (float)std::pow(0.9, (double)net->step);
     bc2 = 1.f - (float)std::pow(0.999, (double)net->step);
   }
-  k_reduce_adam<<<blocks_for(kCapParams + 1, 256), 256, 0, s>>>(net->params, net->adam_m, net->adam_v, net->partial,
+  k_reduce_adam<<<blocks_for(kCapParams + 1, kRedParams), kRedParams * kRedSlices, 0, s>>>(net->params, net->adam_m, net->adam_v, net->partial,
                                                                  blocks, lr, bc1, bc2, grad_dev, loss_dev);
   return ck(cudaGetLastError(), "capnet train launch");
 }
@@ -768,7 +975,7 @@ dem_status dem_capnet_create(unsigned long long seed, dem_capnet** out) {
   *out = nullptr;
   static bool attr = false;
   if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(k_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrainSmem);
+    cudaError_t e = cudaFuncSetAttribute(k_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrainSmem));
     if (e != cudaSuccess) return cuda_check(e, "capnet: shared-memory attribute");
     attr = true;
   }
@@ -777,7 +984,10 @@ dem_status dem_capnet_create(unsigned long long seed, dem_capnet** out) {
   dem_status st = cuda_alloc((void**)&net->params, sizeof(float) * kCapParams);
   if (st == DEM_OK) st = cuda_alloc((void**)&net->adam_m, sizeof(float) * kCapParams);
   if (st == DEM_OK) st = cuda_alloc((void**)&net->adam_v, sizeof(float) * kCapParams);
+  if (st == DEM_OK) st = cuda_alloc((void**)&net->grad, sizeof(float) * (kCapParams + 1));
   if (st == DEM_OK) st = cuda_alloc((void**)&net->packed, sizeof(CapNetSmem));
+  if (st == DEM_OK) st = cuda_alloc((void**)&net->gave_up, sizeof(int));
+  if (st == DEM_OK) st = ck(cudaMemset(net->gave_up, 0, sizeof(int)), "capnet init");
   if (st != DEM_OK) {
     dem_capnet_destroy(net);
     return st;
@@ -811,6 +1021,8 @@ void dem_capnet_destroy(dem_capnet* net) {
   cudaFree(net->params);
   cudaFree(net->adam_m);
   cudaFree(net->adam_v);
+  cudaFree(net->grad);
+  cudaFree(net->gave_up);
   cudaFree(net->partial);
   cudaFree(net->packed);
   delete net;
@@ -842,7 +1054,7 @@ dem_status dem_capnet_set(dem_capnet* net, const float* params, const float* nor
     std::memcpy(net->norm, norm, sizeof(net->norm));
     net->has_norm = true;
   }
-  net->packed_valid = false;
+  params_changed(net);
   return DEM_OK;
 }
 
@@ -850,16 +1062,12 @@ dem_status dem_capnet_grad(dem_capnet* net, const float* x_dev, const float* y_d
                            float* loss) {
   if (!net || !x_dev || !y_dev || n <= 0) return fail(DEM_ERR_ARG, "dem_capnet_grad: bad arguments");
   if (!net->has_norm) return fail(DEM_ERR_STATE, "dem_capnet_grad: set the standardisation first");
-  float* buf = nullptr;
-  dem_status st = cuda_alloc((void**)&buf, sizeof(float) * (kCapParams + 1));
-  if (st != DEM_OK) return st;
-  st = train_step(net, x_dev, y_dev, nullptr, n, 0.f, buf, buf + kCapParams, 0);
-  if (st == DEM_OK) st = ck(cudaDeviceSynchronize(), "dem_capnet_grad");
-  if (st == DEM_OK && grad)
-    st = ck(cudaMemcpy(grad, buf, sizeof(float) * kCapParams, cudaMemcpyDeviceToHost), "dem_capnet_grad");
-  if (st == DEM_OK && loss)
-    st = ck(cudaMemcpy(loss, buf + kCapParams, sizeof(float), cudaMemcpyDeviceToHost), "dem_capnet_grad");
-  cudaFree(buf);
+  /* gradient and loss lie together: one copy brings both (and waits) */
+  dem_status st = train_step(net, x_dev, y_dev, nullptr, n, 0.f, net->grad, net->grad + kCapParams, 0);
+  float h[kCapParams + 1];
+  if (st == DEM_OK) st = ck(cudaMemcpy(h, net->grad, sizeof(h), cudaMemcpyDeviceToHost), "dem_capnet_grad");
+  if (st == DEM_OK && grad) std::memcpy(grad, h, sizeof(float) * kCapParams);
+  if (st == DEM_OK && loss) *loss = h[kCapParams];
   return st;
 }
 
@@ -871,21 +1079,18 @@ dem_status dem_capnet_infer(dem_capnet* net, const float* x_dev, long long n, in
     /* the 5th-generation tensor cores: 128-row tiles, tcgen05.mma into tensor memory */
     dem_status st = ensure_packed(net);
     if (st != DEM_OK) return st;
-    int* err = nullptr;
-    st = cuda_alloc((void**)&err, sizeof(int));
-    if (st != DEM_OK) return st;
-    st = ck(cudaMemset(err, 0, sizeof(int)), "dem_capnet_infer");
     const long long tiles = (n + kTcRows - 1) / kTcRows;
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
-    const int blocks = (int)std::min<long long>(tiles, (long long)std::max(1, sms) * 4);
-    if (st == DEM_OK) k_infer_tc5<<<blocks, kTcRows>>>(net->packed, x_dev, n, y_dev, err);
-    if (st == DEM_OK) st = ck(cudaGetLastError(), "dem_capnet_infer launch");
-    if (st == DEM_OK) st = ck(cudaDeviceSynchronize(), "dem_capnet_infer");
-    int h = 0;
-    if (st == DEM_OK) st = ck(cudaMemcpy(&h, err, sizeof(int), cudaMemcpyDeviceToHost), "dem_capnet_infer");
-    cudaFree(err);
-    if (st == DEM_OK && h) st = fail(DEM_ERR_CUDA, "dem_capnet_infer: tensor-core completion not seen in time");
+    const int blocks = (int)std::min<long long>(tiles, (long long)std::max(1, sms) * kTcBlocks);
+    k_infer_tc5<<<blocks, kTcRows>>>(net->packed, x_dev, n, y_dev, net->gave_up);
+    st = ck(cudaGetLastError(), "dem_capnet_infer launch");
+    int h = 0; /* the copy waits for the kernel */
+    if (st == DEM_OK) st = ck(cudaMemcpy(&h, net->gave_up, sizeof(int), cudaMemcpyDeviceToHost), "dem_capnet_infer");
+    if (st == DEM_OK && h) {
+      cudaMemset(net->gave_up, 0, sizeof(int));
+      st = fail(DEM_ERR_CUDA, "dem_capnet_infer: tensor-core completion not seen in time");
+    }
     return st;
   } else if (tensor_cores) {
     dem_status st = ensure_packed(net);
@@ -894,7 +1099,14 @@ dem_status dem_capnet_infer(dem_capnet* net, const float* x_dev, long long n, in
     const int blocks = (int)std::min<long long>((tiles + 3) / 4, 152LL * 16);
     k_infer_tc<<<blocks, 128>>>(net->packed, x_dev, n, y_dev);
   } else {
-    k_infer32<<<blocks_for(n, 128), 128>>>(net->params, x_dev, n, norm_of(net), y_dev);
+    dem_status st = ensure_host_params(net);
+    if (st != DEM_OK) return st;
+    const CapParams& P = *reinterpret_cast<const CapParams*>(net->host_params);
+    /* few rows: a row a thread in four partial sums, for the latency of its
+     * chain (a call on 1,000 rows 35 us, two a thread 61); from 100,000 rows on
+     * two a thread (1M rows: 289 a call, one a thread 316) */
+    if (n < 100000) k_infer32<1, 4><<<blocks_for(n, kInferThreads), kInferThreads>>>(P, x_dev, n, norm_of(net), y_dev);
+    else k_infer32<2, 1><<<blocks_for(n, 2 * kInferThreads), kInferThreads>>>(P, x_dev, n, norm_of(net), y_dev);
   }
   dem_status st = ck(cudaGetLastError(), "dem_capnet_infer launch");
   if (st == DEM_OK) st = ck(cudaDeviceSynchronize(), "dem_capnet_infer");
@@ -1003,7 +1215,7 @@ dem_status dem_capnet_fit(dem_capnet* net, const float* x_dev, const float* y_de
     if (ep < 64) r.train_mse[ep] = nsteps ? (float)(ep_loss / (double)nsteps) : 0.f;
     r.epochs = ep + 1;
   }
-  net->packed_valid = false;
+  params_changed(net);
   /* validation: standardised MSE of the FP32 network, relative errors of the
    * BF16 tensor-core network against the formula's outputs */
   if (st == DEM_OK && n_val > 0) {
