@@ -30,7 +30,6 @@ namespace dem {
 
 namespace {
 
-constexpr int kRowBatch = 8; /* cell rows whose ranges the neighbour search reads at once */
 constexpr int kScanThreads = 256;
 constexpr int kScanPerThread = 8;
 constexpr int kScanTile = kScanThreads * kScanPerThread; /* cells per scan tile */
@@ -207,56 +206,91 @@ __global__ void k_cell_order(const int* __restrict__ sorted_hash, int* __restric
 /* NeighborFindG (kernel.cu:729-855).  sorted_src == NULL means the particle
  * arrays are themselves in sorted order.
  *
- * Optional prefilter (pre.hi != NULL, particle arrays in sorted order): pre.hi
- * holds (x, y, z, r) as the high floats of (coordinate + offset) with every
- * coordinate in one binade, so hi_i - hi_j is exact in FP32; the FP32 distance
- * from those differences is within pre.tol of the exact one.  A candidate
- * farther than pre.tol from the cut-off is decided in FP32; only the band
- * around it takes the reference's FP64 test, so the list is bit-identical to
- * the all-FP64 build while almost no FP64 square roots are taken.
+ * Optional prefilter (pre.hi != NULL): pre.hi holds (x, y, z, r) as the high
+ * floats of (coordinate + offset) with every coordinate in one binade, so
+ * hi_i - hi_j is exact in FP32; the FP32 distance from those differences is
+ * within pre.tol of the exact one.  A candidate farther than pre.tol from the
+ * cut-off is decided in FP32; only the band around it takes the reference's
+ * FP64 test, so the list is bit-identical to the all-FP64 build while almost no
+ * FP64 square roots are taken.  Likewise the particle's own cell and the reach
+ * in cells: an FP32 quotient farther than its error from an integer has the
+ * FP64 one's floor, the others take the FP64 division.
+ *
+ * With the prefilter and radii bounded by their level's (pre.prune), rows and
+ * row ends farther away than any partner of that level can touch are skipped:
+ * the reference searches a box of cells, rounded up from the ratio of the
+ * levels, of which the sphere that matters fills a quarter (a level-1 sphere
+ * has 88 candidates in the boxes of the packed bed's four levels).  What is
+ * skipped fails the distance test, so the list and its order stay.
  *
  * Optional cell_off (every cell's offset in sorted order, empty cells
  * included, and the total after the last): a row's particles are then
  * [cell_off[first cell], cell_off[last cell + 1]) -- the same range, in the
- * same order, from two loads instead of two per cell of the row.  The search
- * is bound by these scattered loads, not by its arithmetic. */
-__global__ void k_neighbor_find(const double3* __restrict__ pos, const double* __restrict__ rad,
-                                const int* __restrict__ sorted_src, const int* __restrict__ cell_start,
-                                const int* __restrict__ cell_end, const int* __restrict__ cell_off,
-                                const int* __restrict__ plevel,
-                                const int* __restrict__ nebor_idx, LevelView lv, double3 origin,
-                                double search_gap, int* __restrict__ nebor,
-                                int* __restrict__ num_nebor, int n, int* __restrict__ err, Prefilter pre) {
+ * same order, from two loads instead of two per cell of the row. */
+
+/* ceil(a / b) in cells, as the FP64 quotient gives it: from FP32 unless that
+ * quotient is within its error of an integer (an FP64 division is ten
+ * instructions of a pipe that takes 17 cycles each) */
+__device__ __forceinline__ int reach(double a, double b) {
+  if (a == b) return 1;
+  const float t = d2f(a) / d2f(b), f = floorf(t), tol = 4.0e-7f * t;
+  if (t - f > tol && f + 1.0f - t > tol) return (int)f + 1;
+  return (int)ceil(a / b);
+}
+
+/* the cell of x (cells of size 1 / rc, eps a margin in cells), clamped into the
+ * grid: its first and last cells hold what lies outside */
+__device__ __forceinline__ int near_cell(float x, float rc, float eps, int last) {
+  return max(0, min(__float2int_rd(fmaf(x, rc, eps)), last));
+}
+
+/* the hardware square root (a few ulp) */
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float r;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+/* distance from x to the cells [k, k + 1) of size cs, the first and last of a
+ * grid reaching outward without end (they hold what lies outside) */
+__device__ __forceinline__ float cell_gap(float x, int k, int last, float cs) {
+  const float lo = k <= 0 ? -3.0e38f : (float)k * cs, hi = k >= last ? 3.0e38f : (float)(k + 1) * cs;
+  return fmaxf(0.0f, fmaxf(lo - x, x - hi));
+}
+
+__global__ void __launch_bounds__(128) k_neighbor_find(
+    const double3* __restrict__ pos, const double* __restrict__ rad, const int* __restrict__ sorted_src,
+    const int* __restrict__ cell_start, const int* __restrict__ cell_end, const int* __restrict__ cell_off,
+    const int* __restrict__ plevel, const int* __restrict__ nebor_idx, LevelView lv, double3 origin,
+    double search_gap, int* __restrict__ nebor, int* __restrict__ num_nebor, int n, int* __restrict__ err,
+    Prefilter pre) {
   const int i = reversed_block_thread(); /* the largest spheres' long searches first */
   if (i >= n) return;
-  const double3 o = pos[i];
-  const double ri = rad[i];
   const float4 hi_i = pre.hi ? pre.hi[i] : make_float4(0.f, 0.f, 0.f, 0.f);
   const float sg = (float)search_gap;
   const int L = plevel[i];
   const long long base = slot_base(L, lv.level_npars, lv.level_nnebors) + nebor_idx[i];
   const long long stride = lv.level_npars[L];
   const int cap = lv.level_nnebors[L];
+  /* the position from the grid's origin, exactly hi - 2^k: within pre.ulp */
+  const float xf = hi_i.x - pre.base, yf = hi_i.y - pre.base, zf = hi_i.z - pre.base;
   int count = 0;
   bool over = false;
   /* candidate q (sorted position): the distance test, then the append */
   auto visit = [&](int q) {
     const int j = sorted_src ? sorted_src[q] : q;
-    if (j == i) return;
     bool in = false, decided = false;
     if (pre.hi) {
       const float4 hj = pre.hi[j];
       const float dx = hi_i.x - hj.x, dy = hi_i.y - hj.y, dz = hi_i.z - hj.z;
-      const float dc = sqrtf(dx * dx + dy * dy + dz * dz);
-      const float cut = (hj.w + hi_i.w) + sg;
-      if (dc > cut + pre.tol) decided = true; /* certainly outside */
-      else if (dc < cut - pre.tol) {          /* certainly inside */
-        decided = true;
-        in = true;
-      }
+      const float d2 = dx * dx + dy * dy + dz * dz;
+      /* squared: within 2e-7 of the squares' ratio, well inside pre.tol's allowance */
+      const float cut = (hj.w + hi_i.w) + sg, lo = cut - pre.tol, hi = cut + pre.tol;
+      in = lo > 0.f && d2 < lo * lo; /* certainly inside */
+      decided = in || d2 > hi * hi;  /* or outside */
     }
-    if (!decided) in = len3(sub3(o, pos[j])) < rad[j] + ri + search_gap;
-    if (!in) return;
+    if (!decided) in = len3(sub3(pos[i], pos[j])) < rad[j] + rad[i] + search_gap;
+    if (!in || j == i) return;
     if (count >= cap) {
       over = true;
       return;
@@ -265,60 +299,96 @@ __global__ void k_neighbor_find(const double3* __restrict__ pos, const double* _
     count++;
   };
   for (int iL = 0; iL < lv.n_levels; iL++) {
-    const int3 g = grid_pos(o, iL, lv, origin);
-    const int off = (int)ceil(lv.level_size[L] / lv.level_size[iL]);
-    const int cell_sum = iL != 0 ? lv.ncell_idx[iL - 1] : 0;
+    const double csd = lv.cell_size[iL];
+    const float cs = d2f(csd), rc = 1.0f / cs;
     const int3 gs = lv.grid_size[iL];
-    if (cell_off) {
-      /* rows r = (z + off) W + (y + off), in the reference's (z, y) order;
-       * the ranges of kRowBatch rows are read with independent loads before
-       * their particles are visited in order */
-      const int W = 2 * off + 1, R = W * W;
-      for (int r0 = 0; r0 < R; r0 += kRowBatch) {
-        int rf[kRowBatch], rl[kRowBatch];
-#pragma unroll
-        for (int b = 0; b < kRowBatch; b++) {
-          rf[b] = rl[b] = 0;
-          const int r = r0 + b;
-          const int z = r / W - off, y = r % W - off;
-          int3 s = make_int3(g.x - off, g.y + y, g.z + z);
-          int3 e = make_int3(g.x + off, g.y + y, g.z + z);
-          if (s.x < 0) s.x = 0;
-          if (e.x > gs.x - 1) e.x = gs.x - 1;
-          if (r < R && !(s.y < 0 || s.z < 0 || s.y > gs.y - 1 || s.z > gs.z - 1) && e.x >= s.x) {
-            const int row = grid_hash(s, iL, lv) + cell_sum;
-            rf[b] = __ldg(cell_off + row);
-            rl[b] = __ldg(cell_off + row + (e.x - s.x) + 1);
+    int3 g;
+    bool sure = false;
+    if (pre.hi) {
+      const float tx = xf * rc, ty = yf * rc, tz = zf * rc;
+      const float fx = floorf(tx), fy = floorf(ty), fz = floorf(tz);
+      const float ex = pre.ulp * rc;
+      const float ox = ex + 4.0e-7f * fabsf(tx), oy = ex + 4.0e-7f * fabsf(ty), oz = ex + 4.0e-7f * fabsf(tz);
+      sure = tx - fx > ox && fx + 1.0f - tx > ox && ty - fy > oy && fy + 1.0f - ty > oy && tz - fz > oz &&
+             fz + 1.0f - tz > oz;
+      g = make_int3(max(0, min((int)fx, gs.x)), max(0, min((int)fy, gs.y)), max(0, min((int)fz, gs.z)));
+    }
+    if (!sure) g = grid_pos(pos[i], iL, lv, origin);
+    const int off = reach(lv.level_size[L], lv.level_size[iL]);
+    const int cell_sum = iL != 0 ? lv.ncell_idx[iL - 1] : 0;
+    /* no partner of this level farther than this touches the cut-off: the
+     * radii's bounds and the gap, and a margin for FP32 (distances, cells) */
+    const float far = pre.prune ? (hi_i.w + d2f(lv.level_size[iL]) + sg) * 1.0001f + 8.0f * pre.ulp +
+                                      1.0e-6f * (fabsf(xf) + fabsf(yf) + fabsf(zf))
+                                : 0.f;
+    /* planes and rows in the reference's (z, y) order, from those that `far`
+     * reaches; the next row's range is in flight while the current one's
+     * particles are visited.  One copy of the loop's body: unrolled over a
+     * batch of rows it ran from beyond the instruction cache (3.8 of 11 stall
+     * cycles an instruction) */
+    int z = max(g.z - off, 0), z1 = min(g.z + off, gs.z - 1);
+    if (pre.prune) {
+      z = max(z, near_cell(zf - far, rc, -1.0e-4f, gs.z - 1));
+      z1 = min(z1, near_cell(zf + far, rc, 1.0e-4f, gs.z - 1));
+    }
+    int y = 0, y1 = -1; /* the rows left of the current plane */
+    float left_z = 0.f;
+    z--;
+    int f0 = 0, l0 = 0;
+    bool more = true;
+#pragma unroll 1
+    while (more || f0 < l0) {
+      int f1 = 0, l1 = 0;
+      if (more) {
+        if (y > y1) {
+          more = ++z <= z1;
+          y = max(g.y - off, 0);
+          y1 = min(g.y + off, gs.y - 1);
+          if (pre.prune && more) {
+            const float dz = cell_gap(zf, z, gs.z - 1, cs);
+            left_z = far * far - dz * dz;
+            const float ry = sqrt_approx(fmaxf(left_z, 0.f)) * 1.0001f + 4.0f * pre.ulp;
+            y = max(y, near_cell(yf - ry, rc, -1.0e-4f, gs.y - 1));
+            y1 = min(y1, near_cell(yf + ry, rc, 1.0e-4f, gs.y - 1));
           }
         }
-#pragma unroll
-        for (int b = 0; b < kRowBatch; b++)
-          for (int q = rf[b]; q < rl[b]; q++) visit(q);
-      }
-      continue;
-    }
-    for (int z = -off; z <= off; z++) {
-      for (int y = -off; y <= off; y++) {
-        int3 s = make_int3(g.x - off, g.y + y, g.z + z);
-        int3 e = make_int3(g.x + off, g.y + y, g.z + z);
-        if (s.x < 0) s.x = 0;
-        if (e.x > gs.x - 1) e.x = gs.x - 1;
-        if (s.y < 0 || s.z < 0 || s.y > gs.y - 1 || s.z > gs.z - 1) continue;
-        /* the row's particles: from the start of its first non-empty cell to
-         * the end of its last one (cells of a row are consecutive in sorted
-         * order).  The reference walks in from both ends one dependent load
-         * at a time (kernel.cu:775-790); every cell's range is read here
-         * with independent loads -- the same range, the same append order. */
-        int first = -1, last = -1;
-        const int row = grid_hash(s, iL, lv) + cell_sum;
-        for (int x = 0; x <= e.x - s.x; x++) {
-          const int cs = __ldg(cell_start + row + x), ce = __ldg(cell_end + row + x);
-          if (first == -1) first = cs;
-          if (ce != -1) last = ce;
+        if (more && y <= y1) {
+          int x = max(g.x - off, 0), x1 = min(g.x + off, gs.x - 1);
+          if (pre.prune) {
+            const float dy = cell_gap(yf, y, gs.y - 1, cs);
+            const float rx = sqrt_approx(fmaxf(left_z - dy * dy, 0.f)) * 1.0001f + 4.0f * pre.ulp;
+            x = max(x, near_cell(xf - rx, rc, -1.0e-4f, gs.x - 1));
+            x1 = min(x1, near_cell(xf + rx, rc, 1.0e-4f, gs.x - 1));
+          }
+          if (x <= x1) {
+            const int row = (z * gs.y + y) * gs.x + x + cell_sum;
+            if (cell_off) {
+              f1 = __ldg(cell_off + row);
+              l1 = __ldg(cell_off + row + (x1 - x) + 1);
+            } else {
+              /* the row's particles: from the start of its first non-empty
+               * cell to the end of its last one (cells of a row are
+               * consecutive in sorted order; the reference walks in from both
+               * ends, kernel.cu:775-790) */
+              int first = -1, last = -1;
+              for (int k = 0; k <= x1 - x; k++) {
+                const int c0 = __ldg(cell_start + row + k), c1 = __ldg(cell_end + row + k);
+                if (first == -1) first = c0;
+                if (c1 != -1) last = c1;
+              }
+              if (first != -1 && last != -1) {
+                f1 = first;
+                l1 = last;
+              }
+            }
+          }
+          y++;
         }
-        if (first == -1 || last == -1) continue;
-        for (int q = first; q < last; q++) visit(q);
       }
+#pragma unroll 1
+      for (int q = f0; q < l0; q++) visit(q);
+      f0 = f1;
+      l0 = l1;
     }
   }
   num_nebor[i] = count;

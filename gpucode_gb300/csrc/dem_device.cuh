@@ -55,6 +55,29 @@ __device__ __forceinline__ int reversed_block_thread() {
   return (int)((gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x);
 }
 
+/* ---- FP32 <-> FP64 through the integer pipe ----
+ * On GB300 FP64 conversions issue on the scarce FP64 pipe; these move the bits
+ * with integer operations instead.  d2f truncates the mantissa (error below one
+ * FP32 ulp) and flushes results below the FP32 normal range to zero; f2d is
+ * exact for normal floats.  Infinities and NaNs stay non-finite. */
+__device__ __forceinline__ float d2f(double x) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+  const unsigned sign = (unsigned)(u >> 32) & 0x80000000u;
+  const int e = (int)((u >> 52) & 0x7ff);
+  const int fe = e - 1023 + 127;
+  if (fe <= 0) return __uint_as_float(sign);
+  if (fe >= 255) return __uint_as_float(sign | 0x7f800000u | (e == 0x7ff && (u & 0xfffffffffffffull) ? 1u : 0u));
+  return __uint_as_float(sign | ((unsigned)fe << 23) | (unsigned)((u >> 29) & 0x7fffffu));
+}
+__device__ __forceinline__ double f2d(float f) {
+  const unsigned b = __float_as_uint(f);
+  const unsigned e = (b >> 23) & 0xffu;
+  const unsigned long long sign = (unsigned long long)(b & 0x80000000u) << 32;
+  if (e == 0) return __longlong_as_double((long long)sign);
+  const unsigned long long de = (e == 255) ? 0x7ffull : (unsigned long long)(e - 127 + 1023);
+  return __longlong_as_double((long long)(sign | (de << 52) | ((unsigned long long)(b & 0x7fffffu) << 29)));
+}
+
 /* ---- cell hash (kernel.cu:617-641) ---- */
 __device__ __forceinline__ int3 grid_pos(double3 p, int lvl, const LevelView& lv, double3 origin) {
   const double cs = lv.cell_size[lvl];

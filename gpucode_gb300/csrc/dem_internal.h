@@ -114,10 +114,14 @@ dem_status cell_sort(const double3* pos, const int* plevel, const int* order_key
                      cudaStream_t stream, int* cell_off = nullptr);
 
 /* FP32 prefilter of the neighbour test (see build.cu): the high floats of
- * (position + offset, radius) and the bound of their distance error */
+ * (position + offset, radius), the bound of their distance error, the value of
+ * the offset coordinate at the origin (a power of two) and the bound of a high
+ * float's own error; prune: every radius is at most its level's */
 struct Prefilter {
   const float4* hi;
   float tol;
+  float base, ulp;
+  int prune;
 };
 
 /* NeighborFindG semantics (kernel.cu:729-855) on AoS positions; sorted_src
@@ -128,7 +132,7 @@ dem_status neighbor_find(const double3* pos, const double* rad, const int* sorte
                          const int* cell_start, const int* cell_end, const int* plevel,
                          const int* nebor_idx, LevelView lv, const DevConsts& k, int* nebor,
                          int* num_nebor, int n, int* err, cudaStream_t stream,
-                         Prefilter pre = Prefilter{nullptr, 0.f}, const int* cell_off = nullptr);
+                         Prefilter pre = Prefilter{nullptr, 0.f, 0.f, 0.f, 0}, const int* cell_off = nullptr);
 
 /* CirWallListG (kernel.cu:1034-1073); wall list pitched rows.  Batched
  * systems: sys_of_id[id[i]] selects particle i's cylinder in cyl[] (NULL: cyl[0]). */

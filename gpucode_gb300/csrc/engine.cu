@@ -322,7 +322,7 @@ dem_status enqueue_rebuild(dem_ctx* c, cudaStream_t s, int parity) {
     cudaError_t e = cudaMemsetAsync(b.pmove, 0, sizeof(double) * (size_t)n, s);
     if (e != cudaSuccess) return cuda_check(e, "pmove reset");
   }
-  Prefilter pre{nullptr, 0.f};
+  Prefilter pre{nullptr, 0.f, 0.f, 0.f, 0};
   if (c->opt.precision == DEM_PREC_MIXED) {
     /* the permuted state's shadows: read by the next step and by the build's prefilter */
     st = mixed_shadows(c, parity, s);
@@ -689,6 +689,9 @@ extern "C" dem_status dem_create(const dem_setup* s, const double* rad, const in
   c->graph_exec[0] = c->graph_exec[1] = nullptr;
   c->graph_one[0] = c->graph_one[1] = nullptr;
   c->moving_walls = s->cyl.topv != 0.0 ? 1 : 0;
+  c->radii_bounded = 1;
+  for (int i = 0; i < s->np && c->radii_bounded; i++)
+    c->radii_bounded = plevel[i] >= 0 && plevel[i] < s->n_levels && rad[i] <= s->level_size[plevel[i]] * 1.00001;
   c->marks = nullptr;
   c->parity = 0;
   c->cap_w = nullptr;

@@ -109,6 +109,7 @@ struct dem_ctx {
   cudaGraphExec_t graph_exec[2];
   cudaGraphExec_t graph_one[2];
   int parity; /* mixed: which shadow buffer the next step reads */
+  int radii_bounded; /* every radius is at most its level's size: the neighbour search may skip far rows */
   int moving_walls; /* a cylinder's top wall moves (topv != 0): moved before every step's wall contacts */
   /* device-side step chaining (mixed precision): 0 not built yet, 1 built,
    * -1 unavailable (the conditional-node graphs run instead); the graphs

@@ -60,6 +60,7 @@ struct MixedState {
   double3 off;
   float coarse_tol;
   int bin_exp;    /* FP64 biased exponent of the binade [2^k, 2^(k+1)) */
+  float base;     /* 2^k: the offset coordinate of the domain's origin */
   float lo_scale; /* 2^(k-52): the weight of the last significand bit */
 };
 
@@ -186,29 +187,6 @@ __device__ __forceinline__ float exact_gap(float4 hi, float4 lo, float4 hj, floa
   const float inv = __frcp_rn(dist);
   u = make_float3(dx * inv, dy * inv, dz * inv);
   return __fdividef(D, dist + (Sh + Sl));
-}
-
-/* ---- FP32 <-> FP64 through the integer pipe ----
- * On GB300 FP64 conversions issue on the scarce FP64 pipe; these move the bits
- * with integer operations instead.  d2f truncates the mantissa (error below one
- * FP32 ulp) and flushes results below the FP32 normal range to zero; f2d is
- * exact for normal floats.  Infinities and NaNs stay non-finite. */
-__device__ __forceinline__ float d2f(double x) {
-  const unsigned long long u = (unsigned long long)__double_as_longlong(x);
-  const unsigned sign = (unsigned)(u >> 32) & 0x80000000u;
-  const int e = (int)((u >> 52) & 0x7ff);
-  const int fe = e - 1023 + 127;
-  if (fe <= 0) return __uint_as_float(sign);
-  if (fe >= 255) return __uint_as_float(sign | 0x7f800000u | (e == 0x7ff && (u & 0xfffffffffffffull) ? 1u : 0u));
-  return __uint_as_float(sign | ((unsigned)fe << 23) | (unsigned)((u >> 29) & 0x7fffffu));
-}
-__device__ __forceinline__ double f2d(float f) {
-  const unsigned b = __float_as_uint(f);
-  const unsigned e = (b >> 23) & 0xffu;
-  const unsigned long long sign = (unsigned long long)(b & 0x80000000u) << 32;
-  if (e == 0) return __longlong_as_double((long long)sign);
-  const unsigned long long de = (e == 255) ? 0x7ffull : (unsigned long long)(e - 127 + 1023);
-  return __longlong_as_double((long long)(sign | (de << 52) | ((unsigned long long)(b & 0x7fffffu) << 29)));
 }
 
 /* the elasto-plastic normal law, damping and tangential spring of
@@ -1455,6 +1433,7 @@ dem_status mixed_create(dem_ctx* c) {
    * axis, below two ulps of the binade: four ulps is a safe candidate margin */
   m->coarse_tol = (float)(4.0 * std::ldexp(1.0, k2 - 23));
   m->bin_exp = 1023 + k2;
+  m->base = (float)base;
   m->lo_scale = (float)std::ldexp(1.0, k2 - 52);
   return DEM_OK;
 }
@@ -1506,7 +1485,8 @@ Prefilter mixed_prefilter(dem_ctx* c, int which) {
   /* |(hi_i - hi_j) - (x_i - x_j)| <= one binade ulp per axis (the lo parts are
    * below half an ulp each): sqrt(3) ulps, plus FP32 rounding of the distance
    * and of the cut-off (~3e-7 relative, distances < 4 reduced units) */
-  return Prefilter{c->mx->phi[which], 0.5f * c->mx->coarse_tol + 2.0e-6f};
+  return Prefilter{c->mx->phi[which], 0.5f * c->mx->coarse_tol + 2.0e-6f, c->mx->base, 0.25f * c->mx->coarse_tol,
+                   c->radii_bounded};
 }
 
 const char* mixed_step_kernel_name(const dem_ctx* c) {
