@@ -121,3 +121,44 @@ def test_lists_and_forces_at_block_edges(cuda, n):
     assert np.abs(a[2] - b[2]).max() <= 2e-5 * np.abs(a[2]).max()
     for k in ("nb_entries", "contacts", "bridges", "wall_contacts"):
         assert a[3][k] == b[3][k], k
+
+
+@pytest.mark.parametrize("levels, spread", [(1, 1.0), (4, 1.0), (4, 6.0), (3, 0.3)])
+@pytest.mark.parametrize("bounded", [True, False])
+def test_pruned_search_lists_what_the_full_search_lists(cuda, levels, spread, bounded):
+    """The mixed engine's neighbour search skips cells no partner can reach from
+    (when every radius is within its level's); the FP64 engine searches the
+    reference's boxes.  The same lists, entry for entry, for spheres strewn
+    through the whole computing zone and beyond its faces, equal sizes to a
+    ratio of 12, and with radii above their level's (which turn the skipping
+    off)."""
+    from gpucode_gb300 import configs
+
+    rng = np.random.default_rng(levels + int(10 * spread))
+    n = 3000
+    dia = 0.25e-3 * np.exp(np.minimum(spread, 2.5) * rng.random(n)) if levels > 1 else np.full(n, 1e-3)
+    real = float(dia.max())
+    inp = configs.make_input(n, levels, real, 0.1 * dia.max() / dia.min(), 4e-3, 8e-3, configs.RHO, configs.E_YOUNG,
+                             configs.NU, configs.MU, 6.6e-6, configs.yldp_for_yield_overlap(0.01, 1e7, 0.3), 0,
+                             dt=1e-9)
+    setup = configs.Setup.build(inp, dia)
+    s = setup.s
+    if not bounded:
+        # (the slots' counts stay the level's: a sphere too large for its level)
+        big = np.flatnonzero(setup.rad > 0.9 * np.array(list(s.level_size))[setup.plevel])[::7]
+        setup.rad[big] = np.array(list(s.level_size))[setup.plevel[big]] * 1.2
+    lo = np.array([s.prm.Origin.x, s.prm.Origin.y, s.prm.Origin.z])
+    hi = np.array([s.prm.EndPoint.x, s.prm.EndPoint.y, s.prm.EndPoint.z])
+    pos = lo + (hi - lo) * rng.random((n, 3))
+    pos[::50] = lo - 0.4 * rng.random((len(pos[::50]), 3))  # outside: kept in the first cells
+    got = []
+    for precision in ("fp64", "mixed"):
+        e = Engine(setup, precision=precision)
+        e.set_state(pos)
+        e.step(1)
+        c, p = e.neighbors(1024)
+        got.append((c, p))
+        e.close()
+    np.testing.assert_array_equal(got[0][0], got[1][0])
+    np.testing.assert_array_equal(got[0][1], got[1][1])
+    assert got[0][0].sum() > n // 4
