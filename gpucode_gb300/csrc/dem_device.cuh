@@ -12,6 +12,7 @@
 
 #include "dem_internal.h"
 #include "liquid.cuh"
+#include "pairs.cuh"
 
 namespace dem {
 
@@ -111,6 +112,7 @@ struct HistRec {
 /* history access, reference SoA layout */
 struct HistSoAAcc {
   HistSoA h;
+  __device__ __forceinline__ long long at(long long slot) const { return slot; } /* a slot's record */
   __device__ __forceinline__ HistRec load(long long i) const {
     HistRec r;
     r.dispt = h.dispt[i];
@@ -163,15 +165,39 @@ struct HistAoSAcc {
   }
 };
 
-/* Differences between the p-p law (ContactForceD, kernel.cu:89-228) and the
- * wall law (PWcontactD, kernel.cu:236-359). */
-struct LawCfg64 {
-  const calParaPP* cal;
-  bool hertz_le;   /* p-p: nrm <= ydsp*R; wall: nrm < ydsp*R */
-  double rot_eps;  /* 1e-7 (p-p) / 1e-10 (wall): spring rotation guard */
-  double dsmx_eps; /* 1e-7 (p-p) / 1e-10 (wall): slip-ratio and rescale guard */
-  bool damp_on;    /* p-p: stage == 1; wall: stage == 1 || 7 */
-  double dmp;      /* sqrt of the dmpn product (the reference takes it per contact) */
+/* history access, the engine's pair list with a record and a flag a side */
+struct HistPairAcc {
+  PairSet ps;
+  __device__ __forceinline__ HistAoSAcc set() const {
+    return pair_ctl(ps).x ? HistAoSAcc{ps.rec[1], ps.brg[1]} : HistAoSAcc{ps.rec[0], ps.brg[0]};
+  }
+  __device__ __forceinline__ long long at(long long slot) const {
+    const int e = ps.eidx[slot];
+    return e == kNoPair ? -1 : e < 0 ? 2LL * ~e + 1 : 2LL * e;
+  }
+  __device__ __forceinline__ HistRec load(long long i) const { return set().load(i); }
+  __device__ __forceinline__ void store(long long i, const HistRec& r) const { set().store(i, r); }
+  __device__ __forceinline__ int brg(long long i) const { return set().brg(i); }
+  __device__ __forceinline__ void set_brg(long long i, int v) const { set().set_brg(i, v); }
+};
+
+/* The constants of the p-p law (ContactForceD, kernel.cu:89-228) or the wall law
+ * (PWcontactD, kernel.cu:236-359): products and quotients of the material alone,
+ * taken once on the host by the same operations in the same order (IEEE, so the
+ * same values), not by every thread -- a root, two divisions and a dozen
+ * products of some 350 FP64 instructions a contact. */
+struct LawK64 {
+  double k43;             /* 4/3 E* */
+  double ydsp_t, yforce_t, ystiff_t;
+  double damp;            /* -2 sqrt(dmpn product) E* */
+  double sfrc3, nsfrc;    /* 3 mu, -mu */
+  double kt;              /* 16 (1 - nu) E* / (4 - 2 nu) */
+  double roll;            /* 0.5 (rfrc + rfrc) */
+  double dt;
+  double film;            /* 2 x the liquid layer */
+  double eps;             /* spring rotation, slip-ratio and rescale guard: 1e-7 (p-p) / 1e-10 (wall) */
+  int hertz_le;           /* p-p: nrm <= ydsp*R; wall: nrm < ydsp*R */
+  int damp_on;            /* p-p: stage == 1; wall: stage == 1 || 7 */
 };
 
 /* elasto-plastic Hertz normal force + damping + tangential spring with slip
@@ -184,10 +210,8 @@ struct LawCfg64 {
  * The exponent 2/3 (plastic loading only) stays pow.  On
  * GB300 the law is bound by FP64 issue, where each pow is some tens of FP64
  * instructions. */
-__device__ __forceinline__ void contact_law64(const LawCfg64& c, double ijRad, double nrm, double3 u,
-                                              double3 cpv, HistRec& h, double iRad, double rfrc,
-                                              double dt, double3& dF, double3& dM, double& dR) {
-  const calParaPP& cal = *c.cal;
+__device__ __forceinline__ void contact_law64(const LawK64& c, double ijRad, double nrm, double3 u, double3 cpv,
+                                              HistRec& h, double iRad, double3& dF, double3& dM, double& dR) {
   /* pow(ijRad * nrm, 0.5) (twice in the reference's law) and the damping's
    * sqrt(ijRad * nrm): one value */
   const double sq = sqrt(ijRad * nrm);
@@ -201,56 +225,55 @@ __device__ __forceinline__ void contact_law64(const LawCfg64& c, double ijRad, d
   if (st == 1) {
     fN = 0.0;
   } else if (st == 2) {
-    bool elastic = c.hertz_le ? (nrm <= cal.ydsp_t * ijRad) : (nrm < (cal.ydsp_t * ijRad));
+    bool elastic = c.hertz_le ? (nrm <= c.ydsp_t * ijRad) : (nrm < (c.ydsp_t * ijRad));
     if (elastic) {
-      fN = 4.0 / 3.0 * cal.emod * sq * nrm;
+      fN = c.k43 * sq * nrm;
       h.plstRad = ijRad;
       h.plstDfm = 0.0;
     } else {
-      fN = cal.yforce_t * (ijRad * ijRad) + cal.ystiff_t * ijRad * (nrm - cal.ydsp_t * ijRad);
-      h.plstRad = ijRad * (4.0 / 3.0 * cal.emod * sq * nrm) / fN;
-      h.plstDfm = nrm - pow((fN / (4.0 / 3.0 * cal.emod * sqrt(ijRad))), 2.0 / 3.0);
+      fN = c.yforce_t * (ijRad * ijRad) + c.ystiff_t * ijRad * (nrm - c.ydsp_t * ijRad);
+      h.plstRad = ijRad * (c.k43 * sq * nrm) / fN;
+      h.plstDfm = nrm - pow((fN / (c.k43 * sqrt(ijRad))), 2.0 / 3.0);
     }
     h.nDsp_mx = nrm;
   } else {
-    fN = 4.0 / 3.0 * cal.emod * sqrt(h.plstRad) * pow1_5(nrm - h.plstDfm);
+    fN = c.k43 * sqrt(h.plstRad) * pow1_5(nrm - h.plstDfm);
   }
   h.nDsp = nrm;
 
   const double vn = dot3(cpv, u);
   double fD = 0.0;
-  if (c.damp_on) fD = -2.0 * c.dmp * cal.emod * sq * vn;
+  if (c.damp_on) fD = c.damp * sq * vn;
 
   const double3 vt = sub3(cpv, smul3(vn, u));
   const double3 old = h.dispt;
   double3 dT = cross3(smul3(-1.0, u), cross3(u, old));
-  if (len3(dT) > c.rot_eps)
-    dT = add3(div3(mul3(dT, len3(old)), len3(dT)), mul3(vt, dt));
+  if (len3(dT) > c.eps)
+    dT = add3(div3(mul3(dT, len3(old)), len3(dT)), mul3(vt, c.dt));
   else
-    dT = add3(dT, mul3(vt, dt));
+    dT = add3(dT, mul3(vt, c.dt));
 
-  const double dsmx = 3.0 * cal.sfrc * fN /
-                      (16.0 * (1 - cal.pois) * cal.emod / (4.0 - 2.0 * cal.pois) * sq);
+  const double dsmx = c.sfrc3 * fN / (c.kt * sq);
   double ratio = 1.0;
   if (len3(dT) < dsmx) {
-    if (dsmx > c.dsmx_eps) ratio = 1.0 - pow1_5(1.0 - len3(dT) / dsmx);
+    if (dsmx > c.eps) ratio = 1.0 - pow1_5(1.0 - len3(dT) / dsmx);
   } else {
     ratio = 1.0;
-    if (len3(dT) > c.dsmx_eps) dT = div3(smul3(dsmx, dT), len3(dT));
+    if (len3(dT) > c.eps) dT = div3(smul3(dsmx, dT), len3(dT));
     else dT = smul3(dsmx, dT);
   }
   h.dispt = dT;
 
   double3 fT = d3(0.0, 0.0, 0.0);
   if (len3(dT) < dsmx) {
-    if (len3(dT) > 1.0e-10) fT = div3(smul3(-1.0 * cal.sfrc * fN * ratio, dT), len3(dT));
+    if (len3(dT) > 1.0e-10) fT = div3(smul3(c.nsfrc * fN * ratio, dT), len3(dT));
   } else {
-    if (len3(vt) > 1.0e-10) fT = div3(smul3(-1.0 * cal.sfrc * fN * ratio, vt), len3(vt));
+    if (len3(vt) > 1.0e-10) fT = div3(smul3(c.nsfrc * fN * ratio, vt), len3(vt));
   }
   dF = add3(smul3(fN + fD, u), fT);
   const double arm = iRad - nrm / 2.0;
   dM = cross3(smul3(-arm, u), fT);
-  dR = 0.5 * (rfrc + rfrc) * fN * iRad;
+  dR = c.roll * fN * iRad;
 }
 
 /* capillary bridge force, kernel.cu:65-81 (the closed-form fit of Willett et

@@ -368,9 +368,9 @@ dem_status enqueue_step(dem_ctx* c, cudaStream_t s, int parity) {
   dem_status st = var_init(b.force, b.mom, b.rmom, b.lqd, b.lqd_old, n, s);
   if (st != DEM_OK) return st;
   /* the export staging is idle during a step: it holds the spheres' liquid shares */
-  st = pair_force64(b.ps, b.pair_out, b.pos, b.vel, b.angv, b.rad, b.plevel, b.npars, b.nneb, b.nidx, b.num_nebor,
-                    b.lqd, b.lqd_old, b.force, b.mom, b.rmom, n, c->s.force_cap, c->s.load_stage, c->k, b.counters,
-                    reinterpret_cast<double*>(b.tmp_out), s, b.id, c->lm);
+  st = pp_force64<PairSet>(b.pos, b.vel, b.angv, b.rad, b.nebor, b.plevel, b.npars, b.nneb, b.nidx, b.ps,
+                           b.num_nebor, b.lqd, b.lqd_old, b.force, b.mom, b.rmom, n, c->s.force_cap,
+                           c->s.load_stage, c->k, b.counters, reinterpret_cast<double*>(b.tmp_out), s, b.id, c->lm);
   if (st != DEM_OK) return st;
   st = wall_force64<HistAoS>(b.pos, b.vel, b.angv, b.force, b.mom, b.rmom, b.rad, b.cyl, hist_pw(c), b.nwall,
                              b.wlist, 3 * sizeof(int), n, n, c->s.load_stage, c->k, b.counters,
@@ -589,9 +589,9 @@ dem_memory memory_of(long long N, long long S, long long C, const dem_options* o
   /* the list entry and the slot's pair index (8), and for half a pair a slot two
    * sets of pair (16), record (128) and bridge flag (2), and the pair's result
    * (48): 105 in mixed precision, where 138 covers the wall results and the
-   * reserve of unmirrored pairs too; FP64 has a record and flag a side, and 160
-   * bytes of result */
-  m.per_slot = o && o->precision == DEM_PREC_MIXED ? 138 : 240;
+   * reserve of unmirrored pairs too; FP64 has a record and flag a side and no
+   * result: 146, and the reserve */
+  m.per_slot = o && o->precision == DEM_PREC_MIXED ? 138 : 152;
   m.per_cell = 3 * 4;                         /* cell start, end, offset */
   m.slots = S;
   const long long allocations = 64;
@@ -748,7 +748,7 @@ extern "C" dem_status dem_create(const dem_setup* s, const double* rad, const in
   }
   A(b.ps.eidx, S); A(b.ps.ctl, 8);
   char* pair_out = nullptr;
-  A(pair_out, P * (c->opt.precision == DEM_PREC_MIXED ? kPairOut32 : kPairOut64));
+  if (c->opt.precision == DEM_PREC_MIXED) A(pair_out, P * kPairOut32);
   b.pair_out = pair_out;
   A(b.sorted_hash, N); A(b.sorted_src, N); A(b.old_to_new, N); A(b.cell_start, C); A(b.cell_end, C);
   A(b.cell_off, C + 1);

@@ -13,8 +13,8 @@ namespace dem {
 /* a slot without a pair: the pair arrays were full (reported as an overflow) */
 constexpr int kNoPair = (int)0x80000000;
 
-/* bytes of one pair's result in a step: mixed (mixed.cu) and FP64 (step64.cu) */
-constexpr size_t kPairOut32 = 48, kPairOut64 = 160;
+/* bytes of one pair's result in a mixed step (mixed.cu) */
+constexpr size_t kPairOut32 = 48;
 
 /* The pair arrays (device pointers), twice: ctl[0] is the current set,
  * ctl[1 + set] the number of pairs in it; ctl[3] counts the wall slots in use
@@ -61,15 +61,6 @@ dem_status pair_build(const PairSet& ps, const NeborLists& nl, int n, int* cnt, 
 dem_status pair_carry(const PairSet& ps, const NeborLists& nl, int n, const int* src, int* err, cudaStream_t s);
 /* make it the current set */
 dem_status pair_flip(const PairSet& ps, cudaStream_t s);
-
-/* PPForceCalcG (kernel.cu:413-552) over the pair list in FP64 (step64.cu):
- * adds to force, mom, rmom and lqd; out: kPairOut64 bytes per pair */
-dem_status pair_force64(const PairSet& ps, void* out, const double3* pos, const double3* vel, const double3* angvel,
-                        const double* rad, const int* plevel, const int* level_npars, const int* level_nnebors,
-                        const int* nebor_idx, const int* num_nebor, int* lqd, const int* lqd_old, double3* force,
-                        double3* mom, double* rmom, int n, int force_cap, int stage, const DevConsts& k,
-                        unsigned long long* counters, double* pvol, cudaStream_t stream, const int* id,
-                        LiquidModel lm);
 
 /* out[set][i] = sum of in[0 .. i) for i <= n, set = the one that is not
  * current (build.cu); scratch: a scan tile's total per 2048 entries */

@@ -100,7 +100,7 @@ def test_an_entry_without_mirror_image_acts_on_its_own_sphere(cuda, precision):
     assert np.abs(f - want)[free].max() <= tol * scale
 
 
-@pytest.mark.parametrize("n", [1, 2, 31, 33, 127, 128, 129, 255, 257])
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 127, 128, 129, 255, 256, 257, 511, 513])
 def test_lists_and_forces_at_block_edges(cuda, n):
     """the mixed engine against the FP64 one at sizes around the kernels' warps
     and blocks: the same lists, forces to the FP32 law's tolerance"""
@@ -162,3 +162,28 @@ def test_pruned_search_lists_what_the_full_search_lists(cuda, levels, spread, bo
     np.testing.assert_array_equal(got[0][0], got[1][0])
     np.testing.assert_array_equal(got[0][1], got[1][1])
     assert got[0][0].sum() > n // 4
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_longer_lists_change_no_force(cuda, precision):
+    """A wider skin lists several times the partners (a warp's entries then fill
+    several of the FP64 kernel's chunks) but, on the same cells, the same
+    contacts in the same order: a dry bed's forces keep their bits"""
+    from gpucode_gb300 import configs
+
+    w = _workloads.small_dry()
+    pos, vel, ang = _workloads.stirred(w, vscale=0.05, wscale=0.1)
+    got = []
+    w.inp.cut_gap = 1.5
+    for skin in (0.1, 0.6, 1.5):
+        setup = configs.Setup.build(w.inp, w.dia)
+        setup.s.prm.SearchGap = skin
+        e = Engine(setup, precision=precision)
+        e.set_state(pos, vel, ang)
+        e.step(1)
+        e.sync()
+        got.append((int(e.neighbors(512)[0].sum()), e.get_state()["force"]))
+        e.close()
+    assert got[2][0] * 32 / w.setup.n > 2 * 320 > got[0][0] * 32 / w.setup.n
+    for _, f in got[1:]:
+        np.testing.assert_array_equal(f, got[0][1])
