@@ -45,6 +45,7 @@ struct CompatDevice {
   int* err = nullptr;
 };
 CompatDevice g_dev;
+std::mutex g_scratch; /* held from a wrapper's first launch on the scratch to its last */
 
 /* the arithmetic of PpInterCalc / CirPWCalc / UpdateSystem: DEM_PREC_FP64 (the
  * reference's) unless DEM_COMPAT_PRECISION=mixed is set in the environment or
@@ -75,6 +76,20 @@ void* ensure_scratch(size_t bytes) {
     g_dev.scratch_bytes = bytes;
   }
   return g_dev.scratch;
+}
+
+/* scratch that a kernel can do without: NULL where the device has no room */
+void* optional_scratch(size_t bytes) {
+  if (bytes <= g_dev.scratch_bytes) return g_dev.scratch;
+  void* p = nullptr;
+  if (cudaMalloc(&p, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (g_dev.scratch) DEM_REF_CHECK(cudaFree(g_dev.scratch));
+  g_dev.scratch = p;
+  g_dev.scratch_bytes = bytes;
+  return p;
 }
 
 dem::HistSoA soa(const PPCONTACT_HISTORY& h) {
@@ -293,6 +308,7 @@ void BldNeborList(int* hash, int* index, int* cellStart, int* cellEnd, int* d_pL
                   int TotalParticle, double* rad) {
   ensure_small();
   dem::LevelView lv = view(d_cell, d_Ncell_Idx, d_Level_size, d_level_nPars, d_level_nNebors, nLevels);
+  std::lock_guard<std::mutex> lock(g_scratch);
   void* scratch = ensure_scratch(dem::sort_scratch_bytes(TotalParticle, Sys_nCells));
   ok_or_exit(dem::cell_sort(pos, d_pLevel, nullptr, TotalParticle, lv, g_consts, Sys_nCells, hash, index,
                             cellStart, cellEnd, scratch, g_dev.err, 0));
@@ -326,10 +342,12 @@ void PpInterCalc(double3* pos, double3* vel, double3* angvel, double* rad, int* 
                  int* d_Num_Nebor, int* d_lqdCnt, int* d_lqdCnt_Old, double3* force, double3* mom, double* rmom,
                  int TotalParticle, int NP, int ForceCap, int stage) {
   (void)NP;
+  std::lock_guard<std::mutex> lock(g_scratch);
   if (compat_precision() == DEM_PREC_MIXED) {
+    void* bodies = optional_scratch(dem::ref_mixed_scratch(TotalParticle));
     ok_or_exit(dem::pp_force_ref_mixed(pos, vel, angvel, rad, d_Nebor1, d_pLevel, d_level_nPars, d_level_nNebors,
                                        d_Nebor_Idx, soa(h), d_Num_Nebor, d_lqdCnt, d_lqdCnt_Old, force, mom, rmom,
-                                       TotalParticle, ForceCap, stage, g_consts, 0));
+                                       TotalParticle, ForceCap, stage, g_consts, bodies, 0));
     return;
   }
   /* the spheres' liquid shares go to the library's scratch (the neighbour

@@ -194,7 +194,10 @@ dem_status pp_force_ref_mixed(const double3* pos, const double3* vel, const doub
                               const int* nebor, const int* plevel, const int* level_npars, const int* level_nnebors,
                               const int* nebor_idx, HistSoA h, const int* num_nebor, int* lqd, const int* lqd_old,
                               double3* force, double3* mom, double* rmom, int n, int force_cap, int stage,
-                              const DevConsts& k, cudaStream_t s);
+                              const DevConsts& k, void* bodies, cudaStream_t s);
+/* device scratch `bodies` of ref_mixed_scratch(n) bytes: the spheres packed as
+ * their partners read them (NULL: read from the arrays, slower) */
+size_t ref_mixed_scratch(int n);
 dem_status wall_force_ref_mixed(const double3* pos, const double3* vel, const double3* angvel, double3* force,
                                 double3* mom, double* rmom, const double* rad, CylinderBC* cyl, HistSoA h,
                                 const int* nwall, const int* wlist, size_t pitch, int n, int NP, int stage,

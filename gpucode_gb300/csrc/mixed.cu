@@ -1171,157 +1171,310 @@ __device__ __forceinline__ double3 add_sum(double3 v, const KSum3& s) {
   return make_double3(v.x + f2d(s.x.s - s.x.c), v.y + f2d(s.y.s - s.y.c), v.z + f2d(s.z.s - s.z.c));
 }
 
-/* 6 resident blocks (80 registers, a few bytes of spills) measured 15 % faster
- * on the packed 200k bed than 5 (98 registers, no spills); 8 no better */
-#ifndef DEM_REF_MIXED_BLOCKS
-#define DEM_REF_MIXED_BLOCKS 6
-#endif
+/* A sphere as its partners read it: position and radius in one 32-byte sector,
+ * velocity, spin (FP32) and bridge count in the next, where the caller's five
+ * arrays are seven sectors a partner */
+struct __align__(32) RefBody {
+  double x, y, z, r;
+  float vx, vy, vz, wx;
+  float wy, wz;
+  int nl, pad;
+};
+static_assert(sizeof(RefBody) == 64, "two sectors a sphere");
+constexpr size_t kRefBody = sizeof(RefBody);
 
-__global__ void __launch_bounds__(128, DEM_REF_MIXED_BLOCKS) k_pp_ref_mixed(MixArgs a, RefArrays r) {
+__device__ __forceinline__ RefBody ref_body(const RefArrays& r, int i, bool wet) {
+  const double3 p = r.pos[i], v = r.vel[i], w = r.angv[i];
+  RefBody b;
+  b.x = p.x;
+  b.y = p.y;
+  b.z = p.z;
+  b.r = r.rad[i];
+  b.vx = d2f(v.x);
+  b.vy = d2f(v.y);
+  b.vz = d2f(v.z);
+  b.wx = d2f(w.x);
+  b.wy = d2f(w.y);
+  b.wz = d2f(w.z);
+  b.nl = wet ? max(r.lqd_old[i], 12) : 12;
+  b.pad = 0;
+  return b;
+}
+__global__ void k_ref_bodies(RefArrays r, int n, int wet, RefBody* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = ref_body(r, i, wet != 0);
+}
+/* sphere i, packed or (no scratch to pack into) from the caller's arrays */
+__device__ __forceinline__ RefBody load_body(const RefArrays& r, const RefBody* pk, int i, bool wet) {
+  return pk ? pk[i] : ref_body(r, i, wet);
+}
+
+/* PPForceCalcG on the reference's layouts.  Bound by latency: a thread per
+ * sphere chained index -> partner -> history -> law per slot with 16 of 32
+ * lanes at work (249 us cold on the packed wet bed of 200,000).  Now a warp
+ * walks its 32 spheres' lists row by row (the caller's arrays are contiguous
+ * along a row; the next row's indexes are in flight), keeps the slots that
+ * touch or are wet as one dense list, and takes contacts and bridges from it
+ * with all lanes; the sums then go by sphere, in slot order, so every result
+ * keeps its bits (174 us).  A list of 64 leaves the L1 to the partners' records
+ * (96: no better, 128: 25 us slower); 24 warps of 80 registers an SM
+ * run the bed in two waves (20: three waves, 28: spills, both slower). */
+constexpr int kRefCap = 64, kRefBlocks = 24;
+static_assert(kRefCap >= 32 && kRefCap <= 256, "a row has to fit; entries are numbered in a byte");
+struct RefWarp {
+  float4 u[kRefCap];  /* normal, gap */
+  float4 f[kRefCap];  /* tangential force, normal and damping force */
+  float n[kRefCap];   /* normal force */
+  int j[kRefCap];     /* partner, then the bridge force */
+  unsigned row[kRefCap]; /* lanes with an entry, by row */
+  unsigned short slot[kRefCap];
+  unsigned char owner[kRefCap], flags[kRefCap]; /* flags: 1 touches, 2 forms a bridge, 4 wet, 8 was wet */
+  unsigned char contact[kRefCap];
+};
+__global__ void __launch_bounds__(32, kRefBlocks)
+    k_pp_ref_mixed(MixArgs a, RefArrays r, const RefBody* __restrict__ pk) {
+  __shared__ RefWarp sm;
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x;
+  const unsigned below = (1u << lane) - 1u;
   const int i = reversed_block_thread();
-  if (i >= a.n) return;
-  const double3 ip = r.pos[i];
-  const double ird = r.rad[i];
-  const float ri = d2f(ird);
-  const float3 iv = d2f3(r.vel[i]), iw = d2f3(r.angv[i]);
-  const bool wet_i = a.force_cap == 1;
-  float iVol = 0.f;
-  if (wet_i) {
-    const int inl = max(r.lqd_old[i], 12);
-    const float ti = 2.0f * ri;
-    iVol = __fdividef(a.lqd_vol * (ti * ti * ti), (float)inl);
-  }
+  const bool live = i < a.n;
+  const int ii = live ? i : a.n - 1;
+  const int first = i - lane;
+  const bool wet_on = a.force_cap == 1;
+  const int L = r.plevel[ii];
+  const int stride = r.npars[L];
+  const long long base = slot_base(L, r.npars, r.nneb) + r.nidx[ii];
+  const int nn = live ? r.num_nebor[ii] : 0;
+  const int rows = __reduce_max_sync(FULL, nn);
+  const double3 ip = r.pos[ii];
+  const double ird = r.rad[ii];
+  const float ri0 = d2f(ird);
   KSum3 F, M;
   KSum R;
   int wet = 0;
-  const int L = r.plevel[i];
-  const long long stride = r.npars[L];
-  const long long base = slot_base(L, r.npars, r.nneb) + r.nidx[i];
-  const int nn = r.num_nebor[i];
-  for (int k = 0; k < nn; k++) {
-    const long long s = base + k * stride;
-    const int j = r.nebor[s];
-    const double3 jp = r.pos[j];
-    const double jrd = r.rad[j];
-    const double dx = ip.x - jp.x, dy = ip.y - jp.y, dz = ip.z - jp.z;
-    const double d2 = dx * dx + dy * dy + dz * dz;
-    const double S = ird + jrd;
-    const double D = d2 - S * S;
-    if (!wet_i && D >= 0.0) continue; /* apart: nothing to do on a dry bed */
-    const float dist = sqrtf(d2f(d2));
-    const float rj = d2f(jrd);
-    const float gap = __fdividef(d2f(D), dist + d2f(S));
-    const float inv = __frcp_rn(dist);
-    const float3 u = f3(d2f(dx) * inv, d2f(dy) * inv, d2f(dz) * inv);
-    if (gap < 0.f) {
+  int k = 0;
+  int jn, bn; /* the next row */
+  auto fetch = [&]() {
+    const long long s = base + (long long)k * stride;
+    jn = k < nn ? r.nebor[s] : ii;
+    bn = wet_on && k < nn ? r.h.lqdBrg[s] : 0;
+  };
+  fetch();
+  while (k < rows) {
+    int ne = 0, nc = 0, nr = 0;
+    const int kc = k;
+    do {
+      const int j = jn, bprev = bn;
+      const bool in = k < nn;
+      double4 q;
+      if (pk) {
+        q = *reinterpret_cast<const double4*>(pk + j);
+      } else {
+        const double3 p = r.pos[j];
+        q = make_double4(p.x, p.y, p.z, r.rad[j]);
+      }
+      k++;
+      fetch();
+      const double dx = ip.x - q.x, dy = ip.y - q.y, dz = ip.z - q.z;
+      const double d2 = dx * dx + dy * dy + dz * dz;
+      const double S = ird + q.w;
+      const double D = d2 - S * S;
+      const float dist = sqrtf(d2f(d2));
+      const float gap = __fdividef(d2f(D), dist + d2f(S));
+      const bool touch = in && (wet_on || D < 0.0) && gap < 0.f;
+      const bool form = in && wet_on && gap < 2.0f * a.lqd_layer * (ri0 + d2f(q.w));
+      const bool keep = touch || form || bprev != 0;
+      const unsigned mk = __ballot_sync(FULL, keep), mc = __ballot_sync(FULL, touch);
+      if (keep) {
+        const int e = ne + __popc(mk & below);
+        const float inv = __frcp_rn(dist);
+        sm.u[e] = make_float4(d2f(dx) * inv, d2f(dy) * inv, d2f(dz) * inv, gap);
+        sm.j[e] = j;
+        sm.slot[e] = (unsigned short)(k - 1 - kc);
+        sm.owner[e] = (unsigned char)lane;
+        sm.flags[e] = (unsigned char)((touch ? 1 : 0) | (form ? 2 : 0) | (bprev != 0 ? 8 : 0));
+        if (touch) sm.contact[nc + __popc(mc & below)] = (unsigned char)e;
+      }
+      if (mk) {
+        if (lane == 0) sm.row[nr] = mk;
+        nr++;
+      }
+      ne += __popc(mk);
+      nc += __popc(mc);
+    } while (k < rows && ne <= kRefCap - 32 && k - kc < 65535);
+    __syncwarp();
+    for (int t0 = 0; t0 < nc; t0 += 32) {
+      const int t = t0 + lane;
+      const int e = sm.contact[min(t, nc - 1)], o = sm.owner[e];
+      const long long bo = __shfl_sync(FULL, base, o);
+      const int so = __shfl_sync(FULL, stride, o);
+      if (t >= nc) continue;
+      const long long s = bo + (long long)(kc + sm.slot[e]) * so;
       MixedRec rc = soa_load(r.h, s);
-      const float3 vj = d2f3(r.vel[j]), wj = d2f3(r.angv[j]);
-      const float3 cpv = (iv - vj) - crossf(iw * ri + wj * rj, u);
+      const RefBody bi = load_body(r, pk, first + o, wet_on), bj = load_body(r, pk, sm.j[e], wet_on);
+      const float ri = d2f(bi.r), rj = d2f(bj.r);
+      const float4 ug = sm.u[e];
+      const float3 u = f3(ug.x, ug.y, ug.z);
+      /* the own spin's part rounded first */
+      const float3 spin = f3(fmaf(bj.wx, rj, __fmul_rn(bi.wx, ri)), fmaf(bj.wy, rj, __fmul_rn(bi.wy, ri)),
+                             fmaf(bj.wz, rj, __fmul_rn(bi.wz, ri)));
+      const float3 cpv = (f3(bi.vx, bi.vy, bi.vz) - f3(bj.vx, bj.vy, bj.vz)) -
+                         crossf(spin, u);
+      float fN, fD;
+      float3 fT;
+      law32_forces(a.pp, ri * rj / (ri + rj), -ug.w, u, cpv, rc, a.dtf, fN, fD, fT);
+      soa_store(r.h, s, rc);
+      sm.f[e] = make_float4(fT.x, fT.y, fT.z, fN + fD);
+      sm.n[e] = fN;
+    }
+    __syncwarp();
+    if (wet_on)
+      for (int t0 = 0; t0 < ne; t0 += 32) {
+        const int e = min(t0 + lane, ne - 1), o = sm.owner[e];
+        const long long bo = __shfl_sync(FULL, base, o);
+        const int so = __shfl_sync(FULL, stride, o);
+        if (t0 + lane >= ne) continue;
+        const int j = sm.j[e];
+        const float ri = d2f(pk ? pk[first + o].r : r.rad[first + o]), rj = d2f(pk ? pk[j].r : r.rad[j]);
+        const int nli = pk ? pk[first + o].nl : max(r.lqd_old[first + o], 12);
+        const int nlj = pk ? pk[j].nl : max(r.lqd_old[j], 12);
+        const float gap = sm.u[e].w;
+        const float ti = 2.0f * ri, tj = 2.0f * rj;
+        const float qi = __fdividef(1.0f, (float)nli), qj = __fdividef(1.0f, (float)nlj);
+        /* the partner's share joins the own one, rounded first */
+        const float ijVol = fmaf(a.lqd_vol * (tj * tj * tj), qj, __fmul_rn(a.lqd_vol * (ti * ti * ti), qi));
+        const int fl = sm.flags[e], bprev = (fl & 8) ? 1 : 0;
+        int b = (fl & 2) ? 1 : bprev;
+        if (!(fl & 2) && gap > bridge_rupture32(a, ijVol, 0.f)) b = 0;
+        if (b != bprev) r.h.lqdBrg[bo + (long long)(kc + sm.slot[e]) * so] = b;
+        if (b == 1) {
+          sm.j[e] = __float_as_int(bridge_force32(a, gap < 0.f ? 0.f : gap, ijVol, 0.f, 2.0f * ri * rj / (ri + rj)));
+          sm.flags[e] = (unsigned char)(fl | 4);
+        }
+      }
+    __syncwarp();
+    int e0 = 0;
+    for (int t = 0; t < nr; t++) {
+      const unsigned mk = sm.row[t];
+      const int e = e0 + __popc(mk & below);
+      e0 += __popc(mk);
+      if (!((mk >> lane) & 1)) continue;
+      const int fl = sm.flags[e];
+      const float4 ug = sm.u[e];
+      const float3 u = f3(ug.x, ug.y, ug.z);
+      if (fl & 1) {
+        const float4 f = sm.f[e];
+        const float3 fT = f3(f.x, f.y, f.z);
+        const float arm = ri0 - -ug.w * 0.5f;
+        F.add(f.w * u + fT);
+        M.add(crossf(u * (-arm), fT));
+        R.add(0.5f * (a.rfrc + a.rfrc) * sm.n[e] * ri0);
+      }
+      if (fl & 4) {
+        F.add(u * (-__int_as_float(sm.j[e])));
+        wet++;
+      }
+    }
+    __syncwarp();
+  }
+  if (!live) return;
+  double3 f = add_sum(r.force[i], F);
+  const double t = 2.0 * r.rad[i];
+  f.z = f.z - t * t * t; /* gravity, m = (2r)^3 */
+  r.force[i] = f;
+  r.mom[i] = add_sum(r.mom[i], M);
+  r.rmom[i] = r.rmom[i] + f2d(R.s - R.c);
+  if (wet_on) r.lqd[i] = r.lqd[i] + wet;
+}
+
+/* The gap of a wall the sphere certainly does not touch, from FP32 copies of
+ * the coordinates: within tol of the exact one (a few FP32 ulps of the largest
+ * coordinate involved, taken 8x), so such a wall costs no FP64 work.  Any
+ * other kind of wall exerts nothing. */
+__device__ __forceinline__ bool wall_apart(const CylinderBC& cy, int kind, float px, float py, float pz, float ri) {
+  if (kind == 0 || kind == 1) {
+    const float wz = d2f(kind == 0 ? cy.Tw : cy.Bw);
+    return fabsf(pz - wz) - ri > 1e-6f * (fabsf(pz) + fabsf(wz) + ri);
+  }
+  if (kind != 2) return true;
+  const float cx = d2f(cy.cir.x), cyy = d2f(cy.cir.y), R = d2f(cy.R);
+  const float dx = px - cx, dy = py - cyy;
+  return fabsf(sqrtf(dx * dx + dy * dy) - R) - ri >
+         1e-6f * (fabsf(px) + fabsf(py) + fabsf(cx) + fabsf(cyy) + R + ri);
+}
+
+/* CirPWInterG on the reference's wall lists (row i of pitch bytes) and wall
+ * histories (slot a * NP + i); the wall point in FP64 as the fused step
+ * takes it, the law in FP32.  The top wall has moved before this launch.
+ * Few spheres touch a wall, and those lie together: a block of kRefWallThreads
+ * sifts kRefWallEach times as many, 32 at a time from all over the bed, and
+ * works on the rest as one dense list (31 us cold on 200,000 spheres; 42 as a
+ * thread per sphere, with 3 of 32 lanes in the law). */
+constexpr int kRefWallThreads = 128, kRefWallEach = 3;
+__global__ void __launch_bounds__(kRefWallThreads) k_wall_ref_mixed(MixArgs a, RefArrays r) {
+  __shared__ int list[kRefWallThreads * kRefWallEach];
+  __shared__ int listed;
+  if (threadIdx.x == 0) listed = 0;
+  __syncthreads();
+  const CylinderBC cy = *r.cyl;
+#pragma unroll
+  for (int e = 0; e < kRefWallEach; e++) {
+    const int i = ((e * (kRefWallThreads / 32) + (threadIdx.x >> 5)) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31);
+    const int nw = i < a.n ? r.nwall[i] : 0;
+    if (nw <= 0) continue;
+    const double3 p = r.pos[i];
+    const float px = d2f(p.x), py = d2f(p.y), pz = d2f(p.z), ri = d2f(r.rad[i]);
+    const int* row = reinterpret_cast<const int*>(reinterpret_cast<const char*>(r.wlist) + (size_t)i * r.pitch);
+    bool near = false;
+    for (int w = 0; w < nw; w++) near = near || !wall_apart(cy, row[w], px, py, pz, ri);
+    if (near) list[atomicAdd(&listed, 1)] = i;
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < listed; t += kRefWallThreads) {
+    const int i = list[t];
+    const int nw = r.nwall[i];
+    const double3 p = r.pos[i];
+    const double rid = r.rad[i];
+    const float ri = d2f(rid);
+    const float3 iv = d2f3(r.vel[i]), iw = d2f3(r.angv[i]);
+    const int* row = reinterpret_cast<const int*>(reinterpret_cast<const char*>(r.wlist) + (size_t)i * r.pitch);
+    KSum3 F, M;
+    KSum R;
+    float3 jv = f3(0.f, 0.f, 0.f); /* persists across walls (kernel.cu:980) */
+    const float pxf = d2f(p.x), pyf = d2f(p.y), pzf = d2f(p.z);
+    for (int w = 0; w < nw; w++) {
+      const int kind = row[w];
+      if (kind == 0) jv = f3(0.f, 0.f, d2f(cy.topv));
+      if (wall_apart(cy, kind, pxf, pyf, pzf, ri)) continue;
+      double3 jp = make_double3(p.x, p.y, kind == 0 ? cy.Tw : cy.Bw);
+      if (kind == 2) {
+        const double ddx = cy.cir.x - p.x, ddy = cy.cir.y - p.y;
+        const double dist = sqrt(ddx * ddx + ddy * ddy);
+        jp = make_double3(cy.R * ((p.x - cy.cir.x) / dist) + cy.cir.x, cy.R * ((p.y - cy.cir.y) / dist) + cy.cir.y,
+                          p.z);
+      }
+      const double3 d = make_double3(p.x - jp.x, p.y - jp.y, p.z - jp.z);
+      const double len = sqrt(d.x * d.x + d.y * d.y + d.z * d.z);
+      const float gapw = d2f(len - rid);
+      if (gapw >= 0.f) continue;
+      const float il = __frcp_rn(d2f(len));
+      const float3 u = f3(d2f(d.x) * il, d2f(d.y) * il, d2f(d.z) * il);
+      const float3 cpv = (iv - jv) - crossf(iw * ri, u);
+      const long long s = (long long)w * r.np + i;
+      MixedRec rc = soa_load(r.h, s);
       float3 dF, dM;
       float dR;
-      law32(a.pp, ri * rj / (ri + rj), -gap, u, cpv, rc, ri, a.rfrc, a.dtf, dF, dM, dR);
+      law32(a.pw, ri, -gapw, u, cpv, rc, ri, a.rfrc, a.dtf, dF, dM, dR);
       soa_store(r.h, s, rc);
       F.add(dF);
       M.add(dM);
       R.add(dR);
     }
-    if (!wet_i) continue;
-    const int bprev = r.h.lqdBrg[s];
-    const bool form = gap < 2.0f * a.lqd_layer * (ri + rj);
-    if (!form && bprev == 0) continue;
-    const int jnl = max(r.lqd_old[j], 12);
-    const float tj = 2.0f * rj;
-    const float ijVol = iVol + __fdividef(a.lqd_vol * (tj * tj * tj), (float)jnl);
-    int b = bprev;
-    if (form) b = 1;
-    else if (gap > bridge_rupture32(a, ijVol, 0.f)) b = 0;
-    if (b != bprev) r.h.lqdBrg[s] = b;
-    if (b == 1) {
-      const float fc = bridge_force32(a, gap < 0.f ? 0.f : gap, ijVol, 0.f, 2.0f * ri * rj / (ri + rj));
-      F.add(u * (-fc));
-      wet++;
-    }
+    r.force[i] = add_sum(r.force[i], F);
+    r.mom[i] = add_sum(r.mom[i], M);
+    r.rmom[i] = r.rmom[i] + f2d(R.s - R.c);
   }
-  double3 f = add_sum(r.force[i], F);
-  const double t = 2.0 * ird;
-  f.z = f.z - t * t * t; /* gravity, m = (2r)^3 */
-  r.force[i] = f;
-  r.mom[i] = add_sum(r.mom[i], M);
-  r.rmom[i] = r.rmom[i] + f2d(R.s - R.c);
-  if (wet_i) r.lqd[i] = r.lqd[i] + wet;
-}
-
-/* CirPWInterG on the reference's wall lists (row i of pitch bytes) and wall
- * histories (slot a * NP + i); the wall point in FP64 as the fused step
- * takes it, the law in FP32.  The top wall has moved before this launch. */
-__global__ void __launch_bounds__(128) k_wall_ref_mixed(MixArgs a, RefArrays r) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n) return;
-  const int nw = r.nwall[i];
-  if (nw <= 0) return;
-  const CylinderBC cy = *r.cyl;
-  const double3 p = r.pos[i];
-  const double rid = r.rad[i];
-  const float ri = d2f(rid);
-  const float3 iv = d2f3(r.vel[i]), iw = d2f3(r.angv[i]);
-  const int* row = reinterpret_cast<const int*>(reinterpret_cast<const char*>(r.wlist) + (size_t)i * r.pitch);
-  KSum3 F, M;
-  KSum R;
-  float3 jv = f3(0.f, 0.f, 0.f); /* persists across walls (kernel.cu:980) */
-  const float pxf = d2f(p.x), pyf = d2f(p.y), pzf = d2f(p.z);
-  for (int w = 0; w < nw; w++) {
-    const int kind = row[w];
-    if (kind == 0) jv = f3(0.f, 0.f, d2f(cy.topv));
-    /* A wall the sphere certainly does not touch costs no FP64 work: the gap
-     * from FP32 copies of the coordinates is within tol of the exact one (a
-     * few FP32 ulps of the largest coordinate involved, taken 8x) */
-    float gc, tol;
-    if (kind == 0 || kind == 1) {
-      const float wz = d2f(kind == 0 ? cy.Tw : cy.Bw);
-      gc = fabsf(pzf - wz) - ri;
-      tol = 1e-6f * (fabsf(pzf) + fabsf(wz) + ri);
-    } else if (kind == 2) {
-      const float cx = d2f(cy.cir.x), cyy = d2f(cy.cir.y), R = d2f(cy.R);
-      const float dx = pxf - cx, dy = pyf - cyy;
-      gc = fabsf(sqrtf(dx * dx + dy * dy) - R) - ri;
-      tol = 1e-6f * (fabsf(pxf) + fabsf(pyf) + fabsf(cx) + fabsf(cyy) + R + ri);
-    } else {
-      continue;
-    }
-    if (gc > tol) continue;
-    double3 jp;
-    if (kind == 0) {
-      jp = make_double3(p.x, p.y, cy.Tw);
-    } else if (kind == 1) {
-      jp = make_double3(p.x, p.y, cy.Bw);
-    } else if (kind == 2) {
-      const double ddx = cy.cir.x - p.x, ddy = cy.cir.y - p.y;
-      const double dist = sqrt(ddx * ddx + ddy * ddy);
-      jp = make_double3(cy.R * ((p.x - cy.cir.x) / dist) + cy.cir.x, cy.R * ((p.y - cy.cir.y) / dist) + cy.cir.y,
-                        p.z);
-    } else {
-      continue;
-    }
-    const double3 d = make_double3(p.x - jp.x, p.y - jp.y, p.z - jp.z);
-    const double len = sqrt(d.x * d.x + d.y * d.y + d.z * d.z);
-    const float gapw = d2f(len - rid);
-    if (gapw >= 0.f) continue;
-    const float il = __frcp_rn(d2f(len));
-    const float3 u = f3(d2f(d.x) * il, d2f(d.y) * il, d2f(d.z) * il);
-    const float3 cpv = (iv - jv) - crossf(iw * ri, u);
-    const long long s = (long long)w * r.np + i;
-    MixedRec rc = soa_load(r.h, s);
-    float3 dF, dM;
-    float dR;
-    law32(a.pw, ri, -gapw, u, cpv, rc, ri, a.rfrc, a.dtf, dF, dM, dR);
-    soa_store(r.h, s, rc);
-    F.add(dF);
-    M.add(dM);
-    R.add(dR);
-  }
-  r.force[i] = add_sum(r.force[i], F);
-  r.mom[i] = add_sum(r.mom[i], M);
-  r.rmom[i] = r.rmom[i] + f2d(R.s - R.c);
 }
 
 /* UpdateSystemG (kernel.cu:563-606) for the reference entry points' mixed
@@ -1593,11 +1746,13 @@ dem_status mixed_force_to_master(dem_ctx* c, cudaStream_t s) {
   return cuda_check(cudaGetLastError(), "mixed_force_to_master launch");
 }
 
+size_t ref_mixed_scratch(int n) { return kRefBody * (size_t)n; }
+
 dem_status pp_force_ref_mixed(const double3* pos, const double3* vel, const double3* angvel, const double* rad,
                               const int* nebor, const int* plevel, const int* level_npars, const int* level_nnebors,
                               const int* nebor_idx, HistSoA h, const int* num_nebor, int* lqd, const int* lqd_old,
                               double3* force, double3* mom, double* rmom, int n, int force_cap, int stage,
-                              const DevConsts& k, cudaStream_t s) {
+                              const DevConsts& k, void* bodies, cudaStream_t s) {
   if (n <= 0) return DEM_OK;
   RefArrays r;
   std::memset(&r, 0, sizeof(r));
@@ -1605,7 +1760,9 @@ dem_status pp_force_ref_mixed(const double3* pos, const double3* vel, const doub
   r.nebor = nebor; r.plevel = plevel; r.npars = level_npars; r.nneb = level_nnebors; r.nidx = nebor_idx;
   r.num_nebor = num_nebor; r.lqd_old = lqd_old; r.lqd = lqd; r.h = h;
   r.force = force; r.mom = mom; r.rmom = rmom;
-  k_pp_ref_mixed<<<grid_for(n, 128), 128, 0, s>>>(ref_args(k, n, force_cap, stage), r);
+  RefBody* pk = static_cast<RefBody*>(bodies);
+  if (pk) k_ref_bodies<<<grid_for(n, 128), 128, 0, s>>>(r, n, force_cap == 1, pk);
+  k_pp_ref_mixed<<<grid_for(n, 32), 32, 0, s>>>(ref_args(k, n, force_cap, stage), r, pk);
   return cuda_check(cudaGetLastError(), "pp_force_ref_mixed launch");
 }
 
@@ -1620,7 +1777,7 @@ dem_status wall_force_ref_mixed(const double3* pos, const double3* vel, const do
   r.force = force; r.mom = mom; r.rmom = rmom;
   r.cyl = cyl; r.nwall = nwall; r.wlist = wlist; r.pitch = pitch; r.np = NP;
   k_move_walls<<<1, 32, 0, s>>>(cyl, 1, k.prm.dt, nullptr);
-  k_wall_ref_mixed<<<grid_for(n, 128), 128, 0, s>>>(ref_args(k, n, 0, stage), r);
+  k_wall_ref_mixed<<<grid_for(n, kRefWallThreads * kRefWallEach), kRefWallThreads, 0, s>>>(ref_args(k, n, 0, stage), r);
   return cuda_check(cudaGetLastError(), "wall_force_ref_mixed launch");
 }
 
