@@ -206,7 +206,7 @@ __global__ void k_cell_order(const int* __restrict__ sorted_hash, int* __restric
 /* NeighborFindG (kernel.cu:729-855).  sorted_src == NULL means the particle
  * arrays are themselves in sorted order.
  *
- * Optional prefilter (pre.hi != NULL): pre.hi holds (x, y, z, r) as the high
+ * Optional prefilter (pre.hi != NULL): pre.hi + 2 * q holds sphere q's (x, y, z, r) as the high
  * floats of (coordinate + offset) with every coordinate in one binade, so
  * hi_i - hi_j is exact in FP32; the FP32 distance from those differences is
  * within pre.tol of the exact one.  A candidate farther than pre.tol from the
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(128) k_neighbor_find(
     Prefilter pre) {
   const int i = reversed_block_thread(); /* the largest spheres' long searches first */
   if (i >= n) return;
-  const float4 hi_i = pre.hi ? pre.hi[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 hi_i = pre.hi ? pre.hi[2 * i] : make_float4(0.f, 0.f, 0.f, 0.f);
   const float sg = (float)search_gap;
   const int L = plevel[i];
   const long long base = slot_base(L, lv.level_npars, lv.level_nnebors) + nebor_idx[i];
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(128) k_neighbor_find(
     const int j = sorted_src ? sorted_src[q] : q;
     bool in = false, decided = false;
     if (pre.hi) {
-      const float4 hj = pre.hi[j];
+      const float4 hj = pre.hi[2 * j];
       const float dx = hi_i.x - hj.x, dy = hi_i.y - hj.y, dz = hi_i.z - hj.z;
       const float d2 = dx * dx + dy * dy + dz * dz;
       /* squared: within 2e-7 of the squares' ratio, well inside pre.tol's allowance */

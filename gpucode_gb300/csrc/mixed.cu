@@ -53,7 +53,10 @@
 namespace dem {
 
 struct MixedState {
-  float4 *phi[2], *plo[2], *vel[2], *angv[2];
+  /* the FP32 shadows, two float4 to a sphere so that what is read together is
+   * one 32-byte sector: the position's high parts and radius, the low parts;
+   * the velocity and bridge count, the spin */
+  float4 *place[2], *motion[2];
   float4* force;
   float4* wall_out; /* the step's wall results, two per wall slot */
   int* wall_entry;  /* the listed wall slots (slot w of sphere q: w * n + q) */
@@ -81,8 +84,8 @@ struct Law32 {
 };
 
 struct MixArgs {
-  const float4 *phi_in, *plo_in, *v_in, *w_in;
-  float4 *phi_out, *plo_out, *v_out, *w_out;
+  const float4 *place_in, *motion_in;
+  float4 *place_out, *motion_out;
   double3 *pos, *vel, *angv;
   const double* rad;
   double* pmove;
@@ -310,6 +313,33 @@ __device__ __forceinline__ float bridge_rupture32(const MixArgs& a, float V, flo
   return a.lq_mode ? rupture32(V, th) : 0.99f * exp2f(0.33f * __log2f(V));
 }
 
+/* Two float4 of one 32-byte sector in one 256-bit access (p a multiple of 32
+ * bytes): the pair kernel's gathers are bound by the L1's wavefronts, and
+ * scattered lanes cost one per sector and instruction.  Shadows, records and
+ * results in this form: 70.6 us a step on the packed 200k bed, 608 on 2M spheres;
+ * as single float4 of separate arrays 75.1 and 664. */
+__device__ __forceinline__ void get2(const float4* p, float4& a, float4& b) {
+  asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(p));
+}
+__device__ __forceinline__ void put2(float4* p, float4 a, float4 b) {
+  asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w),
+               "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+               : "memory");
+}
+/* the same, streaming */
+__device__ __forceinline__ void get2cs(const float4* p, float4& a, float4& b) {
+  asm volatile("ld.global.cs.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(p) : "memory");
+}
+__device__ __forceinline__ void put2cs(float4* p, float4 a, float4 b) {
+  asm volatile("st.global.cs.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z),
+               "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+               : "memory");
+}
+
 /* A contact record is read once and written once per step: streaming
  * (evict-first) loads and stores keep it from displacing the partners'
  * shadows, which a warp's neighbours read again, from L1 (114.6 vs 118.5 us
@@ -318,19 +348,15 @@ __device__ __forceinline__ MixedRec load_rec(const ContactRec* p) {
   const float4* q = reinterpret_cast<const float4*>(p);
   MixedRec r;
   float4* o = reinterpret_cast<float4*>(&r);
-  o[0] = __ldcs(q + 0);
-  o[1] = __ldcs(q + 1);
-  o[2] = __ldcs(q + 2);
-  o[3] = __ldcs(q + 3);
+  get2cs(q, o[0], o[1]);
+  get2cs(q + 2, o[2], o[3]);
   return r;
 }
 __device__ __forceinline__ void store_rec(ContactRec* p, const MixedRec& r) {
   float4* q = reinterpret_cast<float4*>(p);
   const float4* o = reinterpret_cast<const float4*>(&r);
-  __stcs(q + 0, o[0]);
-  __stcs(q + 1, o[1]);
-  __stcs(q + 2, o[2]);
-  __stcs(q + 3, o[3]);
+  put2cs(q, o[0], o[1]);
+  put2cs(q + 2, o[2], o[3]);
 }
 
 /* hi/lo split of a coordinate already shifted into the binade [2^k, 2^(k+1)):
@@ -417,7 +443,8 @@ __device__ __forceinline__ void cap_run_queue(const CapNetSmem& w, CapEntry* qw,
  * per sphere, and the exact distance is two FP64 roots and three divisions. */
 __device__ __forceinline__ void wall_entry(const MixArgs& a, int e) {
   const int w = e / a.n, q = e - w * a.n;
-  const float4 hi = ro(a.phi_in + q), lo = ro(a.plo_in + q);
+  float4 hi, lo;
+  get2(a.place_in + 2 * q, hi, lo);
   const float ri = hi.w + lo.w;
   const CylinderBC cy = a.cyl[a.sys_of_id ? a.sys_of_id[ro(a.id + q)] : 0];
   const int kind = a.wlist[3 * q + w];
@@ -453,7 +480,8 @@ __device__ __forceinline__ void wall_entry(const MixArgs& a, int e) {
     if (gapw < 0.f) {
       const float il = (float)(1.0 / len);
       const float3 u = f3((float)d.x * il, (float)d.y * il, (float)d.z * il);
-      const float4 vi4 = ro(a.v_in + q), wi4 = ro(a.w_in + q);
+      float4 vi4, wi4;
+      get2(a.motion_in + 2 * q, vi4, wi4);
       /* the top wall's velocity carries over to the walls after it in the
        * list, as the reference's jVel does (kernel.cu:987-1020) */
       double jv = 0.0;
@@ -475,11 +503,11 @@ __device__ __forceinline__ void wall_entry(const MixArgs& a, int e) {
   a.wall_out[2 * (size_t)e + 1] = t;
 }
 
-/* resident blocks per SM the pair kernel is built for: 8 (56 registers, no
- * spills) 80.5 us a step on the packed 200k bed, 7 84.5, 6 86.4; 2M spheres 710,
- * 746, 770 us */
+/* resident blocks per SM the pair kernel is built for: 9 (56 registers, no
+ * spills) 72.2 us a step on the packed 200k bed, 8 73.1, 7 75.0, 10 73.9; 2M
+ * spheres 595, 610, 629, 600 us */
 #ifndef DEM_PAIR_BLOCKS
-#define DEM_PAIR_BLOCKS 8
+#define DEM_PAIR_BLOCKS 9
 #endif
 
 /* One thread per pair of the list: overlap, contact law, capillary bridge, the
@@ -528,16 +556,18 @@ __global__ void __launch_bounds__(128, NET ? kNetBlocks : DEM_PAIR_BLOCKS) k_pai
     if (act) {
       const int2 ij = ro(pair + p);
       const int i = ij.x, j = ij.y;
-      const float4 hi = ro(a.phi_in + i), hj = ro(a.phi_in + j);
-      const float4 lo = ro(a.plo_in + i), lj = ro(a.plo_in + j);
-      const float4 vi = ro(a.v_in + i), vj = ro(a.v_in + j);
+      float4 hi, lo, hj, lj;
+      get2(a.place_in + 2 * i, hi, lo);
+      get2(a.place_in + 2 * j, hj, lj);
+      float4 vi, vj, wi, wj;
+      get2(a.motion_in + 2 * i, vi, wi);
+      get2(a.motion_in + 2 * j, vj, wj);
       if (WET) bprev = brg[p];
       const float ax = hi.x - hj.x, ay = hi.y - hj.y, az = hi.z - hj.z; /* exact */
       const float ri = hi.w + lo.w;
       float rj;
       gap = exact_gap(hi, lo, hj, lj, ax, ay, az, u, rj);
       if (gap < 0.f) {
-        const float4 wi = ro(a.w_in + i), wj = ro(a.w_in + j);
         MixedRec rc = load_rec(rec + p);
         const float3 cpv = f3(vi.x - vj.x, vi.y - vj.y, vi.z - vj.z) -
                            crossf(f3(wi.x, wi.y, wi.z) * ri + f3(wj.x, wj.y, wj.z) * rj, u);
@@ -631,8 +661,8 @@ __global__ void __launch_bounds__(128, NET ? kNetBlocks : DEM_PAIR_BLOCKS) k_pai
     }
     if (act) {
       float4* o = a.pair_out + 2 * (size_t)p;
-      o[0] = make_float4(u.x, u.y, u.z, __uint_as_float(__float_as_uint(nrm) | (wet ? 0x80000000u : 0u)));
-      if (nrm > 0.f) o[1] = make_float4(fT.x, fT.y, fT.z, s_n);
+      put2(o, make_float4(u.x, u.y, u.z, __uint_as_float(__float_as_uint(nrm) | (wet ? 0x80000000u : 0u))),
+           make_float4(fT.x, fT.y, fT.z, s_n));
       if (wet || (a.rfrc != 0.f && nrm > 0.f)) a.pair_out[2 * (size_t)a.ps.cap + p] = make_float4(fN, ci, cj, d);
     }
   }
@@ -644,15 +674,18 @@ __global__ void __launch_bounds__(128, NET ? kNetBlocks : DEM_PAIR_BLOCKS) k_pai
 }
 
 /* resident blocks per SM the sphere kernel is built for, and the pair results
- * a sphere has in flight: 6 and 3, 81.8 us a step on the packed 200k bed; 4 in
- * flight 86.4 (a few spills), 2 83.4, 1 89.4; 5 blocks with 4 89.0, 8 with 2 84.0 */
+ * a sphere has in flight: 6 and 3, 73.1 us a step on the packed 200k bed and 610
+ * on 2M spheres; 4 in flight 78.1 and 641 (a few spills), 2 73.0 and 627; 5 blocks with
+ * 4 77.6 and 623, 7 with 2 75.1 and 642, 8 with 1 75.6 and 633.  The indexes of the
+ * next results are read while the present ones are on their way (690 to 664 us
+ * on 2M spheres when this came in) */
 #ifndef DEM_BODY_BLOCKS
 #define DEM_BODY_BLOCKS 6
 #endif
 #ifndef DEM_BODY_BATCH
 #define DEM_BODY_BATCH 3
 #endif
-constexpr int kBodyBatch = DEM_BODY_BATCH;
+constexpr int kBodyBatch = DEM_BODY_BATCH, kNetBatch = 2;
 
 /* a pair's vector as the slot's sphere sees it: the second sphere's (e < 0)
  * points the other way.  Sign bits, not a product, so that no contraction
@@ -687,7 +720,9 @@ __global__ void __launch_bounds__(128, DEM_BODY_BLOCKS) k_body_mixed(MixArgs a) 
   const int nn = live ? ro(a.num_nebor + qq) : 0;
   const long long stride = ro(a.npars + L);
   const long long base = slot_base(L, a.npars, a.nneb) + ro(a.nidx + qq);
-  const float4 hi = ro(a.phi_in + qq), lo = ro(a.plo_in + qq), wi4 = ro(a.w_in + qq);
+  const float4 wi4 = ro(a.motion_in + 2 * qq + 1);
+  float4 hi, lo;
+  get2(a.place_in + 2 * qq, hi, lo);
   const float ri = hi.w + lo.w, twor = 2.0f * ri;
   const float mass_f = __fmul_rn(__fmul_rn(twor, twor), twor);
   KSum3 F, M;
@@ -715,56 +750,77 @@ __global__ void __launch_bounds__(128, DEM_BODY_BLOCKS) k_body_mixed(MixArgs a) 
       }
       since = end;
     };
-    for (int k = 0; k < nloop; k++) {
-      bool net = false;
-      const int e = k < nn ? ro(a.ps.eidx + base + (long long)k * stride) : kNoPair;
-      if (e != kNoPair) {
-        const int p = e < 0 ? ~e : e;
-        const float4 nu = a.pair_out[2 * (size_t)p], ft = a.pair_out[2 * (size_t)p + 1],
-                     br = a.pair_out[2 * (size_t)a.ps.cap + p];
-        const unsigned nb = __float_as_uint(nu.w);
-        const float nrm = fabsf(nu.w);
-        const float3 u = turned(nu, e);
+    int en[kNetBatch];
+#pragma unroll
+    for (int t = 0; t < kNetBatch; t++) en[t] = t < nn ? ro(a.ps.eidx + base + (long long)t * stride) : kNoPair;
+    for (int k0 = 0; k0 < nloop; k0 += kNetBatch) {
+      int e[kNetBatch];
+      float4 nu[kNetBatch], ft[kNetBatch], br[kNetBatch];
+#pragma unroll
+      for (int t = 0; t < kNetBatch; t++) {
+        e[t] = en[t];
+        nu[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+        ft[t] = br[t] = nu[t];
+        if (e[t] != kNoPair) {
+          const int p = e[t] < 0 ? ~e[t] : e[t];
+          get2(a.pair_out + 2 * (size_t)p, nu[t], ft[t]);
+          br[t] = a.pair_out[2 * (size_t)a.ps.cap + p];
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < kNetBatch; t++)
+        en[t] = k0 + kNetBatch + t < nn ? ro(a.ps.eidx + base + (long long)(k0 + kNetBatch + t) * stride) : kNoPair;
+#pragma unroll
+      for (int t = 0; t < kNetBatch; t++) {
+        const unsigned nb = __float_as_uint(nu[t].w);
+        const float nrm = fabsf(nu[t].w);
+        const float3 u = turned(nu[t], e[t]);
+        bool net = false;
         if (nrm > 0.f) {
-          const float3 fT = turned(ft, e);
-          F.add(ft.w * u + fT);
+          const float3 fT = turned(ft[t], e[t]);
+          F.add(ft[t].w * u + fT);
           const float arm = ri - nrm * 0.5f;
           M.add(crossf(u * (-arm), fT));
-          if (a.rfrc != 0.f) R.add(0.5f * (a.rfrc + a.rfrc) * br.x * ri);
+          if (a.rfrc != 0.f) R.add(0.5f * (a.rfrc + a.rfrc) * br[t].x * ri);
           ncont++;
         }
         if (nb >> 31) {
-          net = br.w != 1.0f;
-          if (!net) F.add(u * (e < 0 ? br.z : br.y));
+          net = br[t].w != 1.0f;
+          if (!net) F.add(u * (e[t] < 0 ? br[t].z : br[t].y));
           wet++;
           if (!(nrm > 0.f)) nbr++;
         }
-      }
-      queued += __popc(__ballot_sync(0xffffffffu, net));
-      if (queued > kCapQ - 32) {
-        flush(k + 1);
-        queued = 0;
+        queued += __popc(__ballot_sync(0xffffffffu, net));
+        if (queued > kCapQ - 32) {
+          flush(k0 + t + 1);
+          queued = 0;
+        }
       }
     }
     flush(nloop);
   }
+  int en[kBodyBatch];
+#pragma unroll
+  for (int t = 0; !NET && t < kBodyBatch; t++) en[t] = t < nn ? ro(a.ps.eidx + base + (long long)t * stride) : kNoPair;
   for (int k0 = 0; !NET && k0 < nn; k0 += kBodyBatch) {
     int e[kBodyBatch];
     float4 nu[kBodyBatch], ft[kBodyBatch], br[kBodyBatch];
 #pragma unroll
     for (int t = 0; t < kBodyBatch; t++)
-      e[t] = k0 + t < nn ? ro(a.ps.eidx + base + (long long)(k0 + t) * stride) : kNoPair;
+      e[t] = en[t];
 #pragma unroll
     for (int t = 0; t < kBodyBatch; t++) {
       nu[t] = make_float4(0.f, 0.f, 0.f, 0.f);
       ft[t] = br[t] = nu[t];
       if (e[t] != kNoPair) {
         const int p = e[t] < 0 ? ~e[t] : e[t];
-        nu[t] = a.pair_out[2 * (size_t)p];
-        ft[t] = a.pair_out[2 * (size_t)p + 1];
+        get2(a.pair_out + 2 * (size_t)p, nu[t], ft[t]);
         if (WET || a.rfrc != 0.f) br[t] = a.pair_out[2 * (size_t)a.ps.cap + p];
       }
     }
+#pragma unroll
+    for (int t = 0; t < kBodyBatch; t++)
+      en[t] = k0 + kBodyBatch + t < nn ? ro(a.ps.eidx + base + (long long)(k0 + kBodyBatch + t) * stride) : kNoPair;
 #pragma unroll
     for (int t = 0; t < kBodyBatch; t++) {
       const unsigned nb = __float_as_uint(nu[t].w);
@@ -847,10 +903,9 @@ __global__ void __launch_bounds__(128, DEM_BODY_BLOCKS) k_body_mixed(MixArgs a) 
     split_hi_lo(p.z + a.off.z, a.bin_exp, a.lo_scale, ph.z, pl.z);
     ph.w = hi.w;
     pl.w = lo.w;
-    a.phi_out[q] = ph;
-    a.plo_out[q] = pl;
-    a.v_out[q] = make_float4(vxf, vyf, vzf, __int_as_float(wet));
-    a.w_out[q] = make_float4(d2f(w.x), d2f(w.y), d2f(w.z), 0.f);
+    put2(a.place_out + 2 * q, ph, pl);
+    put2(a.motion_out + 2 * q, make_float4(vxf, vyf, vzf, __int_as_float(wet)),
+         make_float4(d2f(w.x), d2f(w.y), d2f(w.z), 0.f));
     a.force_out[q] = make_float4(fx, fy, fz, 0.f);
   }
   const unsigned fm = __ballot_sync(0xffffffffu, flagged);
@@ -909,8 +964,7 @@ __global__ void k_move_walls(CylinderBC* cyl, int n_cyl, double dt, const int* g
 
 __global__ void k_shadows(int n, const double3* __restrict__ pos, const double3* __restrict__ vel,
                           const double3* __restrict__ angv, const double* __restrict__ rad, const int* __restrict__ lqd,
-                          double3 off, int bin_exp, float lo_scale, float4* __restrict__ phi, float4* __restrict__ plo,
-                          float4* __restrict__ v4, float4* __restrict__ w4) {
+                          double3 off, int bin_exp, float lo_scale, float4* __restrict__ ps, float4* __restrict__ vs) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
   const double3 p = pos[q];
@@ -921,11 +975,10 @@ __global__ void k_shadows(int n, const double3* __restrict__ pos, const double3*
   const double r = rad[q];
   ph.w = (float)r;
   pl.w = (float)(r - (double)ph.w);
-  phi[q] = ph;
-  plo[q] = pl;
+  put2(ps + 2 * q, ph, pl);
   const double3 v = vel[q], w = angv[q];
-  v4[q] = make_float4(d2f(v.x), d2f(v.y), d2f(v.z), __int_as_float(lqd[q]));
-  w4[q] = make_float4(d2f(w.x), d2f(w.y), d2f(w.z), 0.f);
+  put2(vs + 2 * q, make_float4(d2f(v.x), d2f(v.y), d2f(v.z), __int_as_float(lqd[q])),
+       make_float4(d2f(w.x), d2f(w.y), d2f(w.z), 0.f));
 }
 
 /* A state import without a rebuild in one pass: the caller-order arrays
@@ -936,8 +989,7 @@ __global__ void k_import_shadows(int n, const int* __restrict__ id, const double
                                  const double3* __restrict__ hv, const double3* __restrict__ hw, int has_v, int has_w,
                                  double3* __restrict__ pos, double3* __restrict__ vel, double3* __restrict__ angv,
                                  const double* __restrict__ rad, int* __restrict__ lqd, double3 off, int bin_exp,
-                                 float lo_scale, float4* __restrict__ phi, float4* __restrict__ plo,
-                                 float4* __restrict__ v4, float4* __restrict__ w4) {
+                                 float lo_scale, float4* __restrict__ ps, float4* __restrict__ vs) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
   const int i = id[q];
@@ -947,7 +999,7 @@ __global__ void k_import_shadows(int n, const int* __restrict__ id, const double
   pos[q] = p;
   vel[q] = v;
   angv[q] = w;
-  const int lq = __float_as_int(v4[q].w);
+  const int lq = __float_as_int(vs[2 * q].w);
   lqd[q] = lq;
   float4 ph, pl;
   split_hi_lo(p.x + off.x, bin_exp, lo_scale, ph.x, pl.x);
@@ -956,10 +1008,9 @@ __global__ void k_import_shadows(int n, const int* __restrict__ id, const double
   const double r = rad[q];
   ph.w = (float)r;
   pl.w = (float)(r - (double)ph.w);
-  phi[q] = ph;
-  plo[q] = pl;
-  v4[q] = make_float4(d2f(v.x), d2f(v.y), d2f(v.z), __int_as_float(lq));
-  w4[q] = make_float4(d2f(w.x), d2f(w.y), d2f(w.z), 0.f);
+  put2(ps + 2 * q, ph, pl);
+  put2(vs + 2 * q, make_float4(d2f(v.x), d2f(v.y), d2f(v.z), __int_as_float(lq)),
+       make_float4(d2f(w.x), d2f(w.y), d2f(w.z), 0.f));
 }
 
 /* the same import from mapped host arrays read in caller order.  A block
@@ -1028,7 +1079,7 @@ __global__ void __launch_bounds__(kImportThreads) k_import_shadows_mapped(
     int n, const int* __restrict__ inv, const double3* __restrict__ hp, const double3* __restrict__ hv,
     const double3* __restrict__ hw, double3* __restrict__ pos, double3* __restrict__ vel, double3* __restrict__ angv,
     const double* __restrict__ rad, int* __restrict__ lqd, double3 off, int bin_exp, float lo_scale,
-    float4* __restrict__ phi, float4* __restrict__ plo, float4* __restrict__ v4, float4* __restrict__ w4) {
+    float4* __restrict__ ps, float4* __restrict__ vs) {
   __shared__ double sp[kSliceDoubles], sv[kSliceDoubles], sw[kSliceDoubles];
   const long long nsl = ((long long)n + kImportThreads - 1) / kImportThreads;
   const bool ap = (reinterpret_cast<size_t>(hp) & 15) == 0;
@@ -1063,7 +1114,7 @@ __global__ void __launch_bounds__(kImportThreads) k_import_shadows_mapped(
       pos[q] = p;
       vel[q] = v;
       angv[q] = w;
-      const int lq = __float_as_int(v4[q].w);
+      const int lq = __float_as_int(vs[2 * q].w);
       lqd[q] = lq;
       float4 ph, pl;
       split_hi_lo(p.x + off.x, bin_exp, lo_scale, ph.x, pl.x);
@@ -1072,10 +1123,9 @@ __global__ void __launch_bounds__(kImportThreads) k_import_shadows_mapped(
       const double r = rad[q];
       ph.w = (float)r;
       pl.w = (float)(r - (double)ph.w);
-      phi[q] = ph;
-      plo[q] = pl;
-      v4[q] = make_float4(d2f(v.x), d2f(v.y), d2f(v.z), __int_as_float(lq));
-      w4[q] = make_float4(d2f(w.x), d2f(w.y), d2f(w.z), 0.f);
+      put2(ps + 2 * q, ph, pl);
+      put2(vs + 2 * q, make_float4(d2f(v.x), d2f(v.y), d2f(v.z), __int_as_float(lq)),
+           make_float4(d2f(w.x), d2f(w.y), d2f(w.z), 0.f));
     }
     __syncthreads();
   }
@@ -1089,10 +1139,10 @@ __global__ void k_force_out(int n, const float4* __restrict__ f, double3* __rest
   mom[q] = make_double3(0.0, 0.0, 0.0);
 }
 
-__global__ void k_lqd_from_shadow(int n, const float4* __restrict__ v4, int* __restrict__ lqd) {
+__global__ void k_lqd_from_shadow(int n, const float4* __restrict__ vs, int* __restrict__ lqd) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
-  lqd[q] = __float_as_int(v4[q].w);
+  lqd[q] = __float_as_int(vs[2 * q].w);
 }
 
 Law32 make_law(const calParaPP& c, bool pp, double dmp_sq, int stage) {
@@ -1554,13 +1604,13 @@ dem_status mixed_create(dem_ctx* c) {
   std::memset(m, 0, sizeof(*m));
   c->mx = m;
   const size_t N = (size_t)c->n;
-  float4** bufs[9] = {&m->phi[0], &m->phi[1], &m->plo[0], &m->plo[1], &m->vel[0],
-                      &m->vel[1], &m->angv[0], &m->angv[1], &m->force};
+  float4** bufs[5] = {&m->place[0], &m->place[1], &m->motion[0], &m->motion[1], &m->force};
   for (float4** b : bufs) {
     void* p = nullptr;
-    dem_status st = cuda_alloc(&p, sizeof(float4) * N);
+    const size_t bytes = sizeof(float4) * N * (b == &m->force ? 1 : 2);
+    dem_status st = cuda_alloc(&p, bytes);
     if (st != DEM_OK) return st;
-    cudaMemset(p, 0, sizeof(float4) * N);
+    cudaMemset(p, 0, bytes);
     c->allocs.push_back(p);
     *b = (float4*)p;
   }
@@ -1600,8 +1650,7 @@ dem_status mixed_shadows(dem_ctx* c, int which, cudaStream_t s) {
   MixedState* m = c->mx;
   EngineBufs& b = c->b;
   k_shadows<<<grid_for(c->n, 256), 256, 0, s>>>(c->n, b.pos, b.vel, b.angv, b.rad, b.lqd, m->off, m->bin_exp,
-                                                 m->lo_scale, m->phi[which],
-                                                 m->plo[which], m->vel[which], m->angv[which]);
+                                                 m->lo_scale, m->place[which], m->motion[which]);
   return cuda_check(cudaGetLastError(), "mixed_shadows launch");
 }
 
@@ -1610,8 +1659,7 @@ dem_status mixed_import(dem_ctx* c, int which, int has_v, int has_w, cudaStream_
   EngineBufs& b = c->b;
   k_import_shadows<<<grid_for(c->n, 256), 256, 0, s>>>(c->n, b.id, b.tmp_pos, b.tmp_vel, b.tmp_angv, has_v, has_w,
                                                         b.pos, b.vel, b.angv, b.rad, b.lqd, m->off, m->bin_exp,
-                                                        m->lo_scale, m->phi[which], m->plo[which], m->vel[which],
-                                                        m->angv[which]);
+                                                        m->lo_scale, m->place[which], m->motion[which]);
   return cuda_check(cudaGetLastError(), "mixed_import launch");
 }
 
@@ -1629,8 +1677,7 @@ dem_status mixed_import_mapped(dem_ctx* c, int which, const int* inv, const doub
   const long long nsl = ((long long)c->n + kImportThreads - 1) / kImportThreads;
   const int grid = (int)std::min<long long>(nsl, (long long)kImportBlocksPerSM * sms);
   k_import_shadows_mapped<<<grid, kImportThreads, 0, s>>>(c->n, inv, hp, hv, hw, b.pos, b.vel, b.angv, b.rad, b.lqd,
-                                                         m->off, m->bin_exp, m->lo_scale, m->phi[which],
-                                                         m->plo[which], m->vel[which], m->angv[which]);
+                                                         m->off, m->bin_exp, m->lo_scale, m->place[which], m->motion[which]);
   return cuda_check(cudaGetLastError(), "mixed_import_mapped launch");
 }
 
@@ -1638,7 +1685,7 @@ Prefilter mixed_prefilter(dem_ctx* c, int which) {
   /* |(hi_i - hi_j) - (x_i - x_j)| <= one binade ulp per axis (the lo parts are
    * below half an ulp each): sqrt(3) ulps, plus FP32 rounding of the distance
    * and of the cut-off (~3e-7 relative, distances < 4 reduced units) */
-  return Prefilter{c->mx->phi[which], 0.5f * c->mx->coarse_tol + 2.0e-6f, c->mx->base, 0.25f * c->mx->coarse_tol,
+  return Prefilter{c->mx->place[which], 0.5f * c->mx->coarse_tol + 2.0e-6f, c->mx->base, 0.25f * c->mx->coarse_tol,
                    c->radii_bounded};
 }
 
@@ -1654,9 +1701,10 @@ dem_status mixed_step(dem_ctx* c, int which, cudaStream_t s) {
   EngineBufs& b = c->b;
   MixArgs a;
   std::memset(&a, 0, sizeof(a));
-  a.phi_in = m->phi[which]; a.plo_in = m->plo[which]; a.v_in = m->vel[which]; a.w_in = m->angv[which];
-  a.phi_out = m->phi[1 - which]; a.plo_out = m->plo[1 - which]; a.v_out = m->vel[1 - which];
-  a.w_out = m->angv[1 - which];
+  a.place_in = m->place[which];
+  a.motion_in = m->motion[which];
+  a.place_out = m->place[1 - which];
+  a.motion_out = m->motion[1 - which];
   a.pos = b.pos; a.vel = b.vel; a.angv = b.angv; a.rad = b.rad; a.pmove = b.pmove;
   a.num_nebor = b.num_nebor; a.plevel = b.plevel; a.nidx = b.nidx; a.npars = b.npars; a.nneb = b.nneb;
   a.ps = b.ps; a.pair_out = reinterpret_cast<float4*>(b.pair_out);
@@ -1733,7 +1781,7 @@ dem_status mixed_wall_entries(dem_ctx* c, cudaStream_t s) {
 dem_status mixed_pre_rebuild(dem_ctx* c, int which, cudaStream_t s) {
   /* the bridge counts of the last step travel in the shadow the next step
    * reads; bring them to the master array before it is permuted */
-  k_lqd_from_shadow<<<grid_for(c->n, 256), 256, 0, s>>>(c->n, c->mx->vel[which], c->b.lqd);
+  k_lqd_from_shadow<<<grid_for(c->n, 256), 256, 0, s>>>(c->n, c->mx->motion[which], c->b.lqd);
   return cuda_check(cudaGetLastError(), "mixed_pre_rebuild launch");
 }
 
@@ -1742,7 +1790,7 @@ const float4* mixed_force_shadow(const dem_ctx* c) { return c->mx ? c->mx->force
 dem_status mixed_force_to_master(dem_ctx* c, cudaStream_t s) {
   k_force_out<<<grid_for(c->n, 256), 256, 0, s>>>(c->n, c->mx->force, c->b.force, c->b.mom);
   /* the bridge counts of the last step live in the shadow the next step reads */
-  k_lqd_from_shadow<<<grid_for(c->n, 256), 256, 0, s>>>(c->n, c->mx->vel[c->parity], c->b.lqd);
+  k_lqd_from_shadow<<<grid_for(c->n, 256), 256, 0, s>>>(c->n, c->mx->motion[c->parity], c->b.lqd);
   return cuda_check(cudaGetLastError(), "mixed_force_to_master launch");
 }
 
