@@ -112,64 +112,92 @@ __global__ void k_scan_tiles(int* __restrict__ tile_sum, int ntiles) {
   }
 }
 
-/* (2c) cell offsets -> CellStart / CellEnd (-1 for empty cells); count[] is
- * read from cell_end[] and overwritten in place.  cell_off (optional, ncells
- * + 1 entries) receives every cell's offset, empty or not, and the total */
-__global__ void k_cell_ranges(int* __restrict__ cell_start, int* __restrict__ cell_end, int ncells,
-                              const int* __restrict__ tile_off, int* __restrict__ cell_off) {
-  const long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanPerThread;
-  int c[kScanPerThread];
-  int s = 0;
+/* A thread's kScanPerThread consecutive entries of a tile, read and written
+ * through shared memory so that a warp's accesses are contiguous (the ranges of
+ * the packed bed's cells 18.4 -> 4.5 us).  at() keeps a thread's run off its
+ * neighbours' banks. */
+struct ScanTile {
+  int v[kScanTile + kScanTile / kScanPerThread];
+  __device__ __forceinline__ int& at(int i) { return v[i + i / kScanPerThread]; }
+  __device__ __forceinline__ void load(const int* __restrict__ in, long long n) {
+    const long long base = (long long)blockIdx.x * kScanTile;
 #pragma unroll
-  for (int e = 0; e < kScanPerThread; e++) {
-    long long q = base + e;
-    c[e] = q < ncells ? cell_end[q] : 0;
-    s += c[e];
-  }
-  int total;
-  int off = block_exclusive_scan(s, total) + tile_off[blockIdx.x];
-#pragma unroll
-  for (int e = 0; e < kScanPerThread; e++) {
-    long long q = base + e;
-    if (q < ncells) {
-      cell_start[q] = c[e] ? off : -1;
-      cell_end[q] = c[e] ? off + c[e] : -1;
-      if (cell_off) {
-        cell_off[q] = off;
-        if (q == ncells - 1) cell_off[ncells] = off + c[e];
-      }
+    for (int e = 0; e < kScanPerThread; e++) {
+      const int i = e * kScanThreads + threadIdx.x;
+      at(i) = base + i < n ? in[base + i] : 0;
     }
-    off += c[e];
+    __syncthreads();
+  }
+  /* counts -> their exclusive scan, offset by `before`; returns the tile's end */
+  __device__ __forceinline__ int scan(int before) {
+    int c[kScanPerThread], sum = 0;
+#pragma unroll
+    for (int e = 0; e < kScanPerThread; e++) {
+      c[e] = at(threadIdx.x * kScanPerThread + e);
+      sum += c[e];
+    }
+    int total;
+    int off = block_exclusive_scan(sum, total) + before;
+#pragma unroll
+    for (int e = 0; e < kScanPerThread; e++) {
+      at(threadIdx.x * kScanPerThread + e) = off;
+      off += c[e];
+    }
+    __syncthreads();
+    return before + total;
+  }
+};
+
+/* (2c) cell offsets -> CellStart / CellEnd (-1 for empty cells); count[] is
+ * read from cell_end[] and overwritten in place.  With cell_off (ncells + 1
+ * entries) only that is written: every cell's offset, empty or not, and the
+ * total. */
+__global__ void __launch_bounds__(kScanThreads) k_cell_ranges(int* __restrict__ cell_start, int* __restrict__ cell_end,
+                                                              int ncells, const int* __restrict__ tile_off,
+                                                              int* __restrict__ cell_off) {
+  __shared__ ScanTile sm;
+  const long long base = (long long)blockIdx.x * kScanTile;
+  sm.load(cell_end, ncells);
+  const int end = sm.scan(tile_off[blockIdx.x]);
+#pragma unroll
+  for (int e = 0; e < kScanPerThread; e++) {
+    const int i = e * kScanThreads + threadIdx.x;
+    const long long q = base + i;
+    if (q >= ncells) break;
+    const int off = sm.at(i), next = i + 1 < kScanTile ? sm.at(i + 1) : end;
+    if (cell_off) {
+      cell_off[q] = off;
+      if (q == ncells - 1) cell_off[ncells] = next;
+    } else {
+      cell_start[q] = next > off ? off : -1;
+      cell_end[q] = next > off ? next : -1;
+    }
   }
 }
 
 /* the same scan over any counts: out[i] = sum of in[0 .. i), the total last,
  * into the pair set that is not current */
-__global__ void k_scan_apply(const int* __restrict__ in, int n, const int* __restrict__ tile_off, int* out0, int* out1,
-                             const int* __restrict__ ctl) {
+__global__ void __launch_bounds__(kScanThreads) k_scan_apply(const int* __restrict__ in, int n,
+                                                             const int* __restrict__ tile_off, int* out0, int* out1,
+                                                             const int* __restrict__ ctl) {
+  __shared__ ScanTile sm;
   int* __restrict__ out = ctl[0] ? out0 : out1;
-  const long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanPerThread;
-  int c[kScanPerThread];
-  int s = 0;
+  const long long base = (long long)blockIdx.x * kScanTile;
+  sm.load(in, n);
+  const int end = sm.scan(tile_off[blockIdx.x]);
 #pragma unroll
   for (int e = 0; e < kScanPerThread; e++) {
-    c[e] = base + e < n ? in[base + e] : 0;
-    s += c[e];
-  }
-  int total;
-  int off = block_exclusive_scan(s, total) + tile_off[blockIdx.x];
-#pragma unroll
-  for (int e = 0; e < kScanPerThread; e++) {
-    if (base + e < n) out[base + e] = off;
-    off += c[e];
-    if (base + e == n - 1) out[n] = off;
+    const int i = e * kScanThreads + threadIdx.x;
+    if (base + i >= n) break;
+    out[base + i] = sm.at(i);
+    if (base + i == n - 1) out[n] = i + 1 < kScanTile ? sm.at(i + 1) : end;
   }
 }
 
 /* (3) scatter to sorted positions */
 __global__ void k_scatter(const int* __restrict__ key, const int* __restrict__ rank, int n,
                           const int* __restrict__ cell_start, int* __restrict__ sorted_hash,
-                          int* __restrict__ sorted_src) {
+                          int* __restrict__ sorted_src) { /* cell_start: or cell_off */
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int h = key[i];
@@ -182,7 +210,7 @@ __global__ void k_scatter(const int* __restrict__ key, const int* __restrict__ r
  * sort; cells hold a handful of particles) */
 __global__ void k_cell_order(const int* __restrict__ sorted_hash, int* __restrict__ sorted_src,
                              const int* __restrict__ cell_start, const int* __restrict__ cell_end,
-                             const int* __restrict__ order_key, int n) {
+                             const int* __restrict__ order_key, int n) { /* or cell_off and cell_off + 1 */
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
   const int h = sorted_hash[q];
@@ -266,7 +294,7 @@ __global__ void __launch_bounds__(128) k_neighbor_find(
     const int* __restrict__ cell_start, const int* __restrict__ cell_end, const int* __restrict__ cell_off,
     const int* __restrict__ plevel, const int* __restrict__ nebor_idx, LevelView lv, double3 origin,
     double search_gap, int* __restrict__ nebor, int* __restrict__ num_nebor, int n, int* __restrict__ err,
-    Prefilter pre) {
+    Prefilter pre, int* __restrict__ owned) {
   const int i = reversed_block_thread(); /* the largest spheres' long searches first */
   if (i >= n) return;
   const float4 hi_i = pre.hi ? pre.hi[2 * i] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -277,7 +305,9 @@ __global__ void __launch_bounds__(128) k_neighbor_find(
   const int cap = lv.level_nnebors[L];
   /* the position from the grid's origin, exactly hi - 2^k: within pre.ulp */
   const float xf = hi_i.x - pre.base, yf = hi_i.y - pre.base, zf = hi_i.z - pre.base;
-  int count = 0;
+  const double3 pos_i = pre.hi ? make_double3(0.0, 0.0, 0.0) : pos[i];
+  const double rad_i = pre.hi ? 0.0 : rad[i];
+  int count = 0, higher = 0;
   bool over = false;
   /* candidate q (sorted position): the distance test, then the append */
   auto visit = [&](int q) {
@@ -292,6 +322,16 @@ __global__ void __launch_bounds__(128) k_neighbor_find(
       in = lo > 0.f && d2 < lo * lo; /* certainly inside */
       decided = in || d2 > hi * hi;  /* or outside */
     }
+    else {
+      const double3 d = sub3(pos_i, pos[j]);
+      const float dx = d2f(d.x), dy = d2f(d.y), dz = d2f(d.z), cut = d2f(rad[j] + rad_i + search_gap);
+      const float d2 = dx * dx + dy * dy + dz * dz, c2 = cut * cut;
+      /* each term within 2.4e-7, the squares within 1e-6 */
+      if (cut > 1.0e-15f && cut < 1.0e15f) {
+        in = d2 < c2 * (1.0f - 2.0e-6f);
+        decided = in || d2 > c2 * (1.0f + 2.0e-6f);
+      }
+    }
     if (!decided) in = len3(sub3(pos[i], pos[j])) < rad[j] + rad[i] + search_gap;
     if (!in || j == i) return;
     if (count >= cap) {
@@ -300,6 +340,7 @@ __global__ void __launch_bounds__(128) k_neighbor_find(
     }
     nebor[base + (long long)count * stride] = j;
     count++;
+    higher += j > i;
   };
   for (int iL = 0; iL < lv.n_levels; iL++) {
     const double csd = lv.cell_size[iL];
@@ -395,6 +436,7 @@ __global__ void __launch_bounds__(128) k_neighbor_find(
     }
   }
   num_nebor[i] = count;
+  if (owned) owned[i] = higher;
   if (over) atomicOr(err, 1);
 }
 
@@ -535,9 +577,9 @@ dem_status cell_sort(const double3* pos, const int* plevel, const int* order_key
   k_scan_tiles<<<1, kScanThreads, 0, stream>>>(tile, ntiles);
   k_cell_ranges<<<ntiles, kScanThreads, 0, stream>>>(cell_start, cell_end, ncells, tile, cell_off);
   if (n > 0) {
-    k_scatter<<<grid_for(n, 256), 256, 0, stream>>>(key, rank, n, cell_start, sorted_hash, sorted_src);
-    k_cell_order<<<grid_for(n, 256), 256, 0, stream>>>(sorted_hash, sorted_src, cell_start, cell_end,
-                                                      order_key, n);
+    const int *first = cell_off ? cell_off : cell_start, *last = cell_off ? cell_off + 1 : cell_end;
+    k_scatter<<<grid_for(n, 256), 256, 0, stream>>>(key, rank, n, first, sorted_hash, sorted_src);
+    k_cell_order<<<grid_for(n, 256), 256, 0, stream>>>(sorted_hash, sorted_src, first, last, order_key, n);
   }
   return cuda_check(cudaGetLastError(), "cell_sort launch");
 }
@@ -555,11 +597,11 @@ dem_status exclusive_scan(const int* in, int n, int* out0, int* out1, const int*
 dem_status neighbor_find(const double3* pos, const double* rad, const int* sorted_src,
                          const int* cell_start, const int* cell_end, const int* plevel, const int* nebor_idx,
                          LevelView lv, const DevConsts& k, int* nebor, int* num_nebor, int n, int* err,
-                         cudaStream_t stream, Prefilter pre, const int* cell_off) {
+                         cudaStream_t stream, Prefilter pre, const int* cell_off, int* owned) {
   if (n <= 0) return DEM_OK;
   k_neighbor_find<<<grid_for(n, 128), 128, 0, stream>>>(pos, rad, sorted_src, cell_start, cell_end, cell_off, plevel,
                                                        nebor_idx, lv, k.prm.Origin, k.prm.SearchGap, nebor,
-                                                       num_nebor, n, err, pre);
+                                                       num_nebor, n, err, pre, owned);
   return cuda_check(cudaGetLastError(), "neighbor_find launch");
 }
 

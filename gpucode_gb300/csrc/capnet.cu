@@ -1274,7 +1274,7 @@ dem_status dem_capnet_samples(dem_ctx* c, float* x_dev, float* y_dev, long long 
   if (c->s.force_cap != 1) return fail(DEM_ERR_STATE, "dem_capnet_samples: the bed has no capillary bridges");
   cudaStream_t s = c->stream;
   dem_status st = DEM_OK;
-  if (c->opt.precision == DEM_PREC_MIXED) st = mixed_pre_rebuild(c, c->parity, s); /* bridge counts -> lqd */
+  if (c->opt.precision == DEM_PREC_MIXED) st = mixed_bridge_counts(c, c->parity, s); /* bridge counts -> lqd */
   if (st != DEM_OK) return st;
   int* cnt = nullptr;
   long long *off = nullptr, *total = nullptr;

@@ -127,12 +127,14 @@ struct Prefilter {
 /* NeighborFindG semantics (kernel.cu:729-855) on AoS positions; sorted_src
  * maps sorted position -> particle index; writes the level/slot-major list.
  * Slot overflow sets bit 1 of *err and stops appending.  cell_off (from
- * cell_sort, may be NULL) lets a cell row's range be read with two loads. */
+ * cell_sort, may be NULL) lets a cell row's range be read with two loads;
+ * owned (may be NULL) receives each list's number of higher-indexed partners. */
 dem_status neighbor_find(const double3* pos, const double* rad, const int* sorted_src,
                          const int* cell_start, const int* cell_end, const int* plevel,
                          const int* nebor_idx, LevelView lv, const DevConsts& k, int* nebor,
                          int* num_nebor, int n, int* err, cudaStream_t stream,
-                         Prefilter pre = Prefilter{nullptr, 0.f, 0.f, 0.f, 0}, const int* cell_off = nullptr);
+                         Prefilter pre = Prefilter{nullptr, 0.f, 0.f, 0.f, 0}, const int* cell_off = nullptr,
+                         int* owned = nullptr);
 
 /* CirWallListG (kernel.cu:1034-1073); wall list pitched rows.  Batched
  * systems: sys_of_id[id[i]] selects particle i's cylinder in cyl[] (NULL: cyl[0]). */

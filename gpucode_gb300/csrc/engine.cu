@@ -60,10 +60,13 @@ dem_status dalloc(dem_ctx* c, T** p, size_t count) {
 __global__ void k_copy_old(const int* __restrict__ wlist, const int* __restrict__ nwall,
                            const ContactRec* __restrict__ wrec, int* __restrict__ wlist_old,
                            int* __restrict__ nwall_old, ContactRec* __restrict__ wrec_old, int n,
-                           unsigned long long* counters) {
+                           unsigned long long* counters, const float4* __restrict__ motion, int* __restrict__ lqd) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p == 0 && counters) counters[4] += 1; /* rebuilds */
   if (p >= n) return;
+  /* mixed: the bridge counts of the last step travel in the shadow the next
+   * step reads; bring them to the master array before it is permuted */
+  if (motion) lqd[p] = __float_as_int(motion[2 * p].w);
   const int nw = nwall[p];
   nwall_old[p] = nw;
   for (int a = 0; a < nw; a++) {
@@ -104,25 +107,32 @@ __global__ void k_copy_back(int n, const double3* __restrict__ tpos, const doubl
                             const int* __restrict__ tplevel, double3* __restrict__ pos, double3* __restrict__ vel,
                             double3* __restrict__ angv, double* __restrict__ rad, int* __restrict__ lqd,
                             int* __restrict__ id, int* __restrict__ plevel, int* __restrict__ nidx,
-                            double* __restrict__ pmove, LevelStart ls, int* __restrict__ err) {
+                            double* __restrict__ pmove, int* __restrict__ inv, LevelStart ls, int* __restrict__ err,
+                            ShadowOut sh) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
-  pos[q] = tpos[q];
-  vel[q] = tvel[q];
-  angv[q] = tangv[q];
-  rad[q] = trad[q];
-  lqd[q] = tlqd[q];
-  id[q] = tid[q];
+  const double3 p = tpos[q], v = tvel[q], w = tangv[q];
+  const double r = trad[q];
+  const int lq = tlqd[q], i = tid[q];
+  pos[q] = p;
+  vel[q] = v;
+  angv[q] = w;
+  rad[q] = r;
+  lqd[q] = lq;
+  id[q] = i;
+  inv[i] = q; /* the caller-order view of the new cell order, for the state import and export */
+  /* mixed: the shadows the build's prefilter and the next step read */
+  if (sh.place) write_shadow(sh, q, p, v, w, r, lq);
   const int L = tplevel[q];
   plevel[q] = L;
-  int r = q - ls.v[L];
+  int k = q - ls.v[L];
   /* a particle hashed into another level's cell range (only possible on the
    * far face of the grid) would break level-major order */
-  if (r < 0 || r >= ls.cnt[L]) {
+  if (k < 0 || k >= ls.cnt[L]) {
     atomicOr(err, 4);
-    r = 0;
+    k = 0;
   }
-  nidx[q] = r;
+  nidx[q] = k;
   pmove[q] = 0.0;
 }
 
@@ -292,13 +302,9 @@ dem_status enqueue_rebuild(dem_ctx* c, cudaStream_t s, int parity) {
   const int n = c->n;
   const bool reorder = c->opt.reorder != 0;
   dem_status st;
-  if (c->opt.precision == DEM_PREC_MIXED) {
-    st = mixed_pre_rebuild(c, parity, s);
-    if (st != DEM_OK) return st;
-    mark(c, s, "k_lqd_from_shadow");
-  }
+  const bool mixed = c->opt.precision == DEM_PREC_MIXED;
   k_copy_old<<<grid_for(n, 256), 256, 0, s>>>(b.wlist, b.nwall, b.wrec, b.wlist_old, b.nwall_old, b.wrec_old, n,
-                                              b.counters);
+                                              b.counters, mixed ? mixed_motion(c, parity) : nullptr, b.lqd);
   mark(c, s, "k_copy_old");
   st = cell_sort(b.pos, b.plevel, reorder ? b.id : nullptr, n, c->lv, c->k, c->s.sys_ncells, b.sorted_hash,
                  b.sorted_src, b.cell_start, b.cell_end, b.scratch, b.err, s, b.cell_off);
@@ -316,22 +322,25 @@ dem_status enqueue_rebuild(dem_ctx* c, cudaStream_t s, int parity) {
     }
     k_copy_back<<<grid_for(n, 256), 256, 0, s>>>(n, b.tmp_pos, b.tmp_vel, b.tmp_angv, b.tmp_rad, b.tmp_lqd, b.tmp_id,
                                                   b.tmp_plevel, b.pos, b.vel, b.angv, b.rad, b.lqd, b.id, b.plevel,
-                                                  b.nidx, b.pmove, ls, b.err);
+                                                  b.nidx, b.pmove, b.inv, ls, b.err, mixed ? mixed_shadow_out(c, parity) : ShadowOut{});
     mark(c, s, "k_copy_back");
   } else {
     cudaError_t e = cudaMemsetAsync(b.pmove, 0, sizeof(double) * (size_t)n, s);
     if (e != cudaSuccess) return cuda_check(e, "pmove reset");
   }
   Prefilter pre{nullptr, 0.f, 0.f, 0.f, 0};
-  if (c->opt.precision == DEM_PREC_MIXED) {
-    /* the permuted state's shadows: read by the next step and by the build's prefilter */
-    st = mixed_shadows(c, parity, s);
-    if (st != DEM_OK) return st;
+  if (mixed) {
+    if (!reorder) {
+      st = mixed_shadows(c, parity, s);
+      if (st != DEM_OK) return st;
+      mark(c, s, "k_shadows");
+    }
     pre = mixed_prefilter(c, parity);
-    mark(c, s, "k_shadows");
   }
+  /* the sort's scratch is free again */
+  int* owned = reinterpret_cast<int*>(b.scratch);
   st = neighbor_find(b.pos, b.rad, reorder ? nullptr : b.sorted_src, b.cell_start, b.cell_end, b.plevel, b.nidx,
-                     c->lv, c->k, b.nebor, b.num_nebor, n, b.err, s, pre, b.cell_off);
+                     c->lv, c->k, b.nebor, b.num_nebor, n, b.err, s, pre, b.cell_off, owned);
   if (st != DEM_OK) return st;
   mark(c, s, "k_neighbor_find");
   st = wall_list(b.pos, b.rad, b.cyl, b.wlist, 3 * sizeof(int), b.nwall, n, c->k, s, b.id, b.sys_of_id);
@@ -344,17 +353,16 @@ dem_status enqueue_rebuild(dem_ctx* c, cudaStream_t s, int parity) {
   k_carry_walls<<<grid_for(n, 256), 256, 0, s>>>(b.wlist, b.nwall, b.wlist_old, b.nwall_old, b.wrec_old, b.wrec,
                                                  reorder ? b.sorted_src : nullptr, n);
   mark(c, s, "k_carry_walls");
-  /* the sort's scratch is free again */
-  int* cnt = reinterpret_cast<int*>(b.scratch);
-  st = pair_build(b.ps, lists_of(b), n, cnt, cnt + n, b.err, s);
+  st = pair_build(b.ps, lists_of(b), n, owned, owned + n, b.err, s);
   if (st != DEM_OK) return st;
-  mark(c, s, "pair list (k_pair_count .. k_pair_fill)");
+  mark(c, s, "pair list (scan, k_pair_fill)");
   st = pair_carry(b.ps, lists_of(b), n, reorder ? b.sorted_src : nullptr, b.err, s);
   if (st != DEM_OK) return st;
   mark(c, s, "k_carry");
-  /* the caller-order view of the new cell order, for the state import and export */
-  k_inverse<<<grid_for(n, 256), 256, 0, s>>>(n, b.id, b.inv);
-  mark(c, s, "k_inverse");
+  if (!reorder) {
+    k_inverse<<<grid_for(n, 256), 256, 0, s>>>(n, b.id, b.inv);
+    mark(c, s, "k_inverse");
+  }
   st = pair_flip(b.ps, s);
   if (st != DEM_OK) return st;
   return cuda_check(cudaGetLastError(), "rebuild launch");
@@ -1633,7 +1641,8 @@ extern "C" dem_status dem_load(dem_ctx* c, const char* path) {
   {
     EngineBufs& b = c->b;
     int* cnt = reinterpret_cast<int*>(b.scratch);
-    st = pair_build(b.ps, lists_of(b), c->n, cnt, cnt + c->n, b.err, c->stream);
+    st = pair_owned(lists_of(b), c->n, cnt, c->stream);
+    if (st == DEM_OK) st = pair_build(b.ps, lists_of(b), c->n, cnt, cnt + c->n, b.err, c->stream);
     /* links the slots to the pairs; what it carries over is overwritten below */
     if (st == DEM_OK) st = pair_carry(b.ps, lists_of(b), c->n, nullptr, b.err, c->stream);
     if (st == DEM_OK) st = pair_flip(b.ps, c->stream);

@@ -145,7 +145,12 @@ namespace dem {
 dem_status mixed_create(dem_ctx* c);
 void mixed_destroy(dem_ctx* c);
 /* regenerate shadow buffer `which` from the FP64 master state */
+struct ShadowOut;
+ShadowOut mixed_shadow_out(const dem_ctx* c, int which);
+const float4* mixed_motion(const dem_ctx* c, int which);
 dem_status mixed_shadows(dem_ctx* c, int which, cudaStream_t s);
+/* the last step's bridge counts to the master array */
+dem_status mixed_bridge_counts(dem_ctx* c, int which, cudaStream_t s);
 /* the neighbour build's FP32 prefilter over shadow buffer `which` */
 Prefilter mixed_prefilter(dem_ctx* c, int which);
 /* one fused step reading shadows `which`, writing shadows 1 - which */
@@ -163,7 +168,6 @@ const char* mixed_step_kernel_name(const dem_ctx* c);
 /* the compact list of the wall slots in use, from fresh wall lists */
 dem_status mixed_wall_entries(dem_ctx* c, cudaStream_t s);
 /* copy the last step's bridge counts from the shadow `which` to the master */
-dem_status mixed_pre_rebuild(dem_ctx* c, int which, cudaStream_t s);
 /* download the last step's force totals into the FP64 force array */
 dem_status mixed_force_to_master(dem_ctx* c, cudaStream_t s);
 /* the last step's forces, FP32, cell order (x, y, z, unused) */

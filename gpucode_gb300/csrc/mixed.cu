@@ -323,11 +323,6 @@ __device__ __forceinline__ void get2(const float4* p, float4& a, float4& b) {
       : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
       : "l"(p));
 }
-__device__ __forceinline__ void put2(float4* p, float4 a, float4 b) {
-  asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w),
-               "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
-               : "memory");
-}
 /* the same, streaming */
 __device__ __forceinline__ void get2cs(const float4* p, float4& a, float4& b) {
   asm volatile("ld.global.cs.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
@@ -357,21 +352,6 @@ __device__ __forceinline__ void store_rec(ContactRec* p, const MixedRec& r) {
   const float4* o = reinterpret_cast<const float4*>(&r);
   put2cs(q, o[0], o[1]);
   put2cs(q + 2, o[2], o[3]);
-}
-
-/* hi/lo split of a coordinate already shifted into the binade [2^k, 2^(k+1)):
- * hi keeps the top 24 significand bits (exponent fixed), lo the remaining 29
- * bits as an exact integer times 2^(k-52), rounded to 24 bits.  Integer and
- * conversion units only; a value outside the binade takes the FP64 route. */
-__device__ __forceinline__ void split_hi_lo(double xo, int dexp, float lo_scale, float& hi, float& lo) {
-  const unsigned long long u = (unsigned long long)__double_as_longlong(xo);
-  if ((int)((u >> 52) & 0x7ff) == dexp && !(u >> 63)) {
-    hi = __uint_as_float(((unsigned)(dexp - 1023 + 127) << 23) | (unsigned)((u >> 29) & 0x7fffffu));
-    lo = __uint2float_rn((unsigned)(u & 0x1fffffffull)) * lo_scale;
-  } else {
-    hi = (float)xo;
-    lo = (float)(xo - (double)hi);
-  }
 }
 
 /* read-only global loads (inputs of the step: never written by this launch) */
@@ -964,21 +944,9 @@ __global__ void k_move_walls(CylinderBC* cyl, int n_cyl, double dt, const int* g
 
 __global__ void k_shadows(int n, const double3* __restrict__ pos, const double3* __restrict__ vel,
                           const double3* __restrict__ angv, const double* __restrict__ rad, const int* __restrict__ lqd,
-                          double3 off, int bin_exp, float lo_scale, float4* __restrict__ ps, float4* __restrict__ vs) {
+                          ShadowOut sh) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n) return;
-  const double3 p = pos[q];
-  float4 ph, pl;
-  split_hi_lo(p.x + off.x, bin_exp, lo_scale, ph.x, pl.x);
-  split_hi_lo(p.y + off.y, bin_exp, lo_scale, ph.y, pl.y);
-  split_hi_lo(p.z + off.z, bin_exp, lo_scale, ph.z, pl.z);
-  const double r = rad[q];
-  ph.w = (float)r;
-  pl.w = (float)(r - (double)ph.w);
-  put2(ps + 2 * q, ph, pl);
-  const double3 v = vel[q], w = angv[q];
-  put2(vs + 2 * q, make_float4(d2f(v.x), d2f(v.y), d2f(v.z), __int_as_float(lqd[q])),
-       make_float4(d2f(w.x), d2f(w.y), d2f(w.z), 0.f));
+  if (q < n) write_shadow(sh, q, pos[q], vel[q], angv[q], rad[q], lqd[q]);
 }
 
 /* A state import without a rebuild in one pass: the caller-order arrays
@@ -988,8 +956,7 @@ __global__ void k_shadows(int n, const double3* __restrict__ pos, const double3*
 __global__ void k_import_shadows(int n, const int* __restrict__ id, const double3* __restrict__ hp,
                                  const double3* __restrict__ hv, const double3* __restrict__ hw, int has_v, int has_w,
                                  double3* __restrict__ pos, double3* __restrict__ vel, double3* __restrict__ angv,
-                                 const double* __restrict__ rad, int* __restrict__ lqd, double3 off, int bin_exp,
-                                 float lo_scale, float4* __restrict__ ps, float4* __restrict__ vs) {
+                                 const double* __restrict__ rad, int* __restrict__ lqd, ShadowOut sh) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
   const int i = id[q];
@@ -999,18 +966,9 @@ __global__ void k_import_shadows(int n, const int* __restrict__ id, const double
   pos[q] = p;
   vel[q] = v;
   angv[q] = w;
-  const int lq = __float_as_int(vs[2 * q].w);
+  const int lq = __float_as_int(sh.motion[2 * q].w);
   lqd[q] = lq;
-  float4 ph, pl;
-  split_hi_lo(p.x + off.x, bin_exp, lo_scale, ph.x, pl.x);
-  split_hi_lo(p.y + off.y, bin_exp, lo_scale, ph.y, pl.y);
-  split_hi_lo(p.z + off.z, bin_exp, lo_scale, ph.z, pl.z);
-  const double r = rad[q];
-  ph.w = (float)r;
-  pl.w = (float)(r - (double)ph.w);
-  put2(ps + 2 * q, ph, pl);
-  put2(vs + 2 * q, make_float4(d2f(v.x), d2f(v.y), d2f(v.z), __int_as_float(lq)),
-       make_float4(d2f(w.x), d2f(w.y), d2f(w.z), 0.f));
+  write_shadow(sh, q, p, v, w, rad[q], lq);
 }
 
 /* the same import from mapped host arrays read in caller order.  A block
@@ -1078,8 +1036,7 @@ __device__ __forceinline__ void slice_put(const SliceRegs& r, bool al, double* s
 __global__ void __launch_bounds__(kImportThreads) k_import_shadows_mapped(
     int n, const int* __restrict__ inv, const double3* __restrict__ hp, const double3* __restrict__ hv,
     const double3* __restrict__ hw, double3* __restrict__ pos, double3* __restrict__ vel, double3* __restrict__ angv,
-    const double* __restrict__ rad, int* __restrict__ lqd, double3 off, int bin_exp, float lo_scale,
-    float4* __restrict__ ps, float4* __restrict__ vs) {
+    const double* __restrict__ rad, int* __restrict__ lqd, ShadowOut sh) {
   __shared__ double sp[kSliceDoubles], sv[kSliceDoubles], sw[kSliceDoubles];
   const long long nsl = ((long long)n + kImportThreads - 1) / kImportThreads;
   const bool ap = (reinterpret_cast<size_t>(hp) & 15) == 0;
@@ -1114,18 +1071,9 @@ __global__ void __launch_bounds__(kImportThreads) k_import_shadows_mapped(
       pos[q] = p;
       vel[q] = v;
       angv[q] = w;
-      const int lq = __float_as_int(vs[2 * q].w);
+      const int lq = __float_as_int(sh.motion[2 * q].w);
       lqd[q] = lq;
-      float4 ph, pl;
-      split_hi_lo(p.x + off.x, bin_exp, lo_scale, ph.x, pl.x);
-      split_hi_lo(p.y + off.y, bin_exp, lo_scale, ph.y, pl.y);
-      split_hi_lo(p.z + off.z, bin_exp, lo_scale, ph.z, pl.z);
-      const double r = rad[q];
-      ph.w = (float)r;
-      pl.w = (float)(r - (double)ph.w);
-      put2(ps + 2 * q, ph, pl);
-      put2(vs + 2 * q, make_float4(d2f(v.x), d2f(v.y), d2f(v.z), __int_as_float(lq)),
-           make_float4(d2f(w.x), d2f(w.y), d2f(w.z), 0.f));
+      write_shadow(sh, q, p, v, w, rad[q], lq);
     }
     __syncthreads();
   }
@@ -1646,11 +1594,15 @@ void mixed_destroy(dem_ctx* c) {
   c->mx = nullptr;
 }
 
+ShadowOut mixed_shadow_out(const dem_ctx* c, int which) {
+  const MixedState* m = c->mx;
+  return ShadowOut{m->place[which], m->motion[which], m->off, m->bin_exp, m->lo_scale};
+}
+const float4* mixed_motion(const dem_ctx* c, int which) { return c->mx->motion[which]; }
+
 dem_status mixed_shadows(dem_ctx* c, int which, cudaStream_t s) {
-  MixedState* m = c->mx;
   EngineBufs& b = c->b;
-  k_shadows<<<grid_for(c->n, 256), 256, 0, s>>>(c->n, b.pos, b.vel, b.angv, b.rad, b.lqd, m->off, m->bin_exp,
-                                                 m->lo_scale, m->place[which], m->motion[which]);
+  k_shadows<<<grid_for(c->n, 256), 256, 0, s>>>(c->n, b.pos, b.vel, b.angv, b.rad, b.lqd, mixed_shadow_out(c, which));
   return cuda_check(cudaGetLastError(), "mixed_shadows launch");
 }
 
@@ -1658,8 +1610,7 @@ dem_status mixed_import(dem_ctx* c, int which, int has_v, int has_w, cudaStream_
   MixedState* m = c->mx;
   EngineBufs& b = c->b;
   k_import_shadows<<<grid_for(c->n, 256), 256, 0, s>>>(c->n, b.id, b.tmp_pos, b.tmp_vel, b.tmp_angv, has_v, has_w,
-                                                        b.pos, b.vel, b.angv, b.rad, b.lqd, m->off, m->bin_exp,
-                                                        m->lo_scale, m->place[which], m->motion[which]);
+                                                        b.pos, b.vel, b.angv, b.rad, b.lqd, mixed_shadow_out(c, which));
   return cuda_check(cudaGetLastError(), "mixed_import launch");
 }
 
@@ -1677,7 +1628,7 @@ dem_status mixed_import_mapped(dem_ctx* c, int which, const int* inv, const doub
   const long long nsl = ((long long)c->n + kImportThreads - 1) / kImportThreads;
   const int grid = (int)std::min<long long>(nsl, (long long)kImportBlocksPerSM * sms);
   k_import_shadows_mapped<<<grid, kImportThreads, 0, s>>>(c->n, inv, hp, hv, hw, b.pos, b.vel, b.angv, b.rad, b.lqd,
-                                                         m->off, m->bin_exp, m->lo_scale, m->place[which], m->motion[which]);
+                                                         mixed_shadow_out(c, which));
   return cuda_check(cudaGetLastError(), "mixed_import_mapped launch");
 }
 
@@ -1778,11 +1729,9 @@ dem_status mixed_wall_entries(dem_ctx* c, cudaStream_t s) {
   return cuda_check(cudaGetLastError(), "wall entries launch");
 }
 
-dem_status mixed_pre_rebuild(dem_ctx* c, int which, cudaStream_t s) {
-  /* the bridge counts of the last step travel in the shadow the next step
-   * reads; bring them to the master array before it is permuted */
+dem_status mixed_bridge_counts(dem_ctx* c, int which, cudaStream_t s) {
   k_lqd_from_shadow<<<grid_for(c->n, 256), 256, 0, s>>>(c->n, c->mx->motion[which], c->b.lqd);
-  return cuda_check(cudaGetLastError(), "mixed_pre_rebuild launch");
+  return cuda_check(cudaGetLastError(), "mixed_bridge_counts launch");
 }
 
 const float4* mixed_force_shadow(const dem_ctx* c) { return c->mx ? c->mx->force : nullptr; }

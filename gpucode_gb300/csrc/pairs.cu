@@ -55,26 +55,20 @@ __device__ __forceinline__ long long first_slot(const NeborLists& nl, int q, lon
   return slot_base(L, nl.npars, nl.nneb) + nl.nidx[q];
 }
 
-/* the pairs each sphere owns (cnt); the other slots wait for their pair */
-__global__ void k_pair_count(PairSet ps, NeborLists nl, int n, int* __restrict__ cnt) {
-  const int q = reversed_block_thread();
-  int low = 0;
-  if (q < n) {
-    long long stride;
-    const long long base = first_slot(nl, q, stride);
-    const int nn = nl.num[q];
-    for (int k = 0; k < nn; k++) {
-      const long long s = base + k * stride;
-      if (nl.nebor[s] < q) {
-        ps.eidx[s] = kNoPair;
-        low++;
-      }
-    }
-    cnt[q] = nn - low;
-  }
-  const int t = __reduce_add_sync(0xffffffffu, low);
-  if ((threadIdx.x & 31) == 0 && t) atomicAdd(ps.ctl + 4, t);
+/* the pairs each sphere owns, of lists that no search has just counted */
+__global__ void k_owned(NeborLists nl, int n, int* __restrict__ owned) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= n) return;
+  long long stride;
+  const long long base = first_slot(nl, q, stride);
+  const int nn = nl.num[q];
+  int m = 0;
+  for (int k = 0; k < nn; k++) m += nl.nebor[base + k * stride] >= q;
+  owned[q] = m;
 }
+
+/* list entries a sphere's thread has in flight */
+constexpr int kSlotBatch = 4;
 
 /* the pairs and their owners' slots, from the scanned counts (the set that is
  * not current).  Pairs past the arrays' capacity are dropped and reported
@@ -94,13 +88,17 @@ __global__ void k_pair_fill(PairSet ps, NeborLists nl, int n, int* __restrict__ 
   const long long base = first_slot(nl, q, stride);
   const int nn = nl.num[q];
   int p = off[q];
-  for (int k = 0; k < nn; k++) {
-    const long long s = base + k * stride;
-    const int j = nl.nebor[s];
-    if (j < q) continue;
-    if (p < ps.cap) pair[p] = make_int2(q, j);
-    ps.eidx[s] = p < ps.cap ? p : kNoPair;
-    p++;
+  for (int k0 = 0; k0 < nn; k0 += kSlotBatch) {
+    int j[kSlotBatch];
+#pragma unroll
+    for (int t = 0; t < kSlotBatch; t++) j[t] = k0 + t < nn ? nl.nebor[base + (k0 + t) * stride] : -1;
+#pragma unroll
+    for (int t = 0; t < kSlotBatch; t++) {
+      if (j[t] < q) continue;
+      if (p < ps.cap) pair[p] = make_int2(q, j[t]);
+      ps.eidx[base + (k0 + t) * stride] = p < ps.cap ? p : kNoPair;
+      p++;
+    }
   }
 }
 
@@ -113,6 +111,37 @@ __device__ __forceinline__ void mirror(ContactRec& r) {
   m.fx = -m.fx;
   m.fy = -m.fy;
   m.fz = -m.fz;
+}
+
+/* a record in two 256-bit accesses */
+union RecWords {
+  ContactRec r;
+  float f[16];
+  __device__ __forceinline__ RecWords() {}
+};
+__device__ __forceinline__ ContactRec read_rec(const ContactRec* p) {
+  RecWords w;
+  const float* q = reinterpret_cast<const float*>(p);
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    float* f = w.f + 8 * h;
+    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3]), "=f"(f[4]), "=f"(f[5]), "=f"(f[6]), "=f"(f[7])
+        : "l"(q + 8 * h));
+  }
+  return w.r;
+}
+__device__ __forceinline__ void write_rec(ContactRec* p, const ContactRec& r) {
+  RecWords w;
+  w.r = r;
+  float* q = reinterpret_cast<float*>(p);
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const float* f = w.f + 8 * h;
+    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(q + 8 * h), "f"(f[0]), "f"(f[1]), "f"(f[2]),
+                 "f"(f[3]), "f"(f[4]), "f"(f[5]), "f"(f[6]), "f"(f[7])
+                 : "memory");
+  }
 }
 
 /* HstryCopyG (kernel.cu:869-911) for one new pair: the record and bridge flag
@@ -140,42 +169,69 @@ __device__ __forceinline__ void carry_pair(const PairSet& ps, int cur, int n, in
     unsigned char brg = 0;
     if (hit >= 0) {
       const long long from = (long long)ps.sides * hit + (ps.sides == 2 && turned ? 1 - side : side);
-      r = pick(ps.rec, cur)[from];
+      r = read_rec(pick(ps.rec, cur) + from);
       brg = pick(ps.brg, cur)[from];
       if (ps.sides == 1 && turned) mirror(r);
     } else {
       r.dx = r.dy = r.dz = r.nDsp = r.nDsp_mx = r.plstRad = r.plstDfm = 0.0;
       r.stage = 0;
     }
-    pick(ps.rec, 1 - cur)[(long long)ps.sides * p + side] = r;
+    write_rec(pick(ps.rec, 1 - cur) + (long long)ps.sides * p + side, r);
     pick(ps.brg, 1 - cur)[(long long)ps.sides * p + side] = brg;
   }
 }
 
-/* One thread per new pair: its history, and the link from its second sphere's
- * slot.  Bound by the scattered reads of that sphere's list and of the old
- * pair's record. */
-__global__ void __launch_bounds__(256) k_carry(PairSet ps, NeborLists nl, int n,
-                                               const int* __restrict__ src) {
+/* The links from the slots of the pairs' second spheres: a thread per sphere
+ * looks for itself among the few pairs of each lower-indexed partner, which lie
+ * together.  (Looking for the pair's first sphere in the second one's list, a
+ * thread per pair, read a sector per entry of lists that lie apart.) */
+__device__ __forceinline__ void link_slots(const PairSet& ps, const NeborLists& nl, int n, int q, int cur) {
+  int lost = 0;
+  if (q < n) {
+    const int* __restrict__ off = pick(ps.off, 1 - cur);
+    const int2* __restrict__ pair = pick(ps.pair, 1 - cur);
+    long long stride;
+    const long long base = first_slot(nl, q, stride);
+    const int nn = nl.num[q];
+    for (int k0 = 0; k0 < nn; k0 += kSlotBatch) {
+      int j[kSlotBatch], at[kSlotBatch], end[kSlotBatch];
+#pragma unroll
+      for (int t = 0; t < kSlotBatch; t++) j[t] = k0 + t < nn ? nl.nebor[base + (k0 + t) * stride] : n;
+#pragma unroll
+      for (int t = 0; t < kSlotBatch; t++) {
+        at[t] = j[t] < q ? off[j[t]] : 0;
+        end[t] = j[t] < q ? min(off[j[t] + 1], ps.cap) : 0;
+      }
+#pragma unroll
+      for (int t = 0; t < kSlotBatch; t++) {
+        if (j[t] >= q) continue;
+        int p = at[t];
+        while (p < end[t] && pair[p].y != q) p++;
+        const bool hit = p < end[t];
+        ps.eidx[base + (k0 + t) * stride] = hit ? ~p : kNoPair;
+        lost += !hit;
+      }
+    }
+  }
+  lost = __reduce_add_sync(0xffffffffu, lost);
+  if ((threadIdx.x & 31) == 0 && lost) atomicAdd(ps.ctl + 4, lost);
+}
+
+/* One thread per new pair: its history; the first link_blocks blocks link the
+ * slots meanwhile.  Bound by the scattered reads of the old pair and its record:
+ * 53.5 us cold on the packed wet bed, 69 as one pass per pair with plain copies. */
+__global__ void __launch_bounds__(256) k_carry(PairSet ps, NeborLists nl, int n, const int* __restrict__ src,
+                                               int link_blocks) {
   const int cur = ps.ctl[0];
+  if (blockIdx.x < link_blocks) {
+    link_slots(ps, nl, n, (link_blocks - 1 - blockIdx.x) * blockDim.x + threadIdx.x, cur);
+    return;
+  }
   const int P = ps.ctl[2 - cur];
   const int2* __restrict__ pair = pick(ps.pair, 1 - cur);
-  int linked = 0;
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < P; p += gridDim.x * blockDim.x) {
-    const int2 ij = pair[p];
-    long long stride;
-    const long long base = first_slot(nl, ij.y, stride);
-    const int nn = nl.num[ij.y];
-    for (int k = 0; k < nn; k++)
-      if (nl.nebor[base + k * stride] == ij.x) {
-        ps.eidx[base + k * stride] = ~p;
-        linked++;
-        break;
-      }
-    carry_pair(ps, cur, n, p, ij, src);
-  }
-  linked = __reduce_add_sync(0xffffffffu, linked);
-  if ((threadIdx.x & 31) == 0 && linked) atomicSub(ps.ctl + 4, linked);
+  const int step = (gridDim.x - link_blocks) * blockDim.x;
+  for (int p = (blockIdx.x - link_blocks) * blockDim.x + threadIdx.x; p < P; p += step)
+    carry_pair(ps, cur, n, p, pair[p], src);
 }
 
 /* One-sided pairs for the slots that found none: nothing to do on a set of
@@ -212,10 +268,14 @@ __global__ void k_flip(int* ctl) {
 
 }  // namespace
 
-dem_status pair_build(const PairSet& ps, const NeborLists& nl, int n, int* cnt, void* scratch, int* err,
+dem_status pair_owned(const NeborLists& nl, int n, int* owned, cudaStream_t s) {
+  k_owned<<<grid_for(n, 128), 128, 0, s>>>(nl, n, owned);
+  return cuda_check(cudaGetLastError(), "pair count launch");
+}
+
+dem_status pair_build(const PairSet& ps, const NeborLists& nl, int n, const int* owned, void* scratch, int* err,
                       cudaStream_t s) {
-  k_pair_count<<<grid_for(n, 128), 128, 0, s>>>(ps, nl, n, cnt);
-  dem_status st = exclusive_scan(cnt, n, ps.off[0], ps.off[1], ps.ctl, scratch, s);
+  dem_status st = exclusive_scan(owned, n, ps.off[0], ps.off[1], ps.ctl, scratch, s);
   if (st != DEM_OK) return st;
   k_pair_fill<<<grid_for(n, 128), 128, 0, s>>>(ps, nl, n, err);
   return cuda_check(cudaGetLastError(), "pair list launch");
@@ -223,7 +283,8 @@ dem_status pair_build(const PairSet& ps, const NeborLists& nl, int n, int* cnt, 
 
 dem_status pair_carry(const PairSet& ps, const NeborLists& nl, int n, const int* src, int* err, cudaStream_t s) {
   const long long most = 6LL * n; /* beyond it the grid strides */
-  k_carry<<<grid_for(most < ps.cap ? most : ps.cap, 256), 256, 0, s>>>(ps, nl, n, src);
+  const int link = grid_for(n, 256);
+  k_carry<<<link + grid_for(most < ps.cap ? most : ps.cap, 256), 256, 0, s>>>(ps, nl, n, src, link);
   k_one_sided<<<grid_for(n < 152 * 1024 ? n : 152 * 1024, 256), 256, 0, s>>>(ps, nl, n, src, err);
   return cuda_check(cudaGetLastError(), "history carry launch");
 }

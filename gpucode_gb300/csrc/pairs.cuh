@@ -18,7 +18,7 @@ constexpr size_t kPairOut32 = 48;
 
 /* The pair arrays (device pointers), twice: ctl[0] is the current set,
  * ctl[1 + set] the number of pairs in it; ctl[3] counts the wall slots in use
- * (mixed.cu), ctl[4] the list entries that still want their pair.  off: first
+ * (mixed.cu), ctl[4] the list entries that found no pair.  off: first
  * pair of each sphere (n + 1; the pairs after off[n] are one-sided).  eidx: per
  * neighbour slot, the pair's index, ~index where the slot's sphere is the
  * pair's second one.  sides: the records and flags a pair has, 1 (mixed) or 2
@@ -51,10 +51,13 @@ struct NeborLists {
   const int *nebor, *num, *nidx, *plevel, *npars, *nneb;
 };
 
-/* condense fresh neighbour lists into the set that is not current; cnt (n
- * ints) and scratch (n + 64 ints) are free to use */
-dem_status pair_build(const PairSet& ps, const NeborLists& nl, int n, int* cnt, void* scratch, int* err,
+/* condense fresh neighbour lists into the set that is not current; owned: the
+ * higher-indexed partners of each list (neighbor_find); scratch (n + 64 ints) is
+ * free to use */
+dem_status pair_build(const PairSet& ps, const NeborLists& nl, int n, const int* owned, void* scratch, int* err,
                       cudaStream_t s);
+/* the same counts of lists that come from elsewhere */
+dem_status pair_owned(const NeborLists& nl, int n, int* owned, cudaStream_t s);
 /* link the slots of the pairs' second spheres, and fill the pairs' records and
  * flags from the current set's; src[q]: sphere q's position before the rebuild
  * (NULL: unchanged) */
