@@ -28,6 +28,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstddef>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -389,8 +390,9 @@ dem_status enqueue_step(dem_ctx* c, cudaStream_t s, int parity) {
 
 void destroy_graph(dem_ctx* c) {
   for (int p = 0; p < 2; p++) {
-    cudaGraphExec_t* all[6] = {&c->graph_exec[p],   &c->graph_one[p],     &c->chain_step[p],
-                               &c->chain_single[p], &c->chain_rebuild[p], &c->chain_single_host[p]};
+    cudaGraphExec_t* all[5 + kChainSizes] = {&c->graph_exec[p], &c->graph_one[p], &c->chain_single[p],
+                                             &c->chain_rebuild[p], &c->chain_single_host[p]};
+    for (int g = 0; g < kChainSizes; g++) all[5 + g] = &c->chain_step[g][p];
     for (cudaGraphExec_t* g : all) {
       if (*g) cudaGraphExecDestroy(*g);
       *g = nullptr;
@@ -505,9 +507,24 @@ dem_status capture_device_graph(dem_ctx* c, F enqueue, cudaGraphExec_t* out, cud
   return st;
 }
 
-/* the chained step graphs of the mixed path: S[p] (countdown), S1[p] (one
- * step), R[p] (rebuild), and the control block that names them */
-dem_status build_chain(dem_ctx* c) {
+/* capture the steps of one chain graph and what follows them (chain.cu) */
+dem_status chain_steps(dem_ctx* c, int p, int size, bool single, cudaStream_t cs) {
+  EngineBufs& b = c->b;
+  dem_status st = DEM_OK;
+  for (int k = 0; k < 1 << size && st == DEM_OK; k++) {
+    c->step_gate = k ? c->chain_ctl->flag + (k - 1) : b.need;
+    c->step_flag = k + 1 < 1 << size ? c->chain_ctl->flag + k : b.flag;
+    st = enqueue_step(c, cs, (p + k) & 1);
+  }
+  c->step_gate = nullptr;
+  c->step_flag = nullptr;
+  return st == DEM_OK ? chain_launch_tail(c->chain_ctl, b.flag, b.need, b.err, p, size, single, cs) : st;
+}
+
+/* the chained step graphs of the mixed path: S1[p] (one step) and R[p]
+ * (rebuild) at the first step call, S[G][p] (countdown) at the first of several
+ * steps, and the control block that names them */
+dem_status build_chain(dem_ctx* c, bool many) {
   EngineBufs& b = c->b;
   dem_status st = DEM_OK;
   if (!c->chain_ctl) {
@@ -516,36 +533,37 @@ dem_status build_chain(dem_ctx* c) {
     if (st != DEM_OK) return st;
     c->allocs.push_back(p);
     c->chain_ctl = (StepCtl*)p;
+    st = cuda_check(cudaMemset(p, 0, sizeof(StepCtl)), "step chain control");
   }
+  const bool ones = !c->chain_single[0], counted = many && !c->chain_step[0][0];
   for (int p = 0; p < 2 && st == DEM_OK; p++) {
-    st = capture_device_graph(
-        c,
-        [&](cudaStream_t cs) {
-          dem_status r = chain_clear_request(b.flag, b.need, cs);
-          return r == DEM_OK ? enqueue_rebuild(c, cs, p) : r;
-        },
-        &c->chain_rebuild[p]);
-    for (int single = 0; single < 2 && st == DEM_OK; single++) {
+    if (ones) {
       st = capture_device_graph(
           c,
           [&](cudaStream_t cs) {
-            c->step_gate = b.need;
-            dem_status r = enqueue_step(c, cs, p);
-            c->step_gate = nullptr;
-            return r == DEM_OK ? chain_launch_tail(c->chain_ctl, b.flag, b.need, b.err, p, single != 0, cs) : r;
+            dem_status r = chain_clear_request(b.flag, b.need, cs);
+            return r == DEM_OK ? enqueue_rebuild(c, cs, p) : r;
           },
-          single ? &c->chain_single[p] : &c->chain_step[p], single ? &c->chain_single_host[p] : nullptr);
+          &c->chain_rebuild[p]);
+      if (st == DEM_OK)
+        st = capture_device_graph(c, [&](cudaStream_t cs) { return chain_steps(c, p, 0, true, cs); },
+                                  &c->chain_single[p], &c->chain_single_host[p]);
     }
+    for (int g = 0; g < kChainSizes && counted && st == DEM_OK; g++)
+      st = capture_device_graph(c, [&](cudaStream_t cs) { return chain_steps(c, p, g, false, cs); },
+                                &c->chain_step[g][p]);
   }
   if (st == DEM_OK) {
+    /* the names alone: an earlier chain may still count down beside them */
     StepCtl h;
-    std::memset(&h, 0, sizeof(h));
     for (int p = 0; p < 2; p++) {
-      h.step[p] = c->chain_step[p];
+      for (int g = 0; g < kChainSizes; g++) h.step[g][p] = c->chain_step[g][p];
       h.single[p] = c->chain_single[p];
       h.rebuild[p] = c->chain_rebuild[p];
     }
-    st = cuda_check(cudaMemcpy(c->chain_ctl, &h, sizeof(h), cudaMemcpyHostToDevice), "step chain control");
+    const size_t at = offsetof(StepCtl, step);
+    st = cuda_check(cudaMemcpy((char*)c->chain_ctl + at, (char*)&h + at, sizeof(h) - at, cudaMemcpyHostToDevice),
+                    "step chain control");
   }
   return st;
 }
@@ -1077,13 +1095,14 @@ dem_status step_calls(dem_ctx* c, int nsteps) {
   int left = nsteps;
   if (c->opt.use_graph && c->opt.precision == DEM_PREC_MIXED && c->n > 0 && c->chain_state >= 0 && nsteps > 0) {
     /* steps chained on the device: one host launch for the whole call */
-    if (c->chain_state == 0) {
-      st = build_chain(c);
+    if (c->chain_state == 0 || (c->chain_state == 1 && nsteps > 1 && !c->chain_step[0][0])) {
+      st = build_chain(c, nsteps > 1);
       if (st == DEM_OK) {
         c->chain_state = 1;
       } else {
         /* this device or driver cannot launch these graphs from the device:
          * keep the conditional-node graphs */
+        cudaStreamSynchronize(c->stream); /* single steps may be under way */
         destroy_graph(c);
         c->chain_state = -1;
         cudaGetLastError();
@@ -1102,7 +1121,9 @@ dem_status step_calls(dem_ctx* c, int nsteps) {
          * device-launch copy, which outweighs that copy's later start */
         st = chain_set_left(c->chain_ctl, nsteps, c->stream);
         if (st != DEM_OK) return st;
-        e = cudaGraphLaunch(c->chain_step[p], c->stream);
+        int g = 0;
+        while (g + 1 < kChainSizes && 2 << g <= nsteps) g++;
+        e = cudaGraphLaunch(c->chain_step[g][p], c->stream);
       }
       if (e != cudaSuccess) return cuda_check(e, "cudaGraphLaunch");
       c->iter += nsteps;

@@ -32,13 +32,15 @@ namespace dem {
 
 struct MixedState; /* mixed.cu */
 
-/* device-side step chaining (chain.cu): the device-launchable graphs of one
- * step (with and without the countdown) and of a rebuild, per shadow parity,
- * and the countdown of the running chain */
+/* device-side step chaining (chain.cu): the device-launchable graphs of 1, 2, 4
+ * and 8 steps with the countdown, of one step without it and of a rebuild, per shadow
+ * parity, the countdown of the running chain, and the move flags of a graph's
+ * steps but the last */
+constexpr int kChainSizes = 4, kChainMost = 1 << (kChainSizes - 1);
 struct StepCtl {
   int left;
-  int pad;
-  cudaGraphExec_t step[2], single[2], rebuild[2];
+  int flag[kChainMost - 1];
+  cudaGraphExec_t step[kChainSizes][2], single[2], rebuild[2];
 };
 
 struct EngineBufs {
@@ -119,10 +121,11 @@ struct dem_ctx {
    * chained step is captured, the rebuild request word that gates its
    * kernels (NULL otherwise) */
   int chain_state;
-  cudaGraphExec_t chain_step[2], chain_single[2], chain_rebuild[2];
+  cudaGraphExec_t chain_step[dem::kChainSizes][2], chain_single[2], chain_rebuild[2];
   cudaGraphExec_t chain_single_host[2];
   dem::StepCtl* chain_ctl;
-  const int* step_gate;
+  const int* step_gate; /* capture of a chain graph: the word that holds a step back, */
+  int* step_flag;       /* and its move flag (NULL: b.flag) */
   /* dem_profile_kernels: when set, the rebuild and the step record an event
    * after each of their kernels (NULL otherwise, and always during capture) */
   std::vector<std::pair<const char*, cudaEvent_t>>* marks;
@@ -175,7 +178,8 @@ const float4* mixed_force_shadow(const dem_ctx* c);
 
 /* chain.cu: the chaining kernel after a step (tail-launches the rebuild and
  * the next step), the countdown, and the reset of the rebuild request */
-dem_status chain_launch_tail(StepCtl* ctl, int* flag, int* need, int* err, int parity, bool single, cudaStream_t s);
+dem_status chain_launch_tail(StepCtl* ctl, int* flag, int* need, int* err, int parity, int size, bool single,
+                             cudaStream_t s);
 dem_status chain_set_left(StepCtl* ctl, int nsteps, cudaStream_t s);
 dem_status chain_clear_request(int* flag, int* need, cudaStream_t s);
 

@@ -682,7 +682,10 @@ __device__ __forceinline__ float3 turned(float4 v, int e) {
  * next step's shadows and the counters. */
 template <bool WET, bool NET>
 __global__ void __launch_bounds__(128, DEM_BODY_BLOCKS) k_body_mixed(MixArgs a) {
-  if (a.gate && *a.gate) return;
+  if (a.gate && *a.gate) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *a.flag = -1; /* held back (chain.cu) */
+    return;
+  }
   const int q = reversed_block_thread(); /* the spheres with the most pairs first */
   const bool live = q < a.n;
   const int qq = live ? q : a.n - 1;
@@ -1661,7 +1664,7 @@ dem_status mixed_step(dem_ctx* c, int which, cudaStream_t s) {
   a.ps = b.ps; a.pair_out = reinterpret_cast<float4*>(b.pair_out);
   a.wall_out = m->wall_out; a.wall_entry = m->wall_entry;
   a.wlist = b.wlist; a.nwall = b.nwall; a.wrec = b.wrec;
-  a.force_out = m->force; a.flag = b.flag; a.err = b.err; a.counters = b.counters; a.cyl = b.cyl;
+  a.force_out = m->force; a.flag = c->step_flag ? c->step_flag : b.flag; a.err = b.err; a.counters = b.counters; a.cyl = b.cyl;
   a.sys_of_id = b.sys_of_id; a.sys_wet = b.sys_wet;
   a.n = c->n;
   a.force_cap = c->s.force_cap;
