@@ -42,6 +42,7 @@ struct dem_capnet {
   bool packed_valid;
   float host_params[4612]; /* the parameters as the FP32 network's kernel takes them */
   bool host_valid;
+  bool in_pieces; /* layer 2's weights are within the range of k_infer_split */
   int* gave_up; /* device: raised by a tensor-core kernel that gave up waiting */
 };
 
@@ -84,6 +85,12 @@ __device__ __forceinline__ float silu_acc(float z) {
   const float d = 1.0f + expf(fminf(-z, 80.0f));
   const float r = __fdividef(1.0f, d), q = z * r;
   return z > 80.0f ? z : fmaf(fmaf(-d, q, z), r, q);
+}
+/* silu_acc of a finite argument; an infinite one gives NaN */
+__device__ __forceinline__ float silu_finite(float z) {
+  const float d = 1.0f + expf(fminf(-z, 80.0f));
+  const float r = __fdividef(1.0f, d), q = z * r;
+  return fmaf(fmaf(-d, q, z), r, q);
 }
 __device__ __forceinline__ void std_inputs(const float* raw, const Norm& nz, float x[4]) {
   x[0] = (logf(raw[0]) - nz.xm[0]) / nz.xs[0];
@@ -441,84 +448,10 @@ __global__ void __launch_bounds__(kRedParams* kRedSlices) k_reduce_adam(float* P
   }
 }
 
-/* FP32 forward (the training precision) on raw features -> raw outputs, R rows
- * a thread with their hidden units in registers, A partial sums a dot product.
- * The weights are kernel parameters: they reach the FMAs through the constant
- * path, as uniform operands, where a shared-memory broadcast moves 512 bytes
- * into the register file per four weights and bounded the loop.  Bound by
- * instruction issue (82 %): 4,480 FMAs and 128 SiLUs a row.  1M rows: 271 us
- * (one row a thread with the hidden units in local memory and weights in shared
- * memory: 480). */
+/* the parameters as a kernel argument: uniform operands through the constant path */
 struct __align__(16) CapParams {
   float w[kWPad];
 };
-constexpr int kInferThreads = 128;
-template <int R, int A>
-__global__ void __launch_bounds__(kInferThreads) k_infer32(const __grid_constant__ CapParams P,
-                                                           const float* __restrict__ xr, long long n, Norm nz,
-                                                           float* __restrict__ y) {
-  const long long q0 = (long long)blockIdx.x * (kInferThreads * R) + threadIdx.x;
-  float h1[R][kCapH];
-#pragma unroll
-  for (int r = 0; r < R; r++) {
-    const long long q = q0 + r * kInferThreads;
-    float x[4] = {0.f, 0.f, 0.f, 0.f};
-    if (q < n) std_inputs(xr + 4 * q, nz, x);
-#pragma unroll
-    for (int m = 0; m < kCapH; m++) {
-      float z = P.w[kCapB1 + m];
-#pragma unroll
-      for (int i = 0; i < 4; i++) z = fmaf(P.w[kCapW1 + m * 4 + i], x[i], z);
-      h1[r][m] = silu_acc(z);
-    }
-  }
-  float y0[R], y1[R];
-#pragma unroll
-  for (int r = 0; r < R; r++) {
-    y0[r] = P.w[kCapB3];
-    y1[r] = P.w[kCapB3 + 1];
-  }
-#pragma unroll 1
-  for (int nn = 0; nn < kCapH; nn++) {
-    float z[R][A];
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-#pragma unroll
-      for (int k = 0; k < A; k++) z[r][k] = k ? 0.f : P.w[kCapB2 + nn];
-    }
-    const float4* w4 = reinterpret_cast<const float4*>(P.w + kCapW2 + nn * kCapH);
-#pragma unroll
-    for (int m = 0; m < kCapH / 4; m++) {
-      const float4 w = w4[m];
-#pragma unroll
-      for (int r = 0; r < R; r++) {
-        float& c = z[r][m % A];
-        c = fmaf(w.x, h1[r][4 * m], c);
-        c = fmaf(w.y, h1[r][4 * m + 1], c);
-        c = fmaf(w.z, h1[r][4 * m + 2], c);
-        c = fmaf(w.w, h1[r][4 * m + 3], c);
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-      float v = z[r][0];
-#pragma unroll
-      for (int k = 1; k < A; k++) v += z[r][k];
-      const float a = silu_acc(v);
-      y0[r] = fmaf(P.w[kCapW3 + nn], a, y0[r]);
-      y1[r] = fmaf(P.w[kCapW3 + kCapH + nn], a, y1[r]);
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < R; r++) {
-    const long long q = q0 + r * kInferThreads;
-    if (q < n) {
-      y[2 * q] = y0[r] * nz.ys[0] + nz.ym[0];
-      y[2 * q + 1] = y1[r] * nz.ys[1] + nz.ym[1];
-    }
-  }
-}
-
 /* BF16 tensor-core tiles, exactly as the fused step kernel evaluates them.  The
  * next tile's features are in flight while the current one runs (1M rows: 47
  * us, without 54; the 128 hardware tanh a row alone need 25). */
@@ -822,6 +755,229 @@ __global__ void __launch_bounds__(kTcRows, kTcBlocks) k_infer_tc5(const CapNetSm
 
 /* the plain closure on raw features: FP64 as the reference evaluates it
  * (kernel.cu:65-81 with pow/log/exp, :518), or the step kernel's FP32 form */
+/* ---------------- the FP32 network, its wide layer on the tensor cores ----------------
+ * FP32 forward (the training precision) on raw features -> raw outputs.  Layer 1
+ * (4 inputs), the SiLUs and layer 3 (2 outputs) stay FP32 on the CUDA cores; layer
+ * 2, nine tenths of the multiplications, takes both factors as sums of three BF16
+ * numbers, which hold an FP32 significand exactly, and adds the six products
+ * above 2^-24 of the largest in FP32 in tensor memory, the smallest first, each
+ * half of the hidden units in an accumulator of its own.  (The three products
+ * left out change nothing measurable.)  Its error against 64 bits is below that
+ * of 64 FP32 multiply-adds in a row: on the wet pairs' features 5.3e-8 and
+ * 7.9e-8 of the outputs' rms (before 6.5e-8 and 9.2e-8), largest 4.2e-7 and
+ * 5.2e-7 (5.1e-7 and 5.8e-7); with random weights of 0.05 to 3 as well.
+ *
+ * A block takes 128 rows, a thread each, as k_infer_tc5 does; 32 hidden units are
+ * written while the tensor cores work on the other 32, so the operand needs 24
+ * KB and four blocks share a multiprocessor.  The loops over units are not
+ * unrolled: unrolled, the body ran from beyond the instruction cache (206 us at
+ * 1M rows, 2.1 of 5 stall cycles an instruction).  Bound by instruction issue
+ * (76 %): the exponentials of 128 SiLUs a row.  A call on 1M rows 166 us (the
+ * FP32 units alone: 289), 100,000 48 (61), 1,000 34 (42). */
+constexpr int kSplit = 3, kSpUnits = 8, kSpBlocks = 4;
+/* Layer 2's weights are zero or of this size (2^-100 to 2^60), or k_infer_rows takes
+ * the network: the last pieces of smaller ones are subnormal numbers, which the
+ * tensor cores may flush, and larger ones magnify what is lost of an activation
+ * below 2^-110. */
+constexpr float kSpLeast = 7.888609052210118e-31f, kSpMost = 1.152921504606847e18f;
+constexpr uint32_t kSpCols = 2 * kCapH; /* tensor-memory columns: an accumulator for each half of the hidden units */
+struct __align__(128) SplitSmem {
+  __nv_bfloat16 a[kSplit][kTcRows * kCapH / 2];
+  __nv_bfloat16 b[kSplit][kCapH * kCapH];
+  unsigned long long mbar;
+  uint32_t tmem_base;
+};
+
+/* two values into their pieces: piece k of both in w[k] */
+__device__ __forceinline__ void split3(float a, float b, uint32_t (&w)[kSplit]) {
+#pragma unroll
+  for (int k = 0; k < kSplit; k++) {
+    w[k] = pack_bf16(a, b);
+    a -= __uint_as_float(w[k] << 16);
+    b -= __uint_as_float(w[k] & 0xffff0000u);
+  }
+}
+
+/* One row by FP32 multiply-adds alone, for the rows that the pieces cannot hold:
+ * an activation, weight or product beyond FP32's range (the largest BF16 is less
+ * than the largest FP32) leaves its row's outputs infinite or NaN. */
+__device__ __noinline__ void infer_row(const float* __restrict__ P, float x0, float x1, float x2, float x3, float& o0,
+                                       float& o1) {
+  if (isnan(x0) || isnan(x1) || isnan(x2) || isnan(x3)) return; /* NaN it is */
+  float h[kCapH];
+#pragma unroll 1
+  for (int m = 0; m < kCapH; m++) {
+    float z = P[kCapB1 + m];
+    z = fmaf(P[kCapW1 + 4 * m], x0, z);
+    z = fmaf(P[kCapW1 + 4 * m + 1], x1, z);
+    z = fmaf(P[kCapW1 + 4 * m + 2], x2, z);
+    z = fmaf(P[kCapW1 + 4 * m + 3], x3, z);
+    h[m] = silu_acc(z);
+  }
+  o0 = P[kCapB3];
+  o1 = P[kCapB3 + 1];
+#pragma unroll 1
+  for (int nn = 0; nn < kCapH; nn++) {
+    float z = P[kCapB2 + nn];
+#pragma unroll 4
+    for (int m = 0; m < kCapH; m++) z = fmaf(P[kCapW2 + nn * kCapH + m], h[m], z);
+    const float a = silu_acc(z);
+    o0 = fmaf(P[kCapW3 + nn], a, o0);
+    o1 = fmaf(P[kCapW3 + kCapH + nn], a, o1);
+  }
+}
+
+__global__ void __launch_bounds__(128) k_infer_rows(const float* __restrict__ params, const float* __restrict__ xr,
+                                                    long long n, Norm nz, float* __restrict__ y) {
+  const long long row = blockIdx.x * 128LL + threadIdx.x;
+  if (row >= n) return;
+  float x[4], o0 = nanf(""), o1 = o0;
+  std_inputs(xr + 4 * row, nz, x);
+  infer_row(params, x[0], x[1], x[2], x[3], o0, o1);
+  y[2 * row] = o0 * nz.ys[0] + nz.ym[0];
+  y[2 * row + 1] = o1 * nz.ys[1] + nz.ym[1];
+}
+
+/* err as for k_infer_tc5 */
+__global__ void __launch_bounds__(kTcRows, kSpBlocks) k_infer_split(const __grid_constant__ CapParams P,
+                                                                    const float* __restrict__ params,
+                                                                    const float* __restrict__ xr, long long n, Norm nz,
+                                                                    float* __restrict__ y, int* __restrict__ err) {
+  extern __shared__ __align__(128) unsigned char dsm[];
+  SplitSmem& sm = *reinterpret_cast<SplitSmem*>(dsm);
+  const int tid = threadIdx.x, warp = tid >> 5;
+  for (int e = tid; e < kCapH * kCapH / 2; e += kTcRows) {
+    const int nn = e >> 5, k = 2 * (e & 31);
+    const float* w = params + kCapW2 + nn * kCapH + k;
+    uint32_t piece[kSplit];
+    split3(w[0], w[1], piece);
+#pragma unroll
+    for (int t = 0; t < kSplit; t++)
+      *reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(sm.b[t]) + tc_off(nn, k, 8)) = piece[t];
+  }
+  const uint32_t mbar = smem_u32(&sm.mbar);
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem_base)),
+                 "r"(kSpCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  tc_sync();
+  const uint32_t tmem = sm.tmem_base;
+  const uint32_t lane_base = (uint32_t)(32 * warp) << 16; /* this warp's tensor-memory lanes */
+  uint32_t parity = 0;
+  bool ok = true;
+  const long long tiles = (n + kTcRows - 1) / kTcRows;
+  float f[4] = {1.f, 1.f, 0.f, 0.f};
+  {
+    const long long row = blockIdx.x * (long long)kTcRows + tid;
+    if (row < n)
+      for (int t = 0; t < 4; t++) f[t] = xr[4 * row + t];
+  }
+  for (long long tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+    const long long row = tile * kTcRows + tid;
+    float x[4];
+    std_inputs(f, nz, x);
+    {
+      const long long next = row + (long long)gridDim.x * kTcRows;
+      if (next < n)
+        for (int t = 0; t < 4; t++) f[t] = xr[4 * next + t];
+    }
+#pragma unroll 1
+    for (int u = 0; u < kCapH; u += kSpUnits) {
+      uint32_t w[kSpUnits / 2][kSplit];
+#pragma unroll
+      for (int m = 0; m < kSpUnits; m += 4) {
+        const float4 b1 = *reinterpret_cast<const float4*>(P.w + kCapB1 + u + m);
+        float h[4] = {b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          const float4 w1 = *reinterpret_cast<const float4*>(P.w + kCapW1 + 4 * (u + m + e));
+          h[e] = fmaf(w1.x, x[0], h[e]);
+          h[e] = fmaf(w1.y, x[1], h[e]);
+          h[e] = fmaf(w1.z, x[2], h[e]);
+          h[e] = fmaf(w1.w, x[3], h[e]);
+          h[e] = silu_finite(h[e]);
+        }
+        split3(h[0], h[1], w[m / 2]);
+        split3(h[2], h[3], w[m / 2 + 1]);
+      }
+      if (u == kCapH / 2) {
+        /* the first half's MMAs have read the operand that is written next */
+        ok = __syncthreads_and(tc_wait(mbar, parity)) != 0;
+        if (!ok) break;
+        parity ^= 1u;
+      }
+      const int c = u & (kCapH / 2 - 1);
+#pragma unroll
+      for (int t = 0; t < kSplit; t++)
+#pragma unroll
+        for (int m = 0; m < kSpUnits / 2; m += 4)
+          *reinterpret_cast<uint4*>(reinterpret_cast<char*>(sm.a[t]) + tc_off(tid, c + 2 * m, 4)) =
+              make_uint4(w[m][t], w[m + 1][t], w[m + 2][t], w[m + 3][t]);
+      if (c + kSpUnits < kCapH / 2) continue;
+      const int half = u / (kCapH / 2);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      tc_sync();
+      if (tid == 0) {
+        constexpr int pa[6] = {1, 0, 2, 0, 1, 0}, pb[6] = {1, 2, 0, 1, 0, 0};
+#pragma unroll
+        for (int t = 0; t < 6; t++)
+#pragma unroll
+          for (int k = 0; k < 2; k++) {
+            const unsigned long long da = tc_desc(smem_u32(sm.a[pa[t]]) + 256u * k, 128, 4 * 128);
+            const unsigned long long db = tc_desc(smem_u32(sm.b[pb[t]]) + 256u * (2 * half + k), 128, 8 * 128);
+            tc_mma(tmem + 64u * half, da, db, t > 0 || k > 0);
+          }
+        tc_commit(mbar);
+      }
+    }
+    if (!ok) break;
+    ok = __syncthreads_and(tc_wait(mbar, parity)) != 0;
+    if (!ok) break;
+    parity ^= 1u;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    float o0 = P.w[kCapB3], o1 = P.w[kCapB3 + 1];
+#pragma unroll 1
+    for (int c = 0; c < kCapH; c += 16) {
+      float v[16], u[16];
+      tc_ld16(tmem + lane_base + (uint32_t)c, v);
+      tc_ld16(tmem + 64u + lane_base + (uint32_t)c, u);
+#pragma unroll
+      for (int i = 0; i < 16; i++) v[i] += u[i];
+#pragma unroll
+      for (int i = 0; i < 16; i += 4) {
+        const float4 b2 = *reinterpret_cast<const float4*>(P.w + kCapB2 + c + i);
+        const float4 wa = *reinterpret_cast<const float4*>(P.w + kCapW3 + c + i);
+        const float4 wb = *reinterpret_cast<const float4*>(P.w + kCapW3 + kCapH + c + i);
+        const float h0 = silu_finite(v[i] + b2.x), h1 = silu_finite(v[i + 1] + b2.y);
+        const float h2 = silu_finite(v[i + 2] + b2.z), h3 = silu_finite(v[i + 3] + b2.w);
+        o0 = fmaf(wa.w, h3, fmaf(wa.z, h2, fmaf(wa.y, h1, fmaf(wa.x, h0, o0))));
+        o1 = fmaf(wb.w, h3, fmaf(wb.z, h2, fmaf(wb.y, h1, fmaf(wb.x, h0, o1))));
+      }
+    }
+    if (row < n) {
+      if (!isfinite(o0) || !isfinite(o1)) infer_row(params, x[0], x[1], x[2], x[3], o0, o1);
+      y[2 * row] = o0 * nz.ys[0] + nz.ym[0];
+      y[2 * row + 1] = o1 * nz.ys[1] + nz.ym[1];
+    }
+    /* every row is read before the barrier ahead of the next tile's MMAs */
+  }
+  if (!ok) {
+    if (tid == 0) atomicOr(err, 1);
+    tc_wait(mbar, parity);
+  }
+  tc_sync();
+  if (warp == 0) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kSpCols) : "memory");
+  }
+}
+
 __global__ void k_formula64(const float* __restrict__ xr, long long n, float* __restrict__ y, int angle) {
   const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (q >= n) return;
@@ -928,6 +1084,11 @@ dem_status ensure_host_params(dem_capnet* net) {
   dem_status st = ck(cudaMemcpy(net->host_params, net->params, sizeof(float) * kCapParams, cudaMemcpyDeviceToHost),
                      "capnet params download");
   net->host_valid = st == DEM_OK;
+  net->in_pieces = true;
+  for (int k = kCapW2; k < kCapB2; k++) {
+    const float w = std::fabs(net->host_params[k]);
+    if (w != 0.f && !(w >= kSpLeast && w <= kSpMost)) net->in_pieces = false;
+  }
   return st;
 }
 
@@ -1071,6 +1232,26 @@ dem_status dem_capnet_grad(dem_capnet* net, const float* x_dev, const float* y_d
   return st;
 }
 
+namespace {
+/* blocks of a persistent kernel over 128-row tiles, `each` to a multiprocessor */
+int tc_blocks(long long n, int each) {
+  int sms = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
+  return (int)std::min<long long>((n + kTcRows - 1) / kTcRows, (long long)std::max(1, sms) * each);
+}
+/* after the launch of a kernel that may give up: wait, and report */
+dem_status tc_finish(dem_capnet* net) {
+  dem_status st = ck(cudaGetLastError(), "dem_capnet_infer launch");
+  int h = 0; /* the copy waits for the kernel */
+  if (st == DEM_OK) st = ck(cudaMemcpy(&h, net->gave_up, sizeof(int), cudaMemcpyDeviceToHost), "dem_capnet_infer");
+  if (st == DEM_OK && h) {
+    cudaMemset(net->gave_up, 0, sizeof(int));
+    st = fail(DEM_ERR_CUDA, "dem_capnet_infer: tensor-core completion not seen in time");
+  }
+  return st;
+}
+}  // namespace
+
 dem_status dem_capnet_infer(dem_capnet* net, const float* x_dev, long long n, int tensor_cores, float* y_dev) {
   if (!net || !x_dev || !y_dev || n < 0) return fail(DEM_ERR_ARG, "dem_capnet_infer: bad arguments");
   if (!net->has_norm) return fail(DEM_ERR_STATE, "dem_capnet_infer: no standardisation");
@@ -1079,19 +1260,8 @@ dem_status dem_capnet_infer(dem_capnet* net, const float* x_dev, long long n, in
     /* the 5th-generation tensor cores: 128-row tiles, tcgen05.mma into tensor memory */
     dem_status st = ensure_packed(net);
     if (st != DEM_OK) return st;
-    const long long tiles = (n + kTcRows - 1) / kTcRows;
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
-    const int blocks = (int)std::min<long long>(tiles, (long long)std::max(1, sms) * kTcBlocks);
-    k_infer_tc5<<<blocks, kTcRows>>>(net->packed, x_dev, n, y_dev, net->gave_up);
-    st = ck(cudaGetLastError(), "dem_capnet_infer launch");
-    int h = 0; /* the copy waits for the kernel */
-    if (st == DEM_OK) st = ck(cudaMemcpy(&h, net->gave_up, sizeof(int), cudaMemcpyDeviceToHost), "dem_capnet_infer");
-    if (st == DEM_OK && h) {
-      cudaMemset(net->gave_up, 0, sizeof(int));
-      st = fail(DEM_ERR_CUDA, "dem_capnet_infer: tensor-core completion not seen in time");
-    }
-    return st;
+    k_infer_tc5<<<tc_blocks(n, kTcBlocks), kTcRows>>>(net->packed, x_dev, n, y_dev, net->gave_up);
+    return tc_finish(net);
   } else if (tensor_cores) {
     dem_status st = ensure_packed(net);
     if (st != DEM_OK) return st;
@@ -1101,12 +1271,17 @@ dem_status dem_capnet_infer(dem_capnet* net, const float* x_dev, long long n, in
   } else {
     dem_status st = ensure_host_params(net);
     if (st != DEM_OK) return st;
+    if (!net->in_pieces) {
+      k_infer_rows<<<blocks_for(n, 128), 128>>>(net->params, x_dev, n, norm_of(net), y_dev);
+      return tc_finish(net);
+    }
     const CapParams& P = *reinterpret_cast<const CapParams*>(net->host_params);
-    /* few rows: a row a thread in four partial sums, for the latency of its
-     * chain (a call on 1,000 rows 35 us, two a thread 61); from 100,000 rows on
-     * two a thread (1M rows: 289 a call, one a thread 316) */
-    if (n < 100000) k_infer32<1, 4><<<blocks_for(n, kInferThreads), kInferThreads>>>(P, x_dev, n, norm_of(net), y_dev);
-    else k_infer32<2, 1><<<blocks_for(n, 2 * kInferThreads), kInferThreads>>>(P, x_dev, n, norm_of(net), y_dev);
+    st = ck(cudaFuncSetAttribute(k_infer_split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SplitSmem)),
+            "dem_capnet_infer shared memory");
+    if (st != DEM_OK) return st;
+    const int blocks = tc_blocks(n, kSpBlocks);
+    k_infer_split<<<blocks, kTcRows, sizeof(SplitSmem)>>>(P, net->params, x_dev, n, norm_of(net), y_dev, net->gave_up);
+    return tc_finish(net);
   }
   dem_status st = ck(cudaGetLastError(), "dem_capnet_infer launch");
   if (st == DEM_OK) st = ck(cudaDeviceSynchronize(), "dem_capnet_infer");
