@@ -770,7 +770,10 @@ extern "C" dem_status dem_create(const dem_setup* s, const double* rad, const in
   b.ps.sides = c->opt.precision == DEM_PREC_MIXED ? 1 : 2;
   const size_t PS = P * (size_t)b.ps.sides;
   for (int k = 0; k < 2; k++) {
-    A(b.ps.pair[k], P); A(b.ps.off[k], N + 1); A(b.ps.rec[k], PS); A(b.ps.brg[k], PS);
+    A(b.ps.pair[k], P); A(b.ps.off[k], N + 1); A(b.ps.brg[k], PS);
+    char* rec = nullptr;
+    A(rec, b.ps.sides == 1 ? P * kPairRec32 : PS * sizeof(ContactRec));
+    b.ps.rec[k] = reinterpret_cast<ContactRec*>(rec);
   }
   A(b.ps.eidx, S); A(b.ps.ctl, 8);
   char* pair_out = nullptr;
@@ -1416,6 +1419,50 @@ struct HostPairs {
   std::vector<unsigned char> brg;
   std::vector<int> eidx, num, nidx, plevel;
 };
+/* a double as d2f (dem_device.cuh) truncates it: the FP32 copy that a record's spring has */
+float truncated(double x) {
+  unsigned long long u;
+  std::memcpy(&u, &x, sizeof(u));
+  unsigned f = (unsigned)(u >> 32) & 0x80000000u;
+  const int e = (int)((u >> 52) & 0x7ff), fe = e - 1023 + 127;
+  if (fe >= 255) f |= 0x7f800000u | (e == 0x7ff && (u & 0xfffffffffffffull) ? 1u : 0u);
+  else if (fe > 0) f |= ((unsigned)fe << 23) | (unsigned)((u >> 29) & 0x7fffffu);
+  float r;
+  std::memcpy(&r, &f, sizeof(r));
+  return r;
+}
+/* set cur's records to or from the host, mixed ones as the MixedRec of their two parts */
+cudaError_t copy_records(const PairSet& ps, int cur, std::vector<ContactRec>& rec, bool up) {
+  const size_t P = rec.size();
+  char* dev = reinterpret_cast<char*>(ps.rec[cur]);
+  const cudaMemcpyKind kind = up ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
+  auto copy = [&](char* d, void* h, size_t bytes) { return up ? cudaMemcpy(d, h, bytes, kind) : cudaMemcpy(h, d, bytes, kind); };
+  if (ps.sides == 2) return copy(dev, rec.data(), sizeof(ContactRec) * P);
+  struct Spring {
+    double d[4];
+  };
+  struct Law {
+    float nDsp, plstRad, plstDfm;
+    int stage;
+  };
+  static_assert(sizeof(Spring) + sizeof(Law) == kPairRec32, "the two parts of a record");
+  std::vector<Spring> a(P);
+  std::vector<Law> b(P);
+  MixedRec m;
+  for (size_t p = 0; up && p < P; p++) {
+    std::memcpy(&m, &rec[p], sizeof(m));
+    a[p] = Spring{{m.dx, m.dy, m.dz, m.nDsp_mx}};
+    b[p] = Law{m.nDsp, m.plstRad, m.plstDfm, m.stage};
+  }
+  cudaError_t e = copy(dev, a.data(), sizeof(Spring) * P);
+  if (e == cudaSuccess) e = copy(dev + sizeof(Spring) * (size_t)ps.cap, b.data(), sizeof(Law) * P);
+  for (size_t p = 0; !up && p < P; p++) {
+    m = MixedRec{a[p].d[0], a[p].d[1], a[p].d[2], a[p].d[3], truncated(a[p].d[0]), truncated(a[p].d[1]),
+                 truncated(a[p].d[2]), b[p].nDsp, b[p].plstRad, b[p].plstDfm, b[p].stage, 0};
+    std::memcpy(&rec[p], &m, sizeof(m));
+  }
+  return e;
+}
 dem_status fetch_pairs(dem_ctx* c, HostPairs& h, bool history) {
   EngineBufs& b = c->b;
   const size_t N = (size_t)c->n, S = (size_t)c->slots;
@@ -1431,8 +1478,7 @@ dem_status fetch_pairs(dem_ctx* c, HostPairs& h, bool history) {
     const size_t PS = (size_t)P * b.ps.sides;
     h.rec.resize(PS);
     h.brg.resize(PS);
-    if (e == cudaSuccess)
-      e = cudaMemcpy(h.rec.data(), b.ps.rec[cur], sizeof(ContactRec) * PS, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = copy_records(b.ps, cur, h.rec, false);
     if (e == cudaSuccess) e = cudaMemcpy(h.brg.data(), b.ps.brg[cur], PS, cudaMemcpyDeviceToHost);
   }
   if (e == cudaSuccess) e = cudaMemcpy(h.eidx.data(), b.ps.eidx, sizeof(int) * S, cudaMemcpyDeviceToHost);
@@ -1678,7 +1724,7 @@ extern "C" dem_status dem_load(dem_ctx* c, const char* path) {
     int cur = 0;
     cudaError_t e = cudaMemcpy(&cur, b.ps.ctl, sizeof(int), cudaMemcpyDeviceToHost);
     if (e == cudaSuccess)
-      e = cudaMemcpy(b.ps.rec[cur], hp.rec.data(), sizeof(ContactRec) * hp.rec.size(), cudaMemcpyHostToDevice);
+      e = copy_records(b.ps, cur, hp.rec, true);
     if (e == cudaSuccess) e = cudaMemcpy(b.ps.brg[cur], hp.brg.data(), hp.brg.size(), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cuda_check(e, "dem_load pair history");
   }

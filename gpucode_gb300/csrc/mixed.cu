@@ -91,7 +91,7 @@ struct MixArgs {
   double* pmove;
   const int *num_nebor, *plevel, *nidx, *npars, *nneb;
   PairSet ps;
-  float4* pair_out; /* two float4s per pair */
+  float4* pair_out; /* two float4s per pair, then what bridges and rolling add (k_pair_mixed) */
   float4* wall_out; /* the same per wall slot */
   const int* wall_entry; /* the listed wall slots, ctl[3] of them */
   unsigned wall_blocks;
@@ -313,17 +313,7 @@ __device__ __forceinline__ float bridge_rupture32(const MixArgs& a, float V, flo
   return a.lq_mode ? rupture32(V, th) : 0.99f * exp2f(0.33f * __log2f(V));
 }
 
-/* Two float4 of one 32-byte sector in one 256-bit access (p a multiple of 32
- * bytes): the pair kernel's gathers are bound by the L1's wavefronts, and
- * scattered lanes cost one per sector and instruction.  Shadows, records and
- * results in this form: 70.6 us a step on the packed 200k bed, 608 on 2M spheres;
- * as single float4 of separate arrays 75.1 and 664. */
-__device__ __forceinline__ void get2(const float4* p, float4& a, float4& b) {
-  asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-      : "l"(p));
-}
-/* the same, streaming */
+/* get2 and put2 (dem_device.cuh), streaming */
 __device__ __forceinline__ void get2cs(const float4* p, float4& a, float4& b) {
   asm volatile("ld.global.cs.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
       : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
@@ -415,6 +405,28 @@ __device__ __forceinline__ void cap_run_queue(const CapNetSmem& w, CapEntry* qw,
   }
 }
 
+/* pair p's record (pairs.cuh) */
+__device__ __forceinline__ MixedRec load_pair_rec(const float4* base, int cap, int p) {
+  MixedRec r;
+  float4* o = reinterpret_cast<float4*>(&r);
+  get2cs(base + 2 * (size_t)p, o[0], o[1]);
+  const float4 w = __ldcs(base + 2 * (size_t)cap + p);
+  r.fx = d2f(r.dx);
+  r.fy = d2f(r.dy);
+  r.fz = d2f(r.dz);
+  r.nDsp = w.x;
+  r.plstRad = w.y;
+  r.plstDfm = w.z;
+  r.stage = __float_as_int(w.w);
+  r.pad = 0;
+  return r;
+}
+__device__ __forceinline__ void store_pair_rec(float4* base, int cap, int p, const MixedRec& r) {
+  const float4* o = reinterpret_cast<const float4*>(&r);
+  put2cs(base + 2 * (size_t)p, o[0], o[1]);
+  __stcs(base + 2 * (size_t)cap + p, make_float4(r.nDsp, r.plstRad, r.plstDfm, __int_as_float(r.stage)));
+}
+
 /* One entry of the wall list (sphere q's wall slot w) against its cylinder, the
  * distance in FP64 (CirPWInterG, kernel.cu:958-1023).  The result: the force
  * and the normal force, the moment and the overlap (0: no contact).  Listed walls are evaluated from a compact
@@ -483,11 +495,11 @@ __device__ __forceinline__ void wall_entry(const MixArgs& a, int e) {
   a.wall_out[2 * (size_t)e + 1] = t;
 }
 
-/* resident blocks per SM the pair kernel is built for: 9 (56 registers, no
- * spills) 72.2 us a step on the packed 200k bed, 8 73.1, 7 75.0, 10 73.9; 2M
- * spheres 595, 610, 629, 600 us */
+/* resident blocks per SM the pair kernel is built for: 10 (48 registers, no
+ * spills) 60.9 us a step on the packed 200k bed, 9 62.1, 8 62.8; 2M spheres 573,
+ * 585, 598 us (there it moves 1.42 GB in 267 us, 78 % of the copy rate) */
 #ifndef DEM_PAIR_BLOCKS
-#define DEM_PAIR_BLOCKS 9
+#define DEM_PAIR_BLOCKS 10
 #endif
 
 /* One thread per pair of the list: overlap, contact law, capillary bridge, the
@@ -497,7 +509,8 @@ __device__ __forceinline__ void wall_entry(const MixArgs& a, int e) {
  * says that a bridge acts), the friction fT and the normal force with damping,
  * and, where a bridge acts or the material rolls, fN and the bridge's force:
  * u c_i and u c_j for the two spheres (formula, d = 1), or u c_i times the
- * network's output, d for the first sphere and c_j for the second. */
+ * network's output, d for the first sphere and c_j for the second.  Without
+ * rolling and network only c_i and c_j are left: 8 bytes a pair. */
 template <bool WET, bool NET>
 __global__ void __launch_bounds__(128, NET ? kNetBlocks : DEM_PAIR_BLOCKS) k_pair_mixed(const __grid_constant__ MixArgs a) {
   const int4 ct = pair_ctl(a.ps);
@@ -512,7 +525,7 @@ __global__ void __launch_bounds__(128, NET ? kNetBlocks : DEM_PAIR_BLOCKS) k_pai
   CapEntry* qw = reinterpret_cast<CapEntry*>(dsm + ((sizeof(CapNetSmem) + 15) / 16) * 16) + (threadIdx.x >> 5) * 32;
   const int P = ct.x ? ct.z : ct.y;
   const int2* __restrict__ pair = ct.x ? a.ps.pair[1] : a.ps.pair[0];
-  ContactRec* const rec = ct.x ? a.ps.rec[1] : a.ps.rec[0];
+  float4* const rec = reinterpret_cast<float4*>(ct.x ? a.ps.rec[1] : a.ps.rec[0]);
   unsigned char* const brg = ct.x ? a.ps.brg[1] : a.ps.brg[0];
   if (NET) {
     cap_stage(a.capw, reinterpret_cast<CapNetSmem*>(dsm));
@@ -548,13 +561,13 @@ __global__ void __launch_bounds__(128, NET ? kNetBlocks : DEM_PAIR_BLOCKS) k_pai
       float rj;
       gap = exact_gap(hi, lo, hj, lj, ax, ay, az, u, rj);
       if (gap < 0.f) {
-        MixedRec rc = load_rec(rec + p);
+        MixedRec rc = load_pair_rec(rec, a.ps.cap, p);
         const float3 cpv = f3(vi.x - vj.x, vi.y - vj.y, vi.z - vj.z) -
                            crossf(f3(wi.x, wi.y, wi.z) * ri + f3(wj.x, wj.y, wj.z) * rj, u);
         float fD;
         nrm = -gap;
         law32_forces(a.pp, ri * rj / (ri + rj), nrm, u, cpv, rc, a.dtf, fN, fD, fT);
-        store_rec(rec + p, rc);
+        store_pair_rec(rec, a.ps.cap, p, rc);
         s_n = fN + fD;
       }
       if (WET && (!a.sys_wet || a.sys_wet[a.sys_of_id[ro(a.id + i)]])) {
@@ -643,7 +656,12 @@ __global__ void __launch_bounds__(128, NET ? kNetBlocks : DEM_PAIR_BLOCKS) k_pai
       float4* o = a.pair_out + 2 * (size_t)p;
       put2(o, make_float4(u.x, u.y, u.z, __uint_as_float(__float_as_uint(nrm) | (wet ? 0x80000000u : 0u))),
            make_float4(fT.x, fT.y, fT.z, s_n));
-      if (wet || (a.rfrc != 0.f && nrm > 0.f)) a.pair_out[2 * (size_t)a.ps.cap + p] = make_float4(fN, ci, cj, d);
+      float4* more = a.pair_out + 2 * (size_t)a.ps.cap;
+      if (NET || a.rfrc != 0.f) {
+        if (wet || nrm > 0.f) more[p] = make_float4(fN, ci, cj, d);
+      } else if (wet) {
+        reinterpret_cast<float2*>(more)[p] = make_float2(ci, cj);
+      }
     }
   }
   if (NET && a.counters) {
@@ -654,11 +672,11 @@ __global__ void __launch_bounds__(128, NET ? kNetBlocks : DEM_PAIR_BLOCKS) k_pai
 }
 
 /* resident blocks per SM the sphere kernel is built for, and the pair results
- * a sphere has in flight: 6 and 3, 73.1 us a step on the packed 200k bed and 610
- * on 2M spheres; 4 in flight 78.1 and 641 (a few spills), 2 73.0 and 627; 5 blocks with
- * 4 77.6 and 623, 7 with 2 75.1 and 642, 8 with 1 75.6 and 633.  The indexes of the
- * next results are read while the present ones are on their way (690 to 664 us
- * on 2M spheres when this came in) */
+ * a sphere has in flight: 6 and 3, 62.1 us a step on the packed 200k bed and 585
+ * on 2M spheres; 2 in flight 62.8 and 610, 5 blocks with 4 67.0 and 588 (7 with 2 and
+ * 8 with 1 were 3 % slower still).  The indexes of the next results are read while
+ * the present ones are on their way (690 to 664 us on 2M spheres when this came
+ * in).  On 2M spheres it moves 1.49 GB in 288 us, 76 % of the copy rate. */
 #ifndef DEM_BODY_BLOCKS
 #define DEM_BODY_BLOCKS 6
 #endif
@@ -798,7 +816,14 @@ __global__ void __launch_bounds__(128, DEM_BODY_BLOCKS) k_body_mixed(MixArgs a) 
       if (e[t] != kNoPair) {
         const int p = e[t] < 0 ? ~e[t] : e[t];
         get2(a.pair_out + 2 * (size_t)p, nu[t], ft[t]);
-        if (WET || a.rfrc != 0.f) br[t] = a.pair_out[2 * (size_t)a.ps.cap + p];
+        const float4* more = a.pair_out + 2 * (size_t)a.ps.cap;
+        if (a.rfrc != 0.f) {
+          br[t] = more[p];
+        } else if (WET) {
+          const float2 c = reinterpret_cast<const float2*>(more)[p];
+          br[t].y = c.x;
+          br[t].z = c.y;
+        }
       }
     }
 #pragma unroll

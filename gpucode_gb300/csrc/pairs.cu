@@ -102,17 +102,6 @@ __global__ void k_pair_fill(PairSet ps, NeborLists nl, int n, int* __restrict__ 
   }
 }
 
-/* a mixed record's spring as the other sphere sees it */
-__device__ __forceinline__ void mirror(ContactRec& r) {
-  r.dx = -r.dx;
-  r.dy = -r.dy;
-  r.dz = -r.dz;
-  MixedRec& m = reinterpret_cast<MixedRec&>(r);
-  m.fx = -m.fx;
-  m.fy = -m.fy;
-  m.fz = -m.fz;
-}
-
 /* a record in two 256-bit accesses */
 union RecWords {
   ContactRec r;
@@ -164,20 +153,39 @@ __device__ __forceinline__ void carry_pair(const PairSet& ps, int cur, int n, in
       if (old[t].x == b && old[t].y == a) hit = t;
   }
   const bool turned = hit >= 0 && old[hit].x != oi;
-  for (int side = 0; side < ps.sides; side++) {
+  if (ps.sides == 1) {
+    const float4* from = reinterpret_cast<const float4*>(pick(ps.rec, cur));
+    float4* to = reinterpret_cast<float4*>(pick(ps.rec, 1 - cur));
+    float4 a4 = make_float4(0.f, 0.f, 0.f, 0.f), b4 = a4, law = a4;
+    unsigned char brg = 0;
+    if (hit >= 0) {
+      get2(from + 2 * (size_t)hit, a4, b4);
+      law = from[2 * (size_t)ps.cap + hit];
+      brg = pick(ps.brg, cur)[hit];
+      if (turned) { /* the spring as the other sphere sees it: the signs of three doubles */
+        a4.y = __uint_as_float(__float_as_uint(a4.y) ^ 0x80000000u);
+        a4.w = __uint_as_float(__float_as_uint(a4.w) ^ 0x80000000u);
+        b4.y = __uint_as_float(__float_as_uint(b4.y) ^ 0x80000000u);
+      }
+    }
+    put2(to + 2 * (size_t)p, a4, b4);
+    to[2 * (size_t)ps.cap + p] = law;
+    pick(ps.brg, 1 - cur)[p] = brg;
+    return;
+  }
+  for (int side = 0; side < 2; side++) {
     ContactRec r;
     unsigned char brg = 0;
     if (hit >= 0) {
-      const long long from = (long long)ps.sides * hit + (ps.sides == 2 && turned ? 1 - side : side);
+      const long long from = 2LL * hit + (turned ? 1 - side : side);
       r = read_rec(pick(ps.rec, cur) + from);
       brg = pick(ps.brg, cur)[from];
-      if (ps.sides == 1 && turned) mirror(r);
     } else {
       r.dx = r.dy = r.dz = r.nDsp = r.nDsp_mx = r.plstRad = r.plstDfm = 0.0;
       r.stage = 0;
     }
-    write_rec(pick(ps.rec, 1 - cur) + (long long)ps.sides * p + side, r);
-    pick(ps.brg, 1 - cur)[(long long)ps.sides * p + side] = brg;
+    write_rec(pick(ps.rec, 1 - cur) + 2LL * p + side, r);
+    pick(ps.brg, 1 - cur)[2LL * p + side] = brg;
   }
 }
 

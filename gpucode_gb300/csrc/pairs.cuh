@@ -16,13 +16,20 @@ constexpr int kNoPair = (int)0x80000000;
 /* bytes of one pair's result in a mixed step (mixed.cu) */
 constexpr size_t kPairOut32 = 48;
 
+/* A mixed pair's record in rec[]: the spring and the largest overlap in FP64 (32
+ * bytes, one sector, at 32 p) and, after cap of these, the overlap, plastic
+ * radius, plastic offset and load stage (16 bytes, at 16 p).  The FP32 copy of
+ * the spring that MixedRec has beside them is its truncation (d2f): 16 bytes a
+ * pair and direction less to move. */
+constexpr size_t kPairRec32 = 48;
+
 /* The pair arrays (device pointers), twice: ctl[0] is the current set,
  * ctl[1 + set] the number of pairs in it; ctl[3] counts the wall slots in use
  * (mixed.cu), ctl[4] the list entries that found no pair.  off: first
  * pair of each sphere (n + 1; the pairs after off[n] are one-sided).  eidx: per
  * neighbour slot, the pair's index, ~index where the slot's sphere is the
- * pair's second one.  sides: the records and flags a pair has, 1 (mixed) or 2
- * (FP64, one as each sphere sees it: record sides * p + side). */
+ * pair's second one.  sides: the records and flags a pair has, 1 (mixed, in two
+ * parts) or 2 (FP64, one as each sphere sees it: record sides * p + side). */
 struct PairSet {
   int2* pair[2];
   int* off[2];
