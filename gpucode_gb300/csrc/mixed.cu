@@ -694,6 +694,14 @@ __device__ __forceinline__ float3 turned(float4 v, int e) {
             __uint_as_float(__float_as_uint(v.z) ^ m));
 }
 
+/* the network's bridges of a warp's spheres that wait to be added: direction
+ * times reach, the network's output, and the same sphere's entry before */
+constexpr int kCapQ = 128;
+struct NetQueue {
+  float4 f[kCapQ];
+  short before[kCapQ];
+};
+
 /* One thread per sphere: gravity, its pairs' results summed in neighbour order
  * with Kahan compensation, the <= 3 cylinder-wall contacts (CirPWInterG,
  * kernel.cu:958-1023), the integrator (UpdateSystemG, kernel.cu:563-606), the
@@ -734,22 +742,20 @@ __global__ void __launch_bounds__(128, DEM_BODY_BLOCKS) k_body_mixed(MixArgs a) 
   if (NET) {
     /* The network's bridges join the sum a warp's queue at a time, the newest
      * first, once more than kCapQ - 32 wait: the order in which a kernel that
-     * queues them while it walks the slots adds them. */
-    constexpr int kCapQ = 128;
+     * queues them while it walks the slots adds them.  A sphere's entries are
+     * chained (read again from the results: 127.5 us a step, so 118). */
+    __shared__ NetQueue waiting[NET ? 4 : 1];
+    NetQueue& wq = waiting[NET ? threadIdx.x >> 5 : 0];
+    const unsigned below = (1u << (threadIdx.x & 31)) - 1u;
     const int nloop = __reduce_max_sync(0xffffffffu, nn);
-    int queued = 0, since = 0;
-    auto flush = [&](int end) {
-      for (int k = min(end, nn) - 1; k >= since; k--) {
-        const int e = ro(a.ps.eidx + base + (long long)k * stride);
-        if (e == kNoPair) continue;
-        const int p = e < 0 ? ~e : e;
-        const float4 nu = a.pair_out[2 * (size_t)p];
-        if (!(__float_as_uint(nu.w) >> 31)) continue;
-        const float4 br = a.pair_out[2 * (size_t)a.ps.cap + p];
-        if (br.w == 1.0f) continue;
-        F.add((turned(nu, e) * br.y) * (e < 0 ? br.z : br.w));
+    int queued = 0, last = -1; /* this sphere's newest entry */
+    auto flush = [&]() {
+      for (; last >= 0; last = wq.before[last]) {
+        const float4 v = wq.f[last];
+        F.add(f3(v.x, v.y, v.z) * v.w);
       }
-      since = end;
+      queued = 0;
+      __syncwarp(); /* read before the next entries overwrite them */
     };
     int en[kNetBatch];
 #pragma unroll
@@ -791,14 +797,19 @@ __global__ void __launch_bounds__(128, DEM_BODY_BLOCKS) k_body_mixed(MixArgs a) 
           wet++;
           if (!(nrm > 0.f)) nbr++;
         }
-        queued += __popc(__ballot_sync(0xffffffffu, net));
-        if (queued > kCapQ - 32) {
-          flush(k0 + t + 1);
-          queued = 0;
+        const unsigned m = __ballot_sync(0xffffffffu, net);
+        if (net) {
+          const int at = queued + __popc(m & below);
+          const float3 v = u * br[t].y;
+          wq.f[at] = make_float4(v.x, v.y, v.z, e[t] < 0 ? br[t].z : br[t].w);
+          wq.before[at] = (short)last;
+          last = at;
         }
+        queued += __popc(m);
+        if (queued > kCapQ - 32) flush();
       }
     }
-    flush(nloop);
+    flush();
   }
   int en[kBodyBatch];
 #pragma unroll
