@@ -311,71 +311,70 @@ __global__ void k_move_top_wall(CylinderBC* cyl, double dt) {
   if (blockIdx.x == 0 && threadIdx.x == 0) cyl->Tw = cyl->Tw + cyl->topv * dt;
 }
 
-/* The near walls of a block's spheres, compacted: one listed sphere in six
- * lists a wall and one in fifteen touches it, and an FP64 instruction costs a
- * warp the same for one lane as for 32, so the exact distance and the law run
- * over the block's list of walls that an FP32 gap leaves open (a wall farther
- * than its error bound adds nothing).  One pass per wall slot keeps a sphere's
- * walls in order.  A thread per sphere: 135 us on the packed 200k bed, with 3.4
- * of 32 lanes active; this 54 (blocks of 512 threads 63). */
-constexpr int kWallThreads = 256;
+/* One listed sphere in six lists a wall and one in fifteen touches it, those lie
+ * together, and an FP64 instruction costs a warp the same for one lane as for 32.
+ * So a block sifts kWallEach times as many spheres as it has threads, 32 at a time
+ * from all over the bed, by an FP32 gap (a wall farther than its error bound adds
+ * nothing), and takes those left as one dense list, a sphere's walls in order.
+ * A thread per sphere: 135 us on the packed 200k bed, with 3.4 of 32 lanes active;
+ * a block's own spheres compacted per wall slot 50, waiting at barriers; this 38. */
+constexpr int kWallThreads = 128, kWallEach = 3;
 template <class HA>
-__global__ void __launch_bounds__(kWallThreads, 3) k_wall_force64(
+__global__ void __launch_bounds__(kWallThreads) k_wall_force64(
     const double3* __restrict__ pos, const double3* __restrict__ vel, const double3* __restrict__ angvel,
     double3* __restrict__ force, double3* __restrict__ mom, double* __restrict__ rmom,
     const double* __restrict__ rad, const CylinderBC* __restrict__ cyl, HA h,
     const int* __restrict__ nwall, const int* __restrict__ wlist, size_t pitch, int n, int NP, LawK64 law,
     unsigned long long* __restrict__ counters) {
-  __shared__ int list[kWallThreads];
-  __shared__ double out[7][kWallThreads];
+  __shared__ int list[kWallThreads * kWallEach];
   __shared__ int listed;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int nw = i < n ? nwall[i] : 0;
-  if (!__syncthreads_or(nw > 0)) return;
+  if (threadIdx.x == 0) listed = 0;
+  __syncthreads();
   const CylinderBC c = *cyl;
-  const int* row = (const int*)((const char*)wlist + (size_t)(i < n ? i : 0) * pitch);
-  float px = 0.f, py = 0.f, pz = 0.f, ri = 0.f;
-  if (nw > 0) {
+  /* the gap from FP32 copies is within tol of the exact one: a few FP32 ulps of
+   * the largest coordinate involved, taken 8x */
+  auto near = [&](int w, float px, float py, float pz, float ri) {
+    float gc, tol;
+    if (w == 0 || w == 1) {
+      const float wz = d2f(w == 0 ? c.Tw : c.Bw);
+      gc = fabsf(pz - wz) - ri;
+      tol = 1e-6f * (fabsf(pz) + fabsf(wz) + ri);
+    } else if (w == 2) {
+      const float cx = d2f(c.cir.x), cy = d2f(c.cir.y), Rf = d2f(c.R);
+      const float dx = px - cx, dy = py - cy;
+      gc = fabsf(sqrtf(dx * dx + dy * dy) - Rf) - ri;
+      tol = 1e-6f * (fabsf(px) + fabsf(py) + fabsf(cx) + fabsf(cy) + Rf + ri);
+    } else {
+      return false;
+    }
+    return !(gc > tol);
+  };
+#pragma unroll
+  for (int e = 0; e < kWallEach; e++) {
+    const int i = ((e * (kWallThreads / 32) + (threadIdx.x >> 5)) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31);
+    const int nw = i < n ? nwall[i] : 0;
+    if (nw <= 0) continue;
     const double3 p = pos[i];
-    px = d2f(p.x);
-    py = d2f(p.y);
-    pz = d2f(p.z);
-    ri = d2f(rad[i]);
+    const float px = d2f(p.x), py = d2f(p.y), pz = d2f(p.z), ri = d2f(rad[i]);
+    const int* row = (const int*)((const char*)wlist + (size_t)i * pitch);
+    bool any = false;
+    for (int a = 0; a < nw; a++) any = any || near(row[a], px, py, pz, ri);
+    if (any) list[atomicAdd(&listed, 1)] = i;
   }
+  __syncthreads();
   int nc = 0;
-  for (int a = 0; a < 3; a++) {
-    if (threadIdx.x == 0) listed = 0;
-    if (!__syncthreads_or(a < nw)) break;
-    bool near = false;
-    if (a < nw) {
-      /* the gap from FP32 copies is within tol of the exact one: a few FP32
-       * ulps of the largest coordinate involved, taken 8x */
-      const int w = row[a];
-      float gc = 0.f, tol = -1.f;
-      if (w == 0 || w == 1) {
-        const float wz = d2f(w == 0 ? c.Tw : c.Bw);
-        gc = fabsf(pz - wz) - ri;
-        tol = 1e-6f * (fabsf(pz) + fabsf(wz) + ri);
-      } else if (w == 2) {
-        const float cx = d2f(c.cir.x), cy = d2f(c.cir.y), Rf = d2f(c.R);
-        const float dx = px - cx, dy = py - cy;
-        gc = fabsf(sqrtf(dx * dx + dy * dy) - Rf) - ri;
-        tol = 1e-6f * (fabsf(px) + fabsf(py) + fabsf(cx) + fabsf(cy) + Rf + ri);
-      }
-      near = tol >= 0.f && !(gc > tol);
-    }
-    int at = -1;
-    if (near) {
-      at = atomicAdd(&listed, 1);
-      list[at] = threadIdx.x;
-    }
-    __syncthreads();
-    for (int t = threadIdx.x; t < listed; t += kWallThreads) {
-      const int q = blockIdx.x * blockDim.x + list[t];
-      const int* rq = (const int*)((const char*)wlist + (size_t)q * pitch);
+  for (int t = threadIdx.x; t < listed; t += kWallThreads) {
+    const int q = list[t];
+    const int nw = nwall[q];
+    const int* rq = (const int*)((const char*)wlist + (size_t)q * pitch);
+    const double3 ip = pos[q];
+    const double ir = rad[q];
+    const float px = d2f(ip.x), py = d2f(ip.y), pz = d2f(ip.z), rf = d2f(ir);
+    double3 jv = make_double3(0.0, 0.0, 0.0); /* persists across walls (kernel.cu:980) */
+    for (int a = 0; a < nw; a++) {
       const int w = rq[a];
-      const double3 ip = pos[q];
-      const double ir = rad[q];
+      if (w == 0) jv.z = c.topv;
+      if (!near(w, px, py, pz, rf)) continue;
       double3 jp;
       if (w == 2) {
         /* the reference's pow(pow(dx, 2) + pow(dy, 2), 0.5) (kernel.cu:1009) as the
@@ -390,40 +389,23 @@ __global__ void __launch_bounds__(kWallThreads, 3) k_wall_force64(
       } else {
         jp = make_double3(ip.x, ip.y, w == 0 ? c.Tw : c.Bw);
       }
-      /* the top wall's velocity persists across the walls after it (kernel.cu:980) */
-      double3 jv = make_double3(0.0, 0.0, 0.0);
-      for (int b = 0; b <= a; b++)
-        if (rq[b] == 0) jv.z = c.topv;
       const double3 d = sub3(ip, jp);
       const double len = len3(d);
       const double gap = len - ir;
-      out[6][t] = -1.0;
-      if (gap < 0.0) {
-        const double3 u = div3(d, len);
-        const double3 cpv = sub3(sub3(vel[q], jv), cross3(mul3(angvel[q], ir), u));
-        const long long ine = (long long)a * NP + q;
-        HistRec rec = h.load(ine);
-        double3 dF, dM;
-        double dR;
-        contact_law64(law, ir, -gap, u, cpv, rec, ir, dF, dM, dR);
-        h.store(ine, rec);
-        out[0][t] = dF.x;
-        out[1][t] = dF.y;
-        out[2][t] = dF.z;
-        out[3][t] = dM.x;
-        out[4][t] = dM.y;
-        out[5][t] = dM.z;
-        out[6][t] = dR;
-      }
-    }
-    __syncthreads();
-    if (at >= 0 && !(out[6][at] < 0.0)) {
-      force[i] = add3(force[i], d3(out[0][at], out[1][at], out[2][at]));
-      mom[i] = add3(mom[i], d3(out[3][at], out[4][at], out[5][at]));
-      rmom[i] = rmom[i] + out[6][at];
+      if (!(gap < 0.0)) continue;
+      const double3 u = div3(d, len);
+      const double3 cpv = sub3(sub3(vel[q], jv), cross3(mul3(angvel[q], ir), u));
+      const long long ine = (long long)a * NP + q;
+      HistRec rec = h.load(ine);
+      double3 dF, dM;
+      double dR;
+      contact_law64(law, ir, -gap, u, cpv, rec, ir, dF, dM, dR);
+      h.store(ine, rec);
+      force[q] = add3(force[q], dF);
+      mom[q] = add3(mom[q], dM);
+      rmom[q] = rmom[q] + dR;
       nc++;
     }
-    __syncthreads();
   }
   if (counters && nc) atomicAdd(&counters[3], (unsigned long long)nc);
 }
@@ -504,7 +486,7 @@ dem_status wall_force64(const double3* pos, const double3* vel, const double3* a
   if (move_wall) k_move_top_wall<<<1, 32, 0, stream>>>(cyl, k.prm.dt);
   const LawK64 law = make_law64(k.pwcal, false, k.mat[0].dmpn * k.mat[1].dmpn, stage, k.mat[0].rfrc, k.prm.dt,
                                 k.lqd.layer);
-  k_wall_force64<HA><<<grid_for(n, kWallThreads), kWallThreads, 0, stream>>>(
+  k_wall_force64<HA><<<grid_for(n, kWallThreads * kWallEach), kWallThreads, 0, stream>>>(
       pos, vel, angvel, force, mom, rmom, rad, cyl, Acc<H>::make(h), nwall, wlist, pitch, n, NP, law, counters);
   return cuda_check(cudaGetLastError(), "wall_force64 launch");
 }
