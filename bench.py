@@ -15,9 +15,9 @@ One bench "step" is one DEM time step of the whole bed (rebuild when flagged,
 p-p contact + capillary, wall contact, integration).  The timed steps run as a
 run runs them: chained on the device in one dem_step call (each step graph
 launches the next, the rebuild decided on the device), CUDA events around the
-call.  A step moves ~233 MB through DRAM (ncu), more than the 129 MB L2, so the
-timed region evicts nothing: inputs larger than L2 (a chained step measures
-113.3 us, the step kernel alone with L2 evicted before it 113.8 us).  The same
+call.  A step's two kernels move ~163 MB through DRAM (ncu, cold caches), more
+than the 129 MB L2, so the timed region evicts nothing: inputs larger than L2 (a
+chained step measures 60 us, the kernels alone with L2 evicted before them 62).  The same
 steps launched one at a time with L2 evicted before each (a 256 MB write and a
 256 MB read outside the per-step events) are reported beside it
 (run.one_step_l2_evicted_ms_per_step).
@@ -59,7 +59,7 @@ def bed_config(w) -> dict:
     return {"workload": "wet200k-packed", "particles": w.setup.n, "levels": int(w.setup.s.n_levels), "dt_s": 5e-7,
             "bed": "tests/golden/packed_wet200k.npz (phi 0.662, Z 6.6; at rest, empty histories)",
             "start": "warm-up steps from the bed (the first builds the lists), then the timed steps",
-            "l2": "inputs larger than L2: one step moves ~233 MB through DRAM, the L2 holds 129 MB; no eviction"}
+            "l2": "inputs larger than L2: one step moves ~163 MB through DRAM from cold caches, the L2 holds 129 MB; no eviction"}
 
 
 def _peaks() -> tuple[float, str]:
@@ -613,8 +613,8 @@ def kernel_table(e, n: int) -> list:
     peak, _ = _peaks()
     rows = []
     for name, ms in e.profile_kernels():
-        key = "k_step_coop<1,0>" if name == "step kernel" else name
-        b = bpp.get(key)
+        # the table's capture has other kernels under these names
+        b = None if name in ("step kernel", "k_carry", "k_copy_back", "k_neighbor_find") else bpp.get(name)
         gbs = None if (b is None or ms <= 0) else b * n / (ms * 1e-3) / 1e9
         rows.append({"kernel": name, "ms": ms, "dram_bytes_scaled": None if b is None else b * n,
                      "achieved_gbs": gbs, "frac": None if gbs is None else gbs / peak})
@@ -624,7 +624,7 @@ def kernel_table(e, n: int) -> list:
 def traffic_from_profiles(kernel: str) -> float | None:
     """DRAM bytes per launch of the fused step kernel on the packed bed, from the
     committed ncu summary of the same kernel (None for a kernel without one)"""
-    name = {"k_step_mixed<1,0>": "step_mixed_packed200k.md"}.get(kernel)
+    name = {"k_pair_mixed<1,0> + k_body_mixed<1,0>": "step_pairs_packed200k.md"}.get(kernel)
     if name is None:
         return None
     p = ROOT / "profiles" / name
@@ -740,8 +740,7 @@ def run_headline(args, ws, rank):
     def timed_steps(e, steps, all_ranks=True):
         """`steps` steps of engine e chained on the device in one call (dem_step),
         as a run steps, CUDA events on its stream around the call; no L2 eviction:
-        a step's working set is ~233 MB against the 129 MB L2 (the chained step
-        measures the same as the step kernel alone with L2 evicted before it).
+        a step moves ~163 MB with cold caches against the 129 MB L2.
         Returns (ms total, wall s, clocks, stats before, after)"""
         st = torch.cuda.ExternalStream(e.stream())
         e.sync()
@@ -840,11 +839,12 @@ def run_headline(args, ws, rank):
             cpu_val, cpu_sample = cpu_oracle_rate(w, pos0, args.cpu_steps, threads)
         else:
             cpu_val, cpu_sample = None, "skipped (--cpu-steps 0)"
-        launches_per_step = 2  # fused step kernel + k_chain (each step graph launches the next)
-        # a step that finds the rebuild request set: its gated step kernel + k_chain, then the rebuild graph
-        # (clear request, bridge counts, copy_old, hash, 3 scan, scatter, order, permute, copy_back, shadows,
-        # neighbour, wall list, carry, inverse), then the step again (counted in launches_per_step)
-        rebuild_launches = 2 + 16
+        launches_per_step = 2  # pair and sphere kernel
+        # k_chain at the end of each graph of 8, 4, 2 or 1 steps
+        chain_launches = args.steps // 8 + bin(args.steps % 8).count("1")
+        # a rebuild (clear request, copy_old, hash, 2 scan, ranges, scatter, order, permute, copy_back, neighbour,
+        # wall list, wall entries, wall carry, 3 scan, pair fill, carry, one-sided, flip) and the k_chain before it
+        rebuild_launches = 1 + 21
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": ws, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True, "scaling": "weak",
@@ -857,7 +857,7 @@ def run_headline(args, ws, rank):
                     "wall_s": t_wall},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
-                         "kernel": kname + " (fused contact + capillary + wall + integrate)",
+                         "kernel": kname + " (contact + capillary + wall, then sums + integrate)",
                          "bytes_per_particle": bytes_per_particle, "kernel_ms": ms_k.value},
             "rebuild": rebuild,
             "cpu_baseline": {"value": cpu_val, "unit": UNIT, "cores": threads, "kind": "port",
@@ -865,7 +865,7 @@ def run_headline(args, ws, rank):
             "contact_evaluations_per_s": value * n_c,
             "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": n * 72, "d2h_bytes_per_step": n * 96},
             "e2e_parts_ms": e2e_parts,
-            "gpu_launches": launches_per_step * args.steps + rebuild_launches * d["rebuilds"],
+            "gpu_launches": launches_per_step * args.steps + chain_launches + rebuild_launches * d["rebuilds"],
             "clocks": ck,
             "accuracy_vs_fp64": accuracy,
             "reference_kernels_gpu": ref_gpu,

@@ -6,13 +6,13 @@ them directly, and each case holds a few GB on the device at most.
 
     python -m gpucode_gb300.ncu_cases step [--pairs thread|warp] [--steps 4] [--io]
         the packed 200,000-sphere wet bed: `steps` host-launched mixed steps
-        (the first rebuilds the lists); one step kernel per step; with --io
-        then an export, an import and one more step through page-locked host
-        arrays
+        (the first rebuilds the lists), a pair kernel and a sphere kernel each
+        whatever --pairs says; with --io then an export, an import and one more
+        step through page-locked host arrays
     python -m gpucode_gb300.ncu_cases closure [--rows 1000000]
         the packed bed with the per-contact liquid model: a network trained
         for 3 epochs on the bridges of one step, 3 host-launched steps with it
-        fused in the step kernel, then the network's inference on `rows`
+        fused in the pair kernel, then the network's inference on `rows`
         bridges: twice on the tcgen05 path, once on the warp tiles
     python -m gpucode_gb300.ncu_cases dropin [--precision fp64|mixed] [--steps 3]
         the packed bed through the reference's entry points in main.cpp's
