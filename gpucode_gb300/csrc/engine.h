@@ -125,6 +125,7 @@ struct dem_ctx {
   cudaGraphExec_t chain_single_host[2];
   dem::StepCtl* chain_ctl;
   const int* step_gate; /* capture of a chain graph: the word that holds a step back, */
+  int* body_order;      /* the sphere kernel's blocks, levels side by side (NULL: one level, or a small bed) */
   int* step_flag;       /* and its move flag (NULL: b.flag) */
   /* dem_profile_kernels: when set, the rebuild and the step record an event
    * after each of their kernels (NULL otherwise, and always during capture) */
@@ -149,6 +150,14 @@ dem_status mixed_create(dem_ctx* c);
 void mixed_destroy(dem_ctx* c);
 /* regenerate shadow buffer `which` from the FP64 master state */
 struct ShadowOut;
+/* threads per block of the step kernels */
+int mixed_block_size(const dem_ctx* c);
+/* Spheres from which the sphere kernel takes the levels side by side: about where
+ * the pairs' results (40 bytes each, 4.3 pairs a sphere on a packed bed) outgrow
+ * the L2.  Packed beds, us a step with and without: 300,000 spheres 94.1 and 85.5,
+ * 500,000 143.9 and 143.9, 600,000 171.7 and 175.5, 1,000,000 269.7 and 288.4,
+ * 2,000,000 520.2 and 569.9. */
+constexpr int kSideBySide = 600000;
 ShadowOut mixed_shadow_out(const dem_ctx* c, int which);
 const float4* mixed_motion(const dem_ctx* c, int which);
 dem_status mixed_shadows(dem_ctx* c, int which, cudaStream_t s);

@@ -85,6 +85,7 @@ struct Law32 {
 
 struct MixArgs {
   const float4 *place_in, *motion_in;
+  const int* body_order; /* the sphere kernel's blocks, levels side by side (NULL: in reverse) */
   float4 *place_out, *motion_out;
   double3 *pos, *vel, *angv;
   const double* rad;
@@ -712,7 +713,8 @@ __global__ void __launch_bounds__(128, DEM_BODY_BLOCKS) k_body_mixed(MixArgs a) 
     if (blockIdx.x == 0 && threadIdx.x == 0) *a.flag = -1; /* held back (chain.cu) */
     return;
   }
-  const int q = reversed_block_thread(); /* the spheres with the most pairs first */
+  const int q = a.body_order ? ro(a.body_order + blockIdx.x) * blockDim.x + threadIdx.x
+                             : reversed_block_thread(); /* the spheres with the most pairs first */
   const bool live = q < a.n;
   const int qq = live ? q : a.n - 1;
   __shared__ unsigned sums[5];
@@ -1633,6 +1635,12 @@ void mixed_destroy(dem_ctx* c) {
   c->mx = nullptr;
 }
 
+int mixed_block_size(const dem_ctx* c) {
+  /* the option (a multiple of 32 up to 128), else 128 */
+  const int ob = c->opt.block_size;
+  return (ob >= 32 && ob <= 32 * kWarps && ob % 32 == 0) ? ob : 32 * kWarps;
+}
+
 ShadowOut mixed_shadow_out(const dem_ctx* c, int which) {
   const MixedState* m = c->mx;
   return ShadowOut{m->place[which], m->motion[which], m->off, m->bin_exp, m->lo_scale};
@@ -1697,6 +1705,7 @@ dem_status mixed_step(dem_ctx* c, int which, cudaStream_t s) {
   a.motion_out = m->motion[1 - which];
   a.pos = b.pos; a.vel = b.vel; a.angv = b.angv; a.rad = b.rad; a.pmove = b.pmove;
   a.num_nebor = b.num_nebor; a.plevel = b.plevel; a.nidx = b.nidx; a.npars = b.npars; a.nneb = b.nneb;
+  a.body_order = c->body_order;
   a.ps = b.ps; a.pair_out = reinterpret_cast<float4*>(b.pair_out);
   a.wall_out = m->wall_out; a.wall_entry = m->wall_entry;
   a.wlist = b.wlist; a.nwall = b.nwall; a.wrec = b.wrec;
@@ -1735,9 +1744,7 @@ dem_status mixed_step(dem_ctx* c, int which, cudaStream_t s) {
   const bool net = c->s.force_cap == 1 && c->opt.capillary == DEM_CAP_MLP;
   if (net && !c->cap_w) return fail(DEM_ERR_STATE, "DEM_CAP_MLP: no network installed (dem_set_capnet)");
   const bool wet = c->s.force_cap == 1;
-  /* threads per block: the option (a multiple of 32 up to 128), else 128 */
-  const int ob = c->opt.block_size;
-  const int bs = (ob >= 32 && ob <= 32 * kWarps && ob % 32 == 0) ? ob : 32 * kWarps;
+  const int bs = mixed_block_size(c);
   /* The pair count is known on the device only: the grid covers six pairs a
    * sphere (a packed bed lists 4.3) and strides beyond; the closure's blocks
    * stage its weights once, so they are as many as stay resident. */

@@ -187,3 +187,26 @@ def test_longer_lists_change_no_force(cuda, precision):
     assert got[2][0] * 32 / w.setup.n > 2 * 320 > got[0][0] * 32 / w.setup.n
     for _, f in got[1:]:
         np.testing.assert_array_equal(f, got[0][1])
+
+
+def test_levels_side_by_side_step_every_sphere(cuda):
+    """from 600,000 spheres on the sphere kernel takes its blocks level beside
+    level (level sizes that are no multiples of a block): three steps give the
+    FP64 engine's, forces to 2e-5 of their scale as elsewhere, and every sphere
+    has moved once a step (from rest, gravity alone is 5e-7 x 9.8 of velocity a
+    step in the reduced units, far above FP64's resolution)"""
+    from gpucode_gb300 import configs
+
+    w = configs.wet(n=600_053, cyl_r=0.04)
+    out = {}
+    for precision in ("fp64", "mixed"):
+        e = Engine(w.setup, precision=precision)
+        e.set_state(w.pos0_reduced)
+        e.step(3)
+        e.sync()
+        out[precision] = e.get_state()
+        e.close()
+    f, g = out["fp64"], out["mixed"]
+    assert (np.abs(g["vel"]).max(axis=1) > 0).all()
+    np.testing.assert_allclose(g["force"], f["force"], rtol=2e-5, atol=2e-5 * np.abs(f["force"]).max())
+    np.testing.assert_allclose(g["pos"], f["pos"], rtol=0, atol=1e-9)
