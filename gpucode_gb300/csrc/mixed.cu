@@ -366,10 +366,13 @@ __device__ __forceinline__ void warp_add(unsigned long long* ctr, unsigned v) {
 struct __align__(16) CapEntry {
   float sep, vol, theta, ratio; /* raw features */
 };
+/* resident blocks per SM the network variant is built for: 8 (64 registers, some
+ * spills) 114.4 us a closure step on the packed 200k bed, 7 114.6, 6 116.7, 5 122.6, 9
+ * 118.6 */
 #ifndef DEM_NET_BLOCKS
-#define DEM_NET_BLOCKS 6
+#define DEM_NET_BLOCKS 8
 #endif
-constexpr int kNetBlocks = DEM_NET_BLOCKS; /* resident blocks per SM the network variant is built for */
+constexpr int kNetBlocks = DEM_NET_BLOCKS;
 constexpr int kWarps = 4;                  /* warps per block of the step kernels */
 constexpr size_t kCapSmem = ((sizeof(CapNetSmem) + 15) / 16) * 16 + sizeof(CapEntry) * 32 * kWarps;
 
