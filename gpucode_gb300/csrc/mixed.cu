@@ -512,9 +512,10 @@ __device__ __forceinline__ void wall_entry(const MixArgs& a, int e) {
  * but for their sign: the normal u and the overlap (0: no contact; the sign bit
  * says that a bridge acts), the friction fT and the normal force with damping,
  * and, where a bridge acts or the material rolls, fN and the bridge's force:
- * u c_i and u c_j for the two spheres (formula, d = 1), or u c_i times the
- * network's output, d for the first sphere and c_j for the second.  Without
- * rolling and network only c_i and c_j are left: 8 bytes a pair. */
+ * u c_i and u c_j for the two spheres (formula), or u c_i times the network's
+ * output, d for the first sphere and c_j for the second.  Which of the two is
+ * the sign bit of fN, which is never negative: the outputs take any value.
+ * Without rolling and network only c_i and c_j are left: 8 bytes a pair. */
 template <bool WET, bool NET>
 __global__ void __launch_bounds__(128, NET ? kNetBlocks : DEM_PAIR_BLOCKS) k_pair_mixed(const __grid_constant__ MixArgs a) {
   const int4 ct = pair_ctl(a.ps);
@@ -546,7 +547,7 @@ __global__ void __launch_bounds__(128, NET ? kNetBlocks : DEM_PAIR_BLOCKS) k_pai
     bool want = false; /* NET: this lane's bridge goes to the network */
     bool form = false, wet = false;
     int bprev = 0;
-    float gap = 0.f, fN = 0.f, nrm = 0.f, s_n = 0.f, ci = 0.f, cj = 0.f, d = 1.0f;
+    float gap = 0.f, fN = 0.f, nrm = 0.f, s_n = 0.f, ci = 0.f, cj = 0.f, d = 0.f;
     float3 fT = f3(0.f, 0.f, 0.f), u = f3(0.f, 0.f, 0.f);
     CapEntry ent, ent_j;
     bool want_j = false;
@@ -662,7 +663,8 @@ __global__ void __launch_bounds__(128, NET ? kNetBlocks : DEM_PAIR_BLOCKS) k_pai
            make_float4(fT.x, fT.y, fT.z, s_n));
       float4* more = a.pair_out + 2 * (size_t)a.ps.cap;
       if (NET || a.rfrc != 0.f) {
-        if (wet || nrm > 0.f) more[p] = make_float4(fN, ci, cj, d);
+        if (wet || nrm > 0.f)
+          more[p] = make_float4(__uint_as_float(__float_as_uint(fN) | (want ? 0x80000000u : 0u)), ci, cj, d);
       } else if (wet) {
         reinterpret_cast<float2*>(more)[p] = make_float2(ci, cj);
       }
@@ -793,11 +795,11 @@ __global__ void __launch_bounds__(128, DEM_BODY_BLOCKS) k_body_mixed(MixArgs a) 
           F.add(ft[t].w * u + fT);
           const float arm = ri - nrm * 0.5f;
           M.add(crossf(u * (-arm), fT));
-          if (a.rfrc != 0.f) R.add(0.5f * (a.rfrc + a.rfrc) * br[t].x * ri);
+          if (a.rfrc != 0.f) R.add(0.5f * (a.rfrc + a.rfrc) * fabsf(br[t].x) * ri);
           ncont++;
         }
         if (nb >> 31) {
-          net = br[t].w != 1.0f;
+          net = __float_as_uint(br[t].x) >> 31 != 0u; /* the network's, not the formula's */
           if (!net) F.add(u * (e[t] < 0 ? br[t].z : br[t].y));
           wet++;
           if (!(nrm > 0.f)) nbr++;
