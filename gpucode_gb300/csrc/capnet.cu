@@ -73,22 +73,26 @@ Norm norm_of(const dem_capnet* net) {
 /* 1 / (1 + e^-z) and z / (1 + e^-z) in FP32: the hardware reciprocal with one
  * Newton correction (within an ulp of the quotient) instead of the general
  * division, whose range handling costs as much again as the exponential.  The
- * exponent stops at 80, so the divisor stays finite; beyond 80 the SiLU is its
- * argument (infinity included), and -infinity and NaN give NaN, as the plain
- * quotient does.  No branches: a thread's units overlap. */
+ * exponent stops at 88, so the divisor stays finite, and e^88 is above 2^126,
+ * from where __fdividef gives 0: a z below -87.4 has the sigmoid 0 and the SiLU
+ * -0 at any size (stopping below 2^126 left z times a reciprocal of 1e-35, which
+ * is -6136 at z = -3.4e38).  Beyond 80 the SiLU is its argument (infinity
+ * included), and -infinity and NaN give NaN, as the plain quotient does.  No
+ * branches: a thread's units overlap. */
+constexpr float kExpStop = 88.0f;
 __device__ __forceinline__ float sigmoid_acc(float z) {
-  const float d = 1.0f + expf(fminf(-z, 80.0f));
+  const float d = 1.0f + expf(fminf(-z, kExpStop));
   const float r = __fdividef(1.0f, d);
   return fmaf(fmaf(-d, r, 1.0f), r, r);
 }
 __device__ __forceinline__ float silu_acc(float z) {
-  const float d = 1.0f + expf(fminf(-z, 80.0f));
+  const float d = 1.0f + expf(fminf(-z, kExpStop));
   const float r = __fdividef(1.0f, d), q = z * r;
   return z > 80.0f ? z : fmaf(fmaf(-d, q, z), r, q);
 }
 /* silu_acc of a finite argument; an infinite one gives NaN */
 __device__ __forceinline__ float silu_finite(float z) {
-  const float d = 1.0f + expf(fminf(-z, 80.0f));
+  const float d = 1.0f + expf(fminf(-z, kExpStop));
   const float r = __fdividef(1.0f, d), q = z * r;
   return fmaf(fmaf(-d, q, z), r, q);
 }
