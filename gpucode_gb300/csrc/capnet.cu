@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <numeric>
 #include <random>
@@ -27,6 +28,14 @@
 #include "capnet.cuh"
 #include "dem_device.cuh"
 #include "engine.h"
+
+namespace dem {
+constexpr int kWPad = 4612; /* parameters, padded to a multiple of 16 bytes */
+/* the parameters as a kernel argument: uniform operands through the constant path */
+struct __align__(16) CapParams {
+  float w[kWPad];
+};
+}  // namespace dem
 
 struct dem_capnet {
   float* params;   /* device, kCapParams FP32 */
@@ -40,11 +49,12 @@ struct dem_capnet {
   bool has_norm;
   dem::CapNetSmem* packed; /* device, BF16 network as the step kernel stages it */
   bool packed_valid;
-  float host_params[4612]; /* the parameters as the FP32 network's kernel takes them */
+  dem::CapParams host_params; /* the parameters as the FP32 network's kernel takes them */
   bool host_valid;
   bool in_pieces; /* layer 2's weights are within the range of k_infer_split */
   int* gave_up; /* device: raised by a tensor-core kernel that gave up waiting */
 };
+static_assert(offsetof(dem_capnet, host_params) % alignof(dem::CapParams) == 0, "copied by 16-byte accesses");
 
 namespace dem {
 namespace {
@@ -56,7 +66,6 @@ constexpr int kLd = kCapH + 4;     /* padded row of a 64-wide operand, 16-byte a
 /* the gradients other than dW2, as a block collects them */
 constexpr int kSmW1 = 0, kSmB1 = kSmW1 + kCapH * kCapIn, kSmB2 = kSmB1 + kCapH, kSmW3 = kSmB2 + kCapH,
               kSmB3 = kSmW3 + kCapOut * kCapH, kSmLoss = kSmB3 + kCapOut, kSmall = kSmLoss + 1;
-constexpr int kWPad = 4612;        /* parameters in shared memory, 16-byte multiple */
 
 inline int blocks_for(long long n, int b) { return n <= 0 ? 1 : (int)((n + b - 1) / b); }
 
@@ -452,10 +461,6 @@ __global__ void __launch_bounds__(kRedParams* kRedSlices) k_reduce_adam(float* P
   }
 }
 
-/* the parameters as a kernel argument: uniform operands through the constant path */
-struct __align__(16) CapParams {
-  float w[kWPad];
-};
 /* BF16 tensor-core tiles, exactly as the fused step kernel evaluates them.  The
  * next tile's features are in flight while the current one runs (1M rows: 47
  * us, without 54; the 128 hardware tanh a row alone need 25). */
@@ -1085,14 +1090,16 @@ dem_status ensure_packed(dem_capnet* net) {
 
 dem_status ensure_host_params(dem_capnet* net) {
   if (net->host_valid) return DEM_OK;
-  dem_status st = ck(cudaMemcpy(net->host_params, net->params, sizeof(float) * kCapParams, cudaMemcpyDeviceToHost),
+  dem_status st = ck(cudaMemcpy(net->host_params.w, net->params, sizeof(float) * kCapParams, cudaMemcpyDeviceToHost),
                      "capnet params download");
-  net->host_valid = st == DEM_OK;
-  net->in_pieces = true;
+  if (st != DEM_OK) return st;
+  bool fits = true;
   for (int k = kCapW2; k < kCapB2; k++) {
-    const float w = std::fabs(net->host_params[k]);
-    if (w != 0.f && !(w >= kSpLeast && w <= kSpMost)) net->in_pieces = false;
+    const float w = std::fabs(net->host_params.w[k]);
+    if (w != 0.f && !(w >= kSpLeast && w <= kSpMost)) fits = false;
   }
+  net->in_pieces = fits;
+  net->host_valid = true;
   return st;
 }
 
@@ -1279,12 +1286,11 @@ dem_status dem_capnet_infer(dem_capnet* net, const float* x_dev, long long n, in
       k_infer_rows<<<blocks_for(n, 128), 128>>>(net->params, x_dev, n, norm_of(net), y_dev);
       return tc_finish(net);
     }
-    const CapParams& P = *reinterpret_cast<const CapParams*>(net->host_params);
     st = ck(cudaFuncSetAttribute(k_infer_split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SplitSmem)),
             "dem_capnet_infer shared memory");
     if (st != DEM_OK) return st;
     const int blocks = tc_blocks(n, kSpBlocks);
-    k_infer_split<<<blocks, kTcRows, sizeof(SplitSmem)>>>(P, net->params, x_dev, n, norm_of(net), y_dev, net->gave_up);
+    k_infer_split<<<blocks, kTcRows, sizeof(SplitSmem)>>>(net->host_params, net->params, x_dev, n, norm_of(net), y_dev, net->gave_up);
     return tc_finish(net);
   }
   dem_status st = ck(cudaGetLastError(), "dem_capnet_infer launch");
