@@ -389,6 +389,9 @@ dem_status enqueue_step(dem_ctx* c, cudaStream_t s, int parity) {
 }
 
 void destroy_graph(dem_ctx* c) {
+  /* a chain's graphs launch one another from the device: none may be gone while
+   * an earlier call's steps are under way */
+  cudaStreamSynchronize(c->stream);
   for (int p = 0; p < 2; p++) {
     cudaGraphExec_t* all[5 + kChainSizes] = {&c->graph_exec[p], &c->graph_one[p], &c->chain_single[p],
                                              &c->chain_rebuild[p], &c->chain_single_host[p]};
@@ -903,7 +906,6 @@ extern "C" dem_status dem_set_systems(dem_ctx* c, int n_sys, const int* system_o
 
 extern "C" dem_status dem_destroy(dem_ctx* c) {
   if (!c) return DEM_OK;
-  cudaStreamSynchronize(c->stream);
   destroy_graph(c);
   if (c->mx) mixed_destroy(c);
   for (void* p : c->allocs) cudaFree(p);
@@ -1132,7 +1134,6 @@ dem_status step_calls(dem_ctx* c, int nsteps) {
       } else {
         /* this device or driver cannot launch these graphs from the device:
          * keep the conditional-node graphs */
-        cudaStreamSynchronize(c->stream); /* single steps may be under way */
         destroy_graph(c);
         c->chain_state = -1;
         cudaGetLastError();
