@@ -388,7 +388,9 @@ dem_status enqueue_step(dem_ctx* c, cudaStream_t s, int parity) {
   return update64(b.rad, b.pos, b.vel, b.angv, b.force, b.mom, b.rmom, b.flag, b.pmove, n, c->k, s);
 }
 
-void destroy_graph(dem_ctx* c) {
+}  // namespace
+
+void drop_graphs(dem_ctx* c) {
   /* a chain's graphs launch one another from the device: none may be gone while
    * an earlier call's steps are under way */
   cudaStreamSynchronize(c->stream);
@@ -401,9 +403,9 @@ void destroy_graph(dem_ctx* c) {
       *g = nullptr;
     }
   }
-  /* rebuilt on the next step against the new configuration */
-  if (c->chain_state > 0) c->chain_state = 0;
 }
+
+namespace {
 
 /* G steps: [decide -> IF(rebuild) -> step] x G; the mixed path's shadow
  * parity alternates from start_parity */
@@ -899,14 +901,15 @@ extern "C" dem_status dem_set_systems(dem_ctx* c, int n_sys, const int* system_o
   b.n_sys = n_sys;
   /* graphs captured the single-cylinder pointers: rebuild them; and the wall
    * lists must be rebuilt against the new cylinders */
-  destroy_graph(c);
+  drop_graphs(c);
+  if (c->chain_state > 0) c->chain_state = 0;
   const int one = 1;
   return cuda_check(cudaMemcpy(b.need, &one, sizeof(int), cudaMemcpyHostToDevice), "dem_set_systems");
 }
 
 extern "C" dem_status dem_destroy(dem_ctx* c) {
   if (!c) return DEM_OK;
-  destroy_graph(c);
+  drop_graphs(c);
   if (c->mx) mixed_destroy(c);
   for (void* p : c->allocs) cudaFree(p);
   for (cudaEvent_t ev : c->xev) cudaEventDestroy(ev);
@@ -1127,14 +1130,14 @@ dem_status step_calls(dem_ctx* c, int nsteps) {
   int left = nsteps;
   if (c->opt.use_graph && c->opt.precision == DEM_PREC_MIXED && c->n > 0 && c->chain_state >= 0 && nsteps > 0) {
     /* steps chained on the device: one host launch for the whole call */
-    if (c->chain_state == 0 || (c->chain_state == 1 && nsteps > 1 && !c->chain_step[0][0])) {
+    if (!c->chain_single[0] || (nsteps > 1 && !c->chain_step[0][0])) {
       st = build_chain(c, nsteps > 1);
       if (st == DEM_OK) {
         c->chain_state = 1;
       } else {
         /* this device or driver cannot launch these graphs from the device:
          * keep the conditional-node graphs */
-        destroy_graph(c);
+        drop_graphs(c);
         c->chain_state = -1;
         cudaGetLastError();
       }

@@ -113,8 +113,8 @@ struct dem_ctx {
   int parity; /* mixed: which shadow buffer the next step reads */
   int radii_bounded; /* every radius is at most its level's size: the neighbour search may skip far rows */
   int moving_walls; /* a cylinder's top wall moves (topv != 0): moved before every step's wall contacts */
-  /* device-side step chaining (mixed precision): 0 not built yet, 1 built,
-   * -1 unavailable (the conditional-node graphs run instead); the graphs
+  /* device-side step chaining (mixed precision): 0 not built yet, 1 built (its
+   * graphs anew if they were dropped since), -1 unavailable (the conditional-node graphs run instead); the graphs
    * (instantiated for device launch) and a host-instantiated copy of the
    * one-step graph for dem_step(1) (launched from the host, a device-launch
    * graph starts ~5 us later); the control block on the device; and, while a
@@ -144,6 +144,10 @@ struct dem_ctx {
 };
 
 namespace dem {
+
+/* engine.cu: wait for the context's steps and destroy its captured graphs; the
+ * next dem_step captures them again, with the configuration of then */
+void drop_graphs(dem_ctx* c);
 
 /* mixed.cu */
 dem_status mixed_create(dem_ctx* c);
