@@ -249,7 +249,8 @@ __global__ void k_cell_order(const int* __restrict__ sorted_hash, int* __restric
  * the reference searches a box of cells, rounded up from the ratio of the
  * levels, of which the sphere that matters fills a quarter (a level-1 sphere
  * has 88 candidates in the boxes of the packed bed's four levels).  What is
- * skipped fails the distance test, so the list and its order stay.  Bound by
+ * skipped fails the distance test, so the list and its order stay; grids a few
+ * cells wide are searched whole (spheres past their upper faces lie elsewhere).  Bound by
  * instruction issue (60 %, 16 of 32 lanes).  Packed 200k bed 237 -> 108 us, 2M
  * spheres 1305 -> 774; eight lanes a sphere measured 205 and 1919 (shuffles),
  * rows and candidates in unrolled batches 252 and 3334 (instruction cache).
@@ -365,13 +366,17 @@ __global__ void __launch_bounds__(128) k_neighbor_find(
     const float far = pre.prune ? (hi_i.w + d2f(lv.level_size[iL]) + sg) * 1.0001f + 8.0f * pre.ulp +
                                       1.0e-6f * (fabsf(xf) + fabsf(yf) + fabsf(zf))
                                 : 0.f;
+    /* a sphere past the grid's upper x or y face is hashed into the first cell of
+     * the next row or plane: where the grid is so narrow that the box of a sphere
+     * within reach of that face holds such a cell, nothing is skipped */
+    const bool prune = pre.prune && (float)min(gs.x, gs.y) > (float)off + far * rc + 1.01f;
     /* planes and rows in the reference's (z, y) order, from those that `far`
      * reaches; the next row's range is in flight while the current one's
      * particles are visited.  One copy of the loop's body: unrolled over a
      * batch of rows it ran from beyond the instruction cache (3.8 of 11 stall
      * cycles an instruction) */
     int z = max(g.z - off, 0), z1 = min(g.z + off, gs.z - 1);
-    if (pre.prune) {
+    if (prune) {
       z = max(z, near_cell(zf - far, rc, -1.0e-4f, gs.z - 1));
       z1 = min(z1, near_cell(zf + far, rc, 1.0e-4f, gs.z - 1));
     }
@@ -388,7 +393,7 @@ __global__ void __launch_bounds__(128) k_neighbor_find(
           more = ++z <= z1;
           y = max(g.y - off, 0);
           y1 = min(g.y + off, gs.y - 1);
-          if (pre.prune && more) {
+          if (prune && more) {
             const float dz = cell_gap(zf, z, gs.z - 1, cs);
             left_z = far * far - dz * dz;
             const float ry = sqrt_approx(fmaxf(left_z, 0.f)) * 1.0001f + 4.0f * pre.ulp;
@@ -398,7 +403,7 @@ __global__ void __launch_bounds__(128) k_neighbor_find(
         }
         if (more && y <= y1) {
           int x = max(g.x - off, 0), x1 = min(g.x + off, gs.x - 1);
-          if (pre.prune) {
+          if (prune) {
             const float dy = cell_gap(yf, y, gs.y - 1, cs);
             const float rx = sqrt_approx(fmaxf(left_z - dy * dy, 0.f)) * 1.0001f + 4.0f * pre.ulp;
             x = max(x, near_cell(xf - rx, rc, -1.0e-4f, gs.x - 1));
