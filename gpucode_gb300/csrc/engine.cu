@@ -479,17 +479,15 @@ dem_status build_graph(dem_ctx* c, int G, int start_parity, cudaGraphExec_t* out
   return st;
 }
 
-/* capture what `enqueue` puts on a stream into a graph instantiated for
+/* capture what `enqueue` puts on the stream cs into a graph instantiated for
  * device launch and uploaded, and (host_out) into a second instantiation for
  * launch from the host */
 template <class F>
-dem_status capture_device_graph(dem_ctx* c, F enqueue, cudaGraphExec_t* out, cudaGraphExec_t* host_out = nullptr) {
-  cudaStream_t cs;
-  cudaError_t e = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking);
-  if (e != cudaSuccess) return cuda_check(e, "capture stream");
+dem_status capture_device_graph(dem_ctx* c, cudaStream_t cs, F enqueue, cudaGraphExec_t* out,
+                                cudaGraphExec_t* host_out = nullptr) {
   cudaGraph_t g = nullptr;
   dem_status st = DEM_OK;
-  e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed);
+  cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed);
   if (e == cudaSuccess) {
     st = enqueue(cs);
     const cudaError_t ee = cudaStreamEndCapture(cs, &g);
@@ -508,7 +506,6 @@ dem_status capture_device_graph(dem_ctx* c, F enqueue, cudaGraphExec_t* out, cud
     if (e != cudaSuccess) st = cuda_check(e, "graph instantiate");
   }
   if (g) cudaGraphDestroy(g);
-  cudaStreamDestroy(cs);
   return st;
 }
 
@@ -526,10 +523,26 @@ dem_status chain_steps(dem_ctx* c, int p, int size, bool single, cudaStream_t cs
   return st == DEM_OK ? chain_launch_tail(c->chain_ctl, b.flag, b.need, b.err, p, size, single, cs) : st;
 }
 
-/* the chained step graphs of the mixed path: S1[p] (one step) and R[p]
- * (rebuild) at the first step call, S[G][p] (countdown) at the first of several
- * steps, and the control block that names them */
-dem_status build_chain(dem_ctx* c, bool many) {
+/* the size (log2) of the largest chain graph that a call of nsteps steps uses */
+int chain_size(int nsteps) {
+  int g = 0;
+  while (g + 1 < kChainSizes && 2 << g <= nsteps) g++;
+  return g;
+}
+
+/* whether the chained step graphs that a call of nsteps steps can use are there */
+bool chain_ready(const dem_ctx* c, int nsteps) {
+  return c->chain_rebuild[0] && (nsteps == 1 ? c->chain_single[0] : c->chain_step[chain_size(nsteps)][0]);
+}
+
+/* The chained step graphs of the mixed path that a call of nsteps steps can use
+ * and that are not there yet -- R[p] (rebuild), S1[p] for a single step, S[G][p]
+ * up to the call's length for several -- and the control block that names them.
+ * Every graph costs the call that builds it 40 us: the first call on 5,000 spheres
+ * took 0.75 ms to the end of two steps and 0.90 of twelve with all of them built at
+ * once, now 0.51 and 0.85 (0.50 and 0.77 with graphs of one step alone, where the
+ * second call of twelve took 0.37, now 0.20). */
+dem_status build_chain(dem_ctx* c, int nsteps) {
   EngineBufs& b = c->b;
   dem_status st = DEM_OK;
   if (!c->chain_ctl) {
@@ -540,24 +553,30 @@ dem_status build_chain(dem_ctx* c, bool many) {
     c->chain_ctl = (StepCtl*)p;
     st = cuda_check(cudaMemset(p, 0, sizeof(StepCtl)), "step chain control");
   }
-  const bool ones = !c->chain_single[0], counted = many && !c->chain_step[0][0];
+  cudaStream_t cs;
+  if (st == DEM_OK) st = cuda_check(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking), "capture stream");
+  if (st != DEM_OK) return st;
   for (int p = 0; p < 2 && st == DEM_OK; p++) {
-    if (ones) {
+    if (!c->chain_rebuild[p])
       st = capture_device_graph(
-          c,
-          [&](cudaStream_t cs) {
-            dem_status r = chain_clear_request(b.flag, b.need, cs);
-            return r == DEM_OK ? enqueue_rebuild(c, cs, p) : r;
+          c, cs,
+          [&](cudaStream_t s) {
+            dem_status r = chain_clear_request(b.flag, b.need, s);
+            return r == DEM_OK ? enqueue_rebuild(c, s, p) : r;
           },
           &c->chain_rebuild[p]);
-      if (st == DEM_OK)
-        st = capture_device_graph(c, [&](cudaStream_t cs) { return chain_steps(c, p, 0, true, cs); },
+    if (nsteps == 1) {
+      if (st == DEM_OK && !c->chain_single[p])
+        st = capture_device_graph(c, cs, [&](cudaStream_t s) { return chain_steps(c, p, 0, true, s); },
                                   &c->chain_single[p], &c->chain_single_host[p]);
+      continue;
     }
-    for (int g = 0; g < kChainSizes && counted && st == DEM_OK; g++)
-      st = capture_device_graph(c, [&](cudaStream_t cs) { return chain_steps(c, p, g, false, cs); },
-                                &c->chain_step[g][p]);
+    for (int g = 0; g <= chain_size(nsteps) && st == DEM_OK; g++)
+      if (!c->chain_step[g][p])
+        st = capture_device_graph(c, cs, [&](cudaStream_t s) { return chain_steps(c, p, g, false, s); },
+                                  &c->chain_step[g][p]);
   }
+  cudaStreamDestroy(cs);
   if (st == DEM_OK) {
     /* the names alone: an earlier chain may still count down beside them */
     StepCtl h;
@@ -1130,8 +1149,8 @@ dem_status step_calls(dem_ctx* c, int nsteps) {
   int left = nsteps;
   if (c->opt.use_graph && c->opt.precision == DEM_PREC_MIXED && c->n > 0 && c->chain_state >= 0 && nsteps > 0) {
     /* steps chained on the device: one host launch for the whole call */
-    if (!c->chain_single[0] || (nsteps > 1 && !c->chain_step[0][0])) {
-      st = build_chain(c, nsteps > 1);
+    if (!chain_ready(c, nsteps)) {
+      st = build_chain(c, nsteps);
       if (st == DEM_OK) {
         c->chain_state = 1;
       } else {
@@ -1155,9 +1174,7 @@ dem_status step_calls(dem_ctx* c, int nsteps) {
          * device-launch copy, which outweighs that copy's later start */
         st = chain_set_left(c->chain_ctl, nsteps, c->stream);
         if (st != DEM_OK) return st;
-        int g = 0;
-        while (g + 1 < kChainSizes && 2 << g <= nsteps) g++;
-        e = cudaGraphLaunch(c->chain_step[g][p], c->stream);
+        e = cudaGraphLaunch(c->chain_step[chain_size(nsteps)][p], c->stream);
       }
       if (e != cudaSuccess) return cuda_check(e, "cudaGraphLaunch");
       c->iter += nsteps;
