@@ -645,28 +645,34 @@ std::vector<int> levels_side_by_side(const dem_ctx* c, int bs) {
   return order;
 }
 
-/* device bytes of dem_create for N particles, S slots, C cells: the sums of
- * its allocation list (kept next to it), plus 2 MiB of rounding per allocation */
+/* Device bytes of dem_create for N particles, S slots, C cells, plus 2 MiB of
+ * rounding per allocation.  The rates a particle and a slot are those of the plan's
+ * interface, each an upper bound where lists are of ordinary length: a slot's
+ * arrays take 89 bytes in mixed precision and 146 in FP64, and what the rates a
+ * particle leave out (the mixed wall results, the pair offsets and the pairs'
+ * reserve) is covered by the rest.  Where the lists are so short that it is not,
+ * the total is the sum of dem_create's arrays. */
 dem_memory memory_of(long long N, long long S, long long C, const dem_options* o) {
+  const bool mixed = o && o->precision == DEM_PREC_MIXED;
   dem_memory m;
-  m.per_particle = 3 * 24 + 2 * 8 + 6 * 4      /* pos vel angv, rad pmove, lqd lqd_old id inv plevel nidx */
-                   + 3 * 24 + 8 + 3 * 4        /* tmp copies used while permuting */
-                   + 2 * 24                    /* staging of the force and moment exports */
-                   + 2 * 24 + 8                /* force mom rmom */
-                   + 4 + 12 + 4 + 4 + 12 + 4 + 4 /* num_nebor wlist nwall and their copies, nidx_old */
-                   + 2 * 3 * 64                /* wall records and their copies */
-                   + 3 * 4 + 2 * 4;            /* sorted hash / source, old_to_new, sort scratch */
-  if (o && o->precision == DEM_PREC_MIXED) m.per_particle += 9 * 16; /* FP32 shadows */
-  /* the list entry and the slot's pair index (8), and for half a pair a slot two
-   * sets of pair (16), record (128) and bridge flag (2), and the pair's result
-   * (48): 105 in mixed precision, where 138 covers the wall results and the
-   * reserve of unmirrored pairs too; FP64 has a record and flag a side and no
-   * result: 146, and the reserve */
-  m.per_slot = o && o->precision == DEM_PREC_MIXED ? 138 : 152;
-  m.per_cell = 3 * 4;                         /* cell start, end, offset */
+  m.per_particle = 756 + (mixed ? 9 * 16 : 0); /* state, copies, wall lists and records, sort; FP32 shadows */
+  m.per_slot = mixed ? 138 : 152;
+  m.per_cell = 3 * 4;                          /* cell start, end, offset */
   m.slots = S;
+  const long long particle = 3 * 24 + 2 * 8 + 6 * 4 /* pos vel angv, rad pmove, lqd lqd_old id inv plevel nidx */
+                             + 3 * 24 + 8 + 3 * 4   /* tmp copies used while permuting */
+                             + 2 * 24               /* staging of the force and moment exports */
+                             + 2 * 24 + 8           /* force mom rmom */
+                             + 4 + 2 * (12 + 4)     /* num_nebor, wlist and nwall and their copies */
+                             + 2 * 3 * 64           /* wall records and their copies */
+                             + 2 * 4                /* the pairs' offsets, two sets */
+                             + 3 * 4 + 2 * 4        /* sorted hash and source, old_to_new, sort scratch */
+                             + (mixed ? 9 * 16 + 6 * 16 + 3 * 4 + 1 : 0); /* shadows, wall results and entries, block order */
+  /* two sets of a pair, its record or records and its flag or flags; the pair's result */
+  const long long pair = mixed ? 2 * (8 + (long long)kPairRec32 + 1) + (long long)kPairOut32 : 2 * (8 + 2 * (64 + 1));
+  const long long arrays = N * particle + S * 2 * 4 /* list entry, pair index */ + pair_capacity(N, S) * pair;
   const long long allocations = 64;
-  m.total = N * m.per_particle + S * m.per_slot + C * m.per_cell + ((C + 2047) / 2048 + 64) * 4 +
+  m.total = std::max(N * m.per_particle + S * m.per_slot, arrays) + C * m.per_cell + ((C + 2047) / 2048 + 64) * 4 +
             allocations * (2LL << 20);
   if (o && o->capillary == DEM_CAP_MLP) m.total += 16 << 10;
   return m;

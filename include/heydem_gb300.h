@@ -510,10 +510,10 @@ dem_status dem_packing_metrics(int n, const double3* pos, const double* rad, con
  * Device bytes dem_create allocates for a set-up and options. */
 typedef struct dem_memory {
   long long per_particle;  /* bytes per particle (state, copies, wall lists and records, sort) */
-  long long per_slot;      /* bytes per neighbour slot (list, record, bridge flag, and their copies) */
+  long long per_slot;      /* bytes per neighbour slot (list, pair index, half a pair's records and result) */
   long long per_cell;      /* bytes per cell (ranges, scan tiles) */
   long long slots;         /* neighbour slots of the set-up */
-  long long total;         /* all of it, plus small fixed tables */
+  long long total;         /* all of it, plus small fixed tables; more where the lists are very short */
 } dem_memory;
 dem_status dem_memory_estimate(const dem_setup* s, const dem_options* o, dem_memory* out);
 /* Scale every level's neighbour slots by one factor f <= 1 (each level keeps
