@@ -58,13 +58,6 @@ struct CapNetSmem {
   float hull_lo[kCapIn], hull_hi[kCapIn]; /* raw-feature box of the training set */
 };
 
-/* what the engine keeps on the device for DEM_CAP_MLP */
-struct CapNetDev {
-  const CapNetSmem* w; /* device copy, staged into shared memory per block */
-  unsigned long long theta_seed;
-  float theta_max;
-};
-
 /* is a raw feature vector inside the network's training box? */
 __device__ __forceinline__ bool cap_in_hull(const CapNetSmem& w, float sep, float vol, float theta, float ratio) {
   return sep >= w.hull_lo[0] && sep <= w.hull_hi[0] && vol >= w.hull_lo[1] && vol <= w.hull_hi[1] &&

@@ -301,14 +301,6 @@ __device__ __forceinline__ double fcap64(double Splus, double ijVol, double effe
   return 2 * kPiRef * effectR * L.stension * exp(f1 - f2 * exp(f3 * ls + f4 * (ls * ls)));
 }
 
-/* warp-aggregated counter increment */
-__device__ __forceinline__ void warp_count(unsigned long long* ctr, bool pred) {
-  if (!ctr) return;
-  const unsigned act = __activemask();
-  const unsigned mask = __ballot_sync(act, pred);
-  if ((int)(threadIdx.x & 31) == __ffs(act) - 1 && mask) atomicAdd(ctr, (unsigned long long)__popc(mask));
-}
-
 /* Two float4 of one 32-byte sector in one 256-bit access (p a multiple of 32
  * bytes): the pair kernel's gathers are bound by the L1's wavefronts, and
  * scattered lanes cost one per sector and instruction.  Shadows, records and

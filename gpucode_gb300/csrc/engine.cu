@@ -82,7 +82,7 @@ __global__ void k_permute(const int* __restrict__ src, int n, const double3* __r
                           const double* __restrict__ rad, const int* __restrict__ lqd, const int* __restrict__ id,
                           const int* __restrict__ plevel, double3* __restrict__ tpos, double3* __restrict__ tvel,
                           double3* __restrict__ tangv, double* __restrict__ trad, int* __restrict__ tlqd,
-                          int* __restrict__ tid, int* __restrict__ tplevel, int* __restrict__ old_to_new) {
+                          int* __restrict__ tid, int* __restrict__ tplevel) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
   const int p = src[q];
@@ -93,7 +93,6 @@ __global__ void k_permute(const int* __restrict__ src, int n, const double3* __r
   tlqd[q] = lqd[p];
   tid[q] = id[p];
   tplevel[q] = plevel[p];
-  old_to_new[p] = q;
 }
 
 struct LevelStart {
@@ -314,7 +313,7 @@ dem_status enqueue_rebuild(dem_ctx* c, cudaStream_t s, int parity) {
   if (reorder) {
     k_permute<<<grid_for(n, 256), 256, 0, s>>>(b.sorted_src, n, b.pos, b.vel, b.angv, b.rad, b.lqd, b.id, b.plevel,
                                                 b.tmp_pos, b.tmp_vel, b.tmp_angv, b.tmp_rad, b.tmp_lqd, b.tmp_id,
-                                                b.tmp_plevel, b.old_to_new);
+                                                b.tmp_plevel);
     mark(c, s, "k_permute");
     LevelStart ls;
     for (int l = 0; l < DEM_MAX_LEVELS; l++) {
@@ -666,7 +665,7 @@ dem_memory memory_of(long long N, long long S, long long C, const dem_options* o
                              + 4 + 2 * (12 + 4)     /* num_nebor, wlist and nwall and their copies */
                              + 2 * 3 * 64           /* wall records and their copies */
                              + 2 * 4                /* the pairs' offsets, two sets */
-                             + 3 * 4 + 2 * 4        /* sorted hash and source, old_to_new, sort scratch */
+                             + 2 * 4 + 2 * 4        /* sorted hash and source, sort scratch */
                              + (mixed ? 9 * 16 + 6 * 16 + 3 * 4 + 1 : 0); /* shadows, wall results and entries, block order */
   /* two sets of a pair, its record or records and its flag or flags; the pair's result */
   const long long pair = mixed ? 2 * (8 + (long long)kPairRec32 + 1) + (long long)kPairOut32 : 2 * (8 + 2 * (64 + 1));
@@ -835,7 +834,7 @@ extern "C" dem_status dem_create(const dem_setup* s, const double* rad, const in
     body = levels_side_by_side(c, mixed_block_size(c));
     A(c->body_order, body.size());
   }
-  A(b.sorted_hash, N); A(b.sorted_src, N); A(b.old_to_new, N); A(b.cell_start, C); A(b.cell_end, C);
+  A(b.sorted_hash, N); A(b.sorted_src, N); A(b.cell_start, C); A(b.cell_end, C);
   A(b.cell_off, C + 1);
   A(b.cell_size, L); A(b.grid_size, L); A(b.ncell_idx, L); A(b.npars, L); A(b.nneb, L); A(b.level_size, L);
   A(b.cyl, 1); A(b.flag, 1); A(b.need, 1); A(b.err, 1); A(b.counters, 8);

@@ -109,7 +109,7 @@ struct MixArgs {
   int bin_exp;
   float lo_scale;
   double dt, move_limit; /* 0.3 * SearchGap */
-  float dtf, coarse_tol, rfrc;
+  float dtf, rfrc;
   float lqd_vol, lqd_layer, lqd_gapmn, lqd_st;
   Law32 pp, pw;
   /* batched systems (NULL for one system): system of each particle id (its
@@ -1659,7 +1659,6 @@ dem_status mixed_shadows(dem_ctx* c, int which, cudaStream_t s) {
 }
 
 dem_status mixed_import(dem_ctx* c, int which, int has_v, int has_w, cudaStream_t s) {
-  MixedState* m = c->mx;
   EngineBufs& b = c->b;
   k_import_shadows<<<grid_for(c->n, 256), 256, 0, s>>>(c->n, b.id, b.tmp_pos, b.tmp_vel, b.tmp_angv, has_v, has_w,
                                                         b.pos, b.vel, b.angv, b.rad, b.lqd, mixed_shadow_out(c, which));
@@ -1668,7 +1667,6 @@ dem_status mixed_import(dem_ctx* c, int which, int has_v, int has_w, cudaStream_
 
 dem_status mixed_import_mapped(dem_ctx* c, int which, const int* inv, const double3* hp, const double3* hv,
                                const double3* hw, cudaStream_t s) {
-  MixedState* m = c->mx;
   EngineBufs& b = c->b;
   /* a few resident blocks per SM, each walking several slices */
   static int sms = 0;
@@ -1726,7 +1724,6 @@ dem_status mixed_step(dem_ctx* c, int which, cudaStream_t s) {
   a.dt = c->s.prm.dt;
   a.dtf = (float)c->s.prm.dt;
   a.move_limit = 0.3 * c->s.prm.SearchGap;
-  a.coarse_tol = m->coarse_tol;
   a.rfrc = (float)c->s.mat[0].rfrc;
   a.lqd_vol = (float)c->s.lqd.vol;
   a.lqd_layer = (float)c->s.lqd.layer;
