@@ -22,6 +22,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <unordered_map>
 
 #include "dem_internal.h"
 
@@ -37,15 +38,42 @@ namespace {
 
 dem::DevConsts g_consts; /* the constant-memory set (kernel.cu:15-19) */
 
-/* device-side helpers the reference's wrappers never needed: the sort's
- * scratch and the error word */
+/* device-side helpers the reference's wrappers never needed: the scratch (the
+ * sort's, the liquid shares, the packed spheres) and the error word.  They belong
+ * to one CUDA context: a caller that resets the device or changes to another one
+ * gets fresh ones (the addresses of a context that is gone may be the caller's own
+ * arrays in the next). */
 struct CompatDevice {
   void* scratch = nullptr;
   size_t scratch_bytes = 0;
   int* err = nullptr;
 };
-CompatDevice g_dev;
+std::unordered_map<unsigned long long, CompatDevice> g_devs; /* by context id */
 std::mutex g_scratch; /* held from a wrapper's first launch on the scratch to its last */
+
+/* the id of the calling thread's context, unique for the life of the process (0: none yet) */
+unsigned long long context_id() {
+  using Fn = int (*)(void* context, unsigned long long* id); /* cuCtxGetId */
+  static const Fn get = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult r;
+    if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &r) != cudaSuccess ||
+        r != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return reinterpret_cast<Fn>(f);
+  }();
+  unsigned long long id = 0;
+  return get && get(nullptr, &id) == 0 ? id : 0;
+}
+
+/* the current context's helpers; g_scratch is held */
+CompatDevice& device_helpers() {
+  unsigned long long id = context_id();
+  if (!id && cudaFree(nullptr) == cudaSuccess) id = context_id(); /* a thread that has not used the device yet */
+  return g_devs[id];
+}
 
 /* the arithmetic of PpInterCalc / CirPWCalc / UpdateSystem: DEM_PREC_FP64 (the
  * reference's) unless DEM_COMPAT_PRECISION=mixed is set in the environment or
@@ -60,35 +88,36 @@ int compat_precision() {
   return g_precision;
 }
 
-void ensure_small() {
-  if (!g_dev.err) {
-    DEM_REF_CHECK(cudaMalloc((void**)&g_dev.err, sizeof(int)));
-    DEM_REF_CHECK(cudaMemset(g_dev.err, 0, sizeof(int)));
+int* ensure_err(CompatDevice& d) {
+  if (!d.err) {
+    DEM_REF_CHECK(cudaMalloc((void**)&d.err, sizeof(int)));
+    DEM_REF_CHECK(cudaMemset(d.err, 0, sizeof(int)));
   }
+  return d.err;
 }
 
-void* ensure_scratch(size_t bytes) {
-  if (bytes > g_dev.scratch_bytes) {
-    if (g_dev.scratch) DEM_REF_CHECK(cudaFree(g_dev.scratch));
-    g_dev.scratch = nullptr;
-    g_dev.scratch_bytes = 0;
-    DEM_REF_CHECK(cudaMalloc(&g_dev.scratch, bytes));
-    g_dev.scratch_bytes = bytes;
+void* ensure_scratch(CompatDevice& d, size_t bytes) {
+  if (bytes > d.scratch_bytes) {
+    if (d.scratch) DEM_REF_CHECK(cudaFree(d.scratch));
+    d.scratch = nullptr;
+    d.scratch_bytes = 0;
+    DEM_REF_CHECK(cudaMalloc(&d.scratch, bytes));
+    d.scratch_bytes = bytes;
   }
-  return g_dev.scratch;
+  return d.scratch;
 }
 
 /* scratch that a kernel can do without: NULL where the device has no room */
-void* optional_scratch(size_t bytes) {
-  if (bytes <= g_dev.scratch_bytes) return g_dev.scratch;
+void* optional_scratch(CompatDevice& d, size_t bytes) {
+  if (bytes <= d.scratch_bytes) return d.scratch;
   void* p = nullptr;
   if (cudaMalloc(&p, bytes) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
-  if (g_dev.scratch) DEM_REF_CHECK(cudaFree(g_dev.scratch));
-  g_dev.scratch = p;
-  g_dev.scratch_bytes = bytes;
+  if (d.scratch) DEM_REF_CHECK(cudaFree(d.scratch));
+  d.scratch = p;
+  d.scratch_bytes = bytes;
   return p;
 }
 
@@ -128,8 +157,6 @@ dem::LevelView view(SEARCHCELL c, int* ncell_idx, double* level_size, int* npars
 
 extern "C" {
 
-/* reads and clears the compat path's device error word: bit 1 = neighbour-slot
- * overflow, bit 4 = a particle hashed outside the cell grid */
 dem_status dem_compat_set_precision(int precision) {
   if (precision != DEM_PREC_FP64 && precision != DEM_PREC_MIXED)
     return dem::fail(DEM_ERR_ARG, "dem_compat_set_precision: DEM_PREC_FP64 or DEM_PREC_MIXED");
@@ -139,11 +166,15 @@ dem_status dem_compat_set_precision(int precision) {
 
 int dem_compat_precision(void) { return compat_precision(); }
 
+/* reads and clears the compat path's device error word: bit 1 = neighbour-slot
+ * overflow, bit 4 = a particle hashed outside the cell grid */
 int dem_compat_errors(void) {
-  if (!g_dev.err) return 0;
+  std::lock_guard<std::mutex> lock(g_scratch);
+  const auto d = g_devs.find(context_id());
+  if (d == g_devs.end() || !d->second.err) return 0;
   int v = 0;
-  DEM_REF_CHECK(cudaMemcpy(&v, g_dev.err, sizeof(int), cudaMemcpyDeviceToHost));
-  DEM_REF_CHECK(cudaMemset(g_dev.err, 0, sizeof(int)));
+  DEM_REF_CHECK(cudaMemcpy(&v, d->second.err, sizeof(int), cudaMemcpyDeviceToHost));
+  DEM_REF_CHECK(cudaMemset(d->second.err, 0, sizeof(int)));
   return v;
 }
 
@@ -306,14 +337,15 @@ void BldNeborList(int* hash, int* index, int* cellStart, int* cellEnd, int* d_pL
                   int* d_Ncell_Idx, double* d_Level_size, int* d_level_nPars, int* d_level_nNebors, int nLevels,
                   double3* pos, int Sys_nCells, int* d_Nebor1, int* d_Nebor_Idx, int* d_Num_Nebor,
                   int TotalParticle, double* rad) {
-  ensure_small();
   dem::LevelView lv = view(d_cell, d_Ncell_Idx, d_Level_size, d_level_nPars, d_level_nNebors, nLevels);
   std::lock_guard<std::mutex> lock(g_scratch);
-  void* scratch = ensure_scratch(dem::sort_scratch_bytes(TotalParticle, Sys_nCells));
+  CompatDevice& d = device_helpers();
+  int* err = ensure_err(d);
+  void* scratch = ensure_scratch(d, dem::sort_scratch_bytes(TotalParticle, Sys_nCells));
   ok_or_exit(dem::cell_sort(pos, d_pLevel, nullptr, TotalParticle, lv, g_consts, Sys_nCells, hash, index,
-                            cellStart, cellEnd, scratch, g_dev.err, 0));
+                            cellStart, cellEnd, scratch, err, 0));
   ok_or_exit(dem::neighbor_find(pos, rad, index, cellStart, cellEnd, d_pLevel, d_Nebor_Idx, lv, g_consts, d_Nebor1,
-                                d_Num_Nebor, TotalParticle, g_dev.err, 0));
+                                d_Num_Nebor, TotalParticle, err, 0));
 }
 
 void BldCirWall(double3* pos, double* rad, CylinderBC* d_Cir, int* d_StlW_List, size_t pitch_Sw1,
@@ -344,7 +376,7 @@ void PpInterCalc(double3* pos, double3* vel, double3* angvel, double* rad, int* 
   (void)NP;
   std::lock_guard<std::mutex> lock(g_scratch);
   if (compat_precision() == DEM_PREC_MIXED) {
-    void* bodies = optional_scratch(dem::ref_mixed_scratch(TotalParticle));
+    void* bodies = optional_scratch(device_helpers(), dem::ref_mixed_scratch(TotalParticle));
     ok_or_exit(dem::pp_force_ref_mixed(pos, vel, angvel, rad, d_Nebor1, d_pLevel, d_level_nPars, d_level_nNebors,
                                        d_Nebor_Idx, soa(h), d_Num_Nebor, d_lqdCnt, d_lqdCnt_Old, force, mom, rmom,
                                        TotalParticle, ForceCap, stage, g_consts, bodies, 0));
@@ -352,7 +384,7 @@ void PpInterCalc(double3* pos, double3* vel, double3* angvel, double* rad, int* 
   }
   /* the spheres' liquid shares go to the library's scratch (the neighbour
    * build's sort scratch, idle between builds on the same stream) */
-  double* share = ForceCap == 1 ? static_cast<double*>(ensure_scratch((size_t)TotalParticle * sizeof(double)))
+  double* share = ForceCap == 1 ? static_cast<double*>(ensure_scratch(device_helpers(), (size_t)TotalParticle * sizeof(double)))
                                 : nullptr;
   ok_or_exit(dem::pp_force64(pos, vel, angvel, rad, d_Nebor1, d_pLevel, d_level_nPars, d_level_nNebors,
                              d_Nebor_Idx, soa(h), d_Num_Nebor, d_lqdCnt, d_lqdCnt_Old, force, mom, rmom,

@@ -456,6 +456,10 @@ int ParticleFeedDevice(FeedZone* Feedcube, CylinderBC* h_Cir, double InitParSize
  * The environment variable DEM_COMPAT_PRECISION=mixed selects the mixed mode
  * for a driver that is not changed (the reference's main.cpp); this call
  * overrides it.  Lists (BldNeborList) are the same in both modes.
+ * The mixed PpInterCalc packs the spheres into device scratch of the library, 64
+ * bytes each, allocated by its first call on so many (BldNeborListNoAlloc does
+ * not do it); where there is no room it reads the caller's arrays, slower, with
+ * the same results.
  * Returns DEM_ERR_ARG for another value. */
 dem_status dem_compat_set_precision(int precision);
 /* the mode the next reference-compatible call will use (DEM_PREC_*) */
