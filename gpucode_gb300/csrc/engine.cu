@@ -1737,6 +1737,18 @@ extern "C" dem_status dem_load(dem_ctx* c, const char* path) {
     return fail(DEM_ERR_ARG, "dem_load: checkpoint does not match this context");
   }
   dem_status st = DEM_OK;
+  /* a file that is too short is refused before anything of it is loaded: the pair
+   * list below goes with the whole of the neighbour lists (a pipe cannot tell) */
+  const long at = std::ftell(f);
+  if (at >= 0 && std::fseek(f, 0, SEEK_END) == 0) {
+    long long need = 0;
+    for (const Blob& bl : checkpoint_blobs(c)) need += (long long)bl.bytes;
+    const long end = std::ftell(f);
+    if (std::fseek(f, at, SEEK_SET) != 0 || end - at < need) {
+      std::fclose(f);
+      return fail(DEM_ERR_IO, "dem_load: truncated checkpoint");
+    }
+  }
   std::vector<char> slot_rec, slot_brg;
   for (const Blob& bl : checkpoint_blobs(c)) {
     std::vector<char> h(bl.bytes);

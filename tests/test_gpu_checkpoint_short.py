@@ -1,0 +1,47 @@
+"""Checkpoints that are refused."""
+import numpy as np
+import pytest
+
+import _workloads
+from gpucode_gb300 import _abi
+from gpucode_gb300.engine import Engine
+
+pytestmark = pytest.mark.gpu
+
+
+def _engine(precision, steps, seed=7):
+    w = _workloads.small_wet()
+    pos, vel, ang = _workloads.stirred(w, seed=seed, vscale=0.2, wscale=0.5)
+    e = Engine(w.setup, precision=precision)
+    e.set_state(pos, vel, ang)
+    e.step(steps)
+    return e
+
+
+def _equal(a, b):
+    for k in ("pos", "vel", "angvel", "force"):
+        np.testing.assert_array_equal(a[k], b[k])
+
+
+@pytest.mark.parametrize("keep", [0.02, 0.5, 0.999])
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_a_truncated_checkpoint_changes_nothing(cuda, tmp_path, precision, keep):
+    """a file cut anywhere is an error, and the steps after it are those of an
+    engine that never tried"""
+    other = _engine(precision, 40, seed=8)
+    other.save(tmp_path / "whole")
+    other.close()
+    data = (tmp_path / "whole").read_bytes()
+    (tmp_path / "cut").write_bytes(data[: int(len(data) * keep)])
+    out = []
+    for path in ("cut", None):
+        e = _engine(precision, 40)
+        if path:
+            with pytest.raises(_abi.DemError) as err:
+                e.load(tmp_path / path)
+            assert err.value.code == _abi.DEM_ERR_IO
+        e.step(20)
+        e.sync()
+        out.append(e.get_state())
+        e.close()
+    _equal(*out)
