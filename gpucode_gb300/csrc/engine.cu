@@ -1749,6 +1749,12 @@ extern "C" dem_status dem_load(dem_ctx* c, const char* path) {
       return fail(DEM_ERR_IO, "dem_load: truncated checkpoint");
     }
   }
+  /* steps still under way read what is overwritten now */
+  cudaError_t busy = cudaStreamSynchronize(c->stream);
+  if (busy != cudaSuccess) {
+    std::fclose(f);
+    return cuda_check(busy, "dem_load");
+  }
   std::vector<char> slot_rec, slot_brg;
   for (const Blob& bl : checkpoint_blobs(c)) {
     std::vector<char> h(bl.bytes);

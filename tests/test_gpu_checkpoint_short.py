@@ -1,4 +1,4 @@
-"""Checkpoints that are refused."""
+"""Checkpoints that are refused, and a load right behind queued steps."""
 import numpy as np
 import pytest
 
@@ -45,3 +45,19 @@ def test_a_truncated_checkpoint_changes_nothing(cuda, tmp_path, precision, keep)
         out.append(e.get_state())
         e.close()
     _equal(*out)
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_a_load_behind_queued_steps_waits_for_them(cuda, tmp_path, precision):
+    """the loaded state, whatever was still under way"""
+    saved = _engine(precision, 40, seed=8)
+    saved.save(tmp_path / "cp")
+    saved.step(10)
+    want = saved.get_state()
+    saved.close()
+    e = _engine(precision, 300)
+    e.load(tmp_path / "cp")
+    e.step(10)
+    got = e.get_state()
+    e.close()
+    _equal(got, want)
