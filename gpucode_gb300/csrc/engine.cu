@@ -27,8 +27,9 @@
 
 #include <algorithm>
 #include <cmath>
-#include <cstdio>
 #include <cstddef>
+#include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -1527,10 +1528,12 @@ dem_status fetch_pairs(dem_ctx* c, HostPairs& h, bool history) {
   cudaError_t e = cudaStreamSynchronize(c->stream);
   if (e == cudaSuccess) e = cudaMemcpy(ctl, b.ps.ctl, sizeof(ctl), cudaMemcpyDeviceToHost);
   const int cur = ctl[0] & 1, P = ctl[1 + cur];
+  const size_t PS = (size_t)P * b.ps.sides;
+  ContactRec zero;
+  std::memset(&zero, 0, sizeof(zero));
+  h.rec.assign(PS, zero);
+  h.brg.assign(PS, 0);
   if (history) {
-    const size_t PS = (size_t)P * b.ps.sides;
-    h.rec.resize(PS);
-    h.brg.resize(PS);
     if (e == cudaSuccess) e = copy_records(b.ps, cur, h.rec, false);
     if (e == cudaSuccess) e = cudaMemcpy(h.brg.data(), b.ps.brg[cur], PS, cudaMemcpyDeviceToHost);
   }
@@ -1540,24 +1543,37 @@ dem_status fetch_pairs(dem_ctx* c, HostPairs& h, bool history) {
   if (e == cudaSuccess) e = cudaMemcpy(h.plevel.data(), b.plevel, sizeof(int) * N, cudaMemcpyDeviceToHost);
   return cuda_check(e, "pair history download");
 }
+/* In the order in which the slots lie: level by level, entry by entry (sphere by
+ * sphere every entry is megabytes from the one before); row(first slot, slots) after
+ * every entry of a level, used or not. */
+template <class V, class R>
+void visit_slots(const dem_ctx* c, const HostPairs& h, V visit, R row) {
+  std::vector<std::vector<size_t>> spheres(c->s.n_levels); /* those that have the entry */
+  for (size_t q = 0; q < (size_t)c->n; q++) spheres[h.plevel[q]].push_back(q);
+  size_t base = 0;
+  for (int L = 0; L < c->s.n_levels; L++) {
+    std::vector<size_t>& left = spheres[L];
+    const size_t npars = (size_t)c->s.level_npars[L];
+    for (int a = 0; a < c->s.level_nnebors[L]; a++, base += npars) {
+      size_t m = 0;
+      for (const size_t q : left) {
+        if (a >= h.num[q]) continue;
+        left[m++] = q;
+        const size_t sl = base + h.nidx[q];
+        const int e = h.eidx[sl];
+        const long long p = e < 0 ? ~e : e;
+        if (e == kNoPair) visit(q, a, sl, -1LL, true);
+        else if (c->b.ps.sides == 2) visit(q, a, sl, 2 * p + (e < 0 ? 1 : 0), true);
+        else visit(q, a, sl, p, e >= 0);
+      }
+      left.resize(m);
+      row(base, npars);
+    }
+  }
+}
 template <class V>
 void visit_slots(const dem_ctx* c, const HostPairs& h, V visit) {
-  long long base[DEM_MAX_LEVELS];
-  long long acc = 0;
-  for (int l = 0; l < c->s.n_levels; l++) {
-    base[l] = acc;
-    acc += (long long)c->s.level_nnebors[l] * c->s.level_npars[l];
-  }
-  for (size_t q = 0; q < (size_t)c->n; q++)
-    for (int a = 0; a < h.num[q]; a++) {
-      const int L = h.plevel[q];
-      const size_t sl = (size_t)(base[L] + (long long)a * c->s.level_npars[L] + h.nidx[q]);
-      const int e = h.eidx[sl];
-      const long long p = e < 0 ? ~e : e;
-      if (e == kNoPair) visit(q, a, sl, -1LL, true);
-      else if (c->b.ps.sides == 2) visit(q, a, sl, 2 * p + (e < 0 ? 1 : 0), true);
-      else visit(q, a, sl, p, e >= 0);
-    }
+  visit_slots(c, h, visit, [](size_t, size_t) {});
 }
 /* a record as the slot's sphere sees it: the second sphere's spring is the
  * mirror image of the first one's (mixed records) */
@@ -1665,6 +1681,43 @@ std::vector<Blob> checkpoint_blobs(dem_ctx* c) {
           {b.cyl, sizeof(CylinderBC), 0}, {b.counters, sizeof(unsigned long long) * 8, 0}};
 }
 const char kMagic[8] = {'D', 'E', 'M', 'G', 'B', '3', '0', '1'};
+/* host bytes of one array of a checkpoint, not filled beforehand */
+struct HostBytes {
+  char* p = nullptr;
+  ~HostBytes() { std::free(p); }
+  dem_status get(size_t n) {
+    std::free(p);
+    p = static_cast<char*>(std::malloc(n ? n : 1));
+    return p ? DEM_OK : fail(DEM_ERR_NOMEM, "checkpoint: no host memory for " + std::to_string(n) + " bytes");
+  }
+};
+/* The slots' records (64 bytes each, one in twelve used) written a row of a level's
+ * slots at a time, and their flags gathered for the array after them */
+dem_status write_slots(const dem_ctx* c, const HostPairs& hp, std::vector<char>& brg, FILE* f) {
+  std::vector<ContactRec> recs;
+  brg.assign((size_t)c->slots, 0);
+  size_t most = 0, base = 0, written = 0;
+  for (int l = 0; l < c->s.n_levels; l++) most = std::max(most, (size_t)c->s.level_npars[l]);
+  ContactRec zero;
+  std::memset(&zero, 0, sizeof(zero));
+  recs.assign(most, zero);
+  bool used = false;
+  visit_slots(
+      c, hp,
+      [&](size_t, int, size_t sl, long long p, bool own) {
+        used = true;
+        recs[sl - base] = slot_record(hp, p, own);
+        brg[sl] = p >= 0 && (size_t)p < hp.brg.size() ? (char)hp.brg[(size_t)p] : 0;
+      },
+      [&](size_t first, size_t n) {
+        written += std::fwrite(recs.data(), sizeof(ContactRec), n, f);
+        if (used) std::fill(recs.begin(), recs.begin() + n, zero);
+        used = false;
+        base = first + n;
+      });
+  for (; base < (size_t)c->slots; base++) written += std::fwrite(&zero, sizeof(zero), 1, f); /* slots of no level */
+  return written == (size_t)c->slots ? DEM_OK : fail(DEM_ERR_IO, "dem_save: short write");
+}
 }  // namespace
 
 extern "C" dem_status dem_save(dem_ctx* c, const char* path, int nBatch) {
@@ -1684,27 +1737,23 @@ extern "C" dem_status dem_save(dem_ctx* c, const char* path, int nBatch) {
   std::fwrite(hdr, sizeof(hdr), 1, f);
   std::fwrite(&c->ctime, sizeof(double), 1, f);
   HostPairs hp;
+  HostBytes h;
+  std::vector<char> brg;
   st = fetch_pairs(c, hp, true);
   for (const Blob& bl : checkpoint_blobs(c)) {
     if (st != DEM_OK) break;
-    std::vector<char> h(bl.bytes);
-    if (bl.kind == 0) {
-      e = cudaMemcpy(h.data(), bl.dev, bl.bytes, cudaMemcpyDeviceToHost);
-      if (e != cudaSuccess) {
-        st = cuda_check(e, "dem_save copy");
-        break;
-      }
-    } else {
-      visit_slots(c, hp, [&](size_t, int, size_t sl, long long p, bool own) {
-        if (bl.kind == 1) {
-          const ContactRec r = slot_record(hp, p, own);
-          std::memcpy(h.data() + sl * sizeof(r), &r, sizeof(r));
-        } else {
-          h[sl] = p >= 0 && (size_t)p < hp.brg.size() ? (char)hp.brg[(size_t)p] : 0;
-        }
-      });
+    if (bl.kind == 1) {
+      st = write_slots(c, hp, brg, f);
+      continue;
     }
-    if (std::fwrite(h.data(), 1, bl.bytes, f) != bl.bytes) {
+    const char* out = brg.data();
+    if (bl.kind == 0) {
+      st = h.get(bl.bytes);
+      if (st == DEM_OK) st = cuda_check(cudaMemcpy(h.p, bl.dev, bl.bytes, cudaMemcpyDeviceToHost), "dem_save copy");
+      if (st != DEM_OK) break;
+      out = h.p;
+    }
+    if (std::fwrite(out, 1, bl.bytes, f) != bl.bytes) {
       st = fail(DEM_ERR_IO, "dem_save: short write");
       break;
     }
@@ -1755,22 +1804,18 @@ extern "C" dem_status dem_load(dem_ctx* c, const char* path) {
     std::fclose(f);
     return cuda_check(busy, "dem_load");
   }
-  std::vector<char> slot_rec, slot_brg;
+  HostBytes slot_rec, slot_brg, h;
   for (const Blob& bl : checkpoint_blobs(c)) {
-    std::vector<char> h(bl.bytes);
-    if (std::fread(h.data(), 1, bl.bytes, f) != bl.bytes) {
+    HostBytes& to = bl.kind == 1 ? slot_rec : bl.kind == 2 ? slot_brg : h;
+    st = to.get(bl.bytes);
+    if (st != DEM_OK) break;
+    if (std::fread(to.p, 1, bl.bytes, f) != bl.bytes) {
       st = fail(DEM_ERR_IO, "dem_load: truncated checkpoint");
       break;
     }
-    if (bl.kind) {
-      (bl.kind == 1 ? slot_rec : slot_brg).swap(h);
-      continue;
-    }
-    cudaError_t e = cudaMemcpy(bl.dev, h.data(), bl.bytes, cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) {
-      st = cuda_check(e, "dem_load copy");
-      break;
-    }
+    if (bl.kind) continue;
+    st = cuda_check(cudaMemcpy(bl.dev, h.p, bl.bytes, cudaMemcpyHostToDevice), "dem_load copy");
+    if (st != DEM_OK) break;
   }
   std::fclose(f);
   if (st != DEM_OK) return st;
@@ -1785,12 +1830,12 @@ extern "C" dem_status dem_load(dem_ctx* c, const char* path) {
     if (st == DEM_OK) st = pair_carry(b.ps, lists_of(b), c->n, nullptr, b.err, c->stream);
     if (st == DEM_OK) st = pair_flip(b.ps, c->stream);
     HostPairs hp;
-    if (st == DEM_OK) st = fetch_pairs(c, hp, true);
+    if (st == DEM_OK) st = fetch_pairs(c, hp, false);
     if (st != DEM_OK) return st;
     visit_slots(c, hp, [&](size_t, int, size_t sl, long long p, bool own) {
       if (!own || p < 0) return;
-      std::memcpy(&hp.rec[(size_t)p], slot_rec.data() + sl * sizeof(ContactRec), sizeof(ContactRec));
-      hp.brg[(size_t)p] = (unsigned char)slot_brg[sl];
+      std::memcpy(&hp.rec[(size_t)p], slot_rec.p + sl * sizeof(ContactRec), sizeof(ContactRec));
+      hp.brg[(size_t)p] = (unsigned char)slot_brg.p[sl];
     });
     int cur = 0;
     cudaError_t e = cudaMemcpy(&cur, b.ps.ctl, sizeof(int), cudaMemcpyDeviceToHost);

@@ -1,4 +1,4 @@
-"""Checkpoints that are refused, and a load right behind queued steps."""
+"""Checkpoints that are refused, a load right behind queued steps, and what a file holds."""
 import numpy as np
 import pytest
 
@@ -61,3 +61,23 @@ def test_a_load_behind_queued_steps_waits_for_them(cuda, tmp_path, precision):
     got = e.get_state()
     e.close()
     _equal(got, want)
+
+
+@pytest.mark.parametrize("extra", [0, 37])
+def test_slots_of_no_level_are_written_too(cuda, tmp_path, extra):
+    """a set-up with more slots than its levels use: the file has them all, and a
+    resumed run keeps its bits"""
+    w = _workloads.small_wet()
+    w.setup.s.n_pp_slots += extra
+    pos, vel, ang = _workloads.stirred(w, vscale=0.2, wscale=0.5)
+    a, b = Engine(w.setup, precision="mixed"), Engine(w.setup, precision="mixed")
+    a.set_state(pos, vel, ang)
+    a.step(40)
+    a.save(tmp_path / "cp")
+    b.load(tmp_path / "cp")
+    for e in (a, b):
+        e.step(20)
+        e.sync()
+    _equal(a.get_state(), b.get_state())
+    a.close()
+    b.close()
