@@ -669,8 +669,7 @@ def main():
                          "CPU; ensemble: independent packings batched in one engine; wet2m / wet16m: large wet "
                          "beds with the fused learned closure")
     ap.add_argument("--pairs", default="auto", choices=["auto", "warp", "thread"],
-                    help="pair loop of the step kernel: warp-cooperative, one thread per particle, or auto (the "
-                         "library's choice)")
+                    help="dem_options.pair_mode: all three run the same kernels over the pair list")
     ap.add_argument("--block-size", type=int, default=0, help="threads per block of the step kernel (0: default)")
     ap.add_argument("--full-steps", type=int, default=50000)
     ap.add_argument("--large-steps", type=int, default=0, help="steps of wet2m / wet16m (0: 10,000 / 5,000)")

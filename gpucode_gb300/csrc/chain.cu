@@ -32,13 +32,12 @@
  * held back take 4 us, so more than eight would give back what they gain at the
  * first rebuild.
  *
- * The single-step graphs (one host launch per step) are S[1] without the
- * countdown.  For a one-step call the host launches a second,
- * host-instantiated copy of it: launched from the host, a graph instantiated
- * for device launch starts ~5 us later, and a kernel of the host copy
- * tail-launches the device graphs all the same (a chain of many steps started
- * from that copy measured ~1.5 us per step slower, so longer calls launch the
- * device copy).
+ * For a one-step call the host launches a host-instantiated copy of S[1] without
+ * the countdown: launched from the host, a graph instantiated for device launch
+ * starts ~5 us later, and a kernel of the host copy tail-launches the device
+ * graphs all the same: R and, as the rest of a chain of one step, S[1] (a chain of
+ * many steps started from that copy measured ~1.5 us per step slower, so longer
+ * calls launch the device copy).
  *
  * need and the flags are written only by k_chain and k_clear_request (need also
  * by the host between launches) and, its own flag, by a step's sphere kernel, so
@@ -83,8 +82,9 @@ __global__ void k_chain(StepCtl* ctl, int* flag, int* need, int* err, int p, int
   }
   if (done == 0) {
     /* the first step was held back: rebuild, then the same steps */
+    if (single) ctl->left = 1;
     tail(ctl->rebuild[p], err);
-    tail(single ? ctl->single[p] : ctl->step[size][p], err);
+    tail(ctl->step[size][p], err);
     return;
   }
   /* the countdown always moves, so the chain ends after `left` steps */

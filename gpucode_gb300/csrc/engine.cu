@@ -395,9 +395,9 @@ void drop_graphs(dem_ctx* c) {
    * an earlier call's steps are under way */
   cudaStreamSynchronize(c->stream);
   for (int p = 0; p < 2; p++) {
-    cudaGraphExec_t* all[5 + kChainSizes] = {&c->graph_exec[p], &c->graph_one[p], &c->chain_single[p],
-                                             &c->chain_rebuild[p], &c->chain_single_host[p]};
-    for (int g = 0; g < kChainSizes; g++) all[5 + g] = &c->chain_step[g][p];
+    cudaGraphExec_t* all[4 + kChainSizes] = {&c->graph_exec[p], &c->graph_one[p], &c->chain_rebuild[p],
+                                             &c->chain_single_host[p]};
+    for (int g = 0; g < kChainSizes; g++) all[4 + g] = &c->chain_step[g][p];
     for (cudaGraphExec_t* g : all) {
       if (*g) cudaGraphExecDestroy(*g);
       *g = nullptr;
@@ -479,12 +479,10 @@ dem_status build_graph(dem_ctx* c, int G, int start_parity, cudaGraphExec_t* out
   return st;
 }
 
-/* capture what `enqueue` puts on the stream cs into a graph instantiated for
- * device launch and uploaded, and (host_out) into a second instantiation for
- * launch from the host */
+/* capture what `enqueue` puts on the stream cs into a graph, instantiated for launch
+ * from the device or from the host, and uploaded */
 template <class F>
-dem_status capture_device_graph(dem_ctx* c, cudaStream_t cs, F enqueue, cudaGraphExec_t* out,
-                                cudaGraphExec_t* host_out = nullptr) {
+dem_status capture_graph(dem_ctx* c, cudaStream_t cs, F enqueue, bool from_device, cudaGraphExec_t* out) {
   cudaGraph_t g = nullptr;
   dem_status st = DEM_OK;
   cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed);
@@ -496,14 +494,10 @@ dem_status capture_device_graph(dem_ctx* c, cudaStream_t cs, F enqueue, cudaGrap
     st = cuda_check(e, "begin capture");
   }
   if (st == DEM_OK) {
-    e = cudaGraphInstantiateWithFlags(out, g, cudaGraphInstantiateFlagDeviceLaunch);
+    e = from_device ? cudaGraphInstantiateWithFlags(out, g, cudaGraphInstantiateFlagDeviceLaunch)
+                    : cudaGraphInstantiate(out, g, 0);
     if (e == cudaSuccess) e = cudaGraphUpload(*out, c->stream);
-    if (e != cudaSuccess) st = cuda_check(e, "device graph instantiate");
-  }
-  if (st == DEM_OK && host_out) {
-    e = cudaGraphInstantiate(host_out, g, 0);
-    if (e == cudaSuccess) e = cudaGraphUpload(*host_out, c->stream);
-    if (e != cudaSuccess) st = cuda_check(e, "graph instantiate");
+    if (e != cudaSuccess) st = cuda_check(e, "chain graph instantiate");
   }
   if (g) cudaGraphDestroy(g);
   return st;
@@ -530,18 +524,17 @@ int chain_size(int nsteps) {
   return g;
 }
 
-/* whether the chained step graphs that a call of nsteps steps can use are there */
+/* whether the chained step graphs that a call of nsteps steps uses are there */
 bool chain_ready(const dem_ctx* c, int nsteps) {
-  return c->chain_rebuild[0] && (nsteps == 1 ? c->chain_single[0] : c->chain_step[chain_size(nsteps)][0]);
+  return c->chain_single_host[0] && (nsteps == 1 || c->chain_step[kChainSizes - 1][0]);
 }
 
-/* The chained step graphs of the mixed path that a call of nsteps steps can use
- * and that are not there yet -- R[p] (rebuild), S1[p] for a single step, S[G][p]
- * up to the call's length for several -- and the control block that names them.
- * Every graph costs the call that builds it 40 us: the first call on 5,000 spheres
- * took 0.75 ms to the end of two steps and 0.90 of twelve with all of them built at
- * once, now 0.51 and 0.85 (0.50 and 0.77 with graphs of one step alone, where the
- * second call of twelve took 0.37, now 0.20). */
+/* The chained step graphs of the mixed path that are not there yet -- R[p]
+ * (rebuild), S[1][p] and its host copy, and for a call of several steps S[G][p] of
+ * all sizes, so that no later call builds any -- and the control block that names
+ * them.  20 to 75 us a graph, so there is one of each (a second S[1][p] for one-step
+ * calls and a capture stream a graph were a third of it), and the first call's
+ * rebuild runs meanwhile (step_calls). */
 dem_status build_chain(dem_ctx* c, int nsteps) {
   EngineBufs& b = c->b;
   dem_status st = DEM_OK;
@@ -558,23 +551,20 @@ dem_status build_chain(dem_ctx* c, int nsteps) {
   if (st != DEM_OK) return st;
   for (int p = 0; p < 2 && st == DEM_OK; p++) {
     if (!c->chain_rebuild[p])
-      st = capture_device_graph(
+      st = capture_graph(
           c, cs,
           [&](cudaStream_t s) {
             dem_status r = chain_clear_request(b.flag, b.need, s);
             return r == DEM_OK ? enqueue_rebuild(c, s, p) : r;
           },
-          &c->chain_rebuild[p]);
-    if (nsteps == 1) {
-      if (st == DEM_OK && !c->chain_single[p])
-        st = capture_device_graph(c, cs, [&](cudaStream_t s) { return chain_steps(c, p, 0, true, s); },
-                                  &c->chain_single[p], &c->chain_single_host[p]);
-      continue;
-    }
-    for (int g = 0; g <= chain_size(nsteps) && st == DEM_OK; g++)
+          true, &c->chain_rebuild[p]);
+    if (st == DEM_OK && !c->chain_single_host[p])
+      st = capture_graph(c, cs, [&](cudaStream_t s) { return chain_steps(c, p, 0, true, s); }, false,
+                         &c->chain_single_host[p]);
+    for (int g = 0; g < (nsteps > 1 ? kChainSizes : 1) && st == DEM_OK; g++)
       if (!c->chain_step[g][p])
-        st = capture_device_graph(c, cs, [&](cudaStream_t s) { return chain_steps(c, p, g, false, s); },
-                                  &c->chain_step[g][p]);
+        st = capture_graph(c, cs, [&](cudaStream_t s) { return chain_steps(c, p, g, false, s); }, true,
+                           &c->chain_step[g][p]);
   }
   cudaStreamDestroy(cs);
   if (st == DEM_OK) {
@@ -582,7 +572,6 @@ dem_status build_chain(dem_ctx* c, int nsteps) {
     StepCtl h;
     for (int p = 0; p < 2; p++) {
       for (int g = 0; g < kChainSizes; g++) h.step[g][p] = c->chain_step[g][p];
-      h.single[p] = c->chain_single[p];
       h.rebuild[p] = c->chain_rebuild[p];
     }
     const size_t at = offsetof(StepCtl, step);
@@ -771,6 +760,7 @@ extern "C" dem_status dem_create(const dem_setup* s, const double* rad, const in
     c->radii_bounded = plevel[i] >= 0 && plevel[i] < s->n_levels && rad[i] <= s->level_size[plevel[i]] * 1.00001;
   c->marks = nullptr;
   c->parity = 0;
+  c->rebuild_due = 1;
   c->cap_w = nullptr;
   c->theta_max = 0.52359878f; /* 30 degrees */
   c->theta_seed = 0;
@@ -929,6 +919,7 @@ extern "C" dem_status dem_set_systems(dem_ctx* c, int n_sys, const int* system_o
   drop_graphs(c);
   if (c->chain_state > 0) c->chain_state = 0;
   const int one = 1;
+  c->rebuild_due = 1;
   return cuda_check(cudaMemcpy(b.need, &one, sizeof(int), cudaMemcpyHostToDevice), "dem_set_systems");
 }
 
@@ -1014,6 +1005,7 @@ dem_status state_import(dem_ctx* c, const double3* pos, const double3* vel, cons
       e = cudaMemcpyAsync(b.need, &one, sizeof(int), cudaMemcpyHostToDevice, c->stream);
     }
     if (e != cudaSuccess) return cuda_check(e, "dem_set_state import");
+    if (request_rebuild) c->rebuild_due = 1;
     /* the caller's arrays are free again once the import has read them */
     return wait ? cuda_check(cudaEventSynchronize(c->xev[0]), "dem_set_state") : DEM_OK;
   }
@@ -1039,6 +1031,7 @@ dem_status state_import(dem_ctx* c, const double3* pos, const double3* vel, cons
     const int one = 1;
     e = cudaMemcpyAsync(b.need, &one, sizeof(int), cudaMemcpyHostToDevice, c->stream);
     if (e != cudaSuccess) return cuda_check(e, "dem_set_state");
+    c->rebuild_due = 1;
   }
   if (c->trace) cudaEventRecord(c->trace[2], c->stream);
   /* the caller's arrays are free again once the copies are done; the import
@@ -1153,9 +1146,22 @@ namespace {
 dem_status step_calls(dem_ctx* c, int nsteps) {
   dem_status st = DEM_OK;
   int left = nsteps;
+  struct Stepped { /* the steps of any path answer the request */
+    dem_ctx* c;
+    int n;
+    ~Stepped() { if (n > 0) c->rebuild_due = 0; }
+  } stepped{c, nsteps};
   if (c->opt.use_graph && c->opt.precision == DEM_PREC_MIXED && c->n > 0 && c->chain_state >= 0 && nsteps > 0) {
     /* steps chained on the device: one host launch for the whole call */
     if (!chain_ready(c, nsteps)) {
+      if (c->rebuild_due) {
+        /* the rebuild that the first step would start with: it runs while the host
+         * builds the graphs */
+        st = chain_clear_request(c->b.flag, c->b.need, c->stream);
+        if (st == DEM_OK) st = enqueue_rebuild(c, c->stream, c->parity);
+        if (st != DEM_OK) return st;
+        c->rebuild_due = 0;
+      }
       st = build_chain(c, nsteps);
       if (st == DEM_OK) {
         c->chain_state = 1;
@@ -1358,6 +1364,7 @@ extern "C" dem_status dem_profile_kernels(dem_ctx* c, dem_kernel_time* out, int 
   if (e == cudaSuccess) e = cudaMemsetAsync(c->b.need, 0, sizeof(int), c->stream);
   if (e == cudaSuccess) e = cudaEventRecord(e0, c->stream);
   dem_status st = cuda_check(e, "dem_profile_kernels");
+  c->rebuild_due = 0;
   c->marks = &marks;
   if (st == DEM_OK) st = enqueue_rebuild(c, c->stream, c->parity);
   if (st == DEM_OK) st = enqueue_step(c, c->stream, c->parity);
@@ -1847,6 +1854,7 @@ extern "C" dem_status dem_load(dem_ctx* c, const char* path) {
   c->iter = hdr[0];
   c->ctime = ct;
   c->parity = 0;
+  c->rebuild_due = 0; /* the file's request is on the device */
   k_inverse<<<grid_for(c->n, 256), 256, 0, c->stream>>>(c->n, c->b.id, c->b.inv);
   if (c->opt.precision == DEM_PREC_MIXED) {
     st = mixed_shadows(c, 0, c->stream);

@@ -33,14 +33,13 @@ namespace dem {
 struct MixedState; /* mixed.cu */
 
 /* device-side step chaining (chain.cu): the device-launchable graphs of 1, 2, 4
- * and 8 steps with the countdown, of one step without it and of a rebuild, per shadow
- * parity, the countdown of the running chain, and the move flags of a graph's
- * steps but the last */
+ * and 8 steps and of a rebuild, per shadow parity, the countdown of the running chain,
+ * and the move flags of a graph's steps but the last */
 constexpr int kChainSizes = 4, kChainMost = 1 << (kChainSizes - 1);
 struct StepCtl {
   int left;
   int flag[kChainMost - 1];
-  cudaGraphExec_t step[kChainSizes][2], single[2], rebuild[2];
+  cudaGraphExec_t step[kChainSizes][2], rebuild[2];
 };
 
 struct EngineBufs {
@@ -111,17 +110,18 @@ struct dem_ctx {
   cudaGraphExec_t graph_exec[2];
   cudaGraphExec_t graph_one[2];
   int parity; /* mixed: which shadow buffer the next step reads */
+  int rebuild_due; /* the rebuild request on the device is known to be set */
   int radii_bounded; /* every radius is at most its level's size: the neighbour search may skip far rows */
   int moving_walls; /* a cylinder's top wall moves (topv != 0): moved before every step's wall contacts */
   /* device-side step chaining (mixed precision): 0 not built yet, 1 built (its
-   * graphs anew if they were dropped since), -1 unavailable (the conditional-node graphs run instead); the graphs
-   * (instantiated for device launch) and a host-instantiated copy of the
-   * one-step graph for dem_step(1) (launched from the host, a device-launch
-   * graph starts ~5 us later); the control block on the device; and, while a
-   * chained step is captured, the rebuild request word that gates its
-   * kernels (NULL otherwise) */
+   * graphs anew if they were dropped since), -1 unavailable (the conditional-node
+   * graphs run instead); the graphs (instantiated for device launch) and a
+   * host-instantiated one-step graph without the countdown for dem_step(1)
+   * (launched from the host, a device-launch graph starts ~5 us later); the control
+   * block on the device; and, while a chained step is captured, the rebuild request
+   * word that gates its kernels (NULL otherwise) */
   int chain_state;
-  cudaGraphExec_t chain_step[dem::kChainSizes][2], chain_single[2], chain_rebuild[2];
+  cudaGraphExec_t chain_step[dem::kChainSizes][2], chain_rebuild[2];
   cudaGraphExec_t chain_single_host[2];
   dem::StepCtl* chain_ctl;
   const int* step_gate; /* capture of a chain graph: the word that holds a step back, */

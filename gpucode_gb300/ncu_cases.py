@@ -4,16 +4,17 @@ Every kernel launch of these cases comes from the host (no CUDA graphs, no
 device-launched steps), so a profiler's launch counting (-s / -c) addresses
 them directly, and each case holds a few GB on the device at most.
 
-    python -m gpucode_gb300.ncu_cases step [--pairs thread|warp] [--steps 4] [--io]
+    python -m gpucode_gb300.ncu_cases step [--steps 4] [--io]
         the packed 200,000-sphere wet bed: `steps` host-launched mixed steps
-        (the first rebuilds the lists), a pair kernel and a sphere kernel each
-        whatever --pairs says; with --io then an export, an import and one more
-        step through page-locked host arrays
+        (the first rebuilds the lists), a pair kernel and a sphere kernel each;
+        with --io then an export, an import and one more step through
+        page-locked host arrays
     python -m gpucode_gb300.ncu_cases closure [--rows 1000000]
         the packed bed with the per-contact liquid model: a network trained
         for 3 epochs on the bridges of one step, 3 host-launched steps with it
         fused in the pair kernel, then the network's inference on `rows`
-        bridges: twice on the tcgen05 path, once on the warp tiles
+        bridges: twice on the tcgen05 path, once on the warp tiles, once as
+        the FP32 network
     python -m gpucode_gb300.ncu_cases dropin [--precision fp64|mixed] [--steps 3]
         the packed bed through the reference's entry points in main.cpp's
         order (gpucode_gb300.dropin): `steps` steps, the first one building
@@ -83,9 +84,10 @@ def closure_case(rows: int) -> None:
     a = net.infer(big, "tcgen05")
     b = net.infer(big, "tcgen05")
     c = net.infer(big, True)
+    d = net.infer(big, False)
     torch.cuda.synchronize()
     print("ok", m.step_kernel_name(), m.stats(), "tcgen05 vs warp tiles", float((a - c).abs().max()),
-          "repeat", float((a - b).abs().max()))
+          "repeat", float((a - b).abs().max()), "FP32", float((a - d).abs().max()))
     m.close()
     net.close()
 
@@ -111,7 +113,7 @@ def main(argv=None) -> None:
     ap = argparse.ArgumentParser(description=__doc__, formatter_class=argparse.RawDescriptionHelpFormatter)
     ap.add_argument("case", choices=["step", "closure", "dropin"])
     ap.add_argument("--precision", default="fp64", choices=["fp64", "mixed"])
-    ap.add_argument("--pairs", default="auto", choices=["auto", "warp", "thread"])
+    ap.add_argument("--pairs", default="auto", choices=["auto", "warp", "thread"], help="accepted; all run the same kernels")
     ap.add_argument("--steps", type=int, default=4)
     ap.add_argument("--rows", type=int, default=1_000_000)
     ap.add_argument("--io", action="store_true", help="step: then a round trip through page-locked host arrays")
