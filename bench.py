@@ -587,22 +587,20 @@ CELL_SORT = ("k_hash_count", "k_tile_sums", "k_scan_tiles", "k_cell_ranges", "k_
 
 
 def kernel_bytes_per_particle() -> dict:
-    """DRAM bytes per particle of each kernel of a rebuild + step, from the
-    committed ncu table of the deposited 200,000-sphere bed (MB per launch /
-    200,000; the large beds are deposited too); the cell sort's launches summed
-    under the group name the library reports"""
-    p = ROOT / "profiles" / "launches_deposit200k.md"
+    """DRAM bytes per particle of each kernel of a rebuild, from the committed ncu
+    table of the packed 200,000-sphere bed (MB read and written per launch /
+    200,000; a deposited bed's lists are shorter); launches summed under the group
+    names the library reports"""
+    p = ROOT / "profiles" / "kernels_packed200k.md"
     out = {}
     if not p.exists():
         return out
     for line in p.read_text().splitlines():
         f = [x.strip() for x in line.strip().strip("|").split("|")]
-        if len(f) == 6 and f[0].startswith("k_") and f[2].replace(".", "").isdigit():
-            try:
-                out[f[0]] = float(f[3]) * 1e6 / 200_000
-            except ValueError:
-                pass
+        if len(f) == 6 and f[0].startswith("`k_"):
+            out[f[0].split("`")[1]] = (float(f[2]) + float(f[3])) * 1e6 / 200_000
     out["cell sort (k_hash_count .. k_cell_order)"] = sum(out.get(k, 0.0) for k in CELL_SORT)
+    out["pair list (scan, k_pair_fill)"] = sum(out.get(k, 0.0) for k in ("k_scan_apply", "k_pair_fill"))
     return out
 
 
@@ -613,8 +611,7 @@ def kernel_table(e, n: int) -> list:
     peak, _ = _peaks()
     rows = []
     for name, ms in e.profile_kernels():
-        # the table's capture has other kernels under these names
-        b = None if name in ("step kernel", "k_carry", "k_copy_back", "k_neighbor_find") else bpp.get(name)
+        b = bpp.get(name)
         gbs = None if (b is None or ms <= 0) else b * n / (ms * 1e-3) / 1e9
         rows.append({"kernel": name, "ms": ms, "dram_bytes_scaled": None if b is None else b * n,
                      "achieved_gbs": gbs, "frac": None if gbs is None else gbs / peak})
@@ -622,7 +619,7 @@ def kernel_table(e, n: int) -> list:
 
 
 def traffic_from_profiles(kernel: str) -> float | None:
-    """DRAM bytes per launch of the fused step kernel on the packed bed, from the
+    """DRAM bytes of the two step kernels on the packed bed, from the
     committed ncu summary of the same kernel (None for a kernel without one)"""
     name = {"k_pair_mixed<1,0> + k_body_mixed<1,0>": "step_pairs_packed200k.md"}.get(kernel)
     if name is None:
@@ -792,7 +789,7 @@ def run_headline(args, ws, rank):
     n_nb, n_c, n_w, n_wall = d["nb_entries"] / ps, d["contacts"] / ps, d["bridges"] / ps, d["wall_contacts"] / ps
     bytes_per_particle = algorithmic_bytes(n_nb, n_c, n_w, n_wall)
 
-    # the fused step kernel alone, cold L2 per launch
+    # the two step kernels alone, cold L2 per launch
     ms_k = C.c_double()
     check(eng.lib.dem_profile_step(eng.h, args.profile_reps, C.c_void_p(flush.data_ptr()), flush.numel(),
                                    C.byref(ms_k)), "dem_profile_step")

@@ -461,7 +461,7 @@ __global__ void __launch_bounds__(kRedParams* kRedSlices) k_reduce_adam(float* P
   }
 }
 
-/* BF16 tensor-core tiles, exactly as the fused step kernel evaluates them.  The
+/* BF16 tensor-core tiles, exactly as the pair kernel evaluates them.  The
  * next tile's features are in flight while the current one runs (1M rows: 47
  * us, without 54; the 128 hardware tanh a row alone need 25). */
 __global__ void __launch_bounds__(128) k_infer_tc(const CapNetSmem* __restrict__ wsrc, const float* __restrict__ xr,

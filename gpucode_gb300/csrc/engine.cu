@@ -4,23 +4,23 @@
  * One time step is the reference's main.cpp:466-564 sequence -- rebuild when
  * the last integration flagged it, then p-p forces, wall forces, integration
  * -- with three GB300-specific changes:
- *  - the rebuild decision is taken on the device: each step starts with a
- *    one-thread kernel that reads the rebuild flag and sets the condition of a
- *    CUDA-graph IF node whose body is the whole rebuild, so a graph of many
- *    steps replays with no host round trip (the reference copies the flag to
- *    the host every step, main.cpp:470);
+ *  - the rebuild decision is taken on the device, with no host round trip (the
+ *    reference copies the flag to the host every step, main.cpp:470).  Mixed
+ *    precision: steps and rebuilds are graphs that launch one another from the
+ *    device (chain.cu).  FP64, and mixed precision where graphs cannot be launched
+ *    from the device: each step of a graph starts with a one-thread kernel that
+ *    reads the flag and sets the condition of an IF node whose body is the rebuild;
  *  - particles are kept in cell order: every rebuild permutes the particle
  *    state by the cell sort, so neighbours of consecutive particles are close
  *    in memory, and neighbour slots of consecutive particles are adjacent;
- *  - contact history is 64-byte records (one per slot) instead of seven
- *    parallel arrays; a rebuild copies only the used slots to the *_old
- *    buffers and the carry-over writes every used new slot (match -> copy,
- *    else zero), replacing the reference's full-array copy + memset
- *    (ParticleSystem.cu:336-375).
+ *  - contact history is kept per pair of neighbours (pairs.cu), one record in
+ *    mixed precision and one a side in FP64, instead of per slot in seven parallel
+ *    arrays; a rebuild reads the current set of pairs and writes the other (match
+ *    -> copy, else zero), replacing the reference's full-array copy + memset
+ *    (ParticleSystem.cu:336-375).  Wall records alone are copied to *_old buffers.
  *
  * Precision: DEM_PREC_FP64 runs the reference formulas (step64.cu) on these
- * buffers; DEM_PREC_MIXED runs the fused FP32-force / FP64-state kernel of
- * mixed.cu.
+ * buffers; DEM_PREC_MIXED runs the FP32-force / FP64-state kernels of mixed.cu.
  */
 #include <cuda_runtime.h>
 #include <chrono>

@@ -9,8 +9,9 @@
  *  - neighbour lists: nebor[S] level/slot-major (slot(q,k) = base[L] +
  *    k*npars[L] + nidx[q], coalesced across consecutive particles for a fixed
  *    k), num_nebor[N]; wall lists wlist[N][3], nwall[N];
- *  - the pair list (pairs.cuh): every pair of neighbours once, with its 64-byte
- *    ContactRec and bridge byte, in two sets that a rebuild alternates between
+ *  - the pair list (pairs.cuh): every pair of neighbours once, with its record (48
+ *    bytes in mixed precision, two of 64 in FP64) and bridge bytes, in two sets that
+ *    a rebuild alternates between
  *    (fixed pointers, so a rebuild can sit inside a CUDA graph); each slot's
  *    pair index; the pairs' results of the running step;
  *  - 3N wall records (slot (a, q) at a*N + q), with *_old copies a rebuild
@@ -157,10 +158,12 @@ struct ShadowOut;
 /* threads per block of the step kernels */
 int mixed_block_size(const dem_ctx* c);
 /* Spheres from which the sphere kernel takes the levels side by side: about where
- * the pairs' results (40 bytes each, 4.3 pairs a sphere on a packed bed) outgrow
- * the L2.  Packed beds, us a step with and without: 300,000 spheres 94.1 and 85.5,
- * 500,000 143.9 and 143.9, 600,000 171.7 and 175.5, 1,000,000 269.7 and 288.4,
- * 2,000,000 520.2 and 569.9. */
+ * the pairs' results (40 bytes each, 4.3 pairs a sphere on a packed bed) and the
+ * spheres' own state outgrow the L2.  Packed beds, us a step with and without:
+ * 300,000 spheres 94.1 and 85.5, 500,000 143.9 and 143.9, 600,000 171.7 and 175.5,
+ * 1,000,000 269.7 and 288.4, 2,000,000 520.2 and 569.9.  600,000 spheres with
+ * other lists: dry 148.5 and 151.7, spread apart (3.2 pairs a sphere, no contacts)
+ * wet 105.5 and 107.5, dry 97.4 and 97.5; without any pair 56.5 and 55.6. */
 constexpr int kSideBySide = 600000;
 ShadowOut mixed_shadow_out(const dem_ctx* c, int which);
 const float4* mixed_motion(const dem_ctx* c, int which);
@@ -169,7 +172,7 @@ dem_status mixed_shadows(dem_ctx* c, int which, cudaStream_t s);
 dem_status mixed_bridge_counts(dem_ctx* c, int which, cudaStream_t s);
 /* the neighbour build's FP32 prefilter over shadow buffer `which` */
 Prefilter mixed_prefilter(dem_ctx* c, int which);
-/* one fused step reading shadows `which`, writing shadows 1 - which */
+/* one step (pair kernel, sphere kernel) reading shadows `which`, writing shadows 1 - which */
 dem_status mixed_step(dem_ctx* c, int which, cudaStream_t s);
 /* a state import without a rebuild request: the host arrays already in the
  * tmp buffers, gathered into cell order with the shadow buffer `which`

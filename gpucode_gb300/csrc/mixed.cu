@@ -11,11 +11,11 @@
  * Why two: a thread per sphere that walks its own slots evaluates every pair
  * twice, moves its history twice, keeps 18 of 32 lanes busy (lists of 2 to 30
  * entries) and chains index -> shadow -> record -> law per slot.  On the packed
- * 200k wet bed that one kernel took 114 us; the pair kernel takes 35 us (25 of
- * 32 lanes, half the evaluations, 83 + 30 MB of DRAM traffic at 49 % occupancy;
- * bound by the latency of its two rounds of loads) and the sphere kernel 35 us
- * (bound by the gather of the pairs' results), 78 against 116 us a chained step;
- * 2M spheres 710 against 912 us, 5,000 dry spheres 23 against 43 us.
+ * 200k wet bed that one kernel took 114 us; the pair kernel takes 27 us (25 of
+ * 32 lanes, half the evaluations, 68 + 13 MB of DRAM traffic at 56 % occupancy;
+ * bound by issue, 65 %) and the sphere kernel 32 us (bound by the gather of the
+ * pairs' results), 61 against 116 us a chained step; 2M spheres 520 against 912
+ * us, 5,000 dry spheres 15 against 43 us (a graph of several steps among it).
  *
  * Why this shape on GB300: FP64 arithmetic runs at ~0.6 T op/s (1/58 of
  * FP32) and FP64 pow at ~6 G/s, so the reference's all-FP64 pair math is
@@ -36,8 +36,8 @@
  *    increments (projection correction, length-preserving rescale written as
  *    a small difference, v_t dt) so its accumulation error is relative to
  *    the increment, not to the spring;
- *  - contact records are 64 bytes (two DRAM sectors) read and written only for
- *    contacts, streamed past L2's reusable lines; bridge flags are one byte a
+ *  - contact records are 48 bytes (a sector and half a one) read and written only
+ *    for contacts, streamed past L2's reusable lines; bridge flags are one byte a
  *    pair; a pair's two spheres get one evaluation, mirrored by its signs.
  */
 #include <cuda_runtime.h>
